@@ -316,7 +316,7 @@ def stage_kernel(stage, w_path, prec):
     fk = "k_fgemm" if FIBER_FGEMM else "k_fiber"
     tc = "k_tcpanel" if prec == "tf32x3" else "k_pgemm"
     return {"sigma1": tc if panel else "k_bgemm", "sigma2": fk if panel else "k_bgemm",
-            "sigma3": fk if panel else "k_bgemm", "sigma23": fk,
+            "sigma3": fk if panel else "k_bgemm", "sigma23": fk if w_path == "fused" else "k_wsparse",
             "sigma4": tc if panel else "k_bgemm"}.get(stage, "k_bgemm")
 
 

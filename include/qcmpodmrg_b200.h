@@ -186,6 +186,7 @@ int qc_tc_status(void);
  * is written as
  *   C[c_base + c_off + (f/flo)*fhs + (f%flo)*ncols + c]      (colmajor = 0)
  *   C[c_base + c_off + c*F + f]                              (colmajor = 1)
+ *   C[c_base + c_off + (f/flo)*fhs + c*flo + f%flo]          (colmajor = 2)
  *       = alpha * sum_pairs sum_r in[srow+r][f] * W[b_base + w_off + r*ncols + c]
  * (an empty pair range writes zeros)
  * with pairs fpair[pair_b..pair_e) (qc_fpair, 16 B).  fiber_tile (32 or 64) is
@@ -228,6 +229,26 @@ int qc_fgemm_f32(const void *items_dev, long long nitems, const void *groups_dev
 /* W panels of the dense fiber-group GEMM: dst[i] = idx[i] >= 0 ? src[idx[i]] : 0 (once per dot). */
 int qc_wpanel_f64(const double *src, const long long *idx_dev, double *dst, long long n, void *stream);
 int qc_wpanel_f32(const float *src, const long long *idx_dev, float *dst, long long n, void *stream);
+/* Sparse two-site MPO stage: T3 = T1 . (W_i W_{i+1}) for every operator (records qc_wxitem /
+ * qc_wxdelta / qc_wxgrp / qc_wxdop / qc_wxquad of qc_types.h).  qc_wx_build makes the sparse
+ * rows of one operator class on the host (w1 / w2: FP64 values, operator o at off1[o] /
+ * off2[o]; ns / nd / ioff / allowed: the two layouts), qc_wx_fetch copies them out and frees
+ * the handle.  qc_wsparse_*: items of one tile width (fpt fibers per lane: 1, 2 or 4);
+ * ent_w: four coefficients per entry as 16-byte vectors (FP64: all first halves, then all
+ * second halves, nent apart); maxR / maxQ: most T1 rows / quads of any item's charge
+ * difference. */
+int qc_wx_build(int nops, const double *w1, const long long *off1, const int *ns1, const long long *nd1,
+                const long long *ioff1, const int *allowed1, const double *w2, const long long *off2, const int *ns2,
+                const long long *nd2, const long long *ioff2, const int *allowed2, int ndelta, const int *iblk,
+                const int *kblk, const int *row0, const int *R, void **handle, long long *nquads, long long *nents);
+int qc_wx_fetch(void *handle, long long ent0, int quad0, void *dops, void *quads, double *w, int *r);
+int qc_wsparse_f64(const void *items, long long nitems, int fpt, const void *deltas, const void *grps,
+                   const void *rows, const void *dops, const void *quads, const void *ent_w, long long nent,
+                   const void *ent_r, const void *ops, int maxR, int maxQ, const double *A, double *C, void *stream);
+int qc_wsparse_f32(const void *items, long long nitems, int fpt, const void *deltas, const void *grps,
+                   const void *rows, const void *dops, const void *quads, const void *ent_w, long long nent,
+                   const void *ent_r, const void *ops, int maxR, int maxQ, const float *A, float *C, void *stream);
+
 /* W panels of the dense fiber-group GEMM assembled from their W blocks (the form the plan
  * compiler emits; the W blocks are those of the pair lists of tensordotSYM for
  * top2 = tensordot(top1, W_i) / top3 = tensordot(top2, W_j), kernelQt.py:301-306):

@@ -14,7 +14,7 @@ import torch
 
 from . import native
 from .native import check
-from .engine import OP_DT, TASK_DT, CONTRIB_DT, TC_CFG, LOG, FiberStage, CompositeStage, PanelStage
+from .engine import OP_DT, TASK_DT, CONTRIB_DT, TC_CFG, LOG, FiberStage, CompositeStage, PanelStage, upload
 
 
 def _abs_ops(ops, a, b, c):
@@ -70,6 +70,7 @@ class BatchedSigma(object):
         groups = {}
         fibers = {}
         panels = {}
+        sparse = []
         ops_all = [[], [], [], [], []]
         nops_acc = [0, 0, 0, 0, 0]
         for i, s in enumerate(items):
@@ -83,15 +84,23 @@ class BatchedSigma(object):
             P = self.T[3][int(offs[i, 3]):]
             x = self.X[int(self.xoff[i]):]
             abc = [(L, x, T1), (T1, Wi, T2), (T2, Wj, T3), (T3, R, P)]
-            stages = list(s.stages)
+            stages = list(s._stages)
             if s.fused is not None:         # slot 4: fused W stage, T1 -> T3
                 abc.append((T1, s.Wij if kind == "f64" else s.wij32(), T3))
                 stages.append(s.fused)
+            elif s.wx is not None:          # slot 4: sparse two-site stage, T1 -> T3
+                abc.append((T1, T1, T3))
+                stages.append(s.wx)
             for si, st in enumerate(stages):
+                if st is None:
+                    continue
                 ops = _abs_ops(st.host_ops, *abc[si])
                 base = nops_acc[si]
                 nops_acc[si] += len(ops)
                 ops_all[si].append(ops)
+                if st is s.wx:
+                    sparse.append((st, base))
+                    continue
                 for sub in (st.subs if isinstance(st, CompositeStage) else [st]):
                     if isinstance(sub, FiberStage):
                         if sub.ntasks:
@@ -176,7 +185,49 @@ class BatchedSigma(object):
             span = int(max(1, (tk["op_e"] - tk["op_b"]).max()))
             crow = torch.from_numpy(numpy.concatenate(crows).astype(numpy.int64)).to(device)
             self.panel_launches.append((si, cfg, len(tk), span, up(tk), crow))
+        self.sparse_launches, self.sparse = self._merge_sparse(sparse)
         self.graph = None
+
+    def _merge_sparse(self, parts):
+        """The sparse two-site stages of all instances as one: records back to back, indices rebased."""
+        if not parts:
+            return [], None
+        dels, grps, dops, by = [], [], [], {}
+        nd = ng = nr = no = nq = ne = 0
+        for st, base in parts:
+            d, o = st.h_deltas.copy(), st.h_dops.copy()
+            d["grp_b"] += ng
+            d["grp_e"] += ng
+            d["row_b"] += nr
+            d["dop_b"] += no
+            o["ent_b"] += ne
+            o["quad_b"] += nq
+            for (fpt, it, _, maxr, maxq) in st.items(self.kind if self.kind == "f64" else "f32"):
+                it = it.copy()
+                it["delta"] += nd
+                it["grp"] += ng
+                for k in ("op_b", "op_e", "op0"):
+                    it[k] += base
+                by.setdefault(fpt, []).append((it, maxr, maxq))
+            dels.append(d)
+            grps.append(st.h_groups)
+            dops.append(o)
+            nd, ng, nr = nd + len(d), ng + len(st.h_groups), nr + len(st.h_rows)
+            no, nq, ne = no + len(o), nq + len(st.h_quads), ne + len(st.h_ent_r)
+        sts = [st for st, _ in parts]
+        up = lambda a: upload(a if len(a) else numpy.zeros(1, a.dtype), self.device)       # noqa: E731
+        cat = lambda name, dt: up(numpy.concatenate([getattr(st, name) for st in sts]).astype(dt, copy=False))  # noqa: E731
+        w = numpy.concatenate([st.h_ent_w for st in sts]) if ne else numpy.zeros((1, 4))
+        w = w.reshape(-1, 2, 2).transpose(1, 0, 2) if self.kind == "f64" else w.astype(numpy.float32)
+        rec = {"deltas": up(numpy.concatenate(dels)), "groups": up(numpy.concatenate(grps)),
+               "rows": cat("h_rows", numpy.int32), "dops": up(numpy.concatenate(dops)),
+               "quads": cat("h_quads", sts[0].h_quads.dtype), "ent_r": cat("h_ent_r", numpy.int32),
+               "w": upload(w, self.device), "nent": ne}
+        launches = []
+        for fpt, xs in sorted(by.items(), reverse=True):
+            it = numpy.concatenate([x[0] for x in xs])
+            launches.append((fpt, len(it), up(it), max(x[1] for x in xs), max(x[2] for x in xs)))
+        return launches, rec
 
     def _launch_all(self):
         lib = native.lib()
@@ -196,6 +247,14 @@ class BatchedSigma(object):
                     continue
                 check(ffn(dt.data_ptr(), nt, span, dfi.data_ptr(), dfo.data_ptr(), dfp.data_ptr(),
                           self.d_ops[si].data_ptr(), mr, tile, None, None, None, s), "batched qc_fiber")
+                LOG.launches += 1
+            for (fpt, nt, dt, maxr, maxq) in self.sparse_launches if stage == 4 else []:
+                wfn = lib.qc_wsparse_f64 if self.kind == "f64" else lib.qc_wsparse_f32
+                r = self.sparse
+                check(wfn(dt.data_ptr(), nt, fpt, r["deltas"].data_ptr(), r["groups"].data_ptr(), r["rows"].data_ptr(),
+                          r["dops"].data_ptr(), r["quads"].data_ptr(), r["w"].data_ptr(), r["nent"],
+                          r["ent_r"].data_ptr(), self.d_ops[4].data_ptr(), maxr, maxq, None, None, s),
+                      "batched qc_wsparse")
                 LOG.launches += 1
             for (si, cfg, nt, span, dt, dc) in self.launches:
                 if si != stage:

@@ -122,11 +122,12 @@ k_fiber(const qc_ftask *__restrict__ tasks, const qc_fin *__restrict__ fin, cons
       const int fl = lane + 32 * q;
       if (fl < nf) {
         const int fg = t.f0 + fl;
-        if (ob.colmajor) {
-          T *dst = Cb + ob.c_off + (long long)c0 * t.F + fg;
+        if (ob.colmajor) {      // 1: [ncols][F]; 2: [F / flo][ncols][flo]
+          const int split = ob.colmajor == 2 ? ob.flo : t.F;
+          T *dst = Cb + ob.c_off + (long long)(fg / split) * ob.fhs + (long long)c0 * split + fg % split;
 #pragma unroll
           for (int i = 0; i < CB; ++i)
-            if (i < nb) dst[(long long)i * t.F] = alpha * acc[q][i];
+            if (i < nb) dst[(long long)i * split] = alpha * acc[q][i];
         } else {
           T *dst = Cb + ob.c_off + (long long)(fg / ob.flo) * ob.fhs + (long long)(fg % ob.flo) * nc + c0;
 #pragma unroll

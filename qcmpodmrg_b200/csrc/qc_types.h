@@ -71,7 +71,8 @@ static_assert(sizeof(qc_fin) == 32, "qc_fin is 32 bytes");
 struct alignas(16) qc_fout {
   long long c_off;     // output block offset (relative to the operator's C base)
   int fhs;             // (f, c) at c_off + (f / flo)*fhs + (f % flo)*ncols + c, or,
-  int colmajor;        // when colmajor is set, at c_off + c*F + f (block stored [ncols][F])
+  int colmajor;        // when colmajor is 1, at c_off + c*F + f (block stored [ncols][F]); when it
+                       // is 2, at c_off + (f / flo)*fhs + c*flo + f % flo ([F/flo][ncols][flo])
   int ncols;
   int pair_b, pair_e;  // contributions [pair_b, pair_e) of qc_fpair (empty: the block is zeroed)
   int flo;             // >= F for a block stored [F][ncols]
@@ -210,3 +211,49 @@ struct alignas(16) qc_wpair {
   int width, mc, r0, nr, j0, ncol, src_ld, op_b, nops, pad;
 };
 static_assert(sizeof(qc_wpair) == 64, "qc_wpair is 64 bytes");
+
+// ---- sparse two-site MPO stage (k_wsparse) ---------------------------------------
+// T3 = T1 . (W_i W_{i+1}).  A fiber is one (l, r) pair of states; every fiber whose two
+// sectors differ by the same charge meets the same matrix S[k, i] (k = (c, n1', n2') rows
+// of T3, i = (a, n1, n2) rows of T1), which is sparse.  Groups are (l sector, r sector)
+// pairs, a "delta" is the set of groups of one charge difference and operator class.
+struct alignas(16) qc_wxgrp {
+  int start;           // first fiber of the group in its delta
+  int F;               // fibers D_l * D_r
+  int flo;             // D_r: fiber f is (f / flo, f % flo)
+  int pad;
+  int a[16];           // T1 block (n1, n2) at a_base + a[4 n1 + n2], rows F apart; -1: absent (zero)
+  int c[16];           // T3 block (n1', n2'): (f, c) at c_base + c[.] + (f / flo) * h[.] + c * flo + f % flo;
+  int h[16];           //   -1: not needed
+};
+static_assert(sizeof(qc_wxgrp) == 208, "qc_wxgrp is 208 bytes");
+
+struct alignas(16) qc_wxdelta {
+  int R, row_b;        // T1 rows, first row record (block << 16 | a)
+  int grp_b, grp_e;    // groups
+  int dop_b;           // qc_wxdop of the class's first operator
+  int pad0, pad1, pad2;
+};
+static_assert(sizeof(qc_wxdelta) == 32, "qc_wxdelta is 32 bytes");
+
+struct alignas(16) qc_wxitem {
+  int delta;
+  int grp, f0, nf;     // first group, first fiber in it, fibers of the tile
+  int op_b, op_e;      // operators (operator table)
+  int op0;             // first operator of the class: operator op uses qc_wxdop dop_b + op - op0
+  int pad;
+};
+static_assert(sizeof(qc_wxitem) == 32, "qc_wxitem is 32 bytes");
+
+struct alignas(16) qc_wxdop {
+  long long ent_b;     // first entry
+  int quad_b, nquad;   // quads (four consecutive rows k of one T3 block)
+};
+static_assert(sizeof(qc_wxdop) == 16, "qc_wxdop is 16 bytes");
+
+struct alignas(16) qc_wxquad {
+  int ent, cnt;        // entries ent_b + [ent, ent + cnt): a T1 row and its four coefficients
+  int blk;             // T3 block 4 n1' + n2'
+  int c0nc;            // first c << 8 | rows (1 .. 4)
+};
+static_assert(sizeof(qc_wxquad) == 16, "qc_wxquad is 16 bytes");

@@ -149,7 +149,7 @@ def panel_sigma1(Ll, psi, t1, nblks_out):
             "gemm": (pan_off[lkp], psi.ioff[up], t1pan, Mj, Nj, Kj), "tc": tc}
 
 
-def panel_sigma4(t3lay, Rl, psi, t4):
+def panel_sigma4(t3lay, Rl, psi, t4, r_fast=False):
     """Panel form of the .R contraction (HVecQt top4, kernelQt.py:306-316).
 
     sigma block s = (l, n1', n2', r') receives T3 blocks (l, r, n1', c, n2') times
@@ -162,6 +162,9 @@ def panel_sigma4(t3lay, Rl, psi, t4):
     (c, r, c) slabs in R-panel order); and one dense GEMM per sector and operator
     writes its rows straight into the sigma blocks through a row table.  Returns
     None unless every sigma block pairs with all R blocks of its sector.
+
+    Within the slab of one c the K index is (r, c), c fastest, or (c, r) with r_fast (the
+    order the sparse two-site stage writes with contiguous fibers); the R panels follow it.
     """
     if len(t4) == 0:
         return None
@@ -232,14 +235,15 @@ def panel_sigma4(t3lay, Rl, psi, t4):
         if len(us) else numpy.zeros(0, dtype=numpy.int64)
     crow_base = numpy.zeros(nrb, dtype=numpy.int64)
     crow_base[used] = (numpy.cumsum(Mrb) - Mrb)[used]
-    rperm = (Rl.ioff[uR], poff[rbU] + koffU * dU[:, 1], dU)
+    kc, kr = (dU[:, 2], numpy.ones_like(kU)) if r_fast else (numpy.ones_like(kU), dU[:, 0])    # K strides of c and r
+    rperm = (Rl.ioff[uR], poff[rbU] + koffU * dU[:, 1], dU, (kc * dU[:, 1], numpy.ones_like(kU), kr * dU[:, 1]))
     gemm = (t3pan[used], poff[used], numpy.zeros(len(used), dtype=numpy.int64), Mrb[used], Drb_sec[used],
             Krb[used], crow_base[used], Kp[used])
     # the R panels transposed ([D_r' x K_r'], k contiguous, row stride Kp) for the tensor-core
-    # kernel: R block (c, r', r) element -> rtoff[r'] + r' * Kp + koff + r * D_c + c
+    # kernel: R block (c, r', r) element -> rtoff[r'] + r' * Kp + koff + k(c, r)
     rtsz = Drb_sec * Kp
     rtoff = numpy.cumsum(rtsz) - rtsz
-    rperm_t = (Rl.ioff[uR], rtoff[rbU] + koffU, dU, Kp[rbU])
+    rperm_t = (Rl.ioff[uR], rtoff[rbU] + koffU, dU, (kc, Kp[rbU], kr))
     return {"t3off": t3off, "t3fhs": t3fhs, "t3flo": t3flo, "t3size": int(tsz.sum()), "needed": i3,
             "rperm": rperm, "gemm": gemm, "crow": crow.astype(numpy.int64),
             "sectors": {"used": used, "M": Mrb[used], "N": Drb_sec[used], "K": Krb[used], "Kp": Kp[used],
@@ -605,7 +609,7 @@ def fg_col_perm(col, width, mc):
 
 
 def compile_fiber(c, triples, rows_axis, fiber_major, extra_out=None, in_off=None, out_off=None, out_fhs=None,
-                  out_flo=None, out_colmajor=False):
+                  out_flo=None, out_colmajor=False, out_rfast=False):
     """Fiber-group work items of a W contraction (template for one operator).
 
     The first three output axes form the fiber group (their block dims multiply
@@ -616,7 +620,8 @@ def compile_fiber(c, triples, rows_axis, fiber_major, extra_out=None, in_off=Non
     extra_out (output blocks that must be written: those without pairs are
     written as zeros; with out_off, pairs into any other output block are dropped),
     out_colmajor (output blocks stored column by column, [ncols][F]: the next W
-    contraction then reads them with contiguous fibers, fiber_major=0).
+    contraction then reads them with contiguous fibers, fiber_major=0), out_rfast (output
+    blocks with a two-level fiber split stored [F / flo][ncols][flo]).
     """
     empty = (numpy.zeros(0, FTASK_DT), numpy.zeros(0, FIN_DT), numpy.zeros(0, FOUT_DT), numpy.zeros(0, FPAIR_DT), 1,
              0.0, FIBER_TILE)
@@ -694,7 +699,7 @@ def compile_fiber(c, triples, rows_axis, fiber_major, extra_out=None, in_off=Non
     fouts["fhs"] = 0 if out_fhs is None else out_fhs[allo]
     if out_fhs is not None and len(allo) and int(out_fhs[allo].max()) >= 2 ** 31:
         return None
-    fouts["colmajor"] = 1 if out_colmajor else 0
+    fouts["colmajor"] = 1 if out_colmajor else 2 if out_rfast else 0
     fouts["pair_b"] = pb
     fouts["pair_e"] = pe
     pairs = numpy.zeros(len(ob), FPAIR_DT)
@@ -813,13 +818,14 @@ class FiberStage(object):
         c0o = numpy.cumsum(nco) - nco - col_b[go]           # first column of each output in its group
         e, c_in = ranges(nco)
         o_e, g_c = oidx[e], go[e]
-        cm = fo["colmajor"][o_e] != 0
+        cm = fo["colmajor"][o_e]
         nc_e = nco[e]
         cols_rec = numpy.zeros(int(CT.sum()), FGCOL_DT)
-        cols_rec["off"] = fo["c_off"][o_e] + numpy.where(cm, c_in * F[g_c], c_in)
-        cols_rec["fhs"] = numpy.where(cm, 0, fo["fhs"][o_e].astype(i64))
-        cols_rec["fs"] = numpy.where(cm, 1, nc_e)
-        cmo = fo["colmajor"][oidx] != 0
+        cols_rec["off"] = fo["c_off"][o_e] + c_in * numpy.where(cm == 1, F[g_c],
+                                                                numpy.where(cm == 2, fo["flo"][o_e].astype(i64), 1))
+        cols_rec["fhs"] = numpy.where(cm == 1, 0, fo["fhs"][o_e].astype(i64))
+        cols_rec["fs"] = numpy.where(cm != 0, 1, nc_e)
+        cmo = fo["colmajor"][oidx] == 1
         flo_o = numpy.where(cmo | (fo["flo"][oidx].astype(i64) >= F[go]), F[go], fo["flo"][oidx].astype(i64))
         flo = numpy.full(ng, numpy.iinfo(i64).max, dtype=i64)
         numpy.minimum.at(flo, go, flo_o)
@@ -1088,6 +1094,258 @@ def fiber_stages(parts, device, name, ops, budget=None):
     for p in parts:
         by.setdefault(p[6], []).append(p)
     return [FiberStage(v, device, name, ops, budget) for k, v in sorted(by.items())]
+
+
+# ---------------------------------------------------------------- sparse two-site MPO stage (qc_wsparse_*)
+WXGRP_DT = numpy.dtype([("start", "<i4"), ("F", "<i4"), ("flo", "<i4"), ("pad", "<i4"), ("a", "<i4", (16,)),
+                        ("c", "<i4", (16,)), ("h", "<i4", (16,))])
+WXDELTA_DT = numpy.dtype([("R", "<i4"), ("row_b", "<i4"), ("grp_b", "<i4"), ("grp_e", "<i4"), ("dop_b", "<i4"),
+                          ("pad", "<i4", (3,))])
+WXITEM_DT = numpy.dtype([("delta", "<i4"), ("grp", "<i4"), ("f0", "<i4"), ("nf", "<i4"), ("op_b", "<i4"),
+                         ("op_e", "<i4"), ("op0", "<i4"), ("pad", "<i4")])
+WXDOP_DT = numpy.dtype([("ent_b", "<i8"), ("quad_b", "<i4"), ("nquad", "<i4")])
+WXQUAD_DT = numpy.dtype([("ent", "<i4"), ("cnt", "<i4"), ("blk", "<i4"), ("c0nc", "<i4")])
+assert WXGRP_DT.itemsize == 208 and WXDELTA_DT.itemsize == 32 and WXITEM_DT.itemsize == 32
+assert WXDOP_DT.itemsize == 16 and WXQUAD_DT.itemsize == 16
+WX_MAXR = 640             # T1 rows of one charge difference (FP64 rows of a 32-fiber tile: 160 KB)
+WX_MAXQ = 1024            # quads of one (charge difference, operator)
+WX_TILE_BYTES = {"f64": 96 * 1024, "f32": 48 * 1024}
+WX_SMALL = 8 * 148        # 64-fiber tiles of all operators up to which a dot uses one tile width
+WX_ITEMS = 24 * 148       # work items wanted before operators are walked inside one
+
+
+def _unit_axes(lay, axes):
+    d = [numpy.asarray(lay.ndims[k]) for k in axes]
+    return all(len(x) == 4 and bool((x == 1).all()) for x in d)
+
+
+def sparse_w_class(c1, t1, t1off, t3lay, pan4, W1, W2, psi):
+    """Fiber groups of one operator class for the sparse two-site MPO stage.
+
+    T1 blocks (a, l, n1, n2, r) and T3 blocks (l, r, n1', c, n2') are grouped by their (l, r)
+    sectors, the groups by the charge difference q(l) - q(r): the MPO sectors a(n1, n2) and
+    c(n1', n2') are the same for all groups of one difference.  Returns None where that does
+    not hold or an offset does not fit the records (the caller then keeps the two separate
+    stages), else {"groups", "deltas", "rows", "iblk", "kblk", "row0", "R", "fibers"}."""
+    if not (_unit_axes(c1.out, (2, 3)) and _unit_axes(t3lay, (2, 4)) and _unit_axes(W1, (2, 3))
+            and _unit_axes(W2, (2, 3))):
+        return None
+    if 4 * max(int(numpy.max(W1.ndims[0])), int(numpy.max(W1.ndims[1])), int(numpy.max(W2.ndims[1]))) > FIBER_MAX_ROWS:
+        return None                          # the separate stages would leave the panel form
+    i64 = numpy.int64
+    nr = int(psi.nsyms[3])
+    b1 = numpy.unique(numpy.asarray(t1, dtype=i64)[:, 0])
+    a, l, n1, n2, r = c1.out.block_sectors(b1)
+    b3 = numpy.unique(numpy.asarray(pan4["needed"], dtype=i64))
+    l3, r3, m1, cc, m2 = t3lay.block_sectors(b3)
+    if len(b3) == 0:
+        return None
+    lr = numpy.unique(l3 * nr + r3)
+    keep = numpy.isin(l * nr + r, lr)
+    b1, a, l, n1, n2, r = (x[keep] for x in (b1, a, l, n1, n2, r))
+    gl, gr = lr // nr, lr % nr
+    q2 = lambda q: numpy.rint(2 * numpy.asarray(q)).astype(i64)            # noqa: E731
+    dq = q2(psi.qsyms[0])[gl] - q2(psi.qsyms[3])[gr]
+    uq, dinv = numpy.unique(dq, axis=0, return_inverse=True)
+    dinv = dinv.ravel()
+    nd = len(uq)
+    o = numpy.argsort(dinv, kind="stable")                                 # groups delta by delta
+    lr, gl, gr, dinv = lr[o], gl[o], gr[o], dinv[o]
+    pos = numpy.empty(int(psi.nsyms[0]) * nr, dtype=i64)
+    pos[lr] = numpy.arange(len(lr))
+    dl, dr = numpy.asarray(psi.ndims[0], dtype=i64), numpy.asarray(psi.ndims[3], dtype=i64)
+    F = dl[gl] * dr[gr]
+    g = numpy.zeros(len(lr), WXGRP_DT)
+    g["F"], g["flo"] = F, dr[gr]
+    g["a"], g["c"] = -1, -1
+    cs = numpy.cumsum(F) - F
+    first = numpy.searchsorted(dinv, numpy.arange(nd))
+    if int(F.sum()) >= 2 ** 31:
+        return None
+    g["start"] = cs - cs[first][dinv]
+    off1 = (c1.out.ioff if t1off is None else t1off)[b1]
+    off3, fhs3, flo3 = pan4["t3off"][b3], pan4["t3fhs"][b3], pan4["t3flo"][b3]
+    ends1 = off1 + c1.out.ndim[b1]
+    dc = numpy.asarray(W2.ndims[1], dtype=i64)
+    d3 = t3lay.block_dims(b3)
+    ends3 = off3 + numpy.maximum(d3[:, 0] - 1, 0) * fhs3 + d3[:, 1] * d3[:, 3]
+    if max(int(ends1.max()) if len(ends1) else 0, int(ends3.max())) >= 2 ** 31 or int(fhs3.max()) >= 2 ** 31:
+        return None
+    p1, p3 = pos[l * nr + r], pos[l3 * nr + r3]
+    if not numpy.array_equal(flo3, dr[r3]):
+        return None
+    s1, s3 = 4 * n1 + n2, 4 * m1 + m2
+    iblk = numpy.full((nd, 16), -1, dtype=numpy.int32)
+    kblk = numpy.full((nd, 16), -1, dtype=numpy.int32)
+    iblk[dinv[p1], s1] = a
+    kblk[dinv[p3], s3] = cc
+    # one MPO sector per (n1, n2), one block per (group, n1, n2)
+    if not (numpy.array_equal(iblk[dinv[p1], s1], a) and numpy.array_equal(kblk[dinv[p3], s3], cc)):
+        return None
+    if len(numpy.unique(p1 * 16 + s1)) != len(p1) or len(numpy.unique(p3 * 16 + s3)) != len(p3):
+        return None
+    g["a"][p1, s1] = off1
+    g["c"][p3, s3] = off3
+    g["h"][p3, s3] = fhs3
+    da = numpy.asarray(W1.ndims[0], dtype=i64)
+    rows_b = numpy.where(iblk >= 0, da[numpy.maximum(iblk, 0)], 0)          # [delta, 16]
+    R = rows_b.sum(axis=1)
+    row0 = numpy.where(iblk >= 0, numpy.cumsum(rows_b, axis=1) - rows_b, 0).astype(numpy.int32)
+    dcb = numpy.where(kblk >= 0, dc[numpy.maximum(kblk, 0)], 0)
+    if int(R.max()) > WX_MAXR or int(((dcb + 3) // 4).sum(axis=1).max()) > WX_MAXQ:
+        return None
+    d = numpy.zeros(nd, WXDELTA_DT)
+    d["R"] = R
+    d["row_b"] = numpy.cumsum(R) - R
+    d["grp_b"] = first
+    d["grp_e"] = numpy.r_[first[1:], len(lr)]
+    own, loc = _ranges(rows_b.ravel())
+    rows = ((own % 16) << 16 | loc).astype(numpy.int32)
+    return {"groups": g, "deltas": d, "rows": rows, "iblk": iblk, "kblk": kblk, "row0": row0,
+            "R": R.astype(numpy.int32), "fibers": numpy.add.reduceat(F, first), "W": (W1, W2)}
+
+
+class SparseWStage(object):
+    """T3 = T1 . (W_i W_{i+1}) for every operator in one sparse product (qc_wsparse_*).
+
+    parts: [(sparse_w_class result, operator range)] over the stage's operator table ops
+    (a_base: T1, c_base: T3); Wi / Wj: the sites' TensorSets, order: their operator of every
+    table row.  The MPO's values are compiled into the stage: it is a plan for these values."""
+
+    def __init__(self, parts, device, name, ops, Wi, Wj, order, kinds=("f64",)):
+        """kinds: precisions whose work items and coefficients are made now ("f64", "f32")."""
+        self.name, self.device = name, device
+        self.host_ops = ops
+        self.flops = self.bytes = 0.0
+        grps, dels, rows, dops, quads, ws, rs, self.op_ranges = [], [], [], [], [], [], [], []
+        ngrp = nrow = ndop = nq = ne = 0
+        w1, w2 = Wi.host(), Wj.host()
+        lib = native.lib()
+        i64 = numpy.int64
+        for part, (b, e) in parts:
+            W1, W2 = part["W"]
+            d = part["deltas"].copy()
+            nops, nd = e - b, len(d)
+            o1 = numpy.ascontiguousarray(Wi.offsets[order[b:e]], dtype=i64)
+            o2 = numpy.ascontiguousarray(Wj.offsets[order[b:e]], dtype=i64)
+            h, cq, ce = numpy.zeros(1, dtype=i64), numpy.zeros(1, dtype=i64), numpy.zeros(1, dtype=i64)
+            args = []
+            for lay, w, o in ((W1, w1, o1), (W2, w2, o2)):
+                args += [ptr(w), ptr(o), ptr(lay.nsyms), ptr(lay.ndims_cat), ptr(lay.ioff), ptr(lay.allowed)]
+            check(lib.qc_wx_build(nops, *args, nd, ptr(part["iblk"]), ptr(part["kblk"]), ptr(part["row0"]),
+                                  ptr(part["R"]), ptr(h), ptr(cq), ptr(ce)), "qc_wx_build")
+            dp = numpy.zeros(nd * nops, WXDOP_DT)
+            qd = numpy.zeros(int(cq[0]), WXQUAD_DT)
+            ww, rr = numpy.zeros((int(ce[0]), 4)), numpy.zeros(int(ce[0]), dtype=numpy.int32)
+            check(lib.qc_wx_fetch(int(h[0]), ne, nq, ptr(dp), ptr(qd), ptr(ww), ptr(rr)), "qc_wx_fetch")
+            d["grp_b"] += ngrp
+            d["grp_e"] += ngrp
+            d["row_b"] += nrow
+            d["dop_b"] = ndop + numpy.arange(nd) * nops
+            grps.append(part["groups"])
+            dels.append(d)
+            rows.append(part["rows"])
+            dops.append(dp)
+            quads.append(qd)
+            ws.append(ww)
+            rs.append(rr)
+            self.op_ranges.append((b, e, len(d)))
+            ngrp, nrow, ndop, nq, ne = ngrp + len(part["groups"]), nrow + len(part["rows"]), ndop + len(dp), \
+                nq + len(qd), ne + len(rr)
+        self.h_groups, self.h_deltas = numpy.concatenate(grps), numpy.concatenate(dels)
+        self.h_rows, self.h_dops, self.h_quads = (numpy.concatenate(x) for x in (rows, dops, quads))
+        self.h_ent_w, self.h_ent_r = numpy.concatenate(ws), numpy.concatenate(rs)
+        self.fibers = numpy.concatenate([p["fibers"] for p, _ in parts])
+        self.ntasks = len(self.h_groups)
+        up = lambda a, dt: upload(a if len(a) else numpy.zeros(1, dt), device)         # noqa: E731
+        self.d = {"groups": up(self.h_groups, WXGRP_DT), "deltas": up(self.h_deltas, WXDELTA_DT),
+                  "rows": up(self.h_rows, numpy.int32), "dops": up(self.h_dops, WXDOP_DT),
+                  "quads": up(self.h_quads, WXQUAD_DT), "ent_r": up(self.h_ent_r, numpy.int32),
+                  "ops": upload(ops, device)}
+        w = self.h_ent_w if len(self.h_ent_w) else numpy.zeros((1, 4))
+        # coefficients as 16-byte vectors: two per entry in FP64 (all first halves, then all second)
+        self._w = {"f64": torch.from_numpy(numpy.ascontiguousarray(w.reshape(-1, 2, 2).transpose(1, 0, 2))).to(device)}
+        self._launch = {}
+        for kind in kinds:
+            self.items(kind)
+            self.coefficients(kind)
+
+    def items(self, kind):
+        """Work items by fibers per lane, [(fpt, items, T1 rows, quads)], longest first.
+
+        A tile is 32, 64 or 128 fibers wide: as many as its T1 rows leave room for in
+        WX_TILE_BYTES of shared memory, so that two or three CTAs share an SM.  Dots whose
+        tiles fit the GPU at once use one width, in one launch."""
+        hit = self._launch.get(kind)
+        if hit is not None:
+            return hit
+        el = 8 if kind == "f64" else 4
+        d = self.h_deltas
+        R = numpy.maximum(d["R"].astype(numpy.int64), 1)
+        nops = numpy.concatenate([numpy.full(n, e - b) for (b, e, n) in self.op_ranges])
+        fpt = numpy.where(R * 128 * el <= WX_TILE_BYTES[kind], 4, numpy.where(R * 64 * el <= WX_TILE_BYTES[kind], 2, 1))
+        if int((((self.fibers + 63) // 64) * nops).sum()) <= WX_SMALL:
+            fpt[:] = int(fpt.min())
+        ft = 32 * fpt
+        nt = (self.fibers + ft - 1) // ft
+        op0 = numpy.concatenate([numpy.full(n, b) for (b, e, n) in self.op_ranges])
+        chunk = int(max(1, (nt * nops).sum() // WX_ITEMS))      # operators of one item
+        nch = (nops + chunk - 1) // chunk
+        own, loc = _ranges(nt * nch)
+        t, ch = loc // nch[own], loc % nch[own]
+        it = numpy.zeros(len(own), WXITEM_DT)
+        it["delta"] = own
+        p = t * ft[own]
+        it["nf"] = numpy.minimum(ft[own], self.fibers[own] - p)
+        # the tile's first group: groups are stored delta by delta with their first fibers
+        gkey = numpy.repeat(numpy.arange(len(d)), d["grp_e"] - d["grp_b"]).astype(numpy.int64) << 32
+        gkey = gkey + self.h_groups["start"]
+        it["grp"] = numpy.searchsorted(gkey, (own.astype(numpy.int64) << 32) + p, side="right") - 1
+        it["f0"] = p - self.h_groups["start"][it["grp"]]
+        it["op_b"] = op0[own] + ch * chunk
+        it["op_e"] = numpy.minimum(op0[own] + nops[own], it["op_b"] + chunk)
+        it["op0"] = op0[own]
+        nqd = self.h_dops["nquad"][d["dop_b"]].astype(numpy.int64)
+        cost = (it["op_e"] - it["op_b"]) * (R[own] + 2 * nqd[own]) * fpt[own]
+        out = []
+        for k in (4, 2, 1):
+            sel = numpy.flatnonzero(fpt[own] == k)
+            if len(sel) == 0:
+                continue
+            sel = sel[numpy.argsort(-cost[sel], kind="stable")]
+            dd = numpy.unique(own[sel])
+            out.append((k, it[sel], upload(it[sel], self.device), int(R[dd].max()), int(max(1, nqd[dd].max()))))
+        self._launch[kind] = out
+        return out
+
+    def coefficients(self, kind):
+        if kind not in self._w:
+            self._w[kind] = self._w["f64"].transpose(0, 1).contiguous().to(torch.float32)
+        return self._w[kind]
+
+    def run(self, A, B, C, kind="f64", stream=None):
+        """C = T3 from A = T1 (B, the operand of the separate stages, is not read)."""
+        if self.ntasks == 0:
+            return
+        lib = native.lib()
+        s = stream if stream is not None else torch.cuda.current_stream(C.device).cuda_stream
+        k = "f64" if kind == "f64" else "f32"
+        w = self.coefficients(k)
+        fn = lib.qc_wsparse_f64 if k == "f64" else lib.qc_wsparse_f32
+        if LOG.enabled:
+            e0 = torch.cuda.Event(enable_timing=True)
+            e1 = torch.cuda.Event(enable_timing=True)
+            e0.record()
+        d = self.d
+        for (fpt, host, dev, maxr, maxq) in self.items(k):
+            check(fn(dev.data_ptr(), len(host), fpt, d["deltas"].data_ptr(), d["groups"].data_ptr(),
+                     d["rows"].data_ptr(), d["dops"].data_ptr(), d["quads"].data_ptr(), w.data_ptr(),
+                     len(self.h_ent_r), d["ent_r"].data_ptr(), d["ops"].data_ptr(), maxr, maxq, A.data_ptr(), C.data_ptr(), s),
+                  "qc_wsparse_" + k)
+            LOG.launches += 1
+        if LOG.enabled:
+            e1.record()
+            LOG.records.append((self.name, e0, e1, self.flops, self.bytes * (A.element_size() / 8.0)))
 
 
 # ---------------------------------------------------------------- tensor-core panel GEMM (qc_tcpanel_f32)

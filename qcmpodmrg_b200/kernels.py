@@ -20,7 +20,7 @@ from . import native
 from .native import check
 from .engine import (Stage, compile_classes, add_parts, live_blocks, prune, op_table, TASK_DT, CONTRIB_DT, LOG,
                      compile_fiber, FiberStage, CompositeStage, panel_sigma1, compile_panels, BPERM_DT, PanelStage,
-                     fiber_stages, panel_sigma4, upload)
+                     fiber_stages, panel_sigma4, upload, sparse_w_class, SparseWStage)
 from .mpo import case
 from .qtensor import Contraction, Layout, flip_right, flip_horizontal
 
@@ -55,6 +55,9 @@ class TensorSet(object):
             host = numpy.concatenate([numpy.asarray(v, dtype=numpy.float64) for v in values]) \
                 if values else numpy.zeros(0)
             values = torch.from_numpy(host).to(device)
+            self._host = (host, values, values._version)
+        else:
+            self._host = None
         self.values = values
         self._f32 = None
 
@@ -62,6 +65,14 @@ class TensorSet(object):
         if self._f32 is None or self._f32.data_ptr() == 0:
             self._f32 = self.values.to(torch.float32)
         return self._f32
+
+    def host(self):
+        """The values as a host array: those the set was made from while the device tensor is
+        that one and unchanged since, else a copy from the device (which waits for it)."""
+        h = self._host
+        if h is not None and h[1] is self.values and h[2] == self.values._version:
+            return h[0]
+        return numpy.ascontiguousarray(self.values.detach().cpu().numpy(), dtype=numpy.float64)
 
     def op_values(self, i):
         o = int(self.offsets[i])
@@ -177,8 +188,10 @@ class SigmaOperator(object):
 
     def __init__(self, ws, isite, psi_layout, L, R, Wi, Wj, qkey, opers, hpwts, precision="f64",
                  tensor_cores=None, use_fiber=False, fuse_w=True, panel1=True, panel4=True, live=None,
-                 fg_budget=None):
-        """fg_budget: (A, W) shared-memory budgets of the dense fiber-group GEMM (qc_fgemm), as
+                 fg_budget=None, sparse_w=None):
+        """sparse_w: the two MPO-site contractions as one sparse product (qc_wsparse, the fiber
+        path without fuse_w); None: on a GPU, where the plan's blocks allow it.
+        fg_budget: (A, W) shared-memory budgets of the dense fiber-group GEMM (qc_fgemm), as
         chosen by qcmpodmrg_b200.autotune; None keeps the engine's defaults.
         live: optional mask over the wavefunction layout's flat blocks.  Blocks outside it
         are zero in every input vector and discarded in every output (the blocks that N
@@ -204,6 +217,11 @@ class SigmaOperator(object):
         wbase = numpy.zeros(nops, dtype=numpy.int64)
         wtot = 0
         plans = {}
+        self._fiber_args = (ax, groups, qkey, live, fg_budget)
+        if sparse_w is None:
+            sparse_w = torch.device(dev).type == "cuda"
+        sparse_w = bool(sparse_w) and use_fiber and not fuse_w and panel1 and panel4
+        chains, sx = {}, {}
         for key, ops in sorted(groups.items()):
             i0 = ops[0]
             Ll, W1, W2 = L.layouts[i0], Wi.layouts[i0], Wj.layouts[i0]
@@ -212,23 +230,23 @@ class SigmaOperator(object):
                 if (L.layouts[i] is not Ll or Wi.layouts[i] is not W1 or Wj.layouts[i] is not W2
                         or flip_right(R.layouts[i], qkey) is not Rl):
                     raise ValueError("operators of one symmetry class must share their block structure")
-            c1 = Contraction(Ll, psi_layout, ax[0])
-            t1 = c1.triples if live is None else prune(c1.triples, live2=live)
-            # L.psi as dense panel GEMMs (T1 blocks stored panel by panel)
-            pan = panel_sigma1(Ll, psi_layout, t1, c1.out.nblks) if panel1 else None
+            chains[key] = ch = self._chain(Ll, W1, W2, Rl, use_fiber, panel1, panel4, sparse_w)
+            if sparse_w:
+                (c1, t1), _, (c3, _), _, pan, pan4 = ch
+                sx[key] = sparse_w_class(c1, t1, pan["t1off"], c3.out, pan4, W1, W2, psi_layout) \
+                    if pan is not None and pan4 is not None else None
+                sparse_w = sx[key] is not None
+        for key, ops in sorted(groups.items()):
+            i0 = ops[0]
+            W1, W2 = Wi.layouts[i0], Wj.layouts[i0]
+            Rl = flip_right(R.layouts[i0], qkey)
+            if sx and not sparse_w:         # a class has no sparse form: the separate stages' T3 order
+                chains[key] = self._chain(L.layouts[i0], W1, W2, Rl, use_fiber, panel1, panel4)
+            (c1, t1), (c2, t2), (c3, t3), (c4, t4all), pan, pan4 = chains[key]
             t1off = pan["t1off"] if pan is not None else None
-            c2 = Contraction(c1.out, W1, ax[1])
-            t2 = prune(c2.triples, live1=live_blocks(c1.out, t1))
-            c3 = Contraction(c2.out, W2, ax[2])
-            t3 = prune(c3.triples, live1=live_blocks(c2.out, t2))
             # .W_i and .W_{i+1} fused: T3 = T1 . (W_i W_{i+1}) with the two-site MPO
             # block Wij[a, n1', n1, c, n2', n2] = sum_b W_i[a, b, n1', n1] W_{i+1}[b, c, n2', n2]
             # made once per dot, so T2 is never written (fiber-group kernel only)
-            c4 = Contraction(c3.out, Rl, ax[3])
-            t4all = c4.triples if live is None else c4.triples[live[c4.triples[:, 0]]]
-            # .R as dense panel GEMMs (T3 blocks written into sigma-block panels by the
-            # fiber kernel, R blocks permuted into per-sector panels once per dot)
-            pan4 = panel_sigma4(c3.out, Rl, psi_layout, t4all) if (use_fiber and panel4) else None
             o3 = {} if pan4 is None else {"out_off": pan4["t3off"], "out_fhs": pan4["t3fhs"],
                                           "out_flo": pan4["t3flo"], "extra_out": pan4["needed"]}
             fused = None
@@ -241,23 +259,12 @@ class SigmaOperator(object):
                     fp = compile_fiber(cF, tF, 0, 0, in_off=t1off, **o3)
                     if fp is not None:
                         fused = (cW, cF, tF, fp)
-            elif use_fiber:
-                # .W_i and .W_{i+1} on the fiber kernel: T2 stored column by column (its
-                # physical axes have extent 1, so a T2 block's columns are the next
-                # contraction's rows and its fibers that contraction's fibers), read back
-                # with contiguous fibers
-                cm = bool(unit_phys_t2(c2.out))
-                fib2 = compile_fiber(c2, t2, 0, 0, in_off=t1off, out_colmajor=cm)
-                cm = cm and fib2 is not None
-                if pan4 is not None:
-                    fib3 = compile_fiber(c3, t3, 3, 0 if cm else 1, **o3)
-                    if fib3 is None:
-                        pan4 = None
-                if fib3 is None:
-                    fib3 = compile_fiber(c3, t3, 3, 0 if cm else 1)
-                if fib3 is None and cm:
-                    fib2 = compile_fiber(c2, t2, 0, 0, in_off=t1off)       # T2 packed for the grouped GEMM
-            if pan4 is not None and fused is None and fib3 is None:
+            elif use_fiber and not sparse_w:
+                fib2, fib3 = self._fiber_pair(c1, c2, t2, c3, t3, t1off, o3)
+                if fib3 is None and pan4 is not None:
+                    pan4 = None
+                    fib2, fib3 = self._fiber_pair(c1, c2, t2, c3, t3, t1off, {})
+            if pan4 is not None and fused is None and fib3 is None and not sparse_w:
                 pan4 = None                 # T3 comes from the grouped GEMM in the packed layout
             t4 = prune(t4all, live1=live_blocks(c3.out, fused[2] if fused else t3))
             if c4.out is not psi_layout:
@@ -291,8 +298,10 @@ class SigmaOperator(object):
         st = [{}, {}, {}, {}]
         fib = [[], [], [], []]
         fuse_parts, wij_parts = [], {}
-        # how the W contractions of each symmetry class run: fused / fiber / grouped GEMM
-        self.w_paths = {"fused": 0, "fiber": 0, "generic": 0}
+        wx_parts = []
+        # how the W contractions of each symmetry class run: sparse product / fused / fiber /
+        # grouped GEMM
+        self.w_paths = {"sparse": 0, "fused": 0, "fiber": 0, "generic": 0}
         pos = 0
         # W contractions: fiber-group kernel (inputs staged once per fiber tile) where
         # every group fits in shared memory, generic grouped GEMM otherwise
@@ -324,11 +333,11 @@ class SigmaOperator(object):
             if any4:
                 d = numpy.zeros(0, BPERM_DT)
                 if pan4 is not None:
-                    src, dst, dU = pan4["rperm"]
+                    src, dst, dU, st3 = pan4["rperm"]
                     d = numpy.zeros(len(src), BPERM_DT)
                     d["src_off"], d["dst_off"] = src, dst
                     d["d0"], d["d1"], d["d2"] = dU[:, 0], dU[:, 1], dU[:, 2]
-                    d["s0"], d["s1"], d["s2"] = dU[:, 1], 1, dU[:, 0] * dU[:, 1]
+                    d["s0"], d["s1"], d["s2"] = st3
                 else:                       # R blocks copied in place
                     src = dst = Rl.ioff[Rl.idx_allowed]
                     d = numpy.zeros(len(src), BPERM_DT)
@@ -350,6 +359,9 @@ class SigmaOperator(object):
                     add_parts(p4st_tc, tcp)
                 for cfg, part in parts.items():
                     p4st.setdefault(cfg, []).append(part)
+            if sparse_w:
+                wx_parts.append((sx[key], rng))
+                self.w_paths["sparse"] += 1
             if fib3 is not None:
                 fib[2].append(fib3 + (rng,))
                 self.w_paths["fiber"] += 1
@@ -378,12 +390,18 @@ class SigmaOperator(object):
                     fib[1].append(fib2 + (rng,))
                     self.w_paths["fiber"] += 1
                     continue
+                if sparse_w and si in (1, 2):
+                    continue
                 if si in (1, 2):
                     self.w_paths["generic"] += 1
                 add_parts(st[si], compile_classes(c, t, ax[si], tensor_cores=tc if si in (0, 3) else False,
                                                   off1=off1), op_range=rng)
-        self.stages = []
+        self._stages = []
+        self._tabs = tabs
         for si in range(4):
+            if sparse_w and si in (1, 2):
+                self._stages.append(None)       # compiled when the stage list is asked for
+                continue
             g = Stage(st[si], dev, "sigma%d" % (si + 1), tabs[si]) if st[si] else None
             f = fiber_stages(fib[si], dev, "sigma%d" % (si + 1), tabs[si], fg_budget) if fib[si] else []
             if si == 0:
@@ -394,9 +412,12 @@ class SigmaOperator(object):
                 f = [PanelStage(p4st, dev, "sigma4", tabs[3], p4st_tc,
                                 crow=numpy.concatenate(crow_all) if crow_all else None)]
             if not f:
-                self.stages.append(g if g is not None else Stage({}, dev, "sigma%d" % (si + 1), tabs[si]))
+                self._stages.append(g if g is not None else Stage({}, dev, "sigma%d" % (si + 1), tabs[si]))
             else:
-                self.stages.append(CompositeStage(f + [g], "sigma%d" % (si + 1)))
+                self._stages.append(CompositeStage(f + [g], "sigma%d" % (si + 1)))
+        # the two MPO-site contractions as one sparse product, T1 -> T3
+        self.wx = SparseWStage(wx_parts, dev, "sigma23", op_table(bases[0][order], 0, bases[2][order], 1.0), Wi, Wj,
+                               order, ("f64",) if precision == "f64" else ("f64", "f32")) if sparse_w else None
         # per-dot L panels (a block permutation of every operator's L), FP64 and FP32
         self.lperm = None
         if lperm:
@@ -454,34 +475,109 @@ class SigmaOperator(object):
                     continue
                 c, t = cs[si]
                 tot_b += stage_bytes(c, t, len(ops), si == 0)      # psi is read by every operator
-            self.stages[si].bytes = float(tot_b)
+            if self._stages[si] is not None:
+                self._stages[si].bytes = float(tot_b)
+            if self.wx is not None and si in (1, 2):
+                # T1 and the site's MPO in, T3 and the other site's MPO: no T2
+                for key, (ops, *cs, Rl, fused, pan, pan4, fib2, fib3) in sorted(plans.items()):
+                    (ca, ta), (cb, tb) = cs[1], cs[2]
+                    u, wu = (numpy.unique(ta[:, 1]), numpy.unique(ta[:, 2])) if si == 1 else \
+                        (numpy.unique(tb[:, 0]), numpy.unique(tb[:, 2]))
+                    nb = (ca.l1.ndim[u].sum() + ca.l2.ndim[wu].sum()) if si == 1 else \
+                        (cb.out.ndim[u].sum() + cb.l2.ndim[wu].sum())
+                    self.wx.bytes += 8.0 * float(nb) * len(ops)
         for key, (ops, *cs, Rl, fused, pan, pan4, fib2, fib3) in sorted(plans.items()):
             if fused is not None and LOG.enabled:
                 fb += stage_bytes(fused[1], fused[2], len(ops), False)
         if self.fused is not None:
             self.fused.bytes = float(fb)
         if self.tc4 is not None:
-            self.tc4.bytes = self.stages[3].bytes
+            self.tc4.bytes = self._stages[3].bytes
         if self.tc1 is not None:
-            self.tc1.bytes = self.stages[0].bytes
+            self.tc1.bytes = self._stages[0].bytes
         # FLOPs of the reference's four-contraction chain (tensordotCAL pair GEMMs),
         # whatever the fusion used here
         self.flops = 0.0
         for key, (ops, *cs, Rl, fused, pan, pan4, fib2, fib3) in sorted(plans.items()):
-            for (c, t) in cs:
-                self.flops += pair_flops(c, t) * len(ops)
+            for si, (c, t) in enumerate(cs):
+                fl = pair_flops(c, t) * len(ops)
+                self.flops += fl
+                if self.wx is not None and si in (1, 2):
+                    self.wx.flops += fl
         self.ndim0 = psi_layout.size
         # W panels of the dense fiber-group stages, gathered now (per dot) rather than in
         # the first matrix-vector product
         if torch.device(dev).type == "cuda":
             s = torch.cuda.current_stream(dev).cuda_stream
-            wsets = [(self.stages[1], self.Wi), (self.stages[2], self.Wj)]
-            for st, wset in wsets:
+            wsets = [(self._stages[1], self.Wi), (self._stages[2], self.Wj)]
+            for st, wset in wsets if self.wx is None else []:
                 for sub in (st.subs if isinstance(st, CompositeStage) else [st]):
                     if isinstance(sub, FiberStage) and sub.ntasks and sub.fgemm:
                         sub.wpanel(wset.values, s)
                         if precision != "f64":
                             sub.wpanel(wset.f32(), s)
+
+    def _chain(self, Ll, W1, W2, Rl, use_fiber, panel1, panel4, r_fast=False):
+        """The four contractions of one operator class with their block pairs, and the panel
+        forms of the first and the last one (None where a class has none)."""
+        ax, _, _, live, _ = self._fiber_args
+        c1 = Contraction(Ll, self.psi, ax[0])
+        t1 = c1.triples if live is None else prune(c1.triples, live2=live)
+        # L.psi as dense panel GEMMs (T1 blocks stored panel by panel)
+        pan = panel_sigma1(Ll, self.psi, t1, c1.out.nblks) if panel1 else None
+        c2 = Contraction(c1.out, W1, ax[1])
+        t2 = prune(c2.triples, live1=live_blocks(c1.out, t1))
+        c3 = Contraction(c2.out, W2, ax[2])
+        t3 = prune(c3.triples, live1=live_blocks(c2.out, t2))
+        c4 = Contraction(c3.out, Rl, ax[3])
+        t4 = c4.triples if live is None else c4.triples[live[c4.triples[:, 0]]]
+        # .R as dense panel GEMMs (T3 blocks written into sigma-block panels, R blocks
+        # permuted into per-sector panels once per dot)
+        pan4 = panel_sigma4(c3.out, Rl, self.psi, t4, r_fast) if (use_fiber and panel4) else None
+        return (c1, t1), (c2, t2), (c3, t3), (c4, t4), pan, pan4
+
+    @staticmethod
+    def _fiber_pair(c1, c2, t2, c3, t3, t1off, o3):
+        """.W_i and .W_{i+1} on the fiber kernel: T2 stored column by column (its physical
+        axes have extent 1, so a T2 block's columns are the next contraction's rows and its
+        fibers that contraction's fibers), read back with contiguous fibers."""
+        cm = bool(unit_phys_t2(c2.out))
+        fib2 = compile_fiber(c2, t2, 0, 0, in_off=t1off, out_colmajor=cm)
+        cm = cm and fib2 is not None
+        fib3 = compile_fiber(c3, t3, 3, 0 if cm else 1, **o3)
+        if fib3 is None and cm and not o3:
+            fib2 = compile_fiber(c2, t2, 0, 0, in_off=t1off)       # T2 packed for the grouped GEMM
+        return fib2, fib3
+
+    @property
+    def stages(self):
+        """The four contractions as separate stages.  With the sparse product the two
+        MPO-site ones are not part of a matrix-vector product; they are compiled when asked
+        for (lockstep batches run the stages of many operators in common launches)."""
+        if self.wx is not None and self._stages[1] is None:
+            ax, groups, qkey, live, fg_budget = self._fiber_args
+            fib = [[], []]
+            pos = 0
+            for key, ops in sorted(groups.items()):
+                rng = (pos, pos + len(ops))
+                pos += len(ops)
+                i0 = ops[0]
+                (c1, _), (c2, t2), (c3, t3), _, pan, pan4 = self._chain(
+                    self._lays[0][i0], self.Wi.layouts[i0], self.Wj.layouts[i0], flip_right(self._lays[1][i0], qkey),
+                    True, True, True, True)
+                f2, f3 = self._fiber_pair(c1, c2, t2, c3, t3, pan["t1off"],
+                                          {"out_off": pan4["t3off"], "out_fhs": pan4["t3fhs"],
+                                           "out_flo": pan4["t3flo"], "extra_out": pan4["needed"],
+                                           "out_rfast": True})
+                if f2 is None or f3 is None:
+                    raise RuntimeError("fiber groups of a sparse two-site plan could not be compiled")
+                fib[0].append(f2 + (rng,))
+                fib[1].append(f3 + (rng,))
+            for k in (0, 1):
+                name = "sigma%d" % (k + 2)
+                self._stages[k + 1] = CompositeStage(
+                    fiber_stages(fib[k], self.ws.device, name, self._tabs[k + 1], fg_budget), name)
+        return self._stages
 
     def rebind(self, L, R):
         """Use new environment values with the same block layouts (cached plan)."""
@@ -516,11 +612,11 @@ class SigmaOperator(object):
             t3b.append(int(t3bases[ops_c[0]]))
             rtb.append(rt_tot)
             rts.append(opstride)
-            src, dst, dU, kp = pan4["rperm_t"]
+            src, dst, dU, st3 = pan4["rperm_t"]
             d = numpy.zeros(len(src), BPERM_DT)
             d["src_off"], d["dst_off"] = src, dst
             d["d0"], d["d1"], d["d2"] = dU[:, 0], dU[:, 1], dU[:, 2]
-            d["s0"], d["s1"], d["s2"] = 1, kp, dU[:, 0]
+            d["s0"], d["s1"], d["s2"] = st3
             d["op_b"], d["op_e"] = rng
             descs.append(d)
             rt_tot += opstride * len(ops_c)
@@ -565,7 +661,7 @@ class SigmaOperator(object):
             tot += stride * len(poss)
         self._lp_total = (tot + 31) // 32 * 32
         units, maps, segs = tc_sigma1_units(classes, info, cols, lpb, lps, self._lp_total, self._psi_total)
-        self.tc1 = TCPanelStage("sigma1", units, maps, st1_ops, None, self.stages[0].flops, dev, segs=segs)
+        self.tc1 = TCPanelStage("sigma1", units, maps, st1_ops, None, self._stages[0].flops, dev, segs=segs)
         self._lp_descs = numpy.concatenate(descs)
         self._lp_descs_d = upload(self._lp_descs, dev)
         self._lp_ops_d = upload(op_table(L.offsets[order], 0, base, 1.0), dev)
@@ -696,13 +792,16 @@ class SigmaOperator(object):
             y = torch.empty(self.ndim0, dtype=torch.float64, device=ws.device)
         if prec == "f64":
             T1 = ws.get("t1", self.tot[0], torch.float64)
-            T2 = ws.get("t2", self.tot[1], torch.float64)
             T3 = ws.get("t3", self.tot[2], torch.float64)
             P = ws.get("part", self.nops * self.ndim0, torch.float64)
-            s = self.stages
+            s = self._stages
             s[0].run(self.a1("f64"), x, T1, "f64")
-            s[1].run(T1, self.Wi.values, T2, "f64")
-            s[2].run(T2, self.Wj.values, T3, "f64")
+            if self.wx is not None:
+                self.wx.run(T1, None, T3, "f64")
+            else:
+                T2 = ws.get("t2", self.tot[1], torch.float64)
+                s[1].run(T1, self.Wi.values, T2, "f64")
+                s[2].run(T2, self.Wj.values, T3, "f64")
             if self.fused is not None:
                 self.fused.run(T1, self.Wij, T3, "f64")
             P[:self.nops * self.ndim0].zero_()
@@ -710,13 +809,12 @@ class SigmaOperator(object):
             return reduce_ops(P, self.nops, self.ndim0, y)
         kind = prec if prec in ("tf32", "tf32x3") else "f32"
         T1 = ws.get("t1", self.tot[0], torch.float32)
-        T2 = ws.get("t2", self.tot[1], torch.float32)
         T3 = ws.get("t3", self.tot[2], torch.float32)
         x32 = ws.get("x32", self.ndim0, torch.float32)
         y32 = ws.get("y32", self.ndim0, torch.float32)
         convert(x, x32)
         P = ws.get("part32", self.nops * self.ndim0, torch.float32)
-        s = self.stages
+        s = self._stages
         if self.tc1 is not None and kind == "tf32x3":
             pt = ws.get("psiT", 2 * self._psi_total, torch.float32)
             gather_split(x, self._psi_gidx, pt[:self._psi_total], pt[self._psi_total:2 * self._psi_total])
@@ -725,8 +823,12 @@ class SigmaOperator(object):
                 self._s0_generic.run(self.a1("f32"), x32, T1, "f32")
         else:
             s[0].run(self.a1("f32"), x32, T1, kind)
-        s[1].run(T1, self.Wi.f32(), T2, "f32")
-        s[2].run(T2, self.Wj.f32(), T3, "f32")
+        if self.wx is not None:
+            self.wx.run(T1, None, T3, "f32")
+        else:
+            T2 = ws.get("t2", self.tot[1], torch.float32)
+            s[1].run(T1, self.Wi.f32(), T2, "f32")
+            s[2].run(T2, self.Wj.f32(), T3, "f32")
         if self.fused is not None:
             self.fused.run(T1, self.wij32(), T3, "f32")
         P[:self.nops * self.ndim0].zero_()

@@ -1,0 +1,161 @@
+"""The sparse two-site MPO stage (qc_wsparse): its records interpreted in NumPy against the
+oracle-checked separate stages on the CPU, and the kernel against the grouped-GEMM sigma on
+the GPU at the edges of its tiles (one fiber, 31 / 32 / 33, several sectors in one tile, 64
+and 128 fibers, the last partial quad), in FP64, FP32 and split TF32."""
+import numpy
+import pytest
+import torch
+
+from helpers import load, layout_of, tensorset, record_operators
+from emulate import patch_stage_run
+from qcmpodmrg_b200 import engine
+from qcmpodmrg_b200.hamiltonian import make_hamiltonian
+from qcmpodmrg_b200.mpo import QPHYS, build_mpo
+from qcmpodmrg_b200.qtensor import Layout, classification
+
+
+def interpret(st, A, C, kind="f64"):
+    """C written by the items of a SparseWStage, each element once, absent blocks zero."""
+    a, c = A.numpy().astype(numpy.float64), C.numpy()
+    hits = numpy.zeros(len(c), dtype=numpy.int64)
+    for (fpt, items, _, maxr, maxq) in st.items(kind):
+        for it in items:
+            d = st.h_deltas[it["delta"]]
+            assert it["nf"] <= 32 * fpt and d["R"] <= maxr
+            starts = st.h_groups["start"][d["grp_b"]:d["grp_e"]]
+            pos = st.h_groups["start"][it["grp"]] + it["f0"] + numpy.arange(it["nf"])
+            gi = numpy.searchsorted(starts, pos, side="right") - 1
+            f = pos - starts[gi]
+            g = st.h_groups[d["grp_b"] + gi]
+            assert (f < g["F"]).all()
+            rows = st.h_rows[d["row_b"]:d["row_b"] + d["R"]]
+            for op in range(it["op_b"], it["op_e"]):
+                o = st.host_ops[op]
+                T = numpy.zeros((d["R"], it["nf"]))
+                for r, rec in enumerate(rows):
+                    off = g["a"][:, rec >> 16]
+                    ok = off >= 0
+                    T[r, ok] = a[o["a_base"] + off[ok] + f[ok] + (rec & 0xffff) * g["F"][ok]]
+                dop = st.h_dops[d["dop_b"] + op - it["op0"]]
+                assert dop["nquad"] <= maxq
+                for q in st.h_quads[dop["quad_b"]:dop["quad_b"] + dop["nquad"]]:
+                    e = slice(dop["ent_b"] + q["ent"], dop["ent_b"] + q["ent"] + q["cnt"])
+                    val = st.h_ent_w[e].T @ T[st.h_ent_r[e]]                  # [4, nf]
+                    off = g["c"][:, q["blk"]]
+                    ok = off >= 0
+                    dst = o["c_base"] + off + (f // g["flo"]) * g["h"][:, q["blk"]] + f % g["flo"]
+                    for k in range(q["c0nc"] & 0xff):
+                        at = (dst + ((q["c0nc"] >> 8) + k) * g["flo"])[ok]
+                        hits[at] += 1
+                        c[at] = val[k, ok]
+    return hits
+
+
+def sparse_sigma(r, device, sparse_w=True, precision="f64"):
+    from qcmpodmrg_b200.kernels import SigmaOperator, Workspace
+    opers = [int(x) for x in numpy.atleast_1d(r["opers"])]
+    return SigmaOperator(Workspace(torch.device(device)), int(r["key"][2]), layout_of(r["qtmp"]),
+                         tensorset(r["envL"], device), tensorset(r["envR"], device), tensorset(r["mpo_i"], device),
+                         tensorset(r["mpo_j"], device), numpy.asarray(r["qkey"], dtype=numpy.float64), opers,
+                         numpy.atleast_1d(r["hpwts"]).astype(numpy.float64), precision, use_fiber=True, fuse_w=False,
+                         sparse_w=sparse_w)
+
+
+@pytest.mark.parametrize("tag", ["K4", "K5", "K6", "K5N2"])
+def test_sparse_records_reproduce_the_separate_stages(tag, monkeypatch):
+    """T3 of the sparse records equals T3 of the two separate stages, every element of the
+    T3 panels that stage writes is written exactly once, and sigma is the reference's."""
+    patch_stage_run(monkeypatch)
+    monkeypatch.setattr(engine.SparseWStage, "run",
+                        lambda self, A, B, C, kind="f64", stream=None: interpret(self, A, C, kind))
+    used = 0
+    for r in load("kernels_%s.npz" % tag)["records"]:
+        sig = sparse_sigma(r, "cpu")
+        x = torch.from_numpy(numpy.asarray(r["hvec_x"], dtype=numpy.float64))
+        ref = numpy.asarray(r["hvec_y"])
+        assert numpy.abs(sig(x).numpy() - ref).max() <= 1e-12 * max(1.0, numpy.abs(ref).max())
+        if sig.wx is None:
+            continue
+        used += 1
+        T1 = torch.zeros(sig.tot[0] + 64, dtype=torch.float64)
+        T2 = torch.zeros(sig.tot[1] + 64, dtype=torch.float64)
+        sig._stages[0].run(sig.a1("f64"), x, T1, "f64")
+        ta, tb = torch.zeros(sig.tot[2] + 64, dtype=torch.float64), torch.zeros(sig.tot[2] + 64, dtype=torch.float64)
+        sig.stages[1].run(T1, sig.Wi.values, T2, "f64")         # the stages compiled on demand
+        sig.stages[2].run(T2, sig.Wj.values, tb, "f64")
+        for kind in ("f64", "f32"):
+            ta.zero_()
+            hits = interpret(sig.wx, T1, ta, kind)
+            assert hits.max() <= 1
+            assert numpy.abs(ta.numpy() - tb.numpy()).max() <= 1e-13 * max(1.0, tb.abs().max().item())
+            assert (hits[tb.numpy() != 0] == 1).all()
+    assert used
+
+
+def test_changed_mpo_values_are_seen():
+    """The host copy of a TensorSet is not used once the device values were changed in place."""
+    from qcmpodmrg_b200.kernels import TensorSet
+    r = load("kernels_K4.npz")["records"][0]
+    w = tensorset(r["mpo_i"], "cpu")
+    assert w.host() is w.host()
+    w.values[0] += 1.0
+    assert w.host()[0] == float(w.values[0])
+    w2 = TensorSet(w.layouts, w.values.clone(), w.offsets)
+    assert numpy.array_equal(w2.host(), w.host())
+
+
+def _dot(K, isite, nl, nr, dev, precision, seed=0, sparse_w=None):
+    """A dot whose bonds have the given states per (N, Sz) sector, with random environments."""
+    from qcmpodmrg_b200.kernels import SigmaOperator, TensorSet, Workspace
+    N = K
+    ham = make_hamiltonian(K, N, 3, 3.0)
+    W = {i: TensorSet(*v, device=dev) for i, v in build_mpo(ham, (isite, isite + 1)).items()}
+    ql = numpy.array([[n, 0.5 * s] for n, s, c in nl for _ in range(c)])
+    qr = numpy.array([[n, 0.5 * s] for n, s, c in nr for _ in range(c)])
+    qkey = numpy.array([float(N), 0.0])
+    cl = [classification(q) for q in (ql, QPHYS, QPHYS, qkey - qr)]
+    psi = Layout([False, False, False, True], [c[0] for c in cl], [c[1] for c in cl])
+    gen = torch.Generator(device="cpu").manual_seed(seed)
+
+    def env(lays, k, sign, q):
+        c = classification(q)
+        out = [Layout([True, False, True], [sign * l.qsyms[k], c[0], c[0]], [l.ndims[k], c[1], c[1]]) for l in lays]
+        v = torch.randn(sum(l.size for l in out), dtype=torch.float64, generator=gen).to(dev)
+        return TensorSet(out, v, device=dev)
+
+    L, R = env(W[isite].layouts, 0, 1.0, ql), env(W[isite + 1].layouts, 1, -1.0, qr)
+    opers = list(range(2 * K))
+    mk = lambda **kw: SigmaOperator(Workspace(torch.device(dev)), isite, psi, L, R, W[isite], W[isite + 1], qkey,  # noqa: E731
+                                    opers, numpy.ones(2 * K), precision, **kw)
+    x = torch.randn(psi.size, dtype=torch.float64, generator=gen).to(dev)
+    return mk, x
+
+
+SECTORS = [
+    ([(3, 1, 1), (4, 0, 1), (5, -1, 1)], [(3, 1, 1), (4, 0, 1), (3, -1, 1)]),             # one fiber per sector pair
+    ([(4, 0, 31), (3, 1, 1), (5, 1, 1)], [(4, 0, 1), (3, -1, 1), (3, 1, 1)]),             # 31 fibers
+    ([(4, 0, 8), (3, -1, 3), (5, 1, 2)], [(4, 0, 4), (3, 1, 11), (2, 0, 3)]),             # 32 and 33 fibers
+    ([(4, 0, 13), (3, -1, 7), (3, 1, 5), (5, -1, 6), (2, 0, 2), (6, 0, 3)],
+     [(4, 0, 10), (3, 1, 9), (3, -1, 6), (5, 1, 4), (2, 0, 3)]),                          # several tiles, ragged
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", range(len(SECTORS)))
+@pytest.mark.parametrize("precision", ["f64", "f32", "tf32x3"])
+def test_kernel_at_the_edges_of_its_tiles(case, precision, cuda, monkeypatch):
+    """FP64 within 1e-12 of the grouped GEMM, FP32 within 2e-5, at every fiber-tile width
+    (the shared-memory budget forces 32, 64 and 128 fibers)."""
+    nl, nr = SECTORS[case]
+    mk, x = _dot(8, 3, nl, nr, cuda, precision)
+    ref = mk(use_fiber=False, panel1=False)(x, precision="f64").cpu().numpy()
+    for budget in (1, 40 * 1024, 200 * 1024):
+        monkeypatch.setattr(engine, "WX_TILE_BYTES", {"f64": budget, "f32": budget})
+        sig = mk(use_fiber=True, fuse_w=False)
+        assert sig.wx is not None
+        y = sig(x).cpu().numpy()
+        if precision == "f64":
+            assert numpy.abs(y - ref).max() <= 1e-12 * numpy.abs(ref).max(), budget
+        else:
+            assert numpy.linalg.norm(y - ref) <= 2e-5 * numpy.linalg.norm(ref), budget
+        assert numpy.array_equal(y, sig(x).cpu().numpy())
