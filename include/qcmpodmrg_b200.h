@@ -229,6 +229,14 @@ int qc_fgemm_f32(const void *items_dev, long long nitems, const void *groups_dev
 /* W panels of the dense fiber-group GEMM: dst[i] = idx[i] >= 0 ? src[idx[i]] : 0 (once per dot). */
 int qc_wpanel_f64(const double *src, const long long *idx_dev, double *dst, long long n, void *stream);
 int qc_wpanel_f32(const float *src, const long long *idx_dev, float *dst, long long n, void *stream);
+/* FP64 panel GEMM on the tensor pipe (mma.sync f64): work is nwork (unit, operator) int
+ * pairs, units qc_dunit records, ops the operator table.  Exactly one of crow (row form)
+ * and cols (column form, qc_dcol) is given.  A and B are 16-byte aligned. */
+int qc_dpanel_f64(const void *units, const void *work, long long nwork, const void *ops, const long long *crow,
+                  const void *cols, const double *A, const double *B, double *C, void *stream);
+/* out[i] = x[idx[i]], 0 where idx[i] < 0. */
+int qc_gather_pad_f64(const double *x, const long long *idx, long long n, double *out, void *stream);
+
 /* Sparse two-site MPO stage: T3 = T1 . (W_i W_{i+1}) for every operator (records qc_wxitem /
  * qc_wxdelta / qc_wxgrp / qc_wxdop / qc_wxquad of qc_types.h).  qc_wx_build makes the sparse
  * rows of one operator class on the host (w1 / w2: FP64 values, operator o at off1[o] /

@@ -1,0 +1,292 @@
+// FP64 panel GEMM on the tensor pipe: the L.psi and .R contractions of HVecQt
+// (source/mpo_dmrg_kernelQt.py:301, 306-316) in FP64.
+//
+// Both operands are K-major with 16-byte aligned rows: the L panels of one contracted
+// sector [M x Kp] against the wavefunction's panel of that sector [sum_j N_j x Kp] (all psi
+// blocks of the sector side by side, so that narrow blocks share a tile), and the T3 panels
+// [M x Kp] against the transposed R panels [D_r' x Kp].
+//
+// The FP64 tensor pipe runs at the DFMA rate (37 TFLOP/s), but one m8n8k4 product does 256
+// multiply-adds from one register per operand, so neither shared memory nor issue slots
+// bound the loop as they do with DFMA.  Tile: 128 rows x up to 64 columns, eight warps of
+// 16 rows; a warp's column count is compiled for every multiple of 8 (small sectors end a
+// tile early).  Operands come through a three-stage cp.async ring of 16-deep K slices; row pitch 20 doubles: the
+// eight rows x four k of a fragment touch every bank once.  A persistent grid, two CTAs per
+// SM, walks the (tile, operator) list; the ring runs on from one tile into the next, so the
+// short panels of L.psi (a few K slices each) do not wait for their first operands.
+//
+// Measured at the mid-chain dot of K=24, D=500 (160 GFLOP each; DFMA kernel before): L.psi
+// 16.8 -> 7.7 ms (20.8 TFLOP/s, 56 % of the pipe), .R 14.5 -> 6.2 ms (25.9, 70 %).  L.psi is
+// held back by its T1 stores and by K extents that end inside a 16-deep slice, .R by the
+// last wave of tiles and the ring's barriers.
+#include <cuda_runtime.h>
+#include <cstdio>
+#include "qc_types.h"
+
+namespace {
+
+constexpr int DP_BM = 128, DP_BN = 64, DP_BK = 16, DP_ST = 3, DP_THREADS = 256;
+constexpr int DP_P = DP_BK + 4;                                  // row pitch in doubles
+constexpr int DP_STAGE = (DP_BM + DP_BN) * DP_P;                 // doubles of one stage
+constexpr int DP_SMEM = DP_ST * DP_STAGE * 8;
+
+__device__ __forceinline__ void dp_cp16(unsigned dst, const double *src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ void dp_mma(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+// One K slice (k4 groups of four k) of a warp's 16 x 8 NT tile.
+template <int NT>
+__device__ __forceinline__ void dp_slice(const double *as, const double *bs, int k4, double (&acc)[2][DP_BN / 8][2]) {
+#pragma unroll
+  for (int kk = 0; kk < DP_BK / 4; ++kk) {
+    if (kk < k4) {
+      const double a0 = as[4 * kk], a1 = as[8 * DP_P + 4 * kk];
+      double b[NT];
+#pragma unroll
+      for (int j = 0; j < NT; ++j) b[j] = bs[8 * j * DP_P + 4 * kk];
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        dp_mma(acc[0][j], a0, b[j]);
+        dp_mma(acc[1][j], a1, b[j]);
+      }
+    }
+  }
+}
+
+struct DpRec {
+  qc_dunit u;
+  qc_op o;
+};
+static_assert(sizeof(DpRec) == 96, "unit and operator records back to back");
+constexpr int DP_RECS = 8;       // a CTA's records in flight: the loads run at most two tiles ahead
+// place of tile column n in the staged B tile: an accumulator pair of lane l holds the columns
+// l % 4 and l % 4 + 4 of its group of eight, so that four lanes store 32 contiguous bytes
+__device__ __forceinline__ int dp_col_place(int n) { return (n & ~7) | ((n & 3) << 1) | ((n >> 2) & 1); }
+
+template <bool COLS>
+__global__ void __launch_bounds__(DP_THREADS, 2)
+k_dpanel(const qc_dunit *__restrict__ units, const int2 *__restrict__ work, int nwork,
+         const qc_op *__restrict__ ops, const long long *__restrict__ crow, const qc_dcol *__restrict__ cols,
+         const double *__restrict__ A, const double *__restrict__ B, double *__restrict__ C) {
+  extern __shared__ __align__(16) double dp_smem[];
+  __shared__ __align__(16) DpRec recs[DP_RECS];
+  __shared__ __align__(16) qc_dcol scols[COLS ? DP_RECS : 1][DP_BN];
+  __shared__ __align__(16) long long srow[COLS ? 1 : DP_RECS][DP_BM];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int G = (int)gridDim.x;
+  const int ntile = (nwork - (int)blockIdx.x + G - 1) / G;
+  // tile j of this CTA: every other pass over the grid runs backwards (the list is sorted)
+  auto item = [&](int j) {
+    const int i = j * G + ((j & 1) ? G - 1 - (int)blockIdx.x : (int)blockIdx.x);
+    return i < nwork ? i : j * G + (int)blockIdx.x;
+  };
+  auto fetch = [&](int j, int2 w) {            // records of tile j into their slot
+    if (tid < 6) {
+      const char *src = tid < 4 ? reinterpret_cast<const char *>(units + w.x) + 16 * tid
+                                : reinterpret_cast<const char *>(ops + w.y) + 16 * (tid - 4);
+      const unsigned d = (unsigned)__cvta_generic_to_shared(&recs[j & (DP_RECS - 1)]) + 16u * tid;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+    }
+  };
+  for (int j = 0; j < min(3, ntile); ++j) fetch(j, work[item(j)]);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  int2 nw = ntile > 3 ? work[item(3)] : make_int2(0, 0);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+
+  const unsigned sbase = (unsigned)__cvta_generic_to_shared(dp_smem);
+  // this thread copies 16 bytes (two k) of rows r0, r0 + 32, ... of both operands
+  const int ck = 2 * (tid & 7), r0 = tid >> 3;
+  int lt = 0, lk = 0, lnk, lK, lm, ln, lda, ldb;     // loads: tile, K slice, the tile's extents
+  const double *Ab, *Bb;
+  auto open_tile = [&]() {
+    const DpRec &r = recs[lt & (DP_RECS - 1)];
+    lK = r.u.K;
+    lnk = max(1, (lK + DP_BK - 1) / DP_BK);
+    lm = r.u.mrem;
+    ln = r.u.nrem;
+    lda = r.u.lda;
+    ldb = r.u.ldb;
+    Ab = A + r.o.a_base + r.u.a_off + (long long)r0 * lda + ck;
+    Bb = B + r.o.b_base + r.u.b_off + (long long)r0 * ldb + ck;
+    lk = 0;
+    // the tile's column (row) records, read by its epilogue
+    if (COLS ? tid < ln : tid < lm) {
+      const void *src = COLS ? (const void *)(cols + r.u.c_off + tid) : (const void *)(crow + r.u.c_off + tid);
+      const void *dst = COLS ? (const void *)&scols[lt & (DP_RECS - 1)][tid] : (const void *)&srow[lt & (DP_RECS - 1)][tid];
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                   : "memory");
+    }
+    if (lt + 3 < ntile) {
+      fetch(lt + 3, nw);
+      if (lt + 4 < ntile) nw = work[item(lt + 4)];
+    }
+  };
+  int ls = 0;                                        // stage of the next load
+  auto load = [&]() {
+    if (lt < ntile) {
+      const int k0 = lk * DP_BK;
+      const int kb = max(0, min(2, lK - k0 - ck)) * 8;
+      const unsigned s = sbase + (unsigned)(ls * DP_STAGE + r0 * DP_P + ck) * 8u;
+      const unsigned sb = sbase + (unsigned)(ls * DP_STAGE + dp_col_place(r0) * DP_P + ck) * 8u;
+#pragma unroll
+      for (int e = 0; e < DP_BM / 32; ++e) {
+        const int v = r0 + 32 * e < lm ? kb : 0;
+        dp_cp16(s + (unsigned)(32 * e * DP_P) * 8u, v ? Ab + (long long)(32 * e) * lda + k0 : A, v);
+      }
+#pragma unroll
+      for (int e = 0; e < DP_BN / 32; ++e) {
+        const int v = r0 + 32 * e < ln ? kb : 0;
+        dp_cp16(sb + (unsigned)((DP_BM + 32 * e) * DP_P) * 8u, v ? Bb + (long long)(32 * e) * ldb + k0 : B, v);
+      }
+      if (++lk == lnk && ++lt < ntile) open_tile();
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    ls = ls + 1 == DP_ST ? 0 : ls + 1;
+  };
+  open_tile();
+  for (int s = 0; s < DP_ST - 1; ++s) {
+    load();
+    if (lt > 0 && lk == 0) {      // a tile of one K slice: the next records have landed before they are read
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+    }
+  }
+
+  double acc[2][DP_BN / 8][2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < DP_BN / 8; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int gr = lane >> 2, gk = lane & 3;         // fragment row (or column) and k of this lane
+  int st = 0;
+  for (int ct = 0; ct < ntile; ++ct) {
+    const DpRec &rec = recs[ct & (DP_RECS - 1)];
+    const int K = rec.u.K, nk = max(1, (K + DP_BK - 1) / DP_BK);
+    const int nt = (rec.u.nrem + 7) >> 3;
+    const bool live = warp * 16 < rec.u.mrem;
+    for (int kt = 0; kt < nk; ++kt) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(DP_ST - 2) : "memory");
+      __syncthreads();
+      load();
+      if (live) {
+        const double *as = dp_smem + st * DP_STAGE + (warp * 16 + gr) * DP_P + gk;
+        const double *bs = dp_smem + st * DP_STAGE + (DP_BM + gr) * DP_P + gk;
+        const int k4 = min(DP_BK / 4, (K - kt * DP_BK + 3) >> 2);
+        switch (nt) {
+          case 1: dp_slice<1>(as, bs, k4, acc); break;
+          case 2: dp_slice<2>(as, bs, k4, acc); break;
+          case 3: dp_slice<3>(as, bs, k4, acc); break;
+          case 4: dp_slice<4>(as, bs, k4, acc); break;
+          case 5: dp_slice<5>(as, bs, k4, acc); break;
+          case 6: dp_slice<6>(as, bs, k4, acc); break;
+          case 7: dp_slice<7>(as, bs, k4, acc); break;
+          default: dp_slice<8>(as, bs, k4, acc); break;
+        }
+      }
+      st = st + 1 == DP_ST ? 0 : st + 1;
+    }
+    // the accumulator of lane l: row l / 4, columns l % 4 and l % 4 + 4 of every eight
+    double *const Cb = C + rec.o.c_base;
+    const double alpha = rec.o.alpha;
+    const int mrem = rec.u.mrem, nrem = rec.u.nrem;
+    if (COLS) {
+      const long long m0 = rec.u.m0 + warp * 16 + gr;
+      const qc_dcol *cl = scols[ct & (DP_RECS - 1)];
+#pragma unroll
+      for (int j = 0; j < DP_BN / 8; ++j)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int n = 8 * j + 4 * h + gk;
+          if (n < nrem) {
+            const qc_dcol c = cl[n];
+            if (c.off >= 0) {
+              double *dst = Cb + c.off + m0 * c.ld;
+              if (warp * 16 + gr < mrem) dst[0] = alpha * acc[0][j][h];
+              if (warp * 16 + gr + 8 < mrem) dst[8LL * c.ld] = alpha * acc[1][j][h];
+            }
+          }
+        }
+    } else {
+      const int n0 = rec.u.n0;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int m = warp * 16 + 8 * i + gr;
+        if (m < mrem) {
+          double *dst = Cb + srow[ct & (DP_RECS - 1)][m] + n0;
+#pragma unroll
+          for (int j = 0; j < DP_BN / 8; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int n = 8 * j + 4 * h + gk;
+              if (n < nrem) dst[n] = alpha * acc[i][j][h];
+            }
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < DP_BN / 8; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+}
+
+// out[i] = x[idx[i]], 0 where idx < 0
+__global__ void k_gather_pad(const double *__restrict__ x, const long long *__restrict__ idx, long long n,
+                             double *__restrict__ out) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const long long j = idx[i];
+    out[i] = j >= 0 ? x[j] : 0.0;
+  }
+}
+
+}  // namespace
+
+template <bool COLS>
+static cudaError_t launch_dpanel(const void *units, const void *work, int nwork, const void *ops,
+                                 const long long *crow, const void *cols, const double *A, const double *B, double *C,
+                                 cudaStream_t s) {
+  cudaError_t e = cudaFuncSetAttribute(k_dpanel<COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, DP_SMEM);
+  int dev = 0, nsm = 0;
+  if (e == cudaSuccess) e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  // short panels (L.psi) share a persistent grid; the long ones of .R, sorted by length, are
+  // left to the hardware's scheduler, one tile per CTA (K = 24, D = 500: 5.7 against 6.8 ms)
+  k_dpanel<COLS><<<COLS && nwork > 2 * nsm ? 2 * nsm : nwork, DP_THREADS, DP_SMEM, s>>>(
+      (const qc_dunit *)units, (const int2 *)work, nwork, (const qc_op *)ops, crow, (const qc_dcol *)cols, A, B, C);
+  return cudaGetLastError();
+}
+
+extern "C" int qc_dpanel_f64(const void *units, const void *work, long long nwork, const void *ops,
+                             const long long *crow, const void *cols, const double *A, const double *B, double *C,
+                             void *stream) {
+  if (nwork <= 0) return QC_OK;
+  if (nwork > 0x3fffffffLL || !units || !work || !ops || (!crow && !cols) || ((unsigned long long)A & 15) ||
+      ((unsigned long long)B & 15))
+    return QC_ERR_ARG;
+  cudaStream_t s = (cudaStream_t)stream;
+  const cudaError_t e = cols ? launch_dpanel<true>(units, work, (int)nwork, ops, crow, cols, A, B, C, s)
+                             : launch_dpanel<false>(units, work, (int)nwork, ops, crow, cols, A, B, C, s);
+  if (e != cudaSuccess) {
+    fprintf(stderr, "[qcgpu] qc_dpanel: %s\n", cudaGetErrorString(e));
+    return QC_ERR_CUDA;
+  }
+  return QC_OK;
+}
+
+extern "C" int qc_gather_pad_f64(const double *x, const long long *idx, long long n, double *out, void *stream) {
+  if (n <= 0) return QC_OK;
+  if (!x || !idx || !out) return QC_ERR_ARG;
+  long long blocks = (n + 255) / 256;
+  if (blocks > 148 * 32) blocks = 148 * 32;
+  k_gather_pad<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(x, idx, n, out);
+  return cudaGetLastError() == cudaSuccess ? QC_OK : QC_ERR_CUDA;
+}

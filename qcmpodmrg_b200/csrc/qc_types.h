@@ -257,3 +257,24 @@ struct alignas(16) qc_wxquad {
   int c0nc;            // first c << 8 | rows (1 .. 4)
 };
 static_assert(sizeof(qc_wxquad) == 16, "qc_wxquad is 16 bytes");
+
+// ---- FP64 panel GEMM on the tensor pipe (k_dpanel) ---------------------------------
+// One unit = one tile of at most 128 rows x 64 columns of one operator class,
+//   C[m, n] = alpha * sum_k A[m, k] * B[n, k],   A at a_base + a_off + m * lda + k,
+//                                                B at b_base + b_off + n * ldb + k,
+// with 16-byte aligned rows (lda, ldb multiples of 4).  Row form: row m of the tile goes to
+// C + c_base + crow[c_off + m] + n0; column form: column n of the tile, tile row m, goes to
+// C + c_base + cols[c_off + n].off + (m0 + m) * cols[c_off + n].ld (off < 0: not stored).
+struct alignas(16) qc_dunit {
+  long long a_off, b_off, c_off;
+  int lda, ldb, K;
+  int mrem, nrem;      // rows and columns of the tile
+  int m0, n0;
+  int pad0, pad1, pad2;
+};
+static_assert(sizeof(qc_dunit) == 64, "qc_dunit is 64 bytes");
+
+struct qc_dcol {
+  int off, ld;
+};
+static_assert(sizeof(qc_dcol) == 8, "qc_dcol is 8 bytes");

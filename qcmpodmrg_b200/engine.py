@@ -1481,13 +1481,14 @@ def _ranges(n):
     return own, numpy.arange(int(n.sum()), dtype=numpy.int64) - numpy.repeat(numpy.cumsum(n) - n, n)
 
 
-def psi_panels(psi):
-    """The wavefunction as the B operand of the tensor-core L.psi GEMMs: per first-index
+def psi_panels(psi, blocks=None):
+    """The wavefunction (its allowed blocks, or the given ones) as the B operand of the
+    tensor-core L.psi GEMMs: per first-index
     sector l' the psi blocks (l', n1, n2, r) of that sector side by side as columns,
     transposed to [sum_j N_j x Kp] (k = l' index contiguous, rows padded to Kp = D_l'
     rounded up to 4).  Returns (gather index into the packed vector, -1 for padding),
     {sector: (offset, N total, K, Kp)} and {block: (sector, first column)}."""
-    blocks = numpy.asarray(psi.idx_allowed, dtype=numpy.int64)
+    blocks = numpy.asarray(psi.idx_allowed if blocks is None else blocks, dtype=numpy.int64)
     if len(blocks) == 0:
         return numpy.zeros(0, dtype=numpy.int64), {}, {}
     sec = psi.block_sectors(blocks)[0].astype(numpy.int64)
@@ -1597,3 +1598,90 @@ def tc_sigma1_units(classes, psi_info, psi_cols, lp_base, lp_opstride, lp_total,
     sg = numpy.concatenate(segs) if segs and sum(len(x) for x in segs) else numpy.zeros(1, TCSEG_DT)
     return u, maps, sg
 
+
+
+# ---------------------------------------------------------------- FP64 panel GEMM on the tensor pipe (qc_dpanel_f64)
+DUNIT_DT = numpy.dtype([("a_off", "<i8"), ("b_off", "<i8"), ("c_off", "<i8"), ("lda", "<i4"), ("ldb", "<i4"),
+                        ("K", "<i4"), ("mrem", "<i4"), ("nrem", "<i4"), ("m0", "<i4"), ("n0", "<i4"),
+                        ("pad", "<i4", (3,))])
+DCOL_DT = numpy.dtype([("off", "<i4"), ("ld", "<i4")])
+assert DUNIT_DT.itemsize == 64 and DCOL_DT.itemsize == 8
+DP_BM, DP_BN = 128, 64
+
+
+def _even_tiles(n, most, unit):
+    """(index, start, extent) of the tiles of every extent n[i]: as few as fit `most` each, of
+    equal width in multiples of `unit` (no sliver at the end of a panel)."""
+    n = numpy.asarray(n, dtype=numpy.int64)
+    k = (n + most - 1) // most
+    w = -(-n // numpy.maximum(unit * k, 1)) * unit
+    k = -(-n // numpy.maximum(w, 1))
+    own, loc = _ranges(k)
+    return own, loc * w[own], numpy.minimum(w[own], n[own] - loc * w[own])
+
+
+def dpanel_units(M, N, K, lda, ldb, a_off, b_off, c_off, row_form):
+    """Tiles of the panels C_j[M_j x N_j] = A_j . B_j^T.  c_off: row-table index of row 0 (row
+    form) or column-table index of column 0.  Column tiles of one row tile are neighbours."""
+    M, N, K, lda, ldb, a_off, b_off, c_off = (numpy.asarray(x, dtype=numpy.int64) for x in
+                                              (M, N, K, lda, ldb, a_off, b_off, c_off))
+    jm, m0, mw = _even_tiles(M, DP_BM, 16)
+    jn, n0, nw = _even_tiles(N, DP_BN, 8)
+    nfirst = numpy.searchsorted(jn, numpy.arange(len(M)))
+    ncnt = numpy.bincount(jn, minlength=len(M)) if len(M) else numpy.zeros(0, dtype=numpy.int64)
+    i, k = _ranges(ncnt[jm])
+    j, t = jm[i], nfirst[jm[i]] + k
+    u = numpy.zeros(len(i), DUNIT_DT)
+    u["a_off"], u["b_off"] = a_off[j] + m0[i] * lda[j], b_off[j] + n0[t] * ldb[j]
+    u["c_off"] = c_off[j] + (m0[i] if row_form else n0[t])
+    u["lda"], u["ldb"], u["K"] = lda[j], ldb[j], K[j]
+    u["mrem"], u["nrem"], u["m0"], u["n0"] = mw[i], nw[t], m0[i], n0[t]
+    return u
+
+
+class DPanelStage(object):
+    """Panel GEMMs C = A . B^T of every operator in FP64 (qc_dpanel_f64).
+
+    parts: [(units, operator range)]; exactly one of crow (row table) and cols (DCOL_DT)."""
+
+    def __init__(self, name, parts, ops, device, flops, crow=None, cols=None, longest_first=False):
+        self.name, self.host_ops, self.flops, self.bytes = name, ops, flops, 0.0
+        units, work = [], []
+        n = 0
+        for u, (b, e) in parts:
+            w = numpy.empty((e - b, len(u), 2), dtype=numpy.int32)
+            w[:, :, 0] = n + numpy.arange(len(u))[None, :]
+            w[:, :, 1] = numpy.arange(b, e)[:, None]
+            units.append(u)
+            work.append(w.reshape(-1, 2))
+            n += len(u)
+        self.h_units = numpy.concatenate(units) if units else numpy.zeros(0, DUNIT_DT)
+        self.h_work = numpy.concatenate(work) if work else numpy.zeros((0, 2), dtype=numpy.int32)
+        if longest_first and len(self.h_work):
+            x = self.h_units[self.h_work[:, 0]]
+            cost = x["K"].astype(numpy.int64) * ((x["nrem"] + 7) // 8 + 2)
+            self.h_work = numpy.ascontiguousarray(self.h_work[numpy.argsort(-cost, kind="stable")])
+        self.h_crow, self.h_cols = crow, cols
+        self.ntasks = len(self.h_work)
+        if not self.ntasks:
+            return
+        self.d_units, self.d_work, self.d_ops = (upload(x, device) for x in (self.h_units, self.h_work, ops))
+        self.d_crow = torch.from_numpy(numpy.ascontiguousarray(crow, dtype=numpy.int64)).to(device) \
+            if crow is not None else None
+        self.d_cols = upload(cols, device) if cols is not None else None
+
+    def run(self, A, B, C, stream=None):
+        if self.ntasks == 0:
+            return
+        s = stream if stream is not None else torch.cuda.current_stream(C.device).cuda_stream
+        if LOG.enabled:
+            e0 = torch.cuda.Event(enable_timing=True)
+            e1 = torch.cuda.Event(enable_timing=True)
+            e0.record()
+        check(native.lib().qc_dpanel_f64(self.d_units.data_ptr(), self.d_work.data_ptr(), self.ntasks,
+                                         self.d_ops.data_ptr(), ptr(self.d_crow), ptr(self.d_cols), A.data_ptr(),
+                                         B.data_ptr(), C.data_ptr(), s), "qc_dpanel_f64")
+        LOG.launches += 1
+        if LOG.enabled:
+            e1.record()
+            LOG.records.append((self.name, e0, e1, self.flops, self.bytes))

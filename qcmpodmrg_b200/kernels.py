@@ -20,7 +20,8 @@ from . import native
 from .native import check
 from .engine import (Stage, compile_classes, add_parts, live_blocks, prune, op_table, TASK_DT, CONTRIB_DT, LOG,
                      compile_fiber, FiberStage, CompositeStage, panel_sigma1, compile_panels, BPERM_DT, PanelStage,
-                     fiber_stages, panel_sigma4, upload, sparse_w_class, SparseWStage)
+                     fiber_stages, panel_sigma4, upload, sparse_w_class, SparseWStage,
+                     DPanelStage, dpanel_units, DCOL_DT, psi_panels)
 from .mpo import case
 from .qtensor import Contraction, Layout, flip_right, flip_horizontal
 
@@ -129,6 +130,14 @@ def gather_split(x, idx, hi, lo):
                                            _stream(hi.device)), "qc_gather_split_f32")
     LOG.launches += 1
     return hi, lo
+
+
+def gather_pad(x, idx, out):
+    """out[i] = x[idx[i]], 0 where idx is negative (qc_gather_pad_f64)."""
+    check(native.lib().qc_gather_pad_f64(x.data_ptr(), idx.data_ptr(), idx.numel(), out.data_ptr(),
+                                         _stream(out.device)), "qc_gather_pad_f64")
+    LOG.launches += 1
+    return out
 
 
 def tf32_split(hi, lo):
@@ -349,7 +358,7 @@ class SigmaOperator(object):
             if pan4 is not None:
                 g4 = pan4["gemm"]
                 g4 = g4[:6] + (g4[6] + crow_n,) + tuple(g4[7:])     # row-table indices into the stage's table
-                if want_tc4:
+                if want_tc4 or sparse_w:
                     tc4_classes.append((rng, pan4, crow_n))
                 crow_all.append(pan4["crow"])
                 crow_n += len(pan4["crow"])
@@ -376,7 +385,7 @@ class SigmaOperator(object):
                 if (si == 2 and fib3 is not None) or (si == 3 and pan4 is not None):
                     continue
                 if si == 0 and pan is not None:
-                    if want_tc1:
+                    if want_tc1 or sparse_w:
                         tc1_classes.append((rng, pan["tc"]))
                     parts = compile_panels(pan["gemm"], rng, tensor_cores=bool(tc))
                     if tc:
@@ -426,7 +435,7 @@ class SigmaOperator(object):
             self._lperm_ops = op_table(L.offsets[order], 0, L.offsets[order], 1.0)
             self._lperm_ops_d = upload(self._lperm_ops, dev)
             self._lperm_span = int(max(len(v[0]) for v in plans.values()))
-            self._build_lpan()
+            self._build_lpan(sparse_w)
         # per-dot R panels (every operator's R blocks permuted), FP64 and FP32
         self.rperm = None
         if rperm:
@@ -435,16 +444,16 @@ class SigmaOperator(object):
             rops = op_table(R.offsets[order], 0, R.offsets[order], 1.0)
             self._rperm_ops_d = upload(rops, dev)
             self._rperm_span = int(max(len(v[0]) for v in plans.values()))
-            self._build_rpan()
-        # the .R contraction on the tensor cores: R panels transposed and split into TF32
-        # hi / lo planes once per dot, T3 read raw by TMA and split in the kernel
-        self.tc1 = None
+            self._build_rpan(sparse_w)
+        # L.psi and .R on K-major panels with padded rows (the L panels of a contracted sector,
+        # the transposed R panels, the wavefunction's panels): split TF32 on the tcgen05 kernel,
+        # and FP64 on the tensor pipe where the sparse product runs between them
+        self.tc1 = self.tc4 = self.d1 = self.d4 = None
+        crow = numpy.concatenate(crow_all) if crow_all else numpy.zeros(1, numpy.int64)
         if tc1_classes:
-            self._setup_tc1(tc1_classes, order, L, tabs[0])
-        self.tc4 = None
+            self._setup_panels1(tc1_classes, order, L, tabs[0], want_tc1, sparse_w)
         if tc4_classes:
-            self._setup_tc4(tc4_classes, order, bases[2], R, st4_ops=tabs[3],
-                            crow=numpy.concatenate(crow_all) if crow_all else numpy.zeros(1, numpy.int64))
+            self._setup_panels4(tc4_classes, order, bases[2], R, tabs[3], crow, want_tc4, sparse_w)
         # fused W stage (T1 -> T3) and the per-dot two-site MPO blocks it reads
         self.fused = None
         self.wtot = wtot
@@ -491,10 +500,9 @@ class SigmaOperator(object):
                 fb += stage_bytes(fused[1], fused[2], len(ops), False)
         if self.fused is not None:
             self.fused.bytes = float(fb)
-        if self.tc4 is not None:
-            self.tc4.bytes = self._stages[3].bytes
-        if self.tc1 is not None:
-            self.tc1.bytes = self._stages[0].bytes
+        for st, ref in ((self.tc1, 0), (self.d1, 0), (self.tc4, 3), (self.d4, 3)):
+            if st is not None:
+                st.bytes = self._stages[ref].bytes
         # FLOPs of the reference's four-contraction chain (tensordotCAL pair GEMMs),
         # whatever the fusion used here
         self.flops = 0.0
@@ -587,15 +595,15 @@ class SigmaOperator(object):
             raise ValueError("rebind: environment layouts differ from the compiled plan")
         self.L, self.R = L, R
         if self.lperm is not None:
-            self._build_lpan()
+            self._build_lpan(self.d1 is not None)
         if self.rperm is not None:
-            self._build_rpan()
-        if self.tc4 is not None:
-            self._build_rpan_tc()
-        if self.tc1 is not None:
-            self._build_lpan_tc()
+            self._build_rpan(self.d4 is not None)
+        if self.tc4 is not None or self.d4 is not None:
+            self._build_rpan_k()
+        if self.tc1 is not None or self.d1 is not None:
+            self._build_lpan_k()
 
-    def _setup_tc4(self, tc4_classes, order, t3bases, R, st4_ops, crow):
+    def _setup_panels4(self, tc4_classes, order, t3bases, R, st4_ops, crow, tc, f64):
         from .engine import TCPanelStage, tc_sigma4_units
         dev = self.ws.device
         classes, t3b, rtb, rts, descs = [], [], [], [], []
@@ -622,8 +630,9 @@ class SigmaOperator(object):
             rt_tot += opstride * len(ops_c)
             flops += 2.0 * float((sec["M"] * sec["N"] * sec["K"]).sum()) * len(ops_c)
         rt_tot = (rt_tot + 31) // 32 * 32
-        units, maps = tc_sigma4_units(classes, None, t3b, rtb, rts, rt_tot)
-        self.tc4 = TCPanelStage("sigma4", units, maps, st4_ops, crow, flops, dev)
+        if tc:
+            units, maps = tc_sigma4_units(classes, None, t3b, rtb, rts, rt_tot)
+            self.tc4 = TCPanelStage("sigma4", units, maps, st4_ops, crow, flops, dev)
         self._rt_total = rt_tot
         self._rt_descs = numpy.concatenate(descs)
         self._rt_descs_d = upload(self._rt_descs, dev)
@@ -632,12 +641,19 @@ class SigmaOperator(object):
             base[poss] = b0 + st * numpy.arange(len(poss))
         self._rt_ops_d = upload(op_table(R.offsets[order], 0, base, 1.0), dev)
         self._rt_span = int(max(len(c[0]) for c in classes))
-        self._build_rpan_tc()
+        if f64:
+            ops = st4_ops.copy()
+            ops["b_base"] = base
+            parts = [(dpanel_units(sec["M"], sec["N"], sec["K"], sec["Kp"], sec["Kp"], sec["t3pan"], sec["rtoff"],
+                                   sec["crow_base"], True), (poss[0], poss[-1] + 1)) for (poss, sec, _) in classes]
+            self.d4 = DPanelStage("sigma4", parts, ops, dev, flops, crow=crow, longest_first=True)
+        self._build_rpan_k()
 
-    def _setup_tc1(self, tc1_classes, order, L, st1_ops):
-        from .engine import TCPanelStage, tc_sigma1_units, psi_panels
+    def _setup_panels1(self, tc1_classes, order, L, st1_ops, tc, f64):
+        from .engine import TCPanelStage, tc_sigma1_units
         dev = self.ws.device
-        gidx, info, cols = psi_panels(self.psi)
+        live = numpy.unique(numpy.concatenate([t["blocks"] for _, t in tc1_classes]))
+        gidx, info, cols = psi_panels(self.psi, live)
         self._psi_total = (len(gidx) + 31) // 32 * 32
         self._psi_gidx = torch.from_numpy(numpy.concatenate(
             [gidx, numpy.full(self._psi_total - len(gidx), -1, dtype=numpy.int64)])).to(dev)
@@ -660,40 +676,93 @@ class SigmaOperator(object):
             descs.append(d)
             tot += stride * len(poss)
         self._lp_total = (tot + 31) // 32 * 32
-        units, maps, segs = tc_sigma1_units(classes, info, cols, lpb, lps, self._lp_total, self._psi_total)
-        self.tc1 = TCPanelStage("sigma1", units, maps, st1_ops, None, self._stages[0].flops, dev, segs=segs)
+        if tc:
+            units, maps, segs = tc_sigma1_units(classes, info, cols, lpb, lps, self._lp_total, self._psi_total)
+            self.tc1 = TCPanelStage("sigma1", units, maps, st1_ops, None, self._stages[0].flops, dev, segs=segs)
+        if f64:
+            ops = st1_ops.copy()
+            ops["a_base"], ops["b_base"] = base, 0
+            parts, tab = self._dpanel1_units(classes, info, cols)
+            self.d1 = DPanelStage("sigma1", parts, ops, dev, self._stages[0].flops, cols=tab)
         self._lp_descs = numpy.concatenate(descs)
         self._lp_descs_d = upload(self._lp_descs, dev)
         self._lp_ops_d = upload(op_table(L.offsets[order], 0, base, 1.0), dev)
         self._lp_span = int(max(len(c[0]) for c in classes))
-        self._build_lpan_tc()
+        self._build_lpan_k()
 
-    def _build_lpan_tc(self):
-        """L panels of the tensor-core L.psi kernel: [M x Kp] per sector, FP32 hi plane then lo plane."""
+    @staticmethod
+    def _dpanel1_units(classes, info, cols):
+        """Units and column table of L.psi in FP64: the psi panel of a contracted sector times
+        the class's L panel of that sector; column c of psi block j of sector l' is column c of
+        the T1 panel at t1pan_j (rows N_j apart)."""
+        secs = sorted(info)
+        col0 = dict(zip(secs, (numpy.cumsum([info[s][1] for s in secs]) - [info[s][1] for s in secs]).tolist()))
+        ncol = int(sum(info[s][1] for s in secs))
+        parts, tabs = [], []
+        for poss, tc in classes:
+            base = ncol * len(tabs)
+            tab = numpy.zeros(max(ncol, 1), DCOL_DT)
+            tab["off"] = -1
+            nj, pan = numpy.asarray(tc["Nj"], dtype=numpy.int64), numpy.asarray(tc["t1pan"], dtype=numpy.int64)
+            at = numpy.array([col0[cols[b][0]] + cols[b][1] for b in tc["blocks"].tolist()], dtype=numpy.int64)
+            own = numpy.repeat(numpy.arange(len(nj)), nj)
+            loc = numpy.arange(int(nj.sum())) - numpy.repeat(numpy.cumsum(nj) - nj, nj)
+            if len(pan) and int(pan.max()) + int(nj.max()) >= 2 ** 31:
+                raise ValueError("T1 panel offsets exceed the column record")
+            tab["off"][at[own] + loc] = pan[own] + loc
+            tab["ld"][at[own] + loc] = nj[own]
+            tabs.append(tab)
+            sec = [int(s) for s in tc["sectors"]]
+            N = [info[s][1] for s in sec]
+            u = dpanel_units(tc["M"], N, tc["K"], tc["Kp"], [info[s][3] for s in sec], tc["lpoff"],
+                             [info[s][0] for s in sec], [base + col0[s] for s in sec], False)
+            parts.append((u, (poss[0], poss[-1] + 1)))
+        return parts, numpy.concatenate(tabs)
+
+    def _build_lpan_k(self):
+        """K-major L panels [M x Kp] per sector: FP32 hi plane then lo plane for the tcgen05 kernel,
+        FP64 for the FP64 one."""
         n = self._lp_total
+        if self.d1 is not None:
+            self.lpan64 = torch.empty(max(n, 1), dtype=torch.float64, device=self.ws.device)
+            block_permute(self._lp_descs_d, len(self._lp_descs), self._lp_span, self._lp_ops_d, self.L.values,
+                          self.lpan64)
+        if self.tc1 is None:
+            return
         self.lpan_tc = torch.zeros(2 * max(n, 1), dtype=torch.float32, device=self.ws.device)
         block_permute(self._lp_descs_d, len(self._lp_descs), self._lp_span, self._lp_ops_d, self.L.values,
                       self.lpan_tc)
         tf32_split(self.lpan_tc[:n], self.lpan_tc[n:2 * n])
 
-    def _build_rpan_tc(self):
-        """R panels of the tensor-core .R kernel: [D_r' x K_r'] per sector, FP32 hi plane then lo plane."""
+    def _build_rpan_k(self):
+        """K-major R panels [D_r' x Kp] per sector: FP32 hi plane then lo plane for the tcgen05
+        kernel, FP64 for the FP64 one."""
         n = self._rt_total
+        if self.d4 is not None:
+            self.rpan64 = torch.empty(max(n, 1), dtype=torch.float64, device=self.ws.device)
+            block_permute(self._rt_descs_d, len(self._rt_descs), self._rt_span, self._rt_ops_d, self.R.values,
+                          self.rpan64)
+        if self.tc4 is None:
+            return
         self.rpan_tc = torch.zeros(2 * max(n, 1), dtype=torch.float32, device=self.ws.device)
         block_permute(self._rt_descs_d, len(self._rt_descs), self._rt_span, self._rt_ops_d, self.R.values,
                       self.rpan_tc)
         tf32_split(self.rpan_tc[:n], self.rpan_tc[n:2 * n])
 
-    def _build_rpan(self):
-        self.Rpan = torch.empty(max(self.R.total, 1), dtype=torch.float64, device=self.ws.device)
-        block_permute(self.rperm, len(self._rperm_h), self._rperm_span, self._rperm_ops_d, self.R.values,
-                      self.Rpan)
-        self._Rpan32 = None
+    def _build_rpan(self, later=False):
+        """Panels of the separate .R stage; later: made when that stage asks for them."""
+        self.Rpan = self._Rpan32 = None
+        if not later:
+            self.Rpan = torch.empty(max(self.R.total, 1), dtype=torch.float64, device=self.ws.device)
+            block_permute(self.rperm, len(self._rperm_h), self._rperm_span, self._rperm_ops_d, self.R.values,
+                          self.Rpan)
 
     def b4(self, kind):
         """Second operand of the .R contraction (R panels, or R itself without panels)."""
         if self.rperm is not None:
             if kind == "f64":
+                if self.Rpan is None:
+                    self._build_rpan()
                 return self.Rpan
             if self._Rpan32 is None:
                 self._Rpan32 = torch.empty(max(self.R.total, 1), dtype=torch.float32, device=self.ws.device)
@@ -702,11 +771,13 @@ class SigmaOperator(object):
             return self._Rpan32
         return self.R.values if kind == "f64" else self.R.f32()
 
-    def _build_lpan(self):
-        self.Lpan = torch.empty(max(self.L.total, 1), dtype=torch.float64, device=self.ws.device)
-        block_permute(self.lperm, len(self._lperm_h), self._lperm_span, self._lperm_ops_d, self.L.values,
-                      self.Lpan)
-        self._Lpan32 = None
+    def _build_lpan(self, later=False):
+        """Panels of the separate L.psi stage; later: made when that stage asks for them."""
+        self.Lpan = self._Lpan32 = None
+        if not later:
+            self.Lpan = torch.empty(max(self.L.total, 1), dtype=torch.float64, device=self.ws.device)
+            block_permute(self.lperm, len(self._lperm_h), self._lperm_span, self._lperm_ops_d, self.L.values,
+                          self.Lpan)
 
     def lpan32(self):
         if self._Lpan32 is None:
@@ -718,6 +789,8 @@ class SigmaOperator(object):
     def a1(self, kind):
         """First operand of the L.psi contraction (L panels, or L itself without panels)."""
         if self.lperm is not None:
+            if kind == "f64" and self.Lpan is None:
+                self._build_lpan()
             return self.Lpan if kind == "f64" else self.lpan32()
         return self.L.values if kind == "f64" else self.L.f32()
 
@@ -726,8 +799,8 @@ class SigmaOperator(object):
         self.L = self.R = None
         self.Lpan = self._Lpan32 = None
         self.Rpan = self._Rpan32 = None
-        self.rpan_tc = None
-        self.lpan_tc = None
+        self.rpan_tc = self.rpan64 = None
+        self.lpan_tc = self.lpan64 = None
 
     def wij32(self):
         if self._Wij32 is None:
@@ -795,10 +868,16 @@ class SigmaOperator(object):
             T3 = ws.get("t3", self.tot[2], torch.float64)
             P = ws.get("part", self.nops * self.ndim0, torch.float64)
             s = self._stages
-            s[0].run(self.a1("f64"), x, T1, "f64")
             if self.wx is not None:
+                pt = ws.get("psiT64", self._psi_total, torch.float64)
+                gather_pad(x, self._psi_gidx, pt)
+                self.d1.run(self.lpan64, pt, T1)
                 self.wx.run(T1, None, T3, "f64")
+                P[:self.nops * self.ndim0].zero_()
+                self.d4.run(T3, self.rpan64, P)
+                return reduce_ops(P, self.nops, self.ndim0, y)
             else:
+                s[0].run(self.a1("f64"), x, T1, "f64")
                 T2 = ws.get("t2", self.tot[1], torch.float64)
                 s[1].run(T1, self.Wi.values, T2, "f64")
                 s[2].run(T2, self.Wj.values, T3, "f64")

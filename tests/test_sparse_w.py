@@ -51,6 +51,44 @@ def interpret(st, A, C, kind="f64"):
     return hits
 
 
+def interpret_panel(st, A, B, C):
+    """C written by the units of a DPanelStage, each element once."""
+    a, b, c = A.numpy(), B.numpy(), C.numpy()
+    hits = numpy.zeros(len(c), dtype=numpy.int64)
+    for w in st.h_work:
+        u, o = st.h_units[w[0]], st.host_ops[w[1]]
+        assert 0 < u["mrem"] <= 128 and 0 < u["nrem"] <= 64
+        assert (u["a_off"] + o["a_base"]) % 4 == 0 and (u["b_off"] + o["b_base"]) % 4 == 0 and u["lda"] % 4 == 0
+        m, n, k = (numpy.arange(u[x]) for x in ("mrem", "nrem", "K"))
+        am = a[o["a_base"] + u["a_off"] + m[:, None] * u["lda"] + k]
+        bm = b[o["b_base"] + u["b_off"] + n[:, None] * u["ldb"] + k]
+        if st.h_cols is None:
+            at = st.h_crow[u["c_off"] + m][:, None] + u["n0"] + n
+            ok = numpy.ones(len(n), dtype=bool)
+        else:
+            col = st.h_cols[u["c_off"] + n]
+            ok = col["off"] >= 0
+            at = col["off"].astype(numpy.int64) + (u["m0"] + m[:, None]) * col["ld"].astype(numpy.int64)
+        at = (o["c_base"] + at)[:, ok]
+        numpy.add.at(hits, at.ravel(), 1)
+        c[at] = (o["alpha"] * (am @ bm.T))[:, ok]
+    return hits
+
+
+def patch(monkeypatch):
+    from qcmpodmrg_b200 import kernels
+    patch_stage_run(monkeypatch)
+    monkeypatch.setattr(engine.SparseWStage, "run",
+                        lambda self, A, B, C, kind="f64", stream=None: interpret(self, A, C, kind))
+    monkeypatch.setattr(engine.DPanelStage, "run", lambda self, A, B, C, stream=None: interpret_panel(self, A, B, C))
+
+    def gather_pad(x, idx, out):
+        out[:len(idx)] = torch.where(idx >= 0, x[idx.clamp(min=0)], torch.zeros((), dtype=x.dtype))
+        return out
+
+    monkeypatch.setattr(kernels, "gather_pad", gather_pad)
+
+
 def sparse_sigma(r, device, sparse_w=True, precision="f64"):
     from qcmpodmrg_b200.kernels import SigmaOperator, Workspace
     opers = [int(x) for x in numpy.atleast_1d(r["opers"])]
@@ -65,9 +103,7 @@ def sparse_sigma(r, device, sparse_w=True, precision="f64"):
 def test_sparse_records_reproduce_the_separate_stages(tag, monkeypatch):
     """T3 of the sparse records equals T3 of the two separate stages, every element of the
     T3 panels that stage writes is written exactly once, and sigma is the reference's."""
-    patch_stage_run(monkeypatch)
-    monkeypatch.setattr(engine.SparseWStage, "run",
-                        lambda self, A, B, C, kind="f64", stream=None: interpret(self, A, C, kind))
+    patch(monkeypatch)
     used = 0
     for r in load("kernels_%s.npz" % tag)["records"]:
         sig = sparse_sigma(r, "cpu")
@@ -79,7 +115,13 @@ def test_sparse_records_reproduce_the_separate_stages(tag, monkeypatch):
         used += 1
         T1 = torch.zeros(sig.tot[0] + 64, dtype=torch.float64)
         T2 = torch.zeros(sig.tot[1] + 64, dtype=torch.float64)
-        sig._stages[0].run(sig.a1("f64"), x, T1, "f64")
+        psi = torch.zeros(sig._psi_total, dtype=torch.float64)
+        from qcmpodmrg_b200 import kernels
+        kernels.gather_pad(x, sig._psi_gidx, psi)
+        hits = interpret_panel(sig.d1, sig.lpan64, psi, T1)
+        T0 = torch.zeros_like(T1)
+        sig._stages[0].run(sig.a1("f64"), x, T0, "f64")
+        assert hits.max() == 1 and numpy.abs((T1 - T0).numpy()).max() <= 1e-13 * max(1.0, T0.abs().max().item())
         ta, tb = torch.zeros(sig.tot[2] + 64, dtype=torch.float64), torch.zeros(sig.tot[2] + 64, dtype=torch.float64)
         sig.stages[1].run(T1, sig.Wi.values, T2, "f64")         # the stages compiled on demand
         sig.stages[2].run(T2, sig.Wj.values, tb, "f64")
@@ -89,6 +131,34 @@ def test_sparse_records_reproduce_the_separate_stages(tag, monkeypatch):
             assert hits.max() <= 1
             assert numpy.abs(ta.numpy() - tb.numpy()).max() <= 1e-13 * max(1.0, tb.abs().max().item())
             assert (hits[tb.numpy() != 0] == 1).all()
+        part = torch.zeros(sig.nops * sig.ndim0, dtype=torch.float64)
+        ref4 = torch.zeros_like(part)
+        assert interpret_panel(sig.d4, tb, sig.rpan64, part).max() == 1
+        sig._stages[3].run(tb, sig.b4("f64"), ref4, "f64")
+        assert numpy.abs((part - ref4).numpy()).max() <= 1e-13 * max(1.0, ref4.abs().max().item())
+
+
+@pytest.mark.parametrize("tag", ["SP_K4", "SP_K5"])
+def test_sparse_plan_of_the_spin_projected_operators(tag, monkeypatch):
+    """N-only quantum numbers, blocks outside the (N, Sz) wavefunction left out: H and S
+    products equal those of the separate stages."""
+    from helpers import record_sp_operators
+    from qcmpodmrg_b200 import kernels
+    patch(monkeypatch)
+    used = 0
+    for r in load("kernels_%s.npz" % tag)["records"]:
+        ref = record_sp_operators(r, "cpu")
+        make = kernels.SigmaOperator.__init__
+        with monkeypatch.context() as m:
+            m.setattr(kernels.SigmaOperator, "__init__",
+                      lambda self, *a, **k: make(self, *a, **dict(k, sparse_w=True)))
+            new = record_sp_operators(r, "cpu")
+        for a, b in zip(ref[:2], new[:2]):
+            used += b.inner.wx is not None
+            x = torch.from_numpy(numpy.random.default_rng(1).standard_normal(a.ndim0))
+            ya, yb = a(x).numpy(), b(x).numpy()
+            assert numpy.abs(ya - yb).max() <= 1e-12 * max(1.0, numpy.abs(ya).max())
+    assert used
     assert used
 
 
