@@ -1119,119 +1119,185 @@ def _unit_axes(lay, axes):
     return all(len(x) == 4 and bool((x == 1).all()) for x in d)
 
 
-def sparse_w_class(c1, t1, t1off, t3lay, pan4, W1, W2, psi):
-    """Fiber groups of one operator class for the sparse two-site MPO stage.
+def sparse_groups(ins, outs, dx, dz, qx, qz, da, db):
+    """Fiber groups of a sparse MPO stage for one operator class.
 
-    T1 blocks (a, l, n1, n2, r) and T3 blocks (l, r, n1', c, n2') are grouped by their (l, r)
-    sectors, the groups by the charge difference q(l) - q(r): the MPO sectors a(n1, n2) and
-    c(n1', n2') are the same for all groups of one difference.  Returns None where that does
-    not hold or an offset does not fit the records (the caller then keeps the two separate
-    stages), else {"groups", "deltas", "rows", "iblk", "kblk", "row0", "R", "fibers"}."""
-    if not (_unit_axes(c1.out, (2, 3)) and _unit_axes(t3lay, (2, 4)) and _unit_axes(W1, (2, 3))
-            and _unit_axes(W2, (2, 3))):
-        return None
-    if 4 * max(int(numpy.max(W1.ndims[0])), int(numpy.max(W1.ndims[1])), int(numpy.max(W2.ndims[1]))) > FIBER_MAX_ROWS:
-        return None                          # the separate stages would leave the panel form
+    A group is a pair (x sector, z sector) of bond states, its fibers the states (x, z); the
+    groups are collected by the charge difference q(x) - q(z).  ins / outs: arrays (x, z,
+    slot, MPO sector, offset, row stride, end) of the input blocks [bond][fiber] (fibers of
+    one x contiguous, the row stride is not used) and the output blocks (x, c) -> offset +
+    x * stride + c * D_z + z.  dx, dz, qx, qz: extents and quantum numbers of the sectors of
+    the two bonds, da / db: extents of the MPO sectors.  The MPO sector of a slot is the same
+    for all groups of one difference; returns None where that does not hold or an offset does
+    not fit the records, else {"groups", "deltas", "rows", "iblk", "kblk", "row0", "R",
+    "fibers"}."""
     i64 = numpy.int64
-    nr = int(psi.nsyms[3])
-    b1 = numpy.unique(numpy.asarray(t1, dtype=i64)[:, 0])
-    a, l, n1, n2, r = c1.out.block_sectors(b1)
-    b3 = numpy.unique(numpy.asarray(pan4["needed"], dtype=i64))
-    l3, r3, m1, cc, m2 = t3lay.block_sectors(b3)
-    if len(b3) == 0:
+    x1, z1, s1, a1, o1, _, e1 = ins
+    x3, z3, s3, c3, o3, h3, e3 = outs
+    if len(x3) == 0:
         return None
-    lr = numpy.unique(l3 * nr + r3)
-    keep = numpy.isin(l * nr + r, lr)
-    b1, a, l, n1, n2, r = (x[keep] for x in (b1, a, l, n1, n2, r))
-    gl, gr = lr // nr, lr % nr
+    nz = len(dz)
+    xz = numpy.unique(x3 * nz + z3)
+    keep = numpy.isin(x1 * nz + z1, xz)
+    x1, z1, s1, a1, o1, e1 = (v[keep] for v in (x1, z1, s1, a1, o1, e1))
+    gx, gz = xz // nz, xz % nz
     q2 = lambda q: numpy.rint(2 * numpy.asarray(q)).astype(i64)            # noqa: E731
-    dq = q2(psi.qsyms[0])[gl] - q2(psi.qsyms[3])[gr]
+    dq = q2(qx)[gx] - q2(qz)[gz]
     uq, dinv = numpy.unique(dq, axis=0, return_inverse=True)
     dinv = dinv.ravel()
     nd = len(uq)
     o = numpy.argsort(dinv, kind="stable")                                 # groups delta by delta
-    lr, gl, gr, dinv = lr[o], gl[o], gr[o], dinv[o]
-    pos = numpy.empty(int(psi.nsyms[0]) * nr, dtype=i64)
-    pos[lr] = numpy.arange(len(lr))
-    dl, dr = numpy.asarray(psi.ndims[0], dtype=i64), numpy.asarray(psi.ndims[3], dtype=i64)
-    F = dl[gl] * dr[gr]
-    g = numpy.zeros(len(lr), WXGRP_DT)
-    g["F"], g["flo"] = F, dr[gr]
+    xz, gx, gz, dinv = xz[o], gx[o], gz[o], dinv[o]
+    pos = numpy.empty(len(dx) * nz, dtype=i64)
+    pos[xz] = numpy.arange(len(xz))
+    dx, dz, da, db = (numpy.asarray(v, dtype=i64) for v in (dx, dz, da, db))
+    F = dx[gx] * dz[gz]
+    if int(F.sum()) >= 2 ** 31 or max(int(e1.max()) if len(e1) else 0, int(e3.max()), int(h3.max())) >= 2 ** 31:
+        return None
+    g = numpy.zeros(len(xz), WXGRP_DT)
+    g["F"], g["flo"] = F, dz[gz]
     g["a"], g["c"] = -1, -1
     cs = numpy.cumsum(F) - F
     first = numpy.searchsorted(dinv, numpy.arange(nd))
-    if int(F.sum()) >= 2 ** 31:
-        return None
     g["start"] = cs - cs[first][dinv]
-    off1 = (c1.out.ioff if t1off is None else t1off)[b1]
-    off3, fhs3, flo3 = pan4["t3off"][b3], pan4["t3fhs"][b3], pan4["t3flo"][b3]
-    ends1 = off1 + c1.out.ndim[b1]
-    dc = numpy.asarray(W2.ndims[1], dtype=i64)
-    d3 = t3lay.block_dims(b3)
-    ends3 = off3 + numpy.maximum(d3[:, 0] - 1, 0) * fhs3 + d3[:, 1] * d3[:, 3]
-    if max(int(ends1.max()) if len(ends1) else 0, int(ends3.max())) >= 2 ** 31 or int(fhs3.max()) >= 2 ** 31:
-        return None
-    p1, p3 = pos[l * nr + r], pos[l3 * nr + r3]
-    if not numpy.array_equal(flo3, dr[r3]):
-        return None
-    s1, s3 = 4 * n1 + n2, 4 * m1 + m2
+    p1, p3 = pos[x1 * nz + z1], pos[x3 * nz + z3]
     iblk = numpy.full((nd, 16), -1, dtype=numpy.int32)
     kblk = numpy.full((nd, 16), -1, dtype=numpy.int32)
-    iblk[dinv[p1], s1] = a
-    kblk[dinv[p3], s3] = cc
-    # one MPO sector per (n1, n2), one block per (group, n1, n2)
-    if not (numpy.array_equal(iblk[dinv[p1], s1], a) and numpy.array_equal(kblk[dinv[p3], s3], cc)):
+    iblk[dinv[p1], s1] = a1
+    kblk[dinv[p3], s3] = c3
+    # one MPO sector per slot, one block per (group, slot)
+    if not (numpy.array_equal(iblk[dinv[p1], s1], a1) and numpy.array_equal(kblk[dinv[p3], s3], c3)):
         return None
     if len(numpy.unique(p1 * 16 + s1)) != len(p1) or len(numpy.unique(p3 * 16 + s3)) != len(p3):
         return None
-    g["a"][p1, s1] = off1
-    g["c"][p3, s3] = off3
-    g["h"][p3, s3] = fhs3
-    da = numpy.asarray(W1.ndims[0], dtype=i64)
+    g["a"][p1, s1] = o1
+    g["c"][p3, s3] = o3
+    g["h"][p3, s3] = h3
     rows_b = numpy.where(iblk >= 0, da[numpy.maximum(iblk, 0)], 0)          # [delta, 16]
     R = rows_b.sum(axis=1)
     row0 = numpy.where(iblk >= 0, numpy.cumsum(rows_b, axis=1) - rows_b, 0).astype(numpy.int32)
-    dcb = numpy.where(kblk >= 0, dc[numpy.maximum(kblk, 0)], 0)
+    dcb = numpy.where(kblk >= 0, db[numpy.maximum(kblk, 0)], 0)
     if int(R.max()) > WX_MAXR or int(((dcb + 3) // 4).sum(axis=1).max()) > WX_MAXQ:
         return None
     d = numpy.zeros(nd, WXDELTA_DT)
     d["R"] = R
     d["row_b"] = numpy.cumsum(R) - R
     d["grp_b"] = first
-    d["grp_e"] = numpy.r_[first[1:], len(lr)]
+    d["grp_e"] = numpy.r_[first[1:], len(xz)]
     own, loc = _ranges(rows_b.ravel())
     rows = ((own % 16) << 16 | loc).astype(numpy.int32)
     return {"groups": g, "deltas": d, "rows": rows, "iblk": iblk, "kblk": kblk, "row0": row0,
-            "R": R.astype(numpy.int32), "fibers": numpy.add.reduceat(F, first), "W": (W1, W2)}
+            "R": R.astype(numpy.int32), "fibers": numpy.add.reduceat(F, first)}
+
+
+def sparse_w_class(c1, t1, t1off, t3lay, pan4, W1, W2, psi):
+    """Fiber groups of one operator class for the sparse two-site MPO stage: T1 blocks (a, l,
+    n1, n2, r) in, T3 blocks (l, r, n1', c, n2') out (sparse_groups; None where the class has
+    no such form: the caller then keeps the two separate stages)."""
+    if not (_unit_axes(c1.out, (2, 3)) and _unit_axes(t3lay, (2, 4)) and _unit_axes(W1, (2, 3))
+            and _unit_axes(W2, (2, 3))):
+        return None
+    if 4 * max(int(numpy.max(W1.ndims[0])), int(numpy.max(W1.ndims[1])), int(numpy.max(W2.ndims[1]))) > FIBER_MAX_ROWS:
+        return None                          # the separate stages would leave the panel form
+    i64 = numpy.int64
+    b1 = numpy.unique(numpy.asarray(t1, dtype=i64)[:, 0])
+    a, l, n1, n2, r = c1.out.block_sectors(b1)
+    b3 = numpy.unique(numpy.asarray(pan4["needed"], dtype=i64))
+    l3, r3, m1, cc, m2 = t3lay.block_sectors(b3)
+    if len(b3) == 0 or not numpy.array_equal(pan4["t3flo"][b3], numpy.asarray(psi.ndims[3])[r3]):
+        return None
+    off1 = (c1.out.ioff if t1off is None else t1off)[b1]
+    off3, fhs3 = pan4["t3off"][b3], pan4["t3fhs"][b3]
+    d3 = t3lay.block_dims(b3)
+    out = sparse_groups((l, r, 4 * n1 + n2, a, off1, None, off1 + c1.out.ndim[b1]),
+                        (l3, r3, 4 * m1 + m2, cc, off3, fhs3,
+                         off3 + numpy.maximum(d3[:, 0] - 1, 0) * fhs3 + d3[:, 1] * d3[:, 3]),
+                        psi.ndims[0], psi.ndims[3], psi.qsyms[0], psi.qsyms[3], W1.ndims[0], W2.ndims[1])
+    if out is not None:
+        out["W"] = (W1, W2)
+    return out
+
+
+class WSource(object):
+    """One factor of a sparse MPO stage as its builder reads it: host values, operator offsets
+    and block structure (axes: left bond, right bond, bra and ket physical index)."""
+
+    def __init__(self, values, offsets, nsyms, ndims, ioff, allowed):
+        c = numpy.ascontiguousarray
+        self.values, self.offsets = c(values, dtype=numpy.float64), c(offsets, dtype=numpy.int64)
+        self.nsyms, self.nd = c(nsyms, dtype=numpy.int32), c(ndims, dtype=numpy.int64)
+        self.ioff, self.allowed = c(ioff, dtype=numpy.int64), c(allowed, dtype=numpy.int32)
+
+    @staticmethod
+    def of(lay, values, offsets):
+        return WSource(values, offsets, lay.nsyms, lay.ndims_cat, lay.ioff, lay.allowed)
+
+    @staticmethod
+    def transposed(lay, values, offsets):
+        """The bonds exchanged: every block transposed in place (values: the operators' packed
+        values back to back, one row of ``lay.size`` per operator)."""
+        ns = [int(x) for x in lay.nsyms]
+        perm = _W_PERM.get(id(lay))
+        if perm is None or perm[0] is not lay:
+            d = lay.block_dims(lay.idx_allowed)
+            b, e = _ranges(d[:, 0] * d[:, 1])
+            src = lay.ioff[lay.idx_allowed][b]
+            if len(_W_PERM) > 512:
+                _W_PERM.clear()
+            # element e of the transposed block is (e / D_a, e % D_a) = (b, a)
+            perm = _W_PERM[id(lay)] = (lay, src + (e % d[b, 0]) * d[b, 1] + e // d[b, 0])
+        n = len(offsets)
+        vals = numpy.empty((n, lay.size))
+        for k, o in enumerate(offsets):
+            vals[k] = values[o:o + lay.size][perm[1]]
+        nd = numpy.concatenate([lay.ndims[1], lay.ndims[0], lay.ndims[2], lay.ndims[3]])
+        tr = lambda v: numpy.asarray(v).reshape(ns).transpose(1, 0, 2, 3).ravel()          # noqa: E731
+        return WSource(vals.ravel(), numpy.arange(n) * lay.size, [ns[1], ns[0], ns[2], ns[3]], nd, tr(lay.ioff),
+                       tr(lay.allowed))
+
+    @staticmethod
+    def identity(ndims, nops):
+        """The unit matrix of a bond (second factor of a one-site stage)."""
+        n = numpy.asarray(ndims, dtype=numpy.int64)
+        ns = len(n)
+        allowed = numpy.zeros((ns, ns, 4, 4), dtype=numpy.int32)
+        ioff = numpy.zeros((ns, ns, 4, 4), dtype=numpy.int64)
+        k = numpy.arange(ns)
+        allowed[k, k, 0, 0] = 1
+        ioff[k, k, 0, 0] = numpy.cumsum(n * n) - n * n
+        vals = numpy.concatenate([numpy.eye(int(x)).ravel() for x in n]) if ns else numpy.zeros(0)
+        one = numpy.ones(4, dtype=numpy.int64)
+        return WSource(vals, numpy.zeros(nops), [ns, ns, 4, 4], numpy.concatenate([n, n, one, one]), ioff.ravel(),
+                       allowed.ravel())
+
+
+_W_PERM = {}
 
 
 class SparseWStage(object):
     """T3 = T1 . (W_i W_{i+1}) for every operator in one sparse product (qc_wsparse_*).
 
-    parts: [(sparse_w_class result, operator range)] over the stage's operator table ops
-    (a_base: T1, c_base: T3); Wi / Wj: the sites' TensorSets, order: their operator of every
-    table row.  The MPO's values are compiled into the stage: it is a plan for these values."""
+    parts: [(sparse_groups result, operator range, two WSource factors)] over the stage's
+    operator table ops (a_base: T1, c_base: T3).  The MPO's values are compiled into the
+    stage: it is a plan for these values."""
 
-    def __init__(self, parts, device, name, ops, Wi, Wj, order, kinds=("f64",)):
+    def __init__(self, parts, device, name, ops, kinds=("f64",)):
         """kinds: precisions whose work items and coefficients are made now ("f64", "f32")."""
         self.name, self.device = name, device
         self.host_ops = ops
         self.flops = self.bytes = 0.0
         grps, dels, rows, dops, quads, ws, rs, self.op_ranges = [], [], [], [], [], [], [], []
         ngrp = nrow = ndop = nq = ne = 0
-        w1, w2 = Wi.host(), Wj.host()
         lib = native.lib()
         i64 = numpy.int64
-        for part, (b, e) in parts:
-            W1, W2 = part["W"]
+        for part, (b, e), factors in parts:
             d = part["deltas"].copy()
             nops, nd = e - b, len(d)
-            o1 = numpy.ascontiguousarray(Wi.offsets[order[b:e]], dtype=i64)
-            o2 = numpy.ascontiguousarray(Wj.offsets[order[b:e]], dtype=i64)
             h, cq, ce = numpy.zeros(1, dtype=i64), numpy.zeros(1, dtype=i64), numpy.zeros(1, dtype=i64)
             args = []
-            for lay, w, o in ((W1, w1, o1), (W2, w2, o2)):
-                args += [ptr(w), ptr(o), ptr(lay.nsyms), ptr(lay.ndims_cat), ptr(lay.ioff), ptr(lay.allowed)]
+            for w in factors:
+                assert len(w.offsets) == nops
+                args += [ptr(w.values), ptr(w.offsets), ptr(w.nsyms), ptr(w.nd), ptr(w.ioff), ptr(w.allowed)]
             check(lib.qc_wx_build(nops, *args, nd, ptr(part["iblk"]), ptr(part["kblk"]), ptr(part["row0"]),
                                   ptr(part["R"]), ptr(h), ptr(cq), ptr(ce)), "qc_wx_build")
             dp = numpy.zeros(nd * nops, WXDOP_DT)
@@ -1255,7 +1321,7 @@ class SparseWStage(object):
         self.h_groups, self.h_deltas = numpy.concatenate(grps), numpy.concatenate(dels)
         self.h_rows, self.h_dops, self.h_quads = (numpy.concatenate(x) for x in (rows, dops, quads))
         self.h_ent_w, self.h_ent_r = numpy.concatenate(ws), numpy.concatenate(rs)
-        self.fibers = numpy.concatenate([p["fibers"] for p, _ in parts])
+        self.fibers = numpy.concatenate([p["fibers"] for p, _, _ in parts])
         self.ntasks = len(self.h_groups)
         up = lambda a, dt: upload(a if len(a) else numpy.zeros(1, dt), device)         # noqa: E731
         self.d = {"groups": up(self.h_groups, WXGRP_DT), "deltas": up(self.h_deltas, WXDELTA_DT),
@@ -1620,9 +1686,11 @@ def _even_tiles(n, most, unit):
     return own, loc * w[own], numpy.minimum(w[own], n[own] - loc * w[own])
 
 
-def dpanel_units(M, N, K, lda, ldb, a_off, b_off, c_off, row_form):
-    """Tiles of the panels C_j[M_j x N_j] = A_j . B_j^T.  c_off: row-table index of row 0 (row
-    form) or column-table index of column 0.  Column tiles of one row tile are neighbours."""
+def dpanel_units(M, N, K, lda, ldb, a_off, b_off, c_off, form, blk=None):
+    """Tiles of the panels C_j[M_j x N_j] = A_j . B_j^T.  form "row": c_off is the row-table
+    index of row 0; "col": the column-table index of column 0; "blk": the offset of the block
+    [row / blk[0]][column][row % blk[0]] of blk[1] columns, A given as [K x M].  Column tiles of
+    one row tile are neighbours."""
     M, N, K, lda, ldb, a_off, b_off, c_off = (numpy.asarray(x, dtype=numpy.int64) for x in
                                               (M, N, K, lda, ldb, a_off, b_off, c_off))
     jm, m0, mw = _even_tiles(M, DP_BM, 16)
@@ -1632,8 +1700,11 @@ def dpanel_units(M, N, K, lda, ldb, a_off, b_off, c_off, row_form):
     i, k = _ranges(ncnt[jm])
     j, t = jm[i], nfirst[jm[i]] + k
     u = numpy.zeros(len(i), DUNIT_DT)
-    u["a_off"], u["b_off"] = a_off[j] + m0[i] * lda[j], b_off[j] + n0[t] * ldb[j]
-    u["c_off"] = c_off[j] + (m0[i] if row_form else n0[t])
+    u["a_off"] = a_off[j] + m0[i] * (1 if form == "blk" else lda[j])
+    u["b_off"] = b_off[j] + n0[t] * ldb[j]
+    u["c_off"] = c_off[j] + (m0[i] if form == "row" else n0[t] if form == "col" else 0)
+    if form == "blk":
+        u["pad"][:, 0], u["pad"][:, 1] = numpy.asarray(blk[0])[j], numpy.asarray(blk[1])[j]
     u["lda"], u["ldb"], u["K"] = lda[j], ldb[j], K[j]
     u["mrem"], u["nrem"], u["m0"], u["n0"] = mw[i], nw[t], m0[i], n0[t]
     return u
@@ -1642,7 +1713,8 @@ def dpanel_units(M, N, K, lda, ldb, a_off, b_off, c_off, row_form):
 class DPanelStage(object):
     """Panel GEMMs C = A . B^T of every operator in FP64 (qc_dpanel_f64).
 
-    parts: [(units, operator range)]; exactly one of crow (row table) and cols (DCOL_DT)."""
+    parts: [(units, operator range)]; at most one of crow (row table) and cols (DCOL_DT): with
+    neither, the units are in block form (A row-major [K x M])."""
 
     def __init__(self, name, parts, ops, device, flops, crow=None, cols=None, longest_first=False):
         self.name, self.host_ops, self.flops, self.bytes = name, ops, flops, 0.0

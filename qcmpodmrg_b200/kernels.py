@@ -21,7 +21,7 @@ from .native import check
 from .engine import (Stage, compile_classes, add_parts, live_blocks, prune, op_table, TASK_DT, CONTRIB_DT, LOG,
                      compile_fiber, FiberStage, CompositeStage, panel_sigma1, compile_panels, BPERM_DT, PanelStage,
                      fiber_stages, panel_sigma4, upload, sparse_w_class, SparseWStage,
-                     DPanelStage, dpanel_units, DCOL_DT, psi_panels)
+                     DPanelStage, dpanel_units, DCOL_DT, psi_panels, WSource, sparse_groups, _ranges)
 from .mpo import case
 from .qtensor import Contraction, Layout, flip_right, flip_horizontal
 
@@ -134,6 +134,9 @@ def gather_split(x, idx, hi, lo):
 
 def gather_pad(x, idx, out):
     """out[i] = x[idx[i]], 0 where idx is negative (qc_gather_pad_f64)."""
+    if out.device.type != "cuda":           # plans interpreted on the CPU
+        out[:idx.numel()] = torch.where(idx >= 0, x[idx.clamp(min=0)], torch.zeros((), dtype=x.dtype))
+        return out
     check(native.lib().qc_gather_pad_f64(x.data_ptr(), idx.data_ptr(), idx.numel(), out.data_ptr(),
                                          _stream(out.device)), "qc_gather_pad_f64")
     LOG.launches += 1
@@ -369,7 +372,7 @@ class SigmaOperator(object):
                 for cfg, part in parts.items():
                     p4st.setdefault(cfg, []).append(part)
             if sparse_w:
-                wx_parts.append((sx[key], rng))
+                wx_parts.append((sx[key], ops, rng))
                 self.w_paths["sparse"] += 1
             if fib3 is not None:
                 fib[2].append(fib3 + (rng,))
@@ -425,8 +428,13 @@ class SigmaOperator(object):
             else:
                 self._stages.append(CompositeStage(f + [g], "sigma%d" % (si + 1)))
         # the two MPO-site contractions as one sparse product, T1 -> T3
-        self.wx = SparseWStage(wx_parts, dev, "sigma23", op_table(bases[0][order], 0, bases[2][order], 1.0), Wi, Wj,
-                               order, ("f64",) if precision == "f64" else ("f64", "f32")) if sparse_w else None
+        self.wx = None
+        if sparse_w:
+            w1, w2 = Wi.host(), Wj.host()
+            parts = [(x, rng, (WSource.of(x["W"][0], w1, Wi.offsets[ops]), WSource.of(x["W"][1], w2, Wj.offsets[ops])))
+                     for x, ops, rng in wx_parts]
+            self.wx = SparseWStage(parts, dev, "sigma23", op_table(bases[0][order], 0, bases[2][order], 1.0),
+                                   ("f64",) if precision == "f64" else ("f64", "f32"))
         # per-dot L panels (a block permutation of every operator's L), FP64 and FP32
         self.lperm = None
         if lperm:
@@ -645,7 +653,7 @@ class SigmaOperator(object):
             ops = st4_ops.copy()
             ops["b_base"] = base
             parts = [(dpanel_units(sec["M"], sec["N"], sec["K"], sec["Kp"], sec["Kp"], sec["t3pan"], sec["rtoff"],
-                                   sec["crow_base"], True), (poss[0], poss[-1] + 1)) for (poss, sec, _) in classes]
+                                   sec["crow_base"], "row"), (poss[0], poss[-1] + 1)) for (poss, sec, _) in classes]
             self.d4 = DPanelStage("sigma4", parts, ops, dev, flops, crow=crow, longest_first=True)
         self._build_rpan_k()
 
@@ -715,7 +723,7 @@ class SigmaOperator(object):
             sec = [int(s) for s in tc["sectors"]]
             N = [info[s][1] for s in sec]
             u = dpanel_units(tc["M"], N, tc["K"], tc["Kp"], [info[s][3] for s in sec], tc["lpoff"],
-                             [info[s][0] for s in sec], [base + col0[s] for s in sec], False)
+                             [info[s][0] for s in sec], [base + col0[s] for s in sec], "col")
             parts.append((u, (poss[0], poss[-1] + 1)))
         return parts, numpy.concatenate(tabs)
 
@@ -920,46 +928,6 @@ class SigmaOperator(object):
         return y
 
 
-def _dense_tasks(M, N, K, a_off, a_m, a_k, b_off, b_k, b_n, c_off, c_m, alpha, per_group, tile_cfg):
-    """Work items for dense GEMMs C_g = sum_{j in group g} alpha_j A_j B_j (vectorised).
-
-    a_off / b_off / alpha are per contribution, grouped consecutively: group g owns
-    contributions [g*per_group, (g+1)*per_group) and writes at c_off[g].
-    """
-    from .engine import TILES
-    tm, tn = TILES[tile_cfg]
-    a_off = numpy.asarray(a_off, dtype=numpy.int64)
-    ncontr = len(a_off)
-    contribs = numpy.zeros(ncontr, dtype=CONTRIB_DT)
-    contribs["a_off"] = a_off
-    contribs["b_off"] = b_off
-    contribs["alpha"] = alpha
-    contribs["K"] = K
-    contribs["klo"] = K
-    contribs["a_ml"] = a_m
-    contribs["a_kl"] = a_k
-    contribs["b_kl"] = b_k
-    contribs["b_nl"] = b_n
-    contribs["op_b"] = 0
-    contribs["op_e"] = 1
-    c_off = numpy.asarray(c_off, dtype=numpy.int64)
-    ng = len(c_off)
-    m0 = numpy.arange(0, M, tm)
-    n0 = numpy.arange(0, N, tn)
-    nt = len(m0) * len(n0)
-    t = numpy.zeros(ng * nt, dtype=TASK_DT)
-    g = numpy.repeat(numpy.arange(ng), nt)
-    t["c_off"] = c_off[g]
-    t["M"], t["N"], t["mlo"], t["nlo"] = M, N, M, N
-    t["m0"] = numpy.tile(numpy.repeat(m0, len(n0)), ng)
-    t["n0"] = numpy.tile(numpy.tile(n0, len(m0)), ng)
-    t["c_ml"], t["c_nl"] = c_m, 1
-    t["cb"] = g * per_group
-    t["ce"] = g * per_group + per_group
-    t["op_b"], t["op_e"] = 0, 1
-    return t, contribs, 2.0 * M * N * K * ncontr
-
-
 _DENSE_STAGES = {}
 
 
@@ -973,18 +941,22 @@ def _diag_stages(dev, nops, A, Ab, Ac, ldim, rdim, hp):
     p = numpy.repeat(numpy.arange(nops), 16)
     nm = numpy.tile(numpy.arange(16), nops)
     n, m = nm // 4, nm % 4
-    # X[p, n, m, a, c] = sum_b W1[p, a, b, n] W2[p, b, c, m]
-    sX = _dense_tasks(A, Ac, Ab, p * A * Ab * 4 + n, Ab * 4, 4, p * Ab * Ac * 4 + m, Ac * 4, 4,
-                      (p * 16 + nm) * A * Ac, Ac, 1.0, 1, 0)
-    # T[p, nm, c, l] = sum_a X[p, nm, a, c] Ld[p, a, l]
-    sT = _dense_tasks(Ac, ldim, A, (p * 16 + nm) * A * Ac, 1, Ac, p * A * ldim, ldim, 1,
-                      (p * 16 + nm) * Ac * ldim, ldim, 1.0, 1, 0)
-    # D[nm, l, r] = sum_p w_p sum_c T[p, nm, c, l] Rd[p, c, r]   (contributions ordered nm-major)
-    nm2 = numpy.repeat(numpy.arange(16), nops)
-    p2 = numpy.tile(numpy.arange(nops), 16)
-    sD = _dense_tasks(ldim, rdim, Ac, (p2 * 16 + nm2) * Ac * ldim, 1, ldim, p2 * Ac * rdim, rdim, 1,
-                      numpy.arange(16) * ldim * rdim, rdim, hp[p2], nops, 0)
-    out = (Stage({0: [sX]}, dev, "diagX"), Stage({0: [sT]}, dev, "diagT"), Stage({0: [sD]}, dev, "diagD"))
+
+    def stage(name, M, N, K, ops, count, crow=None, lda=None):
+        z = numpy.zeros(1, dtype=numpy.int64)
+        g = (z, z, z, z + M, z + N, z + K, z if crow is not None else z - 1, z + (K if lda is None else lda))
+        return PanelStage({c: [t] for c, t in compile_panels(g, (0, count)).items()}, dev, name, ops, crow=crow)
+
+    # X[p, n, m][a, c] = sum_b W1[p, n][a, b] W2[p, m][b, c]
+    sX = stage("diagX", A, Ac, Ab, op_table((p * 4 + n) * A * Ab, (p * 4 + m) * Ab * Ac, (p * 16 + nm) * A * Ac, 1.0),
+               16 * nops)
+    # T[nm][l, (p, c)] = w_p sum_a Ld[p][l, a] X[p, nm][a, c]
+    sT = stage("diagT", ldim, Ac, A, op_table(p * ldim * A, (p * 16 + nm) * A * Ac, nm * ldim * nops * Ac + p * Ac,
+                                              hp[p]), 16 * nops, crow=numpy.arange(ldim, dtype=numpy.int64) * nops * Ac)
+    # D[nm][l, r] = sum_(p, c) T[nm][l, (p, c)] Rd[(p, c), r]
+    k = numpy.arange(16)
+    sD = stage("diagD", ldim, rdim, nops * Ac, op_table(k * ldim * nops * Ac, 0, k * ldim * rdim, 1.0), 16)
+    out = (sX, sT, sD)
     if len(_DENSE_STAGES) > 256:
         _DENSE_STAGES.clear()
     _DENSE_STAGES[key] = out
@@ -1013,38 +985,49 @@ def _ragged(n):
     return b, e
 
 
-def _env_diag_map(lay, ncol):
-    """Environment E[a, l, l'] -> its diagonal E[a, l, l] as a dense [A x ncol] matrix (src, dst)."""
+def _neutral(lay, axis):
+    """Sector of an MPO bond with quantum number zero (-1: none) and its extent.  Diagonal
+    blocks E[a, l, l] and W[a, b, n, n] between neutral bond states are all that the
+    diagonal of H_eff reads."""
+    z = numpy.flatnonzero((numpy.rint(2 * numpy.asarray(lay.qsyms[axis])) == 0).all(axis=1))
+    return (int(z[0]), int(lay.ndims[axis][z[0]])) if len(z) else (-1, 0)
+
+
+def _env_diag_map(lay, A, ncol, kfast):
+    """Environment E[a, l, l], a neutral -> a dense [ncol x A] (kfast) or [A x ncol] matrix:
+    source index of every dense element, -1 for none."""
     def build():
         idx = lay.idx_allowed
         sa, s1, s2 = numpy.unravel_index(idx, tuple(lay.nsyms))
-        keep = s1 == s2
-        idx, sa, s1 = idx[keep], sa[keep], s1[keep]
+        keep = (s1 == s2) & (sa == _neutral(lay, 0)[0])
+        idx, s1 = idx[keep], s1[keep]
         d = lay.block_dims(idx) if len(idx) else numpy.zeros((0, 3), dtype=numpy.int64)
         da, dl = d[:, 0], d[:, 1]
         b, e = _ragged(da * dl)
         w, u = e // dl[b], e % dl[b]
         src = lay.ioff[idx][b] + w * dl[b] * dl[b] + u * dl[b] + u
-        dst = (lay.secoff[0][sa][b] + w) * ncol + lay.secoff[1][s1][b] + u
-        return src.astype(numpy.int64), dst.astype(numpy.int64)
-    return _cached(("e", id(lay), ncol), lay, build)
+        col = lay.secoff[1][s1][b] + u
+        out = numpy.full(A * ncol, -1, dtype=numpy.int64)
+        out[col * A + w if kfast else w * ncol + col] = src
+        return out
+    return _cached(("e", id(lay), A, ncol, kfast), lay, build)
 
 
-def _w_diag_map(lay, n2):
-    """MPO site operator W[a, b, n, n'] -> its physical diagonal as a dense [A x n2 x 4] array (src, dst)."""
+def _w_diag_map(lay, A, B):
+    """MPO site operator W[a, b, n, n], a and b neutral -> a dense [4 x A x B] array."""
     def build():
         idx = lay.idx_allowed
         sa, sb, n, n_ = numpy.unravel_index(idx, tuple(lay.nsyms))
-        keep = n == n_
-        idx, sa, sb, n = idx[keep], sa[keep], sb[keep], n[keep]
+        keep = (n == n_) & (sa == _neutral(lay, 0)[0]) & (sb == _neutral(lay, 1)[0])
+        idx, n = idx[keep], n[keep]
         d = lay.block_dims(idx) if len(idx) else numpy.zeros((0, 4), dtype=numpy.int64)
         da, db = d[:, 0], d[:, 1]
         b, e = _ragged(da * db)
         w, v = e // db[b], e % db[b]
-        src = lay.ioff[idx][b] + w * db[b] + v
-        dst = ((lay.secoff[0][sa][b] + w) * n2 + lay.secoff[1][sb][b] + v) * 4 + n[b]
-        return src.astype(numpy.int64), dst.astype(numpy.int64)
-    return _cached(("w", id(lay), n2), lay, build)
+        out = numpy.full(4 * A * B, -1, dtype=numpy.int64)
+        out[(n[b] * A + w) * B + v] = lay.ioff[idx][b] + w * db[b] + v
+        return out
+    return _cached(("w", id(lay), A, B), lay, build)
 
 
 def _psi_diag_gather(ql, ldim, rdim):
@@ -1061,7 +1044,12 @@ def _psi_diag_gather(ql, ldim, rdim):
 
 
 class DiagOperator(object):
-    """Davidson diagonal in the packed wavefunction layout (HDiagQt, two-site)."""
+    """Davidson diagonal in the packed wavefunction layout (HDiagQt, two-site).
+
+    Only the neutral sector of the MPO bonds enters (13 of 98 states at K=24): three dense
+    panel GEMMs on FP64 tensor products over it, all operators in the contracted extent of the
+    last one.  K=24, D=300, host result included: 3.03 -> 0.32 ms (218 us on the device, 131
+    of them the last product; the whole bond took 2.8 ms)."""
 
     def __init__(self, ws, isite, psi_layout, L, R, Wi, Wj, qkey, opers, hpwts):
         dev = ws.device
@@ -1070,32 +1058,21 @@ class DiagOperator(object):
         ql = psi_layout
         ldim = int(ql.shape[0])
         rdim = int(ql.shape[3])
-        A = int(L.layouts[0].shape[0])
-        Ab = int(Wi.layouts[0].shape[1])
-        Ac = int(R.layouts[0].shape[0])
+        # extents of the neutral MPO bond sectors (the largest over the operators, zero-padded)
+        A = max(1, max(_neutral(l, 0)[1] for l in L.layouts))
+        Ab = max(1, max(_neutral(l, 1)[1] for l in Wi.layouts))
+        Ac = max(1, max(_neutral(l, 0)[1] for l in R.layouts))
         self.dims = (A, Ab, Ac, ldim, rdim)
-        # ---- index maps for the diagonal elements (host; cached per interned layout) ----
-        Lsrc, Ldst = [], []
-        Rsrc, Rdst = [], []
-        Wsrc1, Wdst1, Wsrc2, Wdst2 = [], [], [], []
-        for i in range(nops):
-            s_, d_ = _env_diag_map(L.layouts[i], ldim)
-            Lsrc.append(s_ + L.offsets[i])
-            Ldst.append(d_ + i * A * ldim)
-            s_, d_ = _env_diag_map(R.layouts[i], rdim)
-            Rsrc.append(s_ + R.offsets[i])
-            Rdst.append(d_ + i * Ac * rdim)
-            s_, d_ = _w_diag_map(Wi.layouts[i], Ab)
-            Wsrc1.append(s_ + Wi.offsets[i])
-            Wdst1.append(d_ + i * A * Ab * 4)
-            s_, d_ = _w_diag_map(Wj.layouts[i], Ac)
-            Wsrc2.append(s_ + Wj.offsets[i])
-            Wdst2.append(d_ + i * Ab * Ac * 4)
-        cat = lambda x: torch.from_numpy(numpy.concatenate(x).astype(numpy.int64)).to(dev)
-        self.maps = [(cat(Lsrc), cat(Ldst), nops * A * ldim, "ld", L),
-                     (cat(Rsrc), cat(Rdst), nops * Ac * rdim, "rd", R),
-                     (cat(Wsrc1), cat(Wdst1), nops * A * Ab * 4, "w1", Wi),
-                     (cat(Wsrc2), cat(Wdst2), nops * Ab * Ac * 4, "w2", Wj)]
+        # ---- source of every element of the dense operands (host; cached per interned layout)
+        def cat(tset, build):
+            m = [build(tset.layouts[i]) for i in range(nops)]
+            return torch.from_numpy(numpy.concatenate([numpy.where(x >= 0, x + o, -1)
+                                                       for x, o in zip(m, tset.offsets)])).to(dev)
+
+        self.maps = [(cat(L, lambda l: _env_diag_map(l, A, ldim, True)), "ld", L),
+                     (cat(R, lambda l: _env_diag_map(l, Ac, rdim, False)), "rd", R),
+                     (cat(Wi, lambda l: _w_diag_map(l, A, Ab)), "w1", Wi),
+                     (cat(Wj, lambda l: _w_diag_map(l, Ab, Ac)), "w2", Wj)]
         # ---- packed output gather: psi block (sl, n, m, sr), element (u, v) ----
         gat = _psi_diag_gather(ql, ldim, rdim)
         self.gather = torch.from_numpy(gat).to(dev)
@@ -1111,8 +1088,7 @@ class DiagOperator(object):
     def rebind(self, L, R):
         """Use new environment values with the same block layouts (cached plan)."""
         sub = {"ld": L, "rd": R}
-        self.maps = [(src, dst, n, name, sub[name] if name in sub else tset)
-                     for (src, dst, n, name, tset) in self.maps]
+        self.maps = [(idx, name, sub[name] if name in sub else tset) for (idx, name, tset) in self.maps]
 
     def release(self):
         self.rebind(None, None)
@@ -1120,17 +1096,13 @@ class DiagOperator(object):
     def __call__(self):
         ws = self.ws
         bufs = {}
-        for (src, dst, n, name, tset) in self.maps:
-            b = ws.get("diag_" + name, n, torch.float64)
-            b[:n].zero_()
-            if src.numel():
-                b[dst] = tset.values[src]
-            bufs[name] = b
+        for (idx, name, tset) in self.maps:
+            bufs[name] = gather_pad(tset.values, idx, ws.get("diag_" + name, idx.numel(), torch.float64))
         X = ws.get("diag_x", self.nX, torch.float64)
         T = ws.get("diag_t", self.nT, torch.float64)
         D = ws.get("diag_d", self.nD, torch.float64)
         self.sX.run(bufs["w1"], bufs["w2"], X, "f64")
-        self.sT.run(X, bufs["ld"], T, "f64")
+        self.sT.run(bufs["ld"], X, T, "f64")
         self.sD.run(T, bufs["rd"], D, "f64")
         out = torch.empty(self.ndim0, dtype=torch.float64, device=ws.device)
         return gather(D, self.gather, out)
