@@ -230,8 +230,8 @@ int qc_fgemm_f32(const void *items_dev, long long nitems, const void *groups_dev
 int qc_wpanel_f64(const double *src, const long long *idx_dev, double *dst, long long n, void *stream);
 int qc_wpanel_f32(const float *src, const long long *idx_dev, float *dst, long long n, void *stream);
 /* FP64 panel GEMM on the tensor pipe (mma.sync f64): work is nwork (unit, operator) int
- * pairs, units qc_dunit records, ops the operator table.  Exactly one of crow (row form)
- * and cols (column form, qc_dcol) is given.  A and B are 16-byte aligned. */
+ * pairs, units qc_dunit records, ops the operator table.  crow: row form; cols (qc_dcol):
+ * column form; neither: block form.  A and B are 16-byte aligned. */
 int qc_dpanel_f64(const void *units, const void *work, long long nwork, const void *ops, const long long *crow,
                   const void *cols, const double *A, const double *B, double *C, void *stream);
 /* out[i] = x[idx[i]], 0 where idx[i] < 0. */

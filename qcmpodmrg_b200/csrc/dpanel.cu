@@ -20,6 +20,7 @@
 // held back by its T1 stores and by K extents that end inside a 16-deep slice, .R by the
 // last wave of tiles and the ring's barriers.
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdio>
 #include "qc_types.h"
 
@@ -27,6 +28,7 @@ namespace {
 
 constexpr int DP_BM = 128, DP_BN = 64, DP_BK = 16, DP_ST = 3, DP_THREADS = 256;
 constexpr int DP_P = DP_BK + 4;                                  // row pitch in doubles
+constexpr int DP_PT = DP_BM + 4;                                 // the same for an A tile staged [k][m]
 constexpr int DP_STAGE = (DP_BM + DP_BN) * DP_P;                 // doubles of one stage
 constexpr int DP_SMEM = DP_ST * DP_STAGE * 8;
 
@@ -41,12 +43,12 @@ __device__ __forceinline__ void dp_mma(double (&c)[2], double a, double b) {
 }
 
 // One K slice (k4 groups of four k) of a warp's 16 x 8 NT tile.
-template <int NT>
+template <int NT, bool AT>
 __device__ __forceinline__ void dp_slice(const double *as, const double *bs, int k4, double (&acc)[2][DP_BN / 8][2]) {
 #pragma unroll
   for (int kk = 0; kk < DP_BK / 4; ++kk) {
     if (kk < k4) {
-      const double a0 = as[4 * kk], a1 = as[8 * DP_P + 4 * kk];
+      const double a0 = as[4 * kk * (AT ? DP_PT : 1)], a1 = as[4 * kk * (AT ? DP_PT : 1) + 8 * (AT ? 1 : DP_P)];
       double b[NT];
 #pragma unroll
       for (int j = 0; j < NT; ++j) b[j] = bs[8 * j * DP_P + 4 * kk];
@@ -69,15 +71,18 @@ constexpr int DP_RECS = 8;       // a CTA's records in flight: the loads run at 
 // l % 4 and l % 4 + 4 of its group of eight, so that four lanes store 32 contiguous bytes
 __device__ __forceinline__ int dp_col_place(int n) { return (n & ~7) | ((n & 3) << 1) | ((n >> 2) & 1); }
 
-template <bool COLS>
+constexpr int DP_ROWS = 0, DP_COLS = 1, DP_BLK = 2;      // where a tile goes (qc_dunit)
+
+template <int MODE>
 __global__ void __launch_bounds__(DP_THREADS, 2)
 k_dpanel(const qc_dunit *__restrict__ units, const int2 *__restrict__ work, int nwork,
          const qc_op *__restrict__ ops, const long long *__restrict__ crow, const qc_dcol *__restrict__ cols,
          const double *__restrict__ A, const double *__restrict__ B, double *__restrict__ C) {
+  constexpr bool COLS = MODE == DP_COLS, AT = MODE == DP_BLK;
   extern __shared__ __align__(16) double dp_smem[];
   __shared__ __align__(16) DpRec recs[DP_RECS];
   __shared__ __align__(16) qc_dcol scols[COLS ? DP_RECS : 1][DP_BN];
-  __shared__ __align__(16) long long srow[COLS ? 1 : DP_RECS][DP_BM];
+  __shared__ __align__(16) long long srow[MODE == DP_ROWS ? DP_RECS : 1][DP_BM];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int G = (int)gridDim.x;
   const int ntile = (nwork - (int)blockIdx.x + G - 1) / G;
@@ -103,6 +108,7 @@ k_dpanel(const qc_dunit *__restrict__ units, const int2 *__restrict__ work, int 
   const unsigned sbase = (unsigned)__cvta_generic_to_shared(dp_smem);
   // this thread copies 16 bytes (two k) of rows r0, r0 + 32, ... of both operands
   const int ck = 2 * (tid & 7), r0 = tid >> 3;
+  const int cm = 2 * (tid & 63), rk = tid >> 6;      // A given as [K x M]: two m of rows rk, rk + 4, ...
   int lt = 0, lk = 0, lnk, lK, lm, ln, lda, ldb;     // loads: tile, K slice, the tile's extents
   const double *Ab, *Bb;
   auto open_tile = [&]() {
@@ -113,11 +119,11 @@ k_dpanel(const qc_dunit *__restrict__ units, const int2 *__restrict__ work, int 
     ln = r.u.nrem;
     lda = r.u.lda;
     ldb = r.u.ldb;
-    Ab = A + r.o.a_base + r.u.a_off + (long long)r0 * lda + ck;
+    Ab = A + r.o.a_base + r.u.a_off + (AT ? (long long)rk * lda + cm : (long long)r0 * lda + ck);
     Bb = B + r.o.b_base + r.u.b_off + (long long)r0 * ldb + ck;
     lk = 0;
     // the tile's column (row) records, read by its epilogue
-    if (COLS ? tid < ln : tid < lm) {
+    if (MODE != DP_BLK && (COLS ? tid < ln : tid < lm)) {
       const void *src = COLS ? (const void *)(cols + r.u.c_off + tid) : (const void *)(crow + r.u.c_off + tid);
       const void *dst = COLS ? (const void *)&scols[lt & (DP_RECS - 1)][tid] : (const void *)&srow[lt & (DP_RECS - 1)][tid];
       asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
@@ -135,10 +141,20 @@ k_dpanel(const qc_dunit *__restrict__ units, const int2 *__restrict__ work, int 
       const int kb = max(0, min(2, lK - k0 - ck)) * 8;
       const unsigned s = sbase + (unsigned)(ls * DP_STAGE + r0 * DP_P + ck) * 8u;
       const unsigned sb = sbase + (unsigned)(ls * DP_STAGE + dp_col_place(r0) * DP_P + ck) * 8u;
+      if (AT) {
+        const unsigned sa = sbase + (unsigned)(ls * DP_STAGE + rk * DP_PT + cm) * 8u;
+        const int mb = max(0, min(2, lm - cm)) * 8;
 #pragma unroll
-      for (int e = 0; e < DP_BM / 32; ++e) {
-        const int v = r0 + 32 * e < lm ? kb : 0;
-        dp_cp16(s + (unsigned)(32 * e * DP_P) * 8u, v ? Ab + (long long)(32 * e) * lda + k0 : A, v);
+        for (int e = 0; e < DP_BK / 4; ++e) {
+          const int v = k0 + rk + 4 * e < lK ? mb : 0;
+          dp_cp16(sa + (unsigned)(4 * e * DP_PT) * 8u, v ? Ab + (long long)(k0 + 4 * e) * lda : A, v);
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < DP_BM / 32; ++e) {
+          const int v = r0 + 32 * e < lm ? kb : 0;
+          dp_cp16(s + (unsigned)(32 * e * DP_P) * 8u, v ? Ab + (long long)(32 * e) * lda + k0 : A, v);
+        }
       }
 #pragma unroll
       for (int e = 0; e < DP_BN / 32; ++e) {
@@ -176,18 +192,18 @@ k_dpanel(const qc_dunit *__restrict__ units, const int2 *__restrict__ work, int 
       __syncthreads();
       load();
       if (live) {
-        const double *as = dp_smem + st * DP_STAGE + (warp * 16 + gr) * DP_P + gk;
+        const double *as = dp_smem + st * DP_STAGE + (AT ? gk * DP_PT + warp * 16 + gr : (warp * 16 + gr) * DP_P + gk);
         const double *bs = dp_smem + st * DP_STAGE + (DP_BM + gr) * DP_P + gk;
         const int k4 = min(DP_BK / 4, (K - kt * DP_BK + 3) >> 2);
         switch (nt) {
-          case 1: dp_slice<1>(as, bs, k4, acc); break;
-          case 2: dp_slice<2>(as, bs, k4, acc); break;
-          case 3: dp_slice<3>(as, bs, k4, acc); break;
-          case 4: dp_slice<4>(as, bs, k4, acc); break;
-          case 5: dp_slice<5>(as, bs, k4, acc); break;
-          case 6: dp_slice<6>(as, bs, k4, acc); break;
-          case 7: dp_slice<7>(as, bs, k4, acc); break;
-          default: dp_slice<8>(as, bs, k4, acc); break;
+          case 1: dp_slice<1, AT>(as, bs, k4, acc); break;
+          case 2: dp_slice<2, AT>(as, bs, k4, acc); break;
+          case 3: dp_slice<3, AT>(as, bs, k4, acc); break;
+          case 4: dp_slice<4, AT>(as, bs, k4, acc); break;
+          case 5: dp_slice<5, AT>(as, bs, k4, acc); break;
+          case 6: dp_slice<6, AT>(as, bs, k4, acc); break;
+          case 7: dp_slice<7, AT>(as, bs, k4, acc); break;
+          default: dp_slice<8, AT>(as, bs, k4, acc); break;
         }
       }
       st = st + 1 == DP_ST ? 0 : st + 1;
@@ -213,6 +229,23 @@ k_dpanel(const qc_dunit *__restrict__ units, const int2 *__restrict__ work, int 
             }
           }
         }
+    } else if (AT) {
+      const int dr = rec.u.pad0, dc = rec.u.pad1, m0 = rec.u.m0, n0 = rec.u.n0;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int m = warp * 16 + 8 * i + gr;
+        if (m < mrem) {
+          const int q = (m0 + m) / dr, r = (m0 + m) - q * dr;
+          double *dst = Cb + rec.u.c_off + (long long)q * dr * dc + (long long)n0 * dr + r;
+#pragma unroll
+          for (int j = 0; j < DP_BN / 8; ++j)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int n = 8 * j + 4 * h + gk;
+              if (n < nrem) dst[(long long)n * dr] = alpha * acc[i][j][h];
+            }
+        }
+      }
     } else {
       const int n0 = rec.u.n0;
 #pragma unroll
@@ -249,18 +282,26 @@ __global__ void k_gather_pad(const double *__restrict__ x, const long long *__re
 
 }  // namespace
 
-template <bool COLS>
+template <int MODE>
 static cudaError_t launch_dpanel(const void *units, const void *work, int nwork, const void *ops,
                                  const long long *crow, const void *cols, const double *A, const double *B, double *C,
                                  cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(k_dpanel<COLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, DP_SMEM);
-  int dev = 0, nsm = 0;
-  if (e == cudaSuccess) e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  // the shared-memory limit of a kernel and the SM count are properties of a device: asked once for each
+  static std::atomic<int> sms[64];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  // short panels (L.psi) share a persistent grid; the long ones of .R, sorted by length, are
-  // left to the hardware's scheduler, one tile per CTA (K = 24, D = 500: 5.7 against 6.8 ms)
-  k_dpanel<COLS><<<COLS && nwork > 2 * nsm ? 2 * nsm : nwork, DP_THREADS, DP_SMEM, s>>>(
+  int nsm = dev < 64 ? sms[dev].load(std::memory_order_relaxed) : 0;
+  if (nsm == 0) {
+    e = cudaFuncSetAttribute(k_dpanel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, DP_SMEM);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 64) sms[dev].store(nsm, std::memory_order_relaxed);
+  }
+  // short panels (L.psi, the renormalisation's) share a persistent grid; the long ones of .R,
+  // sorted by length, are left to the hardware's scheduler, one tile per CTA (K = 24, D = 500:
+  // 5.7 against 6.8 ms)
+  k_dpanel<MODE><<<MODE != DP_ROWS && nwork > 2 * nsm ? 2 * nsm : nwork, DP_THREADS, DP_SMEM, s>>>(
       (const qc_dunit *)units, (const int2 *)work, nwork, (const qc_op *)ops, crow, (const qc_dcol *)cols, A, B, C);
   return cudaGetLastError();
 }
@@ -269,12 +310,13 @@ extern "C" int qc_dpanel_f64(const void *units, const void *work, long long nwor
                              const long long *crow, const void *cols, const double *A, const double *B, double *C,
                              void *stream) {
   if (nwork <= 0) return QC_OK;
-  if (nwork > 0x3fffffffLL || !units || !work || !ops || (!crow && !cols) || ((unsigned long long)A & 15) ||
+  if (nwork > 0x3fffffffLL || !units || !work || !ops || (crow && cols) || ((unsigned long long)A & 15) ||
       ((unsigned long long)B & 15))
     return QC_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  const cudaError_t e = cols ? launch_dpanel<true>(units, work, (int)nwork, ops, crow, cols, A, B, C, s)
-                             : launch_dpanel<false>(units, work, (int)nwork, ops, crow, cols, A, B, C, s);
+  const cudaError_t e = cols   ? launch_dpanel<DP_COLS>(units, work, (int)nwork, ops, crow, cols, A, B, C, s)
+                        : crow ? launch_dpanel<DP_ROWS>(units, work, (int)nwork, ops, crow, cols, A, B, C, s)
+                               : launch_dpanel<DP_BLK>(units, work, (int)nwork, ops, crow, cols, A, B, C, s);
   if (e != cudaSuccess) {
     fprintf(stderr, "[qcgpu] qc_dpanel: %s\n", cudaGetErrorString(e));
     return QC_ERR_CUDA;

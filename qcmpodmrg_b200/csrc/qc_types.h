@@ -265,6 +265,8 @@ static_assert(sizeof(qc_wxquad) == 16, "qc_wxquad is 16 bytes");
 // with 16-byte aligned rows (lda, ldb multiples of 4).  Row form: row m of the tile goes to
 // C + c_base + crow[c_off + m] + n0; column form: column n of the tile, tile row m, goes to
 // C + c_base + cols[c_off + n].off + (m0 + m) * cols[c_off + n].ld (off < 0: not stored).
+// Block form: A is given as [K x M] rows (element (m, k) at a_off + k * lda + m, m0 in a_off),
+// the tile goes to the block [row / pad0][column][row % pad0] of pad1 columns at c_base + c_off.
 struct alignas(16) qc_dunit {
   long long a_off, b_off, c_off;
   int lda, ldb, K;

@@ -1120,35 +1120,42 @@ def _unit_axes(lay, axes):
 
 
 def sparse_groups(ins, outs, dx, dz, qx, qz, da, db):
-    """Fiber groups of a sparse MPO stage for one operator class.
+    """Fiber groups of a sparse MPO stage.
 
-    A group is a pair (x sector, z sector) of bond states, its fibers the states (x, z); the
-    groups are collected by the charge difference q(x) - q(z).  ins / outs: arrays (x, z,
-    slot, MPO sector, offset, row stride, end) of the input blocks [bond][fiber] (fibers of
-    one x contiguous, the row stride is not used) and the output blocks (x, c) -> offset +
-    x * stride + c * D_z + z.  dx, dz, qx, qz: extents and quantum numbers of the sectors of
-    the two bonds, da / db: extents of the MPO sectors.  The MPO sector of a slot is the same
-    for all groups of one difference; returns None where that does not hold or an offset does
-    not fit the records, else {"groups", "deltas", "rows", "iblk", "kblk", "row0", "R",
-    "fibers"}."""
+    A group is a pair (x sector, z sector) of bond states of one operator class, its fibers
+    the states (x, z); the groups of a class are collected by the charge difference q(x) -
+    q(z).  ins / outs: arrays (class, x, z, slot, MPO sector, offset, row stride, end) of the
+    input blocks [bond][fiber] (fibers of one x contiguous, the row stride is not used) and
+    the output blocks (x, c) -> offset + x * stride + c * D_z + z.  dx, dz, qx, qz: extents
+    and quantum numbers of the sectors of the two bonds, da / db: extents of the MPO sectors
+    [class, sector].  The MPO sector of a slot is the same for all groups of one difference;
+    returns None where that does not hold or an offset does not fit the records, else one
+    {"groups", "deltas", "rows", "iblk", "kblk", "row0", "R", "fibers"} per class (None for a
+    class without output)."""
     i64 = numpy.int64
-    x1, z1, s1, a1, o1, _, e1 = ins
-    x3, z3, s3, c3, o3, h3, e3 = outs
+    k1, x1, z1, s1, a1, o1, _, e1 = ins
+    k3, x3, z3, s3, c3, o3, h3, e3 = outs
+    ncls = len(da)
     if len(x3) == 0:
-        return None
-    nz = len(dz)
-    xz = numpy.unique(x3 * nz + z3)
-    keep = numpy.isin(x1 * nz + z1, xz)
-    x1, z1, s1, a1, o1, e1 = (v[keep] for v in (x1, z1, s1, a1, o1, e1))
-    gx, gz = xz // nz, xz % nz
+        return [None] * ncls
+    nz, nxz = len(dz), len(dx) * len(dz)
+    has = numpy.zeros(ncls * nxz, dtype=bool)
+    has[k3 * nxz + x3 * nz + z3] = True
+    xz = numpy.flatnonzero(has)
+    keep = has[k1 * nxz + x1 * nz + z1]
+    k1, x1, z1, s1, a1, o1, e1 = (v[keep] for v in (k1, x1, z1, s1, a1, o1, e1))
+    gk, gx, gz = xz // nxz, xz % nxz // nz, xz % nz
     q2 = lambda q: numpy.rint(2 * numpy.asarray(q)).astype(i64)            # noqa: E731
-    dq = q2(qx)[gx] - q2(qz)[gz]
-    uq, dinv = numpy.unique(dq, axis=0, return_inverse=True)
-    dinv = dinv.ravel()
+    qx, qz = q2(qx), q2(qz)
+    big = 4 * int(max(abs(qx).max(), abs(qz).max())) + 1
+    qkey = gk
+    for c in range(qx.shape[1]):
+        qkey = qkey * big + (qx[gx, c] - qz[gz, c] + big // 2)
+    uq, dinv = numpy.unique(qkey, return_inverse=True)
     nd = len(uq)
-    o = numpy.argsort(dinv, kind="stable")                                 # groups delta by delta
-    xz, gx, gz, dinv = xz[o], gx[o], gz[o], dinv[o]
-    pos = numpy.empty(len(dx) * nz, dtype=i64)
+    o = numpy.argsort(dinv, kind="stable")                                 # groups delta by delta, class by class
+    xz, gk, gx, gz, dinv = xz[o], gk[o], gx[o], gz[o], dinv[o]
+    pos = numpy.empty(ncls * nxz, dtype=i64)
     pos[xz] = numpy.arange(len(xz))
     dx, dz, da, db = (numpy.asarray(v, dtype=i64) for v in (dx, dz, da, db))
     F = dx[gx] * dz[gz]
@@ -1160,7 +1167,7 @@ def sparse_groups(ins, outs, dx, dz, qx, qz, da, db):
     cs = numpy.cumsum(F) - F
     first = numpy.searchsorted(dinv, numpy.arange(nd))
     g["start"] = cs - cs[first][dinv]
-    p1, p3 = pos[x1 * nz + z1], pos[x3 * nz + z3]
+    p1, p3 = pos[k1 * nxz + x1 * nz + z1], pos[k3 * nxz + x3 * nz + z3]
     iblk = numpy.full((nd, 16), -1, dtype=numpy.int32)
     kblk = numpy.full((nd, 16), -1, dtype=numpy.int32)
     iblk[dinv[p1], s1] = a1
@@ -1168,26 +1175,38 @@ def sparse_groups(ins, outs, dx, dz, qx, qz, da, db):
     # one MPO sector per slot, one block per (group, slot)
     if not (numpy.array_equal(iblk[dinv[p1], s1], a1) and numpy.array_equal(kblk[dinv[p3], s3], c3)):
         return None
-    if len(numpy.unique(p1 * 16 + s1)) != len(p1) or len(numpy.unique(p3 * 16 + s3)) != len(p3):
+    if max(numpy.bincount(p1 * 16 + s1, minlength=1).max(), numpy.bincount(p3 * 16 + s3).max()) > 1:
         return None
     g["a"][p1, s1] = o1
     g["c"][p3, s3] = o3
     g["h"][p3, s3] = h3
-    rows_b = numpy.where(iblk >= 0, da[numpy.maximum(iblk, 0)], 0)          # [delta, 16]
+    dk = gk[first]                                                         # class of every delta
+    rows_b = numpy.where(iblk >= 0, da[dk[:, None], numpy.maximum(iblk, 0)], 0)          # [delta, 16]
     R = rows_b.sum(axis=1)
     row0 = numpy.where(iblk >= 0, numpy.cumsum(rows_b, axis=1) - rows_b, 0).astype(numpy.int32)
-    dcb = numpy.where(kblk >= 0, db[numpy.maximum(kblk, 0)], 0)
+    dcb = numpy.where(kblk >= 0, db[dk[:, None], numpy.maximum(kblk, 0)], 0)
     if int(R.max()) > WX_MAXR or int(((dcb + 3) // 4).sum(axis=1).max()) > WX_MAXQ:
         return None
-    d = numpy.zeros(nd, WXDELTA_DT)
-    d["R"] = R
-    d["row_b"] = numpy.cumsum(R) - R
-    d["grp_b"] = first
-    d["grp_e"] = numpy.r_[first[1:], len(xz)]
     own, loc = _ranges(rows_b.ravel())
     rows = ((own % 16) << 16 | loc).astype(numpy.int32)
-    return {"groups": g, "deltas": d, "rows": rows, "iblk": iblk, "kblk": kblk, "row0": row0,
-            "R": R.astype(numpy.int32), "fibers": numpy.add.reduceat(F, first)}
+    fibers = numpy.add.reduceat(F, first)
+    R = R.astype(numpy.int32)
+    rb = numpy.concatenate([[0], numpy.cumsum(R)])
+    gend = numpy.r_[first[1:], len(xz)]
+    out = []
+    for k in range(ncls):
+        b, e = numpy.searchsorted(dk, [k, k + 1])
+        if b == e:
+            out.append(None)
+            continue
+        g0, g1 = int(first[b]), int(gend[e - 1])
+        d = numpy.zeros(e - b, WXDELTA_DT)
+        d["R"], d["row_b"] = R[b:e], rb[b:e] - rb[b]
+        d["grp_b"], d["grp_e"] = first[b:e] - g0, gend[b:e] - g0
+        c = numpy.ascontiguousarray
+        out.append({"groups": g[g0:g1], "deltas": d, "rows": rows[rb[b]:rb[e]], "iblk": c(iblk[b:e]),
+                    "kblk": c(kblk[b:e]), "row0": c(row0[b:e]), "R": c(R[b:e]), "fibers": fibers[b:e]})
+    return out
 
 
 def sparse_w_class(c1, t1, t1off, t3lay, pan4, W1, W2, psi):
@@ -1209,13 +1228,14 @@ def sparse_w_class(c1, t1, t1off, t3lay, pan4, W1, W2, psi):
     off1 = (c1.out.ioff if t1off is None else t1off)[b1]
     off3, fhs3 = pan4["t3off"][b3], pan4["t3fhs"][b3]
     d3 = t3lay.block_dims(b3)
-    out = sparse_groups((l, r, 4 * n1 + n2, a, off1, None, off1 + c1.out.ndim[b1]),
-                        (l3, r3, 4 * m1 + m2, cc, off3, fhs3,
+    out = sparse_groups((0 * l, l, r, 4 * n1 + n2, a, off1, None, off1 + c1.out.ndim[b1]),
+                        (0 * l3, l3, r3, 4 * m1 + m2, cc, off3, fhs3,
                          off3 + numpy.maximum(d3[:, 0] - 1, 0) * fhs3 + d3[:, 1] * d3[:, 3]),
-                        psi.ndims[0], psi.ndims[3], psi.qsyms[0], psi.qsyms[3], W1.ndims[0], W2.ndims[1])
-    if out is not None:
-        out["W"] = (W1, W2)
-    return out
+                        psi.ndims[0], psi.ndims[3], psi.qsyms[0], psi.qsyms[3], W1.ndims[0][None], W2.ndims[1][None])
+    if out is None:
+        return None
+    out[0]["W"] = (W1, W2)
+    return out[0]
 
 
 class WSource(object):
@@ -1547,12 +1567,13 @@ def _ranges(n):
     return own, numpy.arange(int(n.sum()), dtype=numpy.int64) - numpy.repeat(numpy.cumsum(n) - n, n)
 
 
-def psi_panels(psi, blocks=None):
+def psi_panels(psi, blocks=None, index=True):
     """The wavefunction (its allowed blocks, or the given ones) as the B operand of the
     tensor-core L.psi GEMMs: per first-index
     sector l' the psi blocks (l', n1, n2, r) of that sector side by side as columns,
     transposed to [sum_j N_j x Kp] (k = l' index contiguous, rows padded to Kp = D_l'
-    rounded up to 4).  Returns (gather index into the packed vector, -1 for padding),
+    rounded up to 4).  Returns (gather index into the packed vector, -1 for padding; None
+    without index),
     {sector: (offset, N total, K, Kp)} and {block: (sector, first column)}."""
     blocks = numpy.asarray(psi.idx_allowed if blocks is None else blocks, dtype=numpy.int64)
     if len(blocks) == 0:
@@ -1572,14 +1593,16 @@ def psi_panels(psi, blocks=None):
     soff = numpy.cumsum(size) - size
     col = numpy.cumsum(N) - N - numpy.repeat((numpy.cumsum(N) - N)[first], cnt)    # first column in its sector
     sidx = numpy.repeat(numpy.arange(len(us)), cnt)                                   # sector position per block
+    info = {int(s_): (int(a), int(n), int(k), int(kp)) for s_, a, n, k, kp in zip(us, soff, ntot, ks, kps)}
+    cols = {int(bb): (int(s_), int(c)) for bb, s_, c in zip(blocks, sec, col)}
+    if not index:
+        return None, info, cols
     # gather index: panel element (column c, k) of sector s at soff + c * Kp + k
     gidx = numpy.full(int(size.sum()), -1, dtype=numpy.int64)
     b, e = _ranges(N * K[...])                       # (block, local element) over each block's N x K values
     nb, kb = N[b], K[b]
     cc, kk = e % nb, e // nb                         # element (k, column) of the block: psi offset k * N + c
     gidx[soff[sidx[b]] + (col[b] + cc) * kps[sidx[b]] + kk] = psi.ioff[blocks[b]] + kk * nb + cc
-    info = {int(s_): (int(a), int(n), int(k), int(kp)) for s_, a, n, k, kp in zip(us, soff, ntot, ks, kps)}
-    cols = {int(bb): (int(s_), int(c)) for bb, s_, c in zip(blocks, sec, col)}
     return gidx, info, cols
 
 
@@ -1686,11 +1709,11 @@ def _even_tiles(n, most, unit):
     return own, loc * w[own], numpy.minimum(w[own], n[own] - loc * w[own])
 
 
-def dpanel_units(M, N, K, lda, ldb, a_off, b_off, c_off, form, blk=None):
+def dpanel_units(M, N, K, lda, ldb, a_off, b_off, c_off, form, blk=None, owner=False):
     """Tiles of the panels C_j[M_j x N_j] = A_j . B_j^T.  form "row": c_off is the row-table
     index of row 0; "col": the column-table index of column 0; "blk": the offset of the block
     [row / blk[0]][column][row % blk[0]] of blk[1] columns, A given as [K x M].  Column tiles of
-    one row tile are neighbours."""
+    one row tile are neighbours.  owner: also the panel of every tile."""
     M, N, K, lda, ldb, a_off, b_off, c_off = (numpy.asarray(x, dtype=numpy.int64) for x in
                                               (M, N, K, lda, ldb, a_off, b_off, c_off))
     jm, m0, mw = _even_tiles(M, DP_BM, 16)
@@ -1707,7 +1730,7 @@ def dpanel_units(M, N, K, lda, ldb, a_off, b_off, c_off, form, blk=None):
         u["pad"][:, 0], u["pad"][:, 1] = numpy.asarray(blk[0])[j], numpy.asarray(blk[1])[j]
     u["lda"], u["ldb"], u["K"] = lda[j], ldb[j], K[j]
     u["mrem"], u["nrem"], u["m0"], u["n0"] = mw[i], nw[t], m0[i], n0[t]
-    return u
+    return (u, j) if owner else u
 
 
 class DPanelStage(object):

@@ -21,7 +21,8 @@ from .native import check
 from .engine import (Stage, compile_classes, add_parts, live_blocks, prune, op_table, TASK_DT, CONTRIB_DT, LOG,
                      compile_fiber, FiberStage, CompositeStage, panel_sigma1, compile_panels, BPERM_DT, PanelStage,
                      fiber_stages, panel_sigma4, upload, sparse_w_class, SparseWStage,
-                     DPanelStage, dpanel_units, DCOL_DT, psi_panels, WSource, sparse_groups, _ranges)
+                     DPanelStage, dpanel_units, DCOL_DT, psi_panels, WSource, _ranges)
+from .envpanels import EnvPanels, NoPanelForm
 from .mpo import case
 from .qtensor import Contraction, Layout, flip_right, flip_horizontal
 
@@ -1113,13 +1114,30 @@ class Renormalizer(object):
 
     status 'L': L'[b, r, r'] = sum site*[l, n, r] L[a, l, l'] W[a, b, n, n'] site[l', n', r']
     status 'R': the mirror image with W's bond indices flipped (kernelQt.py:723-740).
+
+    With x, y the bra and ket states of the old bond, z, z' those of the new one and S the
+    site tensor, three stages over all operators: T1[a, x, n, z'] = E[a, x, y] S[y, n, z']
+    (panel GEMM), T2[b, x, n', z'] = W T1 (the sparse MPO stage, fibers (x, z')), and
+    E'[b, z, z'] = S*[(x, n'), z] T2[(x, n'), (b, z')] (panel GEMM, T2 as [K x M]).  Dots whose
+    blocks have no such form run three grouped block GEMMs.
     """
 
-    def __init__(self, ws, isite, status, site_layout, E, W, opers):
+    def __init__(self, ws, isite, status, site_layout, E, W, opers, panels=None):
+        """panels: the panel form (None: on a GPU, where the blocks allow it)."""
         self.ws, self.status = ws, status
         dev = ws.device
         groups = _groups(opers, isite, 1)
         nops = len(opers)
+        self.E, self.W = E, W
+        self.ep = None
+        if panels is None:
+            panels = torch.device(dev).type == "cuda"
+        if panels:
+            try:
+                self._setup_panels(groups, site_layout, E, W)
+                return
+            except NoPanelForm:
+                pass
         if status == "L":
             ax = (([0], [1]), ([0, 2], [2, 0]), ([1, 3], [1, 0]))
         else:
@@ -1166,11 +1184,70 @@ class Renormalizer(object):
                 add_parts(st[si], compile_classes(c, t, ax[si]), op_range=rng)
         self.stages = [Stage(st[si], dev, "renorm%d" % (si + 1), tabs[si]) for si in range(3)]
         self.flops = sum(s.flops for s in self.stages)
-        self.E, self.W = E, W
+
+    def _setup_panels(self, groups, site, E, W):
+        """The panel form; raises NoPanelForm where the blocks do not allow it."""
+        left = self.status == "L"
+        old, new = (0, 2) if left else (2, 0)
+        if list(site.status) != ([False, False, True] if left else [True, False, False]):
+            raise NoPanelForm
+        ep = EnvPanels(self.ws, "renorm", groups, site, old, E, W, left, site.qsyms[old], site.qsyms[new])
+        dx, dz = ep.dx, ep.dz
+        i64 = numpy.int64
+        # bra panel of new sector z: [D_z x Kp], K index (x, n') block by block
+        o = numpy.lexsort((ep.kn, ep.ky, ep.kz))
+        bx, bn, bz = ep.ky[o], ep.kn[o], ep.kz[o]
+        cnt = numpy.bincount(bz, minlength=len(dz)).astype(i64)
+        first = numpy.cumsum(cnt) - cnt
+        Kz = numpy.bincount(bz, weights=dx[bx], minlength=len(dz)).astype(i64)
+        ck = numpy.cumsum(dx[bx]) - dx[bx]
+        koff = ck - ck[first[bz]]
+        Kp = (Kz + 3) // 4 * 4
+        boff = numpy.cumsum(dz * Kp) - dz * Kp
+        bra = ep._copy_descs(ep.ksrc[o], dx[bx], dz[bz], ep.ket_size + boff[bz] + koff, Kp[bz], old)
+        # the new environments' blocks (b, z, z'); T2 panel of each: rows (x, n') of z, columns (b, z')
+        wax, sign = (1, 1.0) if left else (0, -1.0)
+        lays = [Layout([True, False, True], [sign * wl.qsyms[wax], site.qsyms[new], site.qsyms[new]],
+                       [wl.ndims[wax], site.ndims[new], site.ndims[new]]) for wl in ep.Wl]
+        sec = [l.block_sectors(l.idx_allowed) for l in lays]
+        ok = numpy.repeat(numpy.arange(len(lays)), [len(l.idx_allowed) for l in lays])
+        ob, oz, oz2 = (numpy.concatenate([s_[k] for s_ in sec]).astype(i64) for k in range(3))
+        ooff = numpy.concatenate([l.ioff[l.idx_allowed] for l in lays])
+        ncol = ep.db[ok, ob] * dz[oz2]
+        ld = (ncol + 3) // 4 * 4
+        size = Kz[oz] * ld
+        cs = numpy.cumsum(size) - size
+        cls0 = numpy.searchsorted(ok, numpy.arange(len(lays)))
+        pan = cs - cs[numpy.minimum(cls0[ok], max(len(cs) - 1, 0))] if len(cs) else cs
+        own, loc = _ranges(cnt[oz])
+        k = first[oz[own]] + loc                                # bra block of every T2 block
+        o2 = pan[own] + koff[k] * ld[own]
+        if len(own) and not numpy.array_equal(ep.b[ok[own], bx[k], oz2[own], bn[k]], ob[own]):
+            raise NoPanelForm
+        ep.finish((ok[own], bx[k], oz2[own], 4 * bn[k], ob[own], o2, ld[own], o2 + dx[bx[k]] * ld[own]),
+                  numpy.bincount(ok, weights=size, minlength=len(lays)).astype(i64), bra, int((dz * Kp).sum()))
+        base, self._nout = ep.slices([l.size for l in lays], 1)
+        u, uj = dpanel_units(ncol, dz[oz], Kz[oz], ld, Kp[oz], pan, boff[oz], ooff, "blk", (dz[oz2], dz[oz]), owner=True)
+        nop = numpy.array([len(x) for x in ep.ops])
+        fl = 2.0 * float((ncol * dz[oz] * Kz[oz] * nop[ok]).sum())
+        self.d3 = DPanelStage("renorm3", ep.by_class(u, ok[uj]), op_table(ep.base_2, 0, base, 1.0), self.ws.device, fl)
+        self.out_layouts = [None] * ep.nops
+        for l, x in zip(lays, ep.ops):
+            for i in x:
+                self.out_layouts[i] = l
+        self.out_offsets = numpy.empty(ep.nops, dtype=i64)
+        self.out_offsets[ep.order] = base
+        self.ep = ep
+        self.flops = fl + ep.flops1 + (ep.wx.flops if ep.wx is not None else 0.0)
 
     def __call__(self, site_values):
         """site_values: packed site tensor (float64, device) -> new TensorSet."""
         ws = self.ws
+        if self.ep is not None:
+            out = torch.empty(max(self._nout, 1), dtype=torch.float64, device=ws.device)
+            T2, S = self.ep.run(site_values)
+            self.d3.run(T2, S[self.ep.ket_size:], out)
+            return TensorSet(self.out_layouts, out, self.out_offsets)
         T1 = ws.get("r1", self.tot[0], torch.float64)
         T2 = ws.get("r2", self.tot[1], torch.float64)
         out = torch.zeros(max(self.tot[2], 1), dtype=torch.float64, device=ws.device)
@@ -1195,11 +1272,23 @@ class NoiseRDM(object):
     with spin projection, with qkey[:1] then).
     """
 
-    def __init__(self, ws, isite, status, psi_layout, E, W, opers, qkey, dense_idl):
+    def __init__(self, ws, isite, status, psi_layout, E, W, opers, qkey, dense_idl, panels=None):
+        """panels: the panel form (None: on a GPU, where the blocks allow it): T2 of the module
+        envpanels with the rows (l, n1') of one merged class in one panel, whose Gram matrix
+        is one panel GEMM of the panel with itself."""
         self.ws, self.status = ws, status
         dev = ws.device
         groups = _groups(opers, isite, 1)
         nops = len(opers)
+        self.ep = None
+        if panels is None:
+            panels = torch.device(dev).type == "cuda"
+        if panels:
+            try:
+                self._setup_panels(groups, psi_layout, E, W, qkey, dense_idl)
+                return
+            except NoPanelForm:
+                pass
         if status == "L":
             ax = (([2], [0]), ([0, 2], [0, 3]), ([1, 2], [1, 2]))
         else:
@@ -1265,9 +1354,80 @@ class NoiseRDM(object):
         self.prj = torch.from_numpy(out.prjmap(dense_idl)).to(dev) if out is not None else None
         self.ndense = n
 
+    def _setup_panels(self, groups, psi, E, W, qkey, dense_idl):
+        left = self.status == "L"
+        if list(psi.status) != [False, False, True]:
+            raise NoPanelForm
+        i64 = numpy.int64
+        qkey = numpy.asarray(qkey, dtype=numpy.float64)
+        if left:
+            old, qx, qz = 0, psi.qsyms[0], psi.qsyms[2]
+        else:           # the right bond's states carry qkey - q(r) in psi, q(r) in the environment
+            old, qx, qz = 2, qkey - psi.qsyms[2], qkey - psi.qsyms[0]
+        ep = EnvPanels(self.ws, "prdm", groups, psi, old, E, W, left, qx, qz)
+        dx, dz = ep.dx, ep.dz
+        ncls, nx, nz = len(ep.ops), len(dx), len(dz)
+        # merged classes of the rows (x, n'): equal quantum number q(x) + q(n')
+        qm = ep.qx[:, None, :] + numpy.rint(2 * psi.qsyms[1]).astype(i64)[None, :, :]
+        _, mc = numpy.unique(qm.reshape(nx * 4, -1), axis=0, return_inverse=True)
+        mc = mc.ravel()
+        nm = int(mc.max()) + 1
+        o = numpy.argsort(mc, kind="stable")                    # row blocks (x, n') class by class
+        rx, rn, rm = o // 4, o % 4, mc[o]
+        K = numpy.bincount(rm, weights=dx[rx], minlength=nm).astype(i64)
+        cr = numpy.cumsum(dx[rx]) - dx[rx]
+        roff = cr - cr[numpy.searchsorted(rm, rm)]
+        # panel of (operator class, merged class): columns (b, z) sector z by sector z
+        lead = o[numpy.searchsorted(rm, numpy.arange(nm))]      # any row block of the merged class
+        b = ep.b[:, lead // 4, :, lead % 4].transpose(1, 0, 2)  # [class, merged class, z]
+        w = numpy.where(b >= 0, ep.db[numpy.arange(ncls)[:, None, None], numpy.maximum(b, 0)] * dz[None, None, :], 0)
+        coff = numpy.cumsum(w, axis=2) - w
+        wide = w.sum(axis=2)
+        ld = (wide + 3) // 4 * 4
+        sz = ld * K[None, :]
+        pan = numpy.cumsum(sz, axis=1) - sz
+        kk, rr, zz = (v.ravel() for v in numpy.nonzero(b[:, rm, :] >= 0))
+        m = rm[rr]
+        o2 = pan[kk, m] + roff[rr] * ld[kk, m] + coff[kk, m, zz]
+        if len(kk) and not numpy.array_equal(ep.b[kk, rx[rr], zz, rn[rr]], b[kk, m, zz]):
+            raise NoPanelForm
+        ep.finish((kk, rx[rr], zz, 4 * rn[rr], b[kk, m, zz], o2, ld[kk, m], o2 + dx[rx[rr]] * ld[kk, m]),
+                  sz.sum(axis=1), numpy.zeros(0, BPERM_DT), 0)
+        # Gram matrices: K_m x K_m per merged class, one partial result per operator
+        gbase = numpy.cumsum(K * K) - K * K
+        self.size = int((K * K).sum())
+        self.nops = ep.nops
+        rowm, rowi = _ranges(K)
+        crow = gbase[rowm] + rowi * K[rowm]
+        ck, cm = (v.ravel() for v in numpy.nonzero(numpy.ones((ncls, nm), dtype=bool)))
+        r0 = numpy.cumsum(K) - K
+        u, uj = dpanel_units(K[cm], K[cm], wide[ck, cm], ld[ck, cm], ld[ck, cm], pan[ck, cm], pan[ck, cm], r0[cm], "row",
+                             owner=True)
+        fl = 2.0 * float((K[cm] ** 2 * wide[ck, cm] * numpy.array([len(x) for x in ep.ops])[ck]).sum())
+        self.d3 = DPanelStage("prdm3", ep.by_class(u, ck[uj]), op_table(ep.base_2, ep.base_2,
+                                                                        numpy.arange(ep.nops) * self.size, 1.0),
+                              self.ws.device, fl, crow=crow, longest_first=True)
+        # dense position of every row: (l, n1) -> 4 l + n1, (n2, r) -> n2 rdim + r
+        ix = [numpy.asarray(v, dtype=i64) for v in (dense_idl[0] if left else dense_idl[1])]
+        jn = numpy.array([int(v[0]) for v in (dense_idl[1] if left else dense_idl[0])], dtype=i64)
+        nxs = int(dx.sum())
+        pos = numpy.concatenate([ix[x] * 4 + jn[n] if left else jn[n] * nxs + ix[x] for x, n in zip(rx, rn)])
+        d = 4 * nxs
+        own, loc = _ranges(K[rowm])
+        self.prj = torch.from_numpy(pos[own] * d + pos[r0[rowm[own]] + loc]).to(self.ws.device)
+        self.dense_shape = (nxs, 4, nxs, 4) if left else (4, nxs, 4, nxs)
+        self.ndense = d * d
+        self.ep = ep
+        self.flops = fl + ep.flops1 + (ep.wx.flops if ep.wx is not None else 0.0)
+
     def __call__(self, psi_values):
         """psi_values: packed rank-3 wavefunction (device FP64) -> dense noise RDM (d x d)."""
         ws = self.ws
+        if self.ep is not None:
+            P = ws.get("npart", self.nops * self.size, torch.float64)
+            T2, _ = self.ep.run(psi_values)
+            self.d3.run(T2, T2, P)
+            return self._dense(P)
         T1 = ws.get("n1", self.tot[0], torch.float64)
         T2 = ws.get("n2", self.tot[1], torch.float64)
         P = ws.get("npart", self.nops * self.size, torch.float64)
@@ -1280,6 +1440,11 @@ class NoiseRDM(object):
             s[1].run(self.W.values, T1, T2, "f64")
         P[:self.nops * self.size].zero_()
         s[2].run(T2, T2, P, "f64")
+        return self._dense(P)
+
+    def _dense(self, P):
+        """The sum over operators as the dense matrix the decimation uses."""
+        ws = self.ws
         vals = torch.empty(max(self.size, 1), dtype=torch.float64, device=ws.device)[:self.size]
         reduce_ops(P, self.nops, self.size, vals)
         dense = torch.empty(self.ndense, dtype=torch.float64, device=ws.device)

@@ -60,11 +60,16 @@ def interpret_panel(st, A, B, C):
         assert 0 < u["mrem"] <= 128 and 0 < u["nrem"] <= 64
         assert (u["a_off"] + o["a_base"]) % 4 == 0 and (u["b_off"] + o["b_base"]) % 4 == 0 and u["lda"] % 4 == 0
         m, n, k = (numpy.arange(u[x]) for x in ("mrem", "nrem", "K"))
-        am = a[o["a_base"] + u["a_off"] + m[:, None] * u["lda"] + k]
+        blk = st.h_cols is None and st.h_crow is None
+        am = a[o["a_base"] + u["a_off"] + (m[:, None] + k * u["lda"] if blk else m[:, None] * u["lda"] + k)]
         bm = b[o["b_base"] + u["b_off"] + n[:, None] * u["ldb"] + k]
-        if st.h_cols is None:
+        ok = numpy.ones(len(n), dtype=bool)
+        if blk:
+            dr, dc = (int(x) for x in u["pad"][:2])
+            mm = u["m0"] + m[:, None]
+            at = u["c_off"] + mm // dr * dr * dc + (u["n0"] + n) * dr + mm % dr
+        elif st.h_cols is None:
             at = st.h_crow[u["c_off"] + m][:, None] + u["n0"] + n
-            ok = numpy.ones(len(n), dtype=bool)
         else:
             col = st.h_cols[u["c_off"] + n]
             ok = col["off"] >= 0
@@ -76,17 +81,11 @@ def interpret_panel(st, A, B, C):
 
 
 def patch(monkeypatch):
-    from qcmpodmrg_b200 import kernels
     patch_stage_run(monkeypatch)
     monkeypatch.setattr(engine.SparseWStage, "run",
                         lambda self, A, B, C, kind="f64", stream=None: interpret(self, A, C, kind))
     monkeypatch.setattr(engine.DPanelStage, "run", lambda self, A, B, C, stream=None: interpret_panel(self, A, B, C))
 
-    def gather_pad(x, idx, out):
-        out[:len(idx)] = torch.where(idx >= 0, x[idx.clamp(min=0)], torch.zeros((), dtype=x.dtype))
-        return out
-
-    monkeypatch.setattr(kernels, "gather_pad", gather_pad)
 
 
 def sparse_sigma(r, device, sparse_w=True, precision="f64"):
@@ -160,6 +159,57 @@ def test_sparse_plan_of_the_spin_projected_operators(tag, monkeypatch):
             assert numpy.abs(ya - yb).max() <= 1e-12 * max(1.0, numpy.abs(ya).max())
     assert used
     assert used
+
+
+@pytest.mark.parametrize("tag", ["K4", "K5", "K6", "K5N2", "SP_K4", "SP_K5"])
+def test_panel_renormalisation_matches_the_grouped_one(tag, monkeypatch):
+    """Both directions: the same layouts, and values within rounding of the grouped block GEMM.
+    Spin projection's N-only site tensors sum several blocks into one intermediate: they keep
+    the grouped form."""
+    from helpers import record_renormalizer, record_sp_renormalizers
+    from qcmpodmrg_b200 import kernels
+    patch(monkeypatch)
+    rec = (lambda r: record_sp_renormalizers(r, "cpu")) if tag.startswith("SP") else \
+        (lambda r: (lambda x: (x[0], x[1]))(record_renormalizer(r, "cpu")))
+    used = 0
+    make = kernels.Renormalizer.__init__
+    for r in load("kernels_%s.npz" % tag)["records"]:
+        if "renorm_site" not in r:
+            continue
+        ref = rec(r)
+        with monkeypatch.context() as m:
+            m.setattr(kernels.Renormalizer, "__init__", lambda self, *a: make(self, *a, panels=True))
+            new = rec(r)
+        site = torch.from_numpy(ref[-1])
+        for a, b in zip(ref[:-1], new[:-1]):
+            used += b.ep is not None
+            ea, eb = a(site), b(site)
+            for i in range(len(ea.layouts)):
+                assert eb.layouts[i] is ea.layouts[i]
+                va, vb = ea.op_values(i).numpy(), eb.op_values(i).numpy()
+                assert numpy.abs(va - vb).max() <= 1e-13 * max(1.0, numpy.abs(va).max())
+    assert bool(used) != tag.startswith("SP")
+
+
+@pytest.mark.parametrize("tag", ["NZ_K5", "NZ_K6", "NZSP_K5"])
+def test_panel_noise_term_matches_the_grouped_one(tag, monkeypatch):
+    """Both directions: the dense noise matrix within rounding of the grouped block GEMM's."""
+    from helpers import record_noise
+    from qcmpodmrg_b200 import kernels
+    patch(monkeypatch)
+    used = 0
+    make = kernels.NoiseRDM.__init__
+    for r in load("kernels_%s.npz" % tag)["records"]:
+        if "prdm_cimat" not in r:
+            continue
+        ref, vals, _ = record_noise(r, "cpu")
+        with monkeypatch.context() as m:
+            m.setattr(kernels.NoiseRDM, "__init__", lambda self, *a: make(self, *a, panels=True))
+            new = record_noise(r, "cpu")[0]
+        used += new.ep is not None
+        a, b = ref(vals).numpy(), new(vals).numpy()
+        assert a.shape == b.shape and numpy.abs(a - b).max() <= 1e-13 * max(1.0, numpy.abs(a).max())
+    assert bool(used) != ("SP" in tag)
 
 
 def test_changed_mpo_values_are_seen():
