@@ -237,25 +237,24 @@ int qc_dpanel_f64(const void *units, const void *work, long long nwork, const vo
 /* out[i] = x[idx[i]], 0 where idx[i] < 0. */
 int qc_gather_pad_f64(const double *x, const long long *idx, long long n, double *out, void *stream);
 
-/* Sparse two-site MPO stage: T3 = T1 . (W_i W_{i+1}) for every operator (records qc_wxitem /
- * qc_wxdelta / qc_wxgrp / qc_wxdop / qc_wxquad of qc_types.h).  qc_wx_build makes the sparse
+/* Sparse MPO stage: T3 = T1 . (W_i W_{i+1}) for every operator (records qc_wxitem /
+ * qc_wxdelta / qc_wxgrp / qc_wxdop / qc_wxoct of qc_types.h).  qc_wx_build makes the sparse
  * rows of one operator class on the host (w1 / w2: FP64 values, operator o at off1[o] /
  * off2[o]; ns / nd / ioff / allowed: the two layouts), qc_wx_fetch copies them out and frees
- * the handle.  qc_wsparse_*: items of one tile width (fpt fibers per lane: 1, 2 or 4);
- * ent_w: four coefficients per entry as 16-byte vectors (FP64: all first halves, then all
- * second halves, nent apart); maxR / maxQ: most T1 rows / quads of any item's charge
- * difference. */
+ * the handle.  qc_wsparse_*: items of one tile width (32, 64 or 128 fibers); ent_w: the
+ * coefficients in the precision's order (qc_wx_fetch: w64 / w32); maxR / maxO: most T1 rows /
+ * octets of any item's charge difference. */
 int qc_wx_build(int nops, const double *w1, const long long *off1, const int *ns1, const long long *nd1,
                 const long long *ioff1, const int *allowed1, const double *w2, const long long *off2, const int *ns2,
                 const long long *nd2, const long long *ioff2, const int *allowed2, int ndelta, const int *iblk,
-                const int *kblk, const int *row0, const int *R, void **handle, long long *nquads, long long *nents);
-int qc_wx_fetch(void *handle, long long ent0, int quad0, void *dops, void *quads, double *w, int *r);
-int qc_wsparse_f64(const void *items, long long nitems, int fpt, const void *deltas, const void *grps,
-                   const void *rows, const void *dops, const void *quads, const void *ent_w, long long nent,
-                   const void *ent_r, const void *ops, int maxR, int maxQ, const double *A, double *C, void *stream);
-int qc_wsparse_f32(const void *items, long long nitems, int fpt, const void *deltas, const void *grps,
-                   const void *rows, const void *dops, const void *quads, const void *ent_w, long long nent,
-                   const void *ent_r, const void *ops, int maxR, int maxQ, const float *A, float *C, void *stream);
+                const int *kblk, const int *row0, const int *R, void **handle, long long *nocts, long long *nents);
+int qc_wx_fetch(void *handle, long long ent0, int oct0, void *dops, void *octs, double *w64, float *w32, int *r);
+int qc_wsparse_f64(const void *items, long long nitems, int tile, const void *deltas, const void *grps,
+                   const void *rows, const void *dops, const void *octs, const void *ent_w, const void *ent_r,
+                   const void *ops, int maxR, int maxO, const double *A, double *C, void *stream);
+int qc_wsparse_f32(const void *items, long long nitems, int tile, const void *deltas, const void *grps,
+                   const void *rows, const void *dops, const void *octs, const void *ent_w, const void *ent_r,
+                   const void *ops, int maxR, int maxO, const float *A, float *C, void *stream);
 
 /* W panels of the dense fiber-group GEMM assembled from their W blocks (the form the plan
  * compiler emits; the W blocks are those of the pair lists of tensordotSYM for

@@ -193,6 +193,7 @@ class BatchedSigma(object):
         if not parts:
             return [], None
         dels, grps, dops, by = [], [], [], {}
+        kind = "f64" if self.kind == "f64" else "f32"
         nd = ng = nr = no = nq = ne = 0
         for st, base in parts:
             d, o = st.h_deltas.copy(), st.h_dops.copy()
@@ -201,32 +202,30 @@ class BatchedSigma(object):
             d["row_b"] += nr
             d["dop_b"] += no
             o["ent_b"] += ne
-            o["quad_b"] += nq
-            for (fpt, it, _, maxr, maxq) in st.items(self.kind if self.kind == "f64" else "f32"):
+            o["oct_b"] += nq
+            for (tile, it, _, maxr, maxo) in st.items(kind):
                 it = it.copy()
                 it["delta"] += nd
                 it["grp"] += ng
                 for k in ("op_b", "op_e", "op0"):
                     it[k] += base
-                by.setdefault(fpt, []).append((it, maxr, maxq))
+                by.setdefault(tile, []).append((it, maxr, maxo))
             dels.append(d)
             grps.append(st.h_groups)
             dops.append(o)
             nd, ng, nr = nd + len(d), ng + len(st.h_groups), nr + len(st.h_rows)
-            no, nq, ne = no + len(o), nq + len(st.h_quads), ne + len(st.h_ent_r)
+            no, nq, ne = no + len(o), nq + len(st.h_octs), ne + len(st.h_ent_r)
         sts = [st for st, _ in parts]
         up = lambda a: upload(a if len(a) else numpy.zeros(1, a.dtype), self.device)       # noqa: E731
-        cat = lambda name, dt: up(numpy.concatenate([getattr(st, name) for st in sts]).astype(dt, copy=False))  # noqa: E731
-        w = numpy.concatenate([st.h_ent_w for st in sts]) if ne else numpy.zeros((1, 4))
-        w = w.reshape(-1, 2, 2).transpose(1, 0, 2) if self.kind == "f64" else w.astype(numpy.float32)
+        cat = lambda get: up(numpy.concatenate([get(st) for st in sts]))                   # noqa: E731
         rec = {"deltas": up(numpy.concatenate(dels)), "groups": up(numpy.concatenate(grps)),
-               "rows": cat("h_rows", numpy.int32), "dops": up(numpy.concatenate(dops)),
-               "quads": cat("h_quads", sts[0].h_quads.dtype), "ent_r": cat("h_ent_r", numpy.int32),
-               "w": upload(w, self.device), "nent": ne}
+               "rows": cat(lambda st: st.h_rows), "dops": up(numpy.concatenate(dops)),
+               "octs": cat(lambda st: st.h_octs), "ent_r": cat(lambda st: st.h_ent_r),
+               "w": cat(lambda st: st.h_w[kind])}
         launches = []
-        for fpt, xs in sorted(by.items(), reverse=True):
+        for tile, xs in sorted(by.items(), reverse=True):
             it = numpy.concatenate([x[0] for x in xs])
-            launches.append((fpt, len(it), up(it), max(x[1] for x in xs), max(x[2] for x in xs)))
+            launches.append((tile, len(it), up(it), max(x[1] for x in xs), max(x[2] for x in xs)))
         return launches, rec
 
     def _launch_all(self):
@@ -248,13 +247,12 @@ class BatchedSigma(object):
                 check(ffn(dt.data_ptr(), nt, span, dfi.data_ptr(), dfo.data_ptr(), dfp.data_ptr(),
                           self.d_ops[si].data_ptr(), mr, tile, None, None, None, s), "batched qc_fiber")
                 LOG.launches += 1
-            for (fpt, nt, dt, maxr, maxq) in self.sparse_launches if stage == 4 else []:
+            for (tile, nt, dt, maxr, maxo) in self.sparse_launches if stage == 4 else []:
                 wfn = lib.qc_wsparse_f64 if self.kind == "f64" else lib.qc_wsparse_f32
                 r = self.sparse
-                check(wfn(dt.data_ptr(), nt, fpt, r["deltas"].data_ptr(), r["groups"].data_ptr(), r["rows"].data_ptr(),
-                          r["dops"].data_ptr(), r["quads"].data_ptr(), r["w"].data_ptr(), r["nent"],
-                          r["ent_r"].data_ptr(), self.d_ops[4].data_ptr(), maxr, maxq, None, None, s),
-                      "batched qc_wsparse")
+                check(wfn(dt.data_ptr(), nt, tile, r["deltas"].data_ptr(), r["groups"].data_ptr(), r["rows"].data_ptr(),
+                          r["dops"].data_ptr(), r["octs"].data_ptr(), r["w"].data_ptr(), r["ent_r"].data_ptr(),
+                          self.d_ops[4].data_ptr(), maxr, maxo, None, None, s), "batched qc_wsparse")
                 LOG.launches += 1
             for (si, cfg, nt, span, dt, dc) in self.launches:
                 if si != stage:

@@ -246,17 +246,17 @@ struct alignas(16) qc_wxitem {
 static_assert(sizeof(qc_wxitem) == 32, "qc_wxitem is 32 bytes");
 
 struct alignas(16) qc_wxdop {
-  long long ent_b;     // first entry
-  int quad_b, nquad;   // quads (four consecutive rows k of one T3 block)
+  long long ent_b;     // first entry (a multiple of four)
+  int oct_b, noct;     // octets (eight rows k)
 };
 static_assert(sizeof(qc_wxdop) == 16, "qc_wxdop is 16 bytes");
 
-struct alignas(16) qc_wxquad {
-  int ent, cnt;        // entries ent_b + [ent, ent + cnt): a T1 row and its four coefficients
-  int blk;             // T3 block 4 n1' + n2'
-  int c0nc;            // first c << 8 | rows (1 .. 4)
+struct alignas(16) qc_wxoct {
+  int ent, cnt;        // entries ent_b + [ent, ent + cnt), cnt a multiple of four: a T1 row (R .. R + 3: zero)
+  int pad0, pad1;      //   and its eight coefficients
+  int row[8];          // T3 row: block 4 n1' + n2' << 16 | c, -1: none
 };
-static_assert(sizeof(qc_wxquad) == 16, "qc_wxquad is 16 bytes");
+static_assert(sizeof(qc_wxoct) == 48, "qc_wxoct is 48 bytes");
 
 // ---- FP64 panel GEMM on the tensor pipe (k_dpanel) ---------------------------------
 // One unit = one tile of at most 128 rows x 64 columns of one operator class,

@@ -7,20 +7,22 @@
 // every fiber of one charge difference q(l) - q(r) meets the same S.  An ab-initio MPO
 // fills about a tenth of the blocks of S that symmetry allows (K = 24: 20 310 of 230 000
 // elements per operator, 13 per row k, against 74 multiply-adds per element of the two
-// dense block contractions), so S is kept as a list: for every quad of four consecutive
-// rows k, the T1 rows that any of the four reads and their four coefficients.
+// dense block contractions), so S is kept as lists: rows k of like pattern in octets, and for
+// every octet the T1 rows that any of the eight reads with their eight coefficients.
 //
-// One CTA takes a tile of 32 * FPT fibers of one charge difference (fibers of several
+// One CTA takes a tile of 32, 64 or 128 fibers of one charge difference (fibers of several
 // sector pairs share a tile, so small sectors fill the lanes) and walks operators: the
-// tile's T1 rows are staged in shared memory (cp.async, rows contiguous over fibers), a
-// warp takes quads of S, lane = fiber, and every entry is one broadcast of (row,
-// coefficients) against one conflict-free row read for 4 * FPT FMAs.  T3 keeps r as its
-// fastest index, so results leave as contiguous rows straight from registers.
+// tile's T1 rows are staged in shared memory (cp.async, rows contiguous over fibers), then
+// every warp takes octets of S.  T3 keeps r as its fastest index, so results leave as
+// contiguous rows straight from registers.  Two CTAs share an SM: one loads while the
+// other multiplies.
 //
-// Bound: T1 read and T3 written once.  Mid-chain dot of K=24, D=500 (1.22e9 elements each):
-// FP64 8.1 ms, 2.4 TB/s, against 30.2 ms of the two dense stages; FP32 4.6 ms, 2.1 TB/s,
-// against 15.5 ms.  The shared-memory pipe (72 % of its wavefronts: row reads and
-// coefficient broadcasts) and the issue slots (71 %) bound it, not HBM.
+// Bound: T1 read and T3 written once.  Mid-chain dot of K=24, D=500 (1.22e9 elements each: 19.5 GB
+// in FP64, 3.0 ms, and half of that in FP32): two dense stages took 30.2 ms in FP64 and 15.5 ms in
+// FP32, lists of four consecutive rows on scalar multiply-adds 8.1 and 4.6 ms (shared-memory pipe
+// 72 % busy: a row read and a coefficient broadcast for every four rows), octets of like rows
+// 6.0 and 4.05 ms (D = 200: 1.37 -> 1.00, 0.78 -> 0.71 ms).  FP32 is still bound by the shared-memory
+// pipe (75 %); copying alone takes 2.2 and 1.3 ms of it.  Twelve warps of deeper prefetch: 5.99, 4.11.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
@@ -33,9 +35,10 @@
 
 namespace {
 
-constexpr int WX_WARPS = 8;
+constexpr int WX_WARPS = 16;
 constexpr int WX_THREADS = 32 * WX_WARPS;
-constexpr int WX_MAXQ = 1024;             // quads of one (delta, operator)
+constexpr int WX_MAXOCT = 512;            // octets of one (delta, operator)
+constexpr int WX_GRPS = 32;               // sector pairs of one tile
 
 __device__ __forceinline__ void cp_async_el(float *dst, const float *src, bool valid) {
   const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
@@ -50,94 +53,52 @@ __device__ __forceinline__ void cp_async_16(void *dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 
-// The four coefficients of an entry: 16-byte vectors, one in FP32 and two in FP64, kept as
-// separate arrays (half h of entry e at [h * n + e]) so that 32 lanes move them without bank
-// conflicts and one broadcast load reads one.
-template <typename T>
-struct Coef;
-template <>
-struct Coef<float> {
-  typedef float4 V;
-  static constexpr int NV = 1;
-  static __device__ __forceinline__ void get(const float4 *p, int, int e, float (&w)[4]) {
-    const float4 x = p[e];
-    w[0] = x.x;
-    w[1] = x.y;
-    w[2] = x.z;
-    w[3] = x.w;
-  }
-  static __device__ __forceinline__ float4 zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
-};
-template <>
-struct Coef<double> {
-  typedef double2 V;
-  static constexpr int NV = 2;
-  static __device__ __forceinline__ void get(const double2 *p, int n, int e, double (&w)[4]) {
-    const double2 x = p[e], y = p[n + e];
-    w[0] = x.x;
-    w[1] = x.y;
-    w[2] = y.x;
-    w[3] = y.y;
-  }
-  static __device__ __forceinline__ double2 zero() { return make_double2(0.0, 0.0); }
-};
+// Row pitch of the staged tile: FP32 lanes read consecutive fibers of one row; an FP64
+// fragment reads eight fibers of four rows, which touch every bank once when the rows differ
+// mod 4 (the entry lists are ordered that way) and the pitch is 4 mod 16.
+template <typename T, int FT>
+__host__ __device__ constexpr int wx_pitch() { return sizeof(T) == 8 ? FT + 4 : FT; }
 
-template <typename T, int FPT>
-__host__ __device__ constexpr size_t wx_fixed_smem() {
-  return 34 * 32 * FPT * sizeof(int) +                                             // tabA, tabC, fibF, fibO
-         (size_t)WX_WARPS * 32 * (16 * Coef<T>::NV + sizeof(int));                // entry rings
+// A warp's units of work: (octet, group of GW of the tile's fibers), octets by decreasing
+// length; every other pass over the warps runs backwards, which evens out their loads.
+__device__ __forceinline__ int wx_unit(int pass, int warp) {
+  return pass * WX_WARPS + ((pass & 1) ? WX_WARPS - 1 - warp : warp);
 }
 
-template <typename T, int FPT>
-__global__ void __launch_bounds__(WX_THREADS)
-k_wsparse(const qc_wxitem *__restrict__ items, const qc_wxdelta *__restrict__ deltas,
-          const qc_wxgrp *__restrict__ grps, const int *__restrict__ rows, const qc_wxdop *__restrict__ dops,
-          const qc_wxquad *__restrict__ quads, const typename Coef<T>::V *__restrict__ ent_w, long long nent,
-          const int *__restrict__ ent_r, const qc_op *__restrict__ ops, int maxR, int maxQ, const T *__restrict__ A,
-          T *__restrict__ C) {
-  typedef typename Coef<T>::V V;
-  constexpr int NV = Coef<T>::NV;
-  constexpr int FT = 32 * FPT;
-  extern __shared__ __align__(16) unsigned char wx_smem[];
-  T *const As = reinterpret_cast<T *>(wx_smem);                                  // [R + 1][FT], row R zero
-  V *const ring_w0 = reinterpret_cast<V *>(As + (size_t)(maxR + 1) * FT);       // [warps][NV][32]
-  qc_wxquad *const sq = reinterpret_cast<qc_wxquad *>(ring_w0 + WX_WARPS * NV * 32);  // [maxQ]
-  int *const ring_r0 = reinterpret_cast<int *>(sq + maxQ);                       // [warps][32]
-  int *const tabA = ring_r0 + WX_WARPS * 32;                                     // [16][FT]
-  int *const tabC = tabA + 16 * FT;                                              // [16][FT]
-  int *const fibF = tabC + 16 * FT;                                              // [FT]
-  int *const fibO = fibF + FT;                                                   // [FT]
-  int *const rowt = fibO + FT;                                                   // [maxR]
-  __shared__ int s_start[FT + 1];
-  __shared__ int s_grp[FT], s_f[FT];
+// Offsets of a tile's fibers: T1 block (n1, n2) and T3 block (n1', n2') of every fiber (-1: absent,
+// or past the tile), its T1 row stride F and its T3 row stride D_r.
+template <int FT>
+struct alignas(16) WxTile {
+  int a[16][FT], c[16][FT];
+  int F[FT], flo[FT];
+};
 
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const qc_wxitem it = items[blockIdx.x];
-  const qc_wxdelta *const dl = deltas + it.delta;
-  const int R = dl->R, row_b = dl->row_b, grp_e = dl->grp_e, dop_b = dl->dop_b;
+template <typename T, int FT>
+__host__ __device__ constexpr size_t wx_fixed_smem() {
+  return sizeof(WxTile<FT>) + (sizeof(T) == 4 ? (size_t)WX_WARPS * 32 * 36 : 0);     // FP32: entry rings
+}
 
-  // ---- the tile's fibers: sector pair and fiber in it, then their block offsets
-  for (int t = tid; t <= FT; t += WX_THREADS) {
-    const int g = it.grp + t;
-    s_start[t] = g < grp_e ? grps[g].start : 0x7fffffff;
-  }
-  for (int r = tid; r < R; r += WX_THREADS) rowt[r] = rows[row_b + r];
+template <int FT>
+__device__ __forceinline__ void wx_open_tile(WxTile<FT> &w, const qc_wxitem &it, const qc_wxgrp *__restrict__ grps,
+                                             int grp_e) {
+  __shared__ int s_start[WX_GRPS + 1], s_slot[FT], s_f[FT];
+  const int tid = threadIdx.x;
+  for (int t = tid; t <= WX_GRPS; t += WX_THREADS)
+    s_start[t] = (t < WX_GRPS && it.grp + t < grp_e) ? grps[it.grp + t].start : 0x7fffffff;
   __syncthreads();
   for (int t = tid; t < FT; t += WX_THREADS) {
     const int pos = s_start[0] + it.f0 + t;
-    int lo = 0, hi = FT;                       // largest k with s_start[k] <= pos
+    int lo = 0, hi = WX_GRPS - 1;                // largest k with start[k] <= pos
     while (lo < hi) {
       const int m = (lo + hi + 1) >> 1;
       if (s_start[m] <= pos) lo = m; else hi = m - 1;
     }
-    s_grp[t] = t < it.nf ? it.grp + lo : -1;
+    s_slot[t] = t < it.nf ? it.grp + lo : -1;
     s_f[t] = pos - s_start[lo];
-    As[R * FT + t] = T(0);
   }
   __syncthreads();
   for (int e = tid; e < 16 * FT; e += WX_THREADS) {
-    const int b = e / FT, t = e - b * FT;
-    const int g = s_grp[t];
+    const int b = e / FT, t = e - b * FT, g = s_slot[t];
     int oa = -1, oc = -1;
     if (g >= 0) {
       const qc_wxgrp *gr = grps + g;
@@ -147,140 +108,309 @@ k_wsparse(const qc_wxitem *__restrict__ items, const qc_wxdelta *__restrict__ de
       oc = gr->c[b];
       if (oc >= 0) oc += (f / flo) * gr->h[b] + f % flo;
       if (b == 0) {
-        fibF[t] = gr->F;
-        fibO[t] = flo;
+        w.F[t] = gr->F;
+        w.flo[t] = flo;
       }
     } else if (b == 0) {
-      fibF[t] = fibO[t] = 0;
+      w.F[t] = w.flo[t] = 0;
     }
-    tabA[e] = oa;
-    tabC[e] = oc;
+    w.a[b][t] = oa;
+    w.c[b][t] = oc;
   }
   __syncthreads();
+}
 
-  V *const ring_w = ring_w0 + warp * NV * 32;
-  int *const ring_r = ring_r0 + warp * 32;
+// The tile's T1 rows and the operator's octet records on their way to shared memory.
+template <typename T, int FT>
+__device__ __forceinline__ void wx_stage(const WxTile<FT> &w, const int *rowt, int R, const T *Ao, T *As,
+                                         const qc_wxoct *go, qc_wxoct *so, int no) {
+  constexpr int P = wx_pitch<T, FT>();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int F[FT / 32];
+#pragma unroll
+  for (int j = 0; j < FT / 32; ++j) F[j] = w.F[lane + 32 * j];
+#pragma unroll 2
+  for (int r = warp; r < R; r += WX_WARPS) {
+    const int rec = rowt[r], a = rec & 0xffff;
+    const int *ta = w.a[rec >> 16] + lane;
+#pragma unroll
+    for (int j = 0; j < FT / 32; ++j) {
+      const int off = ta[32 * j];
+      cp_async_el(As + r * P + lane + 32 * j, Ao + (off >= 0 ? off + a * F[j] : 0), off >= 0);
+    }
+  }
+  for (int e = threadIdx.x; e < no * (int)(sizeof(qc_wxoct) / 16); e += WX_THREADS)
+    cp_async_16(reinterpret_cast<char *>(so) + 16 * e, reinterpret_cast<const char *>(go) + 16 * e);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+__device__ __forceinline__ void wx_ffma2(unsigned long long &c, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+}
+
+// FP32: lane = fiber (FT / 32 of them); an entry is one row read per fiber against eight
+// broadcast coefficients, packed in pairs (fma.rn.f32x2: two multiply-adds an issue slot).
+template <int FT, int GW>
+__global__ void __launch_bounds__(WX_THREADS, 2)
+k_wsparse_f32(const qc_wxitem *__restrict__ items, const qc_wxdelta *__restrict__ deltas,
+              const qc_wxgrp *__restrict__ grps, const int *__restrict__ rows, const qc_wxdop *__restrict__ dops,
+              const qc_wxoct *__restrict__ octs, const float4 *__restrict__ ent_w, const int *__restrict__ ent_r,
+              const qc_op *__restrict__ ops, int maxR, int maxO, const float *__restrict__ A, float *__restrict__ C) {
+  constexpr int NJ = GW / 32, NG = FT / GW;
+  extern __shared__ __align__(16) unsigned char wx_smem[];
+  WxTile<FT> &w = *reinterpret_cast<WxTile<FT> *>(wx_smem);
+  float4 *const ring0 = reinterpret_cast<float4 *>(&w + 1);                            // [warps][2][32]
+  int *const ringr0 = reinterpret_cast<int *>(ring0 + WX_WARPS * 64);                  // [warps][32]
+  qc_wxoct *const so = reinterpret_cast<qc_wxoct *>(ringr0 + WX_WARPS * 32);           // [maxO]
+  float *const As = reinterpret_cast<float *>(so + maxO);                              // [R + 4][FT], last rows zero
+  int *const rowt = reinterpret_cast<int *>(As + (size_t)(maxR + 4) * FT);            // [maxR]
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const qc_wxitem it = items[blockIdx.x];
+  const qc_wxdelta *const dl = deltas + it.delta;
+  const int R = dl->R, dop_b = dl->dop_b;
+  for (int r = tid; r < R; r += WX_THREADS) rowt[r] = rows[dl->row_b + r];
+  for (int t = tid; t < 4 * FT; t += WX_THREADS) As[R * FT + t] = 0.f;
+  wx_open_tile<FT>(w, it, grps, dl->grp_e);
+  float4 *const ring = ring0 + warp * 64;
+  int *const ringr = ringr0 + warp * 32;
   for (int op = it.op_b; op < it.op_e; ++op) {
     const qc_op o = ops[op];
     const qc_wxdop dop = dops[dop_b + op - it.op0];
-    const T *const Ao = A + o.a_base;
-    T *const Co = C + o.c_base;
-    const V *const ew = ent_w + dop.ent_b;
+    const int no = dop.noct;
+    const qc_wxoct *const go = octs + dop.oct_b;
+    wx_stage<float, FT>(w, rowt, R, A + o.a_base, As, go, so, no);
+    const float4 *const ew = ent_w + 2 * dop.ent_b;
     const int *const er = ent_r + dop.ent_b;
-    const qc_wxquad *const gq = quads + dop.quad_b;
-    const int nq = dop.nquad;
-    // ---- stage the tile's T1 rows and the operator's quad records
-    for (int r = warp; r < R; r += WX_WARPS) {
-      const int rec = rowt[r];
-      const int *ta = tabA + (rec >> 16) * FT;
-      const int a = rec & 0xffff;
-#pragma unroll
-      for (int j = 0; j < FPT; ++j) {
-        const int f = lane + 32 * j;
-        const int off = ta[f];
-        cp_async_el(As + r * FT + f, off >= 0 ? Ao + off + (long long)a * fibF[f] : A, off >= 0);
-      }
-    }
-    for (int e = tid; e < nq; e += WX_THREADS) cp_async_16(sq + e, gq + e);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    // the warp's first quad and its first entries, while the rows are in flight; lanes past
-    // the end hold the zero row with zero coefficients
-    V pw[NV];
-    int pr;
-    auto fetch = [&](const qc_wxquad &x, int c0) {
-#pragma unroll
-      for (int h = 0; h < NV; ++h) pw[h] = Coef<T>::zero();
-      pr = R;
-      if (c0 + lane < x.cnt) {
-#pragma unroll
-        for (int h = 0; h < NV; ++h) pw[h] = ew[h * nent + x.ent + c0 + lane];
-        pr = er[x.ent + c0 + lane];
+    float *const Co = C + o.c_base;
+    // the warp's first octet and its first entries, while the rows are in flight (a list's
+    // length is a multiple of four: it ends in zero rows with zero coefficients)
+    float4 p0, p1;
+    int pr = 0;
+    auto fetch = [&](int first, int cnt) {
+      if (lane < cnt) {
+        p0 = ew[2 * (first + lane)];
+        p1 = ew[2 * (first + lane) + 1];
+        pr = er[first + lane];
       }
     };
-    int q = warp;
-    qc_wxquad cur;
-    if (q < nq) {
-      cur = gq[q];
-      fetch(cur, 0);
+    const int nu = no * NG;
+    int pass = 0, u = wx_unit(0, warp), ent = 0, cnt = 0;
+    if (u < nu) {
+      ent = go[u / NG].ent;
+      cnt = go[u / NG].cnt;
+      fetch(ent, cnt);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    while (q < nq) {
-      const qc_wxquad cq = cur;
-      const int qn = q + WX_WARPS;
-      if (qn < nq) cur = sq[qn];
-      T acc[4][FPT];
+    while (u < nu) {
+      const int q = u / NG, g0 = (u % NG) * GW + lane, n0 = cnt;
+      int e0 = ent;
+      u = wx_unit(++pass, warp);
+      if (u < nu) {
+        ent = so[u / NG].ent;
+        cnt = so[u / NG].cnt;
+      } else {
+        cnt = 0;
+      }
+      unsigned long long acc[4][NJ];
 #pragma unroll
       for (int k = 0; k < 4; ++k)
 #pragma unroll
-        for (int j = 0; j < FPT; ++j) acc[k][j] = T(0);
-      for (int c0 = 0;; c0 += 32) {
-        const int n = min(32, cq.cnt - c0);
-#pragma unroll
-        for (int h = 0; h < NV; ++h) ring_w[32 * h + lane] = pw[h];
-        ring_r[lane] = pr * FT;
+        for (int j = 0; j < NJ; ++j) acc[k][j] = 0ull;
+      for (int left = n0;;) {
+        const int n = min(32, left);
+        ring[lane] = p0;
+        ring[32 + lane] = p1;
+        ringr[lane] = pr * FT;
         __syncwarp();
-        const bool more = c0 + 32 < cq.cnt;
-        if (more)
-          fetch(cq, c0 + 32);
-        else if (qn < nq)
-          fetch(cur, 0);
+        left -= n;
+        e0 += n;
+        if (left > 0)
+          fetch(e0, left);
+        else
+          fetch(ent, cnt);
         for (int e = 0; e < n; e += 4) {
-          const int4 r4 = *reinterpret_cast<const int4 *>(ring_r + e);
+          const int4 r4 = *reinterpret_cast<const int4 *>(ringr + e);
           const int rr[4] = {r4.x, r4.y, r4.z, r4.w};
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            T w[4], av[FPT];
-            Coef<T>::get(ring_w, 32, e + u, w);
-            const T *a = As + rr[u] + lane;
+          for (int x = 0; x < 4; ++x) {
+            const ulonglong2 wl = *reinterpret_cast<const ulonglong2 *>(ring + e + x);
+            const ulonglong2 wh = *reinterpret_cast<const ulonglong2 *>(ring + 32 + e + x);
+            const float *a = As + rr[x] + g0;
 #pragma unroll
-            for (int j = 0; j < FPT; ++j) av[j] = a[32 * j];
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-#pragma unroll
-              for (int j = 0; j < FPT; ++j) acc[k][j] = fma(w[k], av[j], acc[k][j]);
+            for (int j = 0; j < NJ; ++j) {
+              const float v = a[32 * j];
+              unsigned long long vv;
+              asm("mov.b64 %0, {%1, %1};" : "=l"(vv) : "f"(v));
+              wx_ffma2(acc[0][j], wl.x, vv);
+              wx_ffma2(acc[1][j], wl.y, vv);
+              wx_ffma2(acc[2][j], wh.x, vv);
+              wx_ffma2(acc[3][j], wh.y, vv);
+            }
           }
         }
         __syncwarp();
-        if (!more) break;
+        if (left <= 0) break;
       }
-      // ---- four rows of the block: fibers of one l are contiguous
-      const int *tc = tabC + cq.blk * FT;
-      const int nc = cq.c0nc & 0xff, cfirst = cq.c0nc >> 8;
+      // ---- eight rows, each of its own block; fibers of one l are contiguous
+      int fl[NJ];
 #pragma unroll
-      for (int j = 0; j < FPT; ++j) {
-        const int off = tc[lane + 32 * j], fl = fibO[lane + 32 * j];
-        if (off >= 0) {
-          T *dst = Co + off + (long long)cfirst * fl;
+      for (int j = 0; j < NJ; ++j) fl[j] = w.flo[g0 + 32 * j];
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (k < nc) dst[(long long)k * fl] = acc[k][j];
+      for (int k = 0; k < 8; ++k) {
+        const int row = so[q].row[k];
+        if (row < 0) break;
+        const int *tc = w.c[row >> 16] + g0;
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          const int off = tc[32 * j];
+          if (off >= 0)
+            Co[off + (row & 0xffff) * fl[j]] = __uint_as_float((unsigned)(acc[k >> 1][j] >> (k & 1 ? 32 : 0)));
         }
       }
-      q = qn;
     }
     __syncthreads();
   }
 }
 
-template <typename T, int FPT>
-size_t wx_smem_bytes(int maxR, int maxQ) {
-  return (size_t)(maxR + 1) * 32 * FPT * sizeof(T) + (size_t)maxQ * sizeof(qc_wxquad) + (size_t)maxR * sizeof(int) +
-         wx_fixed_smem<T, FPT>();
+// FP64: an octet's four entries against eight fibers are one m8n8k4 product on the FP64
+// tensor pipe (T1 rows x coefficients); the coefficients come from global memory in fragment
+// order, one value per lane, three steps ahead.
+template <int FT>
+__global__ void __launch_bounds__(WX_THREADS, 2)
+k_wsparse_f64(const qc_wxitem *__restrict__ items, const qc_wxdelta *__restrict__ deltas,
+              const qc_wxgrp *__restrict__ grps, const int *__restrict__ rows, const qc_wxdop *__restrict__ dops,
+              const qc_wxoct *__restrict__ octs, const double *__restrict__ ent_w, const int *__restrict__ ent_r,
+              const qc_op *__restrict__ ops, int maxR, int maxO, const double *__restrict__ A,
+              double *__restrict__ C) {
+  constexpr int GW = 32, NG = FT / GW, NT = GW / 8, P = wx_pitch<double, FT>();
+  extern __shared__ __align__(16) unsigned char wx_smem[];
+  WxTile<FT> &w = *reinterpret_cast<WxTile<FT> *>(wx_smem);
+  qc_wxoct *const so = reinterpret_cast<qc_wxoct *>(&w + 1);                           // [maxO]
+  double *const As = reinterpret_cast<double *>(so + maxO);                            // [R + 4][P], last rows zero
+  int *const rowt = reinterpret_cast<int *>(As + (size_t)(maxR + 4) * P);             // [maxR]
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int gr = lane >> 2, gk = lane & 3;
+  const qc_wxitem it = items[blockIdx.x];
+  const qc_wxdelta *const dl = deltas + it.delta;
+  const int R = dl->R, dop_b = dl->dop_b;
+  for (int r = tid; r < R; r += WX_THREADS) rowt[r] = rows[dl->row_b + r];
+  for (int t = tid; t < 4 * P; t += WX_THREADS) As[R * P + t] = 0.0;
+  wx_open_tile<FT>(w, it, grps, dl->grp_e);
+  for (int op = it.op_b; op < it.op_e; ++op) {
+    const qc_op o = ops[op];
+    const qc_wxdop dop = dops[dop_b + op - it.op0];
+    const int no = dop.noct;
+    const qc_wxoct *const go = octs + dop.oct_b;
+    wx_stage<double, FT>(w, rowt, R, A + o.a_base, As, go, so, no);
+    const double *const ew = ent_w + 8 * dop.ent_b + lane;       // step s: [32 s]
+    const int *const er = ent_r + dop.ent_b + gk;                // step s: [4 s]
+    double *const Co = C + o.c_base;
+    // the stream of this warp's steps, unit after unit, three steps ahead (an octet has one at
+    // least: fe counts steps from the operator's first, fl ends the current unit's)
+    const qc_wxoct *fo = go;                     // records: global memory until the staged ones are in
+    const int nu = no * NG;
+    int fp = 0, fu = wx_unit(0, warp), fe = 0, fl = 0;
+    if (fu < nu) {
+      fe = go[fu / NG].ent >> 2;
+      fl = fe + (go[fu / NG].cnt >> 2);
+    }
+    auto fetch = [&](double &wv, int &rv) {
+      if (fe < fl) {
+        wv = ew[32 * fe];
+        rv = er[4 * fe];
+        if (++fe == fl) {
+          fu = wx_unit(++fp, warp);
+          if (fu < nu) {
+            fe = fo[fu / NG].ent >> 2;
+            fl = fe + (fo[fu / NG].cnt >> 2);
+          }
+        }
+      }
+    };
+    double w0 = 0.0, w1 = 0.0, w2 = 0.0;
+    int r0 = R, r1 = R, r2 = R;
+    fetch(w0, r0);
+    fetch(w1, r1);
+    fetch(w2, r2);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    fo = so;
+    int pass = 0, u = wx_unit(0, warp), left = 0, g0 = 0;
+    double acc[NT][2];
+    auto open_unit = [&]() {
+      if (u < nu) {
+        left = so[u / NG].cnt >> 2;
+        g0 = (u % NG) * GW + gr;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = 0.0;
+      }
+    };
+    auto step = [&](double wv, int r) {
+      const double *a = As + r * P + g0;
+      double av[NT];
+#pragma unroll
+      for (int t = 0; t < NT; ++t) av[t] = a[8 * t];
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                     : "+d"(acc[t][0]), "+d"(acc[t][1])
+                     : "d"(av[t]), "d"(wv));
+      if (--left == 0) {
+        // lane: fiber 8 t + lane / 4 of every t, rows 2 (lane % 4) and the next one
+        const qc_wxoct &x = so[u / NG];
+        const int ra = x.row[2 * gk], rb = x.row[2 * gk + 1];
+        const int *ta = w.c[max(ra, 0) >> 16] + g0, *tb = w.c[max(rb, 0) >> 16] + g0;
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          const int fl = w.flo[g0 + 8 * t], oa = ta[8 * t], ob = tb[8 * t];
+          if (ra >= 0 && oa >= 0) Co[oa + (ra & 0xffff) * fl] = acc[t][0];
+          if (rb >= 0 && ob >= 0) Co[ob + (rb & 0xffff) * fl] = acc[t][1];
+        }
+        u = wx_unit(++pass, warp);
+        open_unit();
+      }
+    };
+    open_unit();
+    // each of the three prefetched steps keeps its registers: a copy would wait for its load
+    while (u < nu) {
+      step(w0, r0);
+      fetch(w0, r0);
+      if (u >= nu) break;
+      step(w1, r1);
+      fetch(w1, r1);
+      if (u >= nu) break;
+      step(w2, r2);
+      fetch(w2, r2);
+    }
+    __syncthreads();
+  }
 }
 
-template <typename T, int FPT>
-int launch_fpt(const void *items, long long nitems, const void *deltas, const void *grps, const void *rows,
-               const void *dops, const void *quads, const void *ent_w, long long nent, const void *ent_r,
-               const void *ops, int maxR, int maxQ, const T *A, T *C, cudaStream_t s) {
-  const size_t smem = wx_smem_bytes<T, FPT>(maxR, maxQ);
+template <typename T, int FT>
+size_t wx_smem_bytes(int maxR, int maxO) {
+  return (size_t)(maxR + 4) * wx_pitch<T, FT>() * sizeof(T) + (size_t)maxO * sizeof(qc_wxoct) +
+         (size_t)maxR * sizeof(int) + wx_fixed_smem<T, FT>();
+}
+
+struct WxArgs {
+  const void *items;
+  long long nitems;
+  const void *deltas, *grps, *rows, *dops, *octs, *ent_w, *ent_r, *ops;
+  int maxR, maxO;
+};
+
+template <typename T, typename W, typename K>
+int launch_kernel(K kernel, size_t smem, const WxArgs &x, const T *A, T *C, cudaStream_t s) {
   if (smem > 224 * 1024) return QC_ERR_ARG;
-  cudaError_t e = cudaFuncSetAttribute(k_wsparse<T, FPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess) {
-    k_wsparse<T, FPT><<<(unsigned)nitems, WX_THREADS, smem, s>>>(
-        (const qc_wxitem *)items, (const qc_wxdelta *)deltas, (const qc_wxgrp *)grps, (const int *)rows,
-        (const qc_wxdop *)dops, (const qc_wxquad *)quads, (const typename Coef<T>::V *)ent_w, nent,
-        (const int *)ent_r, (const qc_op *)ops, maxR, maxQ, A, C);
+    kernel<<<(unsigned)x.nitems, WX_THREADS, smem, s>>>(
+        (const qc_wxitem *)x.items, (const qc_wxdelta *)x.deltas, (const qc_wxgrp *)x.grps, (const int *)x.rows,
+        (const qc_wxdop *)x.dops, (const qc_wxoct *)x.octs, (const W *)x.ent_w, (const int *)x.ent_r,
+        (const qc_op *)x.ops, x.maxR, x.maxO, A, C);
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) {
@@ -290,20 +420,9 @@ int launch_fpt(const void *items, long long nitems, const void *deltas, const vo
   return QC_OK;
 }
 
-template <typename T>
-int launch_wsparse(const void *items, long long nitems, int fpt, const void *deltas, const void *grps,
-                   const void *rows, const void *dops, const void *quads, const void *ent_w, long long nent,
-                   const void *ent_r, const void *ops, int maxR, int maxQ, const T *A, T *C, cudaStream_t s) {
-  if (nitems <= 0) return QC_OK;
-  if (nitems > 0x7fffffffLL || !items || !deltas || !grps || !rows || !dops || !quads || !ent_w || !ent_r || !ops ||
-      maxR < 0 || maxQ < 0 || maxQ > WX_MAXQ || nent < 0)
-    return QC_ERR_ARG;
-  switch (fpt) {
-    case 1: return launch_fpt<T, 1>(items, nitems, deltas, grps, rows, dops, quads, ent_w, nent, ent_r, ops, maxR, maxQ, A, C, s);
-    case 2: return launch_fpt<T, 2>(items, nitems, deltas, grps, rows, dops, quads, ent_w, nent, ent_r, ops, maxR, maxQ, A, C, s);
-    case 4: return launch_fpt<T, 4>(items, nitems, deltas, grps, rows, dops, quads, ent_w, nent, ent_r, ops, maxR, maxQ, A, C, s);
-    default: return QC_ERR_ARG;
-  }
+bool wx_bad(const WxArgs &x) {
+  return x.nitems > 0x7fffffffLL || !x.items || !x.deltas || !x.grps || !x.rows || !x.dops || !x.octs || !x.ent_w ||
+         !x.ent_r || !x.ops || x.maxR < 0 || x.maxO < 0 || x.maxO > WX_MAXOCT;
 }
 
 // ---- host: the sparse rows of S = W_i W_{i+1} for every (delta, operator) of one class
@@ -323,8 +442,8 @@ struct SparseW {
 
 struct OpLists {
   std::vector<qc_wxdop> dops;
-  std::vector<qc_wxquad> quads;
-  std::vector<double> w;
+  std::vector<qc_wxoct> octs;
+  std::vector<double> w;       // [entry][8]
   std::vector<int> r;
 };
 
@@ -356,24 +475,26 @@ void build_op(const SparseW &W1, const double *v1, const SparseW &W2, const doub
   list_rows(W1, v1, st1, nz1);
   list_rows(W2, v2, st2, nz2);
   const int nsb = W1.ns[1];
-  std::vector<double> S;
+  std::vector<double> S;                 // rows of the current delta, dense in i
   std::vector<uint64_t> mask;
-  std::vector<qc_wxquad> qs;
+  std::vector<int> rowid, nnz, perm;
+  std::vector<qc_wxoct> os;
   for (int d = 0; d < ndelta; ++d) {
     const int R = Rs[d];
     const int words = (R + 63) / 64;
-    qc_wxdop rec;
-    rec.ent_b = (long long)out.r.size();
-    rec.quad_b = (int)out.quads.size();
-    qs.clear();
+    int nrow = 0;
+    for (int kb = 0; kb < 16; ++kb)
+      if (kblk[16 * d + kb] >= 0) nrow += (int)W2.nd[1][kblk[16 * d + kb]];
+    S.assign((size_t)nrow * R, 0.0);
+    mask.assign((size_t)nrow * words, 0);
+    rowid.resize(nrow);
+    int base = 0;
     for (int kb = 0; kb < 16; ++kb) {
       const int sc = kblk[16 * d + kb];
       if (sc < 0) continue;
       const int nc = (int)W2.nd[1][sc];
-      const int nq = (nc + 3) / 4;
-      S.assign((size_t)nq * 4 * R, 0.0);            // [row i][nc padded to quads]
-      mask.assign((size_t)nq * words, 0);
       const int n1p = kb >> 2, n2p = kb & 3;
+      for (int c = 0; c < nc; ++c) rowid[base + c] = kb << 16 | c;
       for (int ib = 0; ib < 16; ++ib) {
         const int sa = iblk[16 * d + ib];
         if (sa < 0) continue;
@@ -389,37 +510,93 @@ void build_op(const SparseW &W1, const double *v1, const SparseW &W2, const doub
               const Nz u = nz1[b1][x];
               for (int y = st2[b2][u.j]; y < st2[b2][u.j + 1]; ++y) {
                 const Nz w = nz2[b2][y];
-                S[((size_t)(w.j >> 2) * R + i) * 4 + (w.j & 3)] += u.v * w.v;
-                mask[(size_t)(w.j >> 2) * words + (i >> 6)] |= 1ull << (i & 63);
+                S[(size_t)(base + w.j) * R + i] += u.v * w.v;
+                mask[(size_t)(base + w.j) * words + (i >> 6)] |= 1ull << (i & 63);
               }
             }
           }
         }
       }
-      for (int q = 0; q < nq; ++q) {
-        qc_wxquad x;
-        x.ent = (int)((long long)out.r.size() - rec.ent_b);
-        x.blk = kb;
-        x.c0nc = (4 * q) << 8 | std::min(4, nc - 4 * q);
-        for (int wd = 0; wd < words; ++wd) {
-          uint64_t m = mask[(size_t)q * words + wd];
-          while (m) {
-            const int i = wd * 64 + __builtin_ctzll(m);
-            m &= m - 1;
-            const double *p = &S[((size_t)q * R + i) * 4];
-            if (p[0] == 0.0 && p[1] == 0.0 && p[2] == 0.0 && p[3] == 0.0) continue;
-            out.w.insert(out.w.end(), p, p + 4);
-            out.r.push_back(i);
-          }
-        }
-        x.cnt = (int)((long long)out.r.size() - rec.ent_b) - x.ent;
-        qs.push_back(x);
-      }
+      base += nc;
     }
-    // longest first: warps take quads round-robin, so their loads come out even
-    std::stable_sort(qs.begin(), qs.end(), [](const qc_wxquad &x, const qc_wxquad &y) { return x.cnt > y.cnt; });
-    out.quads.insert(out.quads.end(), qs.begin(), qs.end());
-    rec.nquad = (int)qs.size();
+    // products that cancelled exactly are no entries
+    nnz.assign(nrow, 0);
+    for (int k = 0; k < nrow; ++k)
+      for (int wd = 0; wd < words; ++wd) {
+        uint64_t m = mask[(size_t)k * words + wd], live = 0;
+        while (m) {
+          const int bit = __builtin_ctzll(m);
+          m &= m - 1;
+          if (S[(size_t)k * R + wd * 64 + bit] != 0.0) live |= 1ull << bit;
+        }
+        mask[(size_t)k * words + wd] = live;
+        nnz[k] += __builtin_popcountll(live);
+      }
+    // rows of like pattern share an octet: longest first, equal patterns side by side
+    perm.resize(nrow);
+    for (int k = 0; k < nrow; ++k) perm[k] = k;
+    std::stable_sort(perm.begin(), perm.end(), [&](int x, int y) {
+      if (nnz[x] != nnz[y]) return nnz[x] > nnz[y];
+      for (int wd = 0; wd < words; ++wd) {
+        const uint64_t mx = mask[(size_t)x * words + wd], my = mask[(size_t)y * words + wd];
+        if (mx != my) return mx > my;
+      }
+      return false;
+    });
+    qc_wxdop rec;
+    rec.ent_b = (long long)out.r.size();
+    rec.oct_b = (int)out.octs.size();
+    os.clear();
+    for (int k0 = 0; k0 < nrow; k0 += 8) {
+      const int nk = std::min(8, nrow - k0);
+      qc_wxoct x;
+      memset(&x, 0, sizeof(x));
+      x.ent = (int)((long long)out.r.size() - rec.ent_b);
+      for (int k = 0; k < 8; ++k) x.row[k] = k < nk ? rowid[perm[k0 + k]] : -1;
+      // the T1 rows any of the eight reads, in fours of different residues mod 4 where possible
+      std::vector<int> bucket[4];
+      for (int wd = 0; wd < words; ++wd) {
+        uint64_t m = 0;
+        for (int k = 0; k < nk; ++k) m |= mask[(size_t)perm[k0 + k] * words + wd];
+        while (m) {
+          const int i = wd * 64 + __builtin_ctzll(m);
+          m &= m - 1;
+          bucket[i & 3].push_back(i);
+        }
+      }
+      int rest = (int)(bucket[0].size() + bucket[1].size() + bucket[2].size() + bucket[3].size());
+      // (one step of zero rows for an octet without entries)
+      for (bool first = true; first || rest > 0; first = false) {
+        bool used[4] = {false, false, false, false};
+        for (int e = 0; e < 4; ++e) {
+          int best = -1;
+          for (int b = 0; b < 4; ++b)
+            if (!used[b] && !bucket[b].empty() && (best < 0 || bucket[b].size() > bucket[best].size())) best = b;
+          if (best < 0) {                         // residues used up: any row that is left
+            for (int b = 0; b < 4; ++b)
+              if (!bucket[b].empty() && (best < 0 || bucket[b].size() > bucket[best].size())) best = b;
+          }
+          if (best < 0) {                         // none left: a zero row of an unused residue
+            int z = 0;
+            while (z < 3 && used[(R + z) & 3]) ++z;
+            used[(R + z) & 3] = true;
+            out.r.push_back(R + z);
+            out.w.insert(out.w.end(), 8, 0.0);
+            continue;
+          }
+          used[best] = true;
+          const int i = bucket[best].back();
+          bucket[best].pop_back();
+          --rest;
+          out.r.push_back(i);
+          for (int k = 0; k < 8; ++k) out.w.push_back(k < nk ? S[(size_t)perm[k0 + k] * R + i] : 0.0);
+        }
+      }
+      x.cnt = (int)((long long)out.r.size() - rec.ent_b) - x.ent;
+      os.push_back(x);
+    }
+    out.octs.insert(out.octs.end(), os.begin(), os.end());
+    rec.noct = (int)os.size();
     out.dops.push_back(rec);
   }
 }
@@ -441,9 +618,9 @@ extern "C" int qc_wx_build(int nops, const double *w1, const long long *off1, co
                            const long long *ioff1, const int *allowed1, const double *w2, const long long *off2,
                            const int *ns2, const long long *nd2, const long long *ioff2, const int *allowed2,
                            int ndelta, const int *iblk, const int *kblk, const int *row0, const int *R, void **handle,
-                           long long *nquads, long long *nents) {
+                           long long *nocts, long long *nents) {
   if (nops < 1 || ndelta < 0 || !w1 || !off1 || !ns1 || !nd1 || !ioff1 || !allowed1 || !w2 || !off2 || !ns2 || !nd2 ||
-      !ioff2 || !allowed2 || (ndelta && (!iblk || !kblk || !row0 || !R)) || !handle || !nquads || !nents)
+      !ioff2 || !allowed2 || (ndelta && (!iblk || !kblk || !row0 || !R)) || !handle || !nocts || !nents)
     return QC_ERR_ARG;
   if (ns1[2] != 4 || ns1[3] != 4 || ns2[2] != 4 || ns2[3] != 4 || ns1[1] != ns2[0]) return QC_ERR_LAYOUT;
   try {
@@ -511,7 +688,7 @@ extern "C" int qc_wx_build(int nops, const double *w1, const long long *off1, co
     }
     long long nq = 0, ne = 0;
     for (const OpLists &l : h->ops) {
-      nq += (long long)l.quads.size();
+      nq += (long long)l.octs.size();
       ne += (long long)l.r.size();
     }
     if (nq > 0x7fffffffLL) {
@@ -519,7 +696,7 @@ extern "C" int qc_wx_build(int nops, const double *w1, const long long *off1, co
       return QC_ERR_CAPACITY;
     }
     *handle = h;
-    *nquads = nq;
+    *nocts = nq;
     *nents = ne;
     return QC_OK;
   } catch (...) {
@@ -527,49 +704,74 @@ extern "C" int qc_wx_build(int nops, const double *w1, const long long *off1, co
   }
 }
 
-// Copies what qc_wx_build made and frees it: dops [ndelta][nops] (entry and quad offsets from
-// ent0 / quad0), quads, coefficients [nents][4] and T1 rows [nents].
-extern "C" int qc_wx_fetch(void *handle, long long ent0, int quad0, void *dops, void *quads, double *w, int *r) {
+// Copies what qc_wx_build made and frees it: dops [ndelta][nops] (entry and octet offsets from
+// ent0 / oct0), octets, T1 rows [nents] and the coefficients in the kernels' orders: FP64
+// fragments (w64: step by step, lane l the coefficient of entry l % 4 and row l / 4) and FP32
+// [nents][8] (w32); either may be null.
+extern "C" int qc_wx_fetch(void *handle, long long ent0, int oct0, void *dops, void *octs, double *w64, float *w32,
+                           int *r) {
   WxBuild *h = (WxBuild *)handle;
   if (!h) return QC_ERR_ARG;
   const int nops = (int)h->ops.size();
   qc_wxdop *pd = (qc_wxdop *)dops;
-  qc_wxquad *pq = (qc_wxquad *)quads;
+  qc_wxoct *po = (qc_wxoct *)octs;
   for (int o = 0; o < nops; ++o) {
     const OpLists &l = h->ops[o];
     for (int d = 0; d < h->ndelta; ++d) {
       qc_wxdop x = l.dops[d];
       x.ent_b += ent0;
-      x.quad_b += quad0;
+      x.oct_b += oct0;
       pd[(long long)d * nops + o] = x;
     }
-    if (!l.quads.empty()) memcpy(pq, l.quads.data(), l.quads.size() * sizeof(qc_wxquad));
-    if (!l.r.empty()) {
-      memcpy(w, l.w.data(), l.w.size() * sizeof(double));
-      memcpy(r, l.r.data(), l.r.size() * sizeof(int));
+    const size_t n = l.r.size();
+    if (!l.octs.empty()) memcpy(po, l.octs.data(), l.octs.size() * sizeof(qc_wxoct));
+    if (n) memcpy(r, l.r.data(), n * sizeof(int));
+    if (w64) {
+      for (size_t e = 0; e < n; ++e)
+        for (int k = 0; k < 8; ++k) w64[(e & ~(size_t)3) * 8 + 4 * k + (e & 3)] = l.w[8 * e + k];
+      w64 += 8 * n;
     }
-    pq += l.quads.size();
-    w += l.w.size();
-    r += l.r.size();
-    ent0 += (long long)l.r.size();
-    quad0 += (int)l.quads.size();
+    if (w32) {
+      for (size_t e = 0; e < 8 * n; ++e) w32[e] = (float)l.w[e];
+      w32 += 8 * n;
+    }
+    po += l.octs.size();
+    r += n;
+    ent0 += (long long)n;
+    oct0 += (int)l.octs.size();
   }
   delete h;
   return QC_OK;
 }
 
-extern "C" int qc_wsparse_f64(const void *items, long long nitems, int fpt, const void *deltas, const void *grps,
-                              const void *rows, const void *dops, const void *quads, const void *ent_w,
-                              long long nent, const void *ent_r, const void *ops, int maxR, int maxQ, const double *A,
-                              double *C, void *stream) {
-  return launch_wsparse<double>(items, nitems, fpt, deltas, grps, rows, dops, quads, ent_w, nent, ent_r, ops, maxR, maxQ,
-                            A, C, (cudaStream_t)stream);
+extern "C" int qc_wsparse_f64(const void *items, long long nitems, int tile, const void *deltas, const void *grps,
+                              const void *rows, const void *dops, const void *octs, const void *ent_w,
+                              const void *ent_r, const void *ops, int maxR, int maxO, const double *A, double *C,
+                              void *stream) {
+  if (nitems <= 0) return QC_OK;
+  const WxArgs x = {items, nitems, deltas, grps, rows, dops, octs, ent_w, ent_r, ops, maxR, maxO};
+  if (wx_bad(x)) return QC_ERR_ARG;
+  cudaStream_t s = (cudaStream_t)stream;
+  switch (tile) {
+    case 32: return launch_kernel<double, double>(k_wsparse_f64<32>, wx_smem_bytes<double, 32>(maxR, maxO), x, A, C, s);
+    case 64: return launch_kernel<double, double>(k_wsparse_f64<64>, wx_smem_bytes<double, 64>(maxR, maxO), x, A, C, s);
+    case 128: return launch_kernel<double, double>(k_wsparse_f64<128>, wx_smem_bytes<double, 128>(maxR, maxO), x, A, C, s);
+    default: return QC_ERR_ARG;
+  }
 }
 
-extern "C" int qc_wsparse_f32(const void *items, long long nitems, int fpt, const void *deltas, const void *grps,
-                              const void *rows, const void *dops, const void *quads, const void *ent_w,
-                              long long nent, const void *ent_r, const void *ops, int maxR, int maxQ, const float *A,
-                              float *C, void *stream) {
-  return launch_wsparse<float>(items, nitems, fpt, deltas, grps, rows, dops, quads, ent_w, nent, ent_r, ops, maxR, maxQ,
-                            A, C, (cudaStream_t)stream);
+extern "C" int qc_wsparse_f32(const void *items, long long nitems, int tile, const void *deltas, const void *grps,
+                              const void *rows, const void *dops, const void *octs, const void *ent_w,
+                              const void *ent_r, const void *ops, int maxR, int maxO, const float *A, float *C,
+                              void *stream) {
+  if (nitems <= 0) return QC_OK;
+  const WxArgs x = {items, nitems, deltas, grps, rows, dops, octs, ent_w, ent_r, ops, maxR, maxO};
+  if (wx_bad(x)) return QC_ERR_ARG;
+  cudaStream_t s = (cudaStream_t)stream;
+  switch (tile) {
+    case 32: return launch_kernel<float, float4>(k_wsparse_f32<32, 32>, wx_smem_bytes<float, 32>(maxR, maxO), x, A, C, s);
+    case 64: return launch_kernel<float, float4>(k_wsparse_f32<64, 64>, wx_smem_bytes<float, 64>(maxR, maxO), x, A, C, s);
+    case 128: return launch_kernel<float, float4>(k_wsparse_f32<128, 64>, wx_smem_bytes<float, 128>(maxR, maxO), x, A, C, s);
+    default: return QC_ERR_ARG;
+  }
 }

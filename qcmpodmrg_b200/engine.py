@@ -1103,13 +1103,14 @@ WXDELTA_DT = numpy.dtype([("R", "<i4"), ("row_b", "<i4"), ("grp_b", "<i4"), ("gr
                           ("pad", "<i4", (3,))])
 WXITEM_DT = numpy.dtype([("delta", "<i4"), ("grp", "<i4"), ("f0", "<i4"), ("nf", "<i4"), ("op_b", "<i4"),
                          ("op_e", "<i4"), ("op0", "<i4"), ("pad", "<i4")])
-WXDOP_DT = numpy.dtype([("ent_b", "<i8"), ("quad_b", "<i4"), ("nquad", "<i4")])
-WXQUAD_DT = numpy.dtype([("ent", "<i4"), ("cnt", "<i4"), ("blk", "<i4"), ("c0nc", "<i4")])
+WXDOP_DT = numpy.dtype([("ent_b", "<i8"), ("oct_b", "<i4"), ("noct", "<i4")])
+WXOCT_DT = numpy.dtype([("ent", "<i4"), ("cnt", "<i4"), ("pad", "<i4", (2,)), ("row", "<i4", (8,))])
 assert WXGRP_DT.itemsize == 208 and WXDELTA_DT.itemsize == 32 and WXITEM_DT.itemsize == 32
-assert WXDOP_DT.itemsize == 16 and WXQUAD_DT.itemsize == 16
+assert WXDOP_DT.itemsize == 16 and WXOCT_DT.itemsize == 48
 WX_MAXR = 640             # T1 rows of one charge difference (FP64 rows of a 32-fiber tile: 160 KB)
-WX_MAXQ = 1024            # quads of one (charge difference, operator)
-WX_TILE_BYTES = {"f64": 96 * 1024, "f32": 48 * 1024}
+WX_MAXOCT = 512           # octets of one (charge difference, operator)
+WX_GRPS = 32              # sector pairs of one tile
+WX_TILE_BYTES = 112 * 1024  # shared memory of a CTA: two share an SM
 WX_SMALL = 8 * 148        # 64-fiber tiles of all operators up to which a dot uses one tile width
 WX_ITEMS = 24 * 148       # work items wanted before operators are walked inside one
 
@@ -1185,7 +1186,7 @@ def sparse_groups(ins, outs, dx, dz, qx, qz, da, db):
     R = rows_b.sum(axis=1)
     row0 = numpy.where(iblk >= 0, numpy.cumsum(rows_b, axis=1) - rows_b, 0).astype(numpy.int32)
     dcb = numpy.where(kblk >= 0, db[dk[:, None], numpy.maximum(kblk, 0)], 0)
-    if int(R.max()) > WX_MAXR or int(((dcb + 3) // 4).sum(axis=1).max()) > WX_MAXQ:
+    if int(R.max()) > WX_MAXR or int(dcb.sum(axis=1).max()) > 8 * WX_MAXOCT or max(int(dx.max()), int(dz.max())) >= 2 ** 15:
         return None
     own, loc = _ranges(rows_b.ravel())
     rows = ((own % 16) << 16 | loc).astype(numpy.int32)
@@ -1306,24 +1307,26 @@ class SparseWStage(object):
         self.name, self.device = name, device
         self.host_ops = ops
         self.flops = self.bytes = 0.0
-        grps, dels, rows, dops, quads, ws, rs, self.op_ranges = [], [], [], [], [], [], [], []
-        ngrp = nrow = ndop = nq = ne = 0
+        grps, dels, rows, dops, octs, w64, w32, rs, self.op_ranges = [], [], [], [], [], [], [], [], []
+        ngrp = nrow = ndop = no = ne = 0
         lib = native.lib()
         i64 = numpy.int64
         for part, (b, e), factors in parts:
             d = part["deltas"].copy()
             nops, nd = e - b, len(d)
-            h, cq, ce = numpy.zeros(1, dtype=i64), numpy.zeros(1, dtype=i64), numpy.zeros(1, dtype=i64)
+            h, co, ce = numpy.zeros(1, dtype=i64), numpy.zeros(1, dtype=i64), numpy.zeros(1, dtype=i64)
             args = []
             for w in factors:
                 assert len(w.offsets) == nops
                 args += [ptr(w.values), ptr(w.offsets), ptr(w.nsyms), ptr(w.nd), ptr(w.ioff), ptr(w.allowed)]
             check(lib.qc_wx_build(nops, *args, nd, ptr(part["iblk"]), ptr(part["kblk"]), ptr(part["row0"]),
-                                  ptr(part["R"]), ptr(h), ptr(cq), ptr(ce)), "qc_wx_build")
-            dp = numpy.zeros(nd * nops, WXDOP_DT)
-            qd = numpy.zeros(int(cq[0]), WXQUAD_DT)
-            ww, rr = numpy.zeros((int(ce[0]), 4)), numpy.zeros(int(ce[0]), dtype=numpy.int32)
-            check(lib.qc_wx_fetch(int(h[0]), ne, nq, ptr(dp), ptr(qd), ptr(ww), ptr(rr)), "qc_wx_fetch")
+                                  ptr(part["R"]), ptr(h), ptr(co), ptr(ce)), "qc_wx_build")
+            n = int(ce[0])
+            dp, oc = numpy.empty(nd * nops, WXDOP_DT), numpy.empty(int(co[0]), WXOCT_DT)
+            wd = numpy.empty(8 * n) if "f64" in kinds else None
+            ws = numpy.empty(8 * n, dtype=numpy.float32) if "f32" in kinds else None
+            rr = numpy.empty(n, dtype=numpy.int32)
+            check(lib.qc_wx_fetch(int(h[0]), ne, no, ptr(dp), ptr(oc), ptr(wd), ptr(ws), ptr(rr)), "qc_wx_fetch")
             d["grp_b"] += ngrp
             d["grp_e"] += ngrp
             d["row_b"] += nrow
@@ -1332,82 +1335,90 @@ class SparseWStage(object):
             dels.append(d)
             rows.append(part["rows"])
             dops.append(dp)
-            quads.append(qd)
-            ws.append(ww)
+            octs.append(oc)
+            w64.append(wd)
+            w32.append(ws)
             rs.append(rr)
-            self.op_ranges.append((b, e, len(d)))
-            ngrp, nrow, ndop, nq, ne = ngrp + len(part["groups"]), nrow + len(part["rows"]), ndop + len(dp), \
-                nq + len(qd), ne + len(rr)
+            self.op_ranges.append((b, e, nd))
+            ngrp, nrow, ndop, no, ne = ngrp + len(part["groups"]), nrow + len(part["rows"]), ndop + len(dp), \
+                no + len(oc), ne + n
         self.h_groups, self.h_deltas = numpy.concatenate(grps), numpy.concatenate(dels)
-        self.h_rows, self.h_dops, self.h_quads = (numpy.concatenate(x) for x in (rows, dops, quads))
-        self.h_ent_w, self.h_ent_r = numpy.concatenate(ws), numpy.concatenate(rs)
+        self.h_rows, self.h_dops, self.h_octs = (numpy.concatenate(x) for x in (rows, dops, octs))
+        self.h_ent_r = numpy.concatenate(rs)
+        self.h_w = {k: numpy.concatenate(w) for k, w in (("f64", w64), ("f32", w32)) if k in kinds}
         self.fibers = numpy.concatenate([p["fibers"] for p, _, _ in parts])
         self.ntasks = len(self.h_groups)
         up = lambda a, dt: upload(a if len(a) else numpy.zeros(1, dt), device)         # noqa: E731
         self.d = {"groups": up(self.h_groups, WXGRP_DT), "deltas": up(self.h_deltas, WXDELTA_DT),
                   "rows": up(self.h_rows, numpy.int32), "dops": up(self.h_dops, WXDOP_DT),
-                  "quads": up(self.h_quads, WXQUAD_DT), "ent_r": up(self.h_ent_r, numpy.int32),
+                  "octs": up(self.h_octs, WXOCT_DT), "ent_r": up(self.h_ent_r, numpy.int32),
                   "ops": upload(ops, device)}
-        w = self.h_ent_w if len(self.h_ent_w) else numpy.zeros((1, 4))
-        # coefficients as 16-byte vectors: two per entry in FP64 (all first halves, then all second)
-        self._w = {"f64": torch.from_numpy(numpy.ascontiguousarray(w.reshape(-1, 2, 2).transpose(1, 0, 2))).to(device)}
+        self._w = {k: up(w, w.dtype) for k, w in self.h_w.items()}
         self._launch = {}
         for kind in kinds:
             self.items(kind)
-            self.coefficients(kind)
 
     def items(self, kind):
-        """Work items by fibers per lane, [(fpt, items, T1 rows, quads)], longest first.
+        """Work items by tile width, [(fibers, items, device items, T1 rows, octets)], longest first.
 
-        A tile is 32, 64 or 128 fibers wide: as many as its T1 rows leave room for in
-        WX_TILE_BYTES of shared memory, so that two or three CTAs share an SM.  Dots whose
-        tiles fit the GPU at once use one width, in one launch."""
+        A tile is 32, 64 or 128 fibers wide: as many as its T1 rows, its offset tables and (in
+        FP32) its entry rings leave room for in WX_TILE_BYTES of shared memory, so that two
+        CTAs share an SM.  Dots whose tiles fit
+        the GPU at once use one width, in one launch."""
         hit = self._launch.get(kind)
         if hit is not None:
             return hit
         el = 8 if kind == "f64" else 4
         d = self.h_deltas
-        R = numpy.maximum(d["R"].astype(numpy.int64), 1)
+        i64 = numpy.int64
+        R = d["R"].astype(i64) + 4
         nops = numpy.concatenate([numpy.full(n, e - b) for (b, e, n) in self.op_ranges])
-        fpt = numpy.where(R * 128 * el <= WX_TILE_BYTES[kind], 4, numpy.where(R * 64 * el <= WX_TILE_BYTES[kind], 2, 1))
+        noct = self.h_dops["noct"][d["dop_b"]].astype(i64)
+        own = 48 * noct + 4 * R + (2048 if kind == "f64" else 20 * 1024)
+        room = lambda f: R * (f + 4) * el + 136 * f + own <= WX_TILE_BYTES              # noqa: E731
+        ft = numpy.where(room(128), 128, numpy.where(room(64), 64, 32))
         if int((((self.fibers + 63) // 64) * nops).sum()) <= WX_SMALL:
-            fpt[:] = int(fpt.min())
-        ft = 32 * fpt
-        nt = (self.fibers + ft - 1) // ft
+            ft[:] = min(64, int(ft.min()))
         op0 = numpy.concatenate([numpy.full(n, b) for (b, e, n) in self.op_ranges])
-        chunk = int(max(1, (nt * nops).sum() // WX_ITEMS))      # operators of one item
-        nch = (nops + chunk - 1) // chunk
-        own, loc = _ranges(nt * nch)
-        t, ch = loc // nch[own], loc % nch[own]
-        it = numpy.zeros(len(own), WXITEM_DT)
-        it["delta"] = own
-        p = t * ft[own]
-        it["nf"] = numpy.minimum(ft[own], self.fibers[own] - p)
+        nt = (self.fibers + ft - 1) // ft
+        own, loc = _ranges(nt)
+        p = loc * ft[own]
+        nf = numpy.minimum(ft[own], self.fibers[own] - p)
         # the tile's first group: groups are stored delta by delta with their first fibers
-        gkey = numpy.repeat(numpy.arange(len(d)), d["grp_e"] - d["grp_b"]).astype(numpy.int64) << 32
+        gkey = numpy.repeat(numpy.arange(len(d)), d["grp_e"] - d["grp_b"]).astype(i64) << 32
         gkey = gkey + self.h_groups["start"]
-        it["grp"] = numpy.searchsorted(gkey, (own.astype(numpy.int64) << 32) + p, side="right") - 1
-        it["f0"] = p - self.h_groups["start"][it["grp"]]
+        grp = numpy.searchsorted(gkey, (own.astype(i64) << 32) + p, side="right") - 1
+        last = numpy.searchsorted(gkey, (own.astype(i64) << 32) + p + nf - 1, side="right") - 1
+        # tiles of more sector pairs than a tile's tables hold are cut
+        cut = (last - grp) // WX_GRPS + 1
+        if int(cut.max()) > 1:
+            t, c = _ranges(cut)
+            first = grp[t] + c * WX_GRPS
+            lo = numpy.where(c > 0, self.h_groups["start"][first], p[t])
+            nxt = numpy.minimum(first + WX_GRPS, len(self.h_groups) - 1)
+            hi = numpy.where(c + 1 < cut[t], self.h_groups["start"][nxt], p[t] + nf[t])
+            own, grp, p, nf = own[t], first, lo, hi - lo
+        chunk = int(max(1, nops[own].sum() // WX_ITEMS))      # operators of one item
+        nch = (nops[own] + chunk - 1) // chunk
+        t, ch = _ranges(nch)
+        own, grp, p, nf = own[t], grp[t], p[t], nf[t]
+        it = numpy.zeros(len(own), WXITEM_DT)
+        it["delta"], it["grp"], it["nf"] = own, grp, nf
+        it["f0"] = p - self.h_groups["start"][grp]
         it["op_b"] = op0[own] + ch * chunk
         it["op_e"] = numpy.minimum(op0[own] + nops[own], it["op_b"] + chunk)
         it["op0"] = op0[own]
-        nqd = self.h_dops["nquad"][d["dop_b"]].astype(numpy.int64)
-        cost = (it["op_e"] - it["op_b"]) * (R[own] + 2 * nqd[own]) * fpt[own]
+        cost = (it["op_e"] - it["op_b"]) * (R[own] + 12 * noct[own]) * ft[own]
         out = []
-        for k in (4, 2, 1):
-            sel = numpy.flatnonzero(fpt[own] == k)
+        for k in (128, 64, 32):
+            sel = numpy.flatnonzero(ft[own] == k)
             if len(sel) == 0:
                 continue
             sel = sel[numpy.argsort(-cost[sel], kind="stable")]
             dd = numpy.unique(own[sel])
-            out.append((k, it[sel], upload(it[sel], self.device), int(R[dd].max()), int(max(1, nqd[dd].max()))))
+            out.append((k, it[sel], upload(it[sel], self.device), int(d["R"][dd].max()), int(max(1, noct[dd].max()))))
         self._launch[kind] = out
         return out
-
-    def coefficients(self, kind):
-        if kind not in self._w:
-            self._w[kind] = self._w["f64"].transpose(0, 1).contiguous().to(torch.float32)
-        return self._w[kind]
 
     def run(self, A, B, C, kind="f64", stream=None):
         """C = T3 from A = T1 (B, the operand of the separate stages, is not read)."""
@@ -1416,17 +1427,17 @@ class SparseWStage(object):
         lib = native.lib()
         s = stream if stream is not None else torch.cuda.current_stream(C.device).cuda_stream
         k = "f64" if kind == "f64" else "f32"
-        w = self.coefficients(k)
+        w = self._w[k]
         fn = lib.qc_wsparse_f64 if k == "f64" else lib.qc_wsparse_f32
         if LOG.enabled:
             e0 = torch.cuda.Event(enable_timing=True)
             e1 = torch.cuda.Event(enable_timing=True)
             e0.record()
         d = self.d
-        for (fpt, host, dev, maxr, maxq) in self.items(k):
-            check(fn(dev.data_ptr(), len(host), fpt, d["deltas"].data_ptr(), d["groups"].data_ptr(),
-                     d["rows"].data_ptr(), d["dops"].data_ptr(), d["quads"].data_ptr(), w.data_ptr(),
-                     len(self.h_ent_r), d["ent_r"].data_ptr(), d["ops"].data_ptr(), maxr, maxq, A.data_ptr(), C.data_ptr(), s),
+        for (tile, host, dev, maxr, maxo) in self.items(k):
+            check(fn(dev.data_ptr(), len(host), tile, d["deltas"].data_ptr(), d["groups"].data_ptr(),
+                     d["rows"].data_ptr(), d["dops"].data_ptr(), d["octs"].data_ptr(), w.data_ptr(),
+                     d["ent_r"].data_ptr(), d["ops"].data_ptr(), maxr, maxo, A.data_ptr(), C.data_ptr(), s),
                   "qc_wsparse_" + k)
             LOG.launches += 1
         if LOG.enabled:

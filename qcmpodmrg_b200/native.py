@@ -80,9 +80,9 @@ _SIGS = {
     "qc_dpanel_f64": (c_int, [c_vp, c_vp, c_ll] + [c_vp] * 7),
     "qc_gather_pad_f64": (c_int, [c_vp, c_vp, c_ll, c_vp, c_vp]),
     "qc_wx_build": (c_int, [c_int] + [c_vp] * 12 + [c_int] + [c_vp] * 7),
-    "qc_wx_fetch": (c_int, [c_vp, c_ll, c_int, c_vp, c_vp, c_vp, c_vp]),
-    "qc_wsparse_f64": (c_int, [c_vp, c_ll, c_int] + [c_vp] * 6 + [c_ll, c_vp, c_vp, c_int, c_int, c_vp, c_vp, c_vp]),
-    "qc_wsparse_f32": (c_int, [c_vp, c_ll, c_int] + [c_vp] * 6 + [c_ll, c_vp, c_vp, c_int, c_int, c_vp, c_vp, c_vp]),
+    "qc_wx_fetch": (c_int, [c_vp, c_ll, c_int, c_vp, c_vp, c_vp, c_vp, c_vp]),
+    "qc_wsparse_f64": (c_int, [c_vp, c_ll, c_int] + [c_vp] * 8 + [c_int, c_int, c_vp, c_vp, c_vp]),
+    "qc_wsparse_f32": (c_int, [c_vp, c_ll, c_int] + [c_vp] * 8 + [c_int, c_int, c_vp, c_vp, c_vp]),
     "qc_wpanel_f64": (c_int, [c_vp, c_vp, c_vp, c_ll, c_vp]),
     "qc_wpanel_f32": (c_int, [c_vp, c_vp, c_vp, c_ll, c_vp]),
     "qc_wpanel_pairs_f64": (c_int, [c_vp, c_ll, c_vp, c_ll, c_int, c_vp, c_vp, c_ll, c_vp]),
