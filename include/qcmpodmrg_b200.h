@@ -229,12 +229,16 @@ int qc_fgemm_f32(const void *items_dev, long long nitems, const void *groups_dev
 /* W panels of the dense fiber-group GEMM: dst[i] = idx[i] >= 0 ? src[idx[i]] : 0 (once per dot). */
 int qc_wpanel_f64(const double *src, const long long *idx_dev, double *dst, long long n, void *stream);
 int qc_wpanel_f32(const float *src, const long long *idx_dev, float *dst, long long n, void *stream);
-/* FP64 panel GEMM on the tensor pipe (mma.sync f64): work is nwork (unit, operator) int
+/* Panel GEMM, FP64 on the tensor pipe (mma.sync f64) or FP32: work is nwork (unit, operator) int
  * pairs, units qc_dunit records, ops the operator table.  crow: row form; cols (qc_dcol):
- * column form; neither: block form.  A and B are 16-byte aligned. */
+ * column form; neither: block form (FP64 only).  A and B and their rows are 16-byte aligned.  Tiles
+ * of up to 128 x 64 (FP64) or 256 x 32 (FP32). */
 int qc_dpanel_f64(const void *units, const void *work, long long nwork, const void *ops, const long long *crow,
                   const void *cols, const double *A, const double *B, double *C, void *stream);
+int qc_dpanel_f32(const void *units, const void *work, long long nwork, const void *ops, const long long *crow,
+                  const void *cols, const float *A, const float *B, float *C, void *stream);
 /* out[i] = x[idx[i]], 0 where idx[i] < 0. */
+int qc_gather_pad_f32(const double *x, const long long *idx, long long n, float *out, void *stream);
 int qc_gather_pad_f64(const double *x, const long long *idx, long long n, double *out, void *stream);
 
 /* Sparse MPO stage: T3 = T1 . (W_i W_{i+1}) for every operator (records qc_wxitem /

@@ -1700,13 +1700,14 @@ def tc_sigma1_units(classes, psi_info, psi_cols, lp_base, lp_opstride, lp_total,
 
 
 
-# ---------------------------------------------------------------- FP64 panel GEMM on the tensor pipe (qc_dpanel_f64)
+# ---------------------------------------------------------------- panel GEMM (qc_dpanel_f64, qc_dpanel_f32)
 DUNIT_DT = numpy.dtype([("a_off", "<i8"), ("b_off", "<i8"), ("c_off", "<i8"), ("lda", "<i4"), ("ldb", "<i4"),
                         ("K", "<i4"), ("mrem", "<i4"), ("nrem", "<i4"), ("m0", "<i4"), ("n0", "<i4"),
                         ("pad", "<i4", (3,))])
 DCOL_DT = numpy.dtype([("off", "<i4"), ("ld", "<i4")])
 assert DUNIT_DT.itemsize == 64 and DCOL_DT.itemsize == 8
-DP_BM, DP_BN = 128, 64
+# rows and columns of a tile, rows of a warp; both fill about 90 KB of a three-stage ring
+DP_TILE = {"f64": (128, 64, 16), "f32": (256, 32, 32)}
 
 
 def _even_tiles(n, most, unit):
@@ -1720,15 +1721,15 @@ def _even_tiles(n, most, unit):
     return own, loc * w[own], numpy.minimum(w[own], n[own] - loc * w[own])
 
 
-def dpanel_units(M, N, K, lda, ldb, a_off, b_off, c_off, form, blk=None, owner=False):
+def dpanel_units(M, N, K, lda, ldb, a_off, b_off, c_off, form, blk=None, owner=False, kind="f64"):
     """Tiles of the panels C_j[M_j x N_j] = A_j . B_j^T.  form "row": c_off is the row-table
     index of row 0; "col": the column-table index of column 0; "blk": the offset of the block
     [row / blk[0]][column][row % blk[0]] of blk[1] columns, A given as [K x M].  Column tiles of
-    one row tile are neighbours.  owner: also the panel of every tile."""
+    one row tile are neighbours.  owner: also the panel of every tile.  kind: the tile's type."""
     M, N, K, lda, ldb, a_off, b_off, c_off = (numpy.asarray(x, dtype=numpy.int64) for x in
                                               (M, N, K, lda, ldb, a_off, b_off, c_off))
-    jm, m0, mw = _even_tiles(M, DP_BM, 16)
-    jn, n0, nw = _even_tiles(N, DP_BN, 8)
+    jm, m0, mw = _even_tiles(M, DP_TILE[kind][0], DP_TILE[kind][2])
+    jn, n0, nw = _even_tiles(N, DP_TILE[kind][1], 8)
     nfirst = numpy.searchsorted(jn, numpy.arange(len(M)))
     ncnt = numpy.bincount(jn, minlength=len(M)) if len(M) else numpy.zeros(0, dtype=numpy.int64)
     i, k = _ranges(ncnt[jm])
@@ -1745,13 +1746,14 @@ def dpanel_units(M, N, K, lda, ldb, a_off, b_off, c_off, form, blk=None, owner=F
 
 
 class DPanelStage(object):
-    """Panel GEMMs C = A . B^T of every operator in FP64 (qc_dpanel_f64).
+    """Panel GEMMs C = A . B^T of every operator (qc_dpanel_f64, qc_dpanel_f32).
 
     parts: [(units, operator range)]; at most one of crow (row table) and cols (DCOL_DT): with
     neither, the units are in block form (A row-major [K x M])."""
 
-    def __init__(self, name, parts, ops, device, flops, crow=None, cols=None, longest_first=False):
-        self.name, self.host_ops, self.flops, self.bytes = name, ops, flops, 0.0
+    def __init__(self, name, parts, ops, device, flops, crow=None, cols=None, longest_first=False,
+                 kind="f64"):
+        self.name, self.host_ops, self.flops, self.bytes, self.kind = name, ops, flops, 0.0, kind
         units, work = [], []
         n = 0
         for u, (b, e) in parts:
@@ -1784,9 +1786,9 @@ class DPanelStage(object):
             e0 = torch.cuda.Event(enable_timing=True)
             e1 = torch.cuda.Event(enable_timing=True)
             e0.record()
-        check(native.lib().qc_dpanel_f64(self.d_units.data_ptr(), self.d_work.data_ptr(), self.ntasks,
-                                         self.d_ops.data_ptr(), ptr(self.d_crow), ptr(self.d_cols), A.data_ptr(),
-                                         B.data_ptr(), C.data_ptr(), s), "qc_dpanel_f64")
+        fn = native.lib().qc_dpanel_f64 if self.kind == "f64" else native.lib().qc_dpanel_f32
+        check(fn(self.d_units.data_ptr(), self.d_work.data_ptr(), self.ntasks, self.d_ops.data_ptr(),
+                 ptr(self.d_crow), ptr(self.d_cols), A.data_ptr(), B.data_ptr(), C.data_ptr(), s), "qc_dpanel")
         LOG.launches += 1
         if LOG.enabled:
             e1.record()

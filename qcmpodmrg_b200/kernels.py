@@ -134,12 +134,12 @@ def gather_split(x, idx, hi, lo):
 
 
 def gather_pad(x, idx, out):
-    """out[i] = x[idx[i]], 0 where idx is negative (qc_gather_pad_f64)."""
+    """out[i] = x[idx[i]] in out's type, 0 where idx is negative (qc_gather_pad_f64, _f32)."""
     if out.device.type != "cuda":           # plans interpreted on the CPU
         out[:idx.numel()] = torch.where(idx >= 0, x[idx.clamp(min=0)], torch.zeros((), dtype=x.dtype))
         return out
-    check(native.lib().qc_gather_pad_f64(x.data_ptr(), idx.data_ptr(), idx.numel(), out.data_ptr(),
-                                         _stream(out.device)), "qc_gather_pad_f64")
+    fn = native.lib().qc_gather_pad_f64 if out.dtype == torch.float64 else native.lib().qc_gather_pad_f32
+    check(fn(x.data_ptr(), idx.data_ptr(), idx.numel(), out.data_ptr(), _stream(out.device)), "qc_gather_pad")
     LOG.launches += 1
     return out
 
@@ -456,8 +456,8 @@ class SigmaOperator(object):
             self._build_rpan(sparse_w)
         # L.psi and .R on K-major panels with padded rows (the L panels of a contracted sector,
         # the transposed R panels, the wavefunction's panels): split TF32 on the tcgen05 kernel,
-        # and FP64 on the tensor pipe where the sparse product runs between them
-        self.tc1 = self.tc4 = self.d1 = self.d4 = None
+        # and FP64 (on the tensor pipe) or FP32 where the sparse product runs between them
+        self.tc1 = self.tc4 = self.d1 = self.d4 = self.f1 = self.f4 = None
         crow = numpy.concatenate(crow_all) if crow_all else numpy.zeros(1, numpy.int64)
         if tc1_classes:
             self._setup_panels1(tc1_classes, order, L, tabs[0], want_tc1, sparse_w)
@@ -509,7 +509,7 @@ class SigmaOperator(object):
                 fb += stage_bytes(fused[1], fused[2], len(ops), False)
         if self.fused is not None:
             self.fused.bytes = float(fb)
-        for st, ref in ((self.tc1, 0), (self.d1, 0), (self.tc4, 3), (self.d4, 3)):
+        for st, ref in ((self.tc1, 0), (self.d1, 0), (self.f1, 0), (self.tc4, 3), (self.d4, 3), (self.f4, 3)):
             if st is not None:
                 st.bytes = self._stages[ref].bytes
         # FLOPs of the reference's four-contraction chain (tensordotCAL pair GEMMs),
@@ -653,9 +653,12 @@ class SigmaOperator(object):
         if f64:
             ops = st4_ops.copy()
             ops["b_base"] = base
-            parts = [(dpanel_units(sec["M"], sec["N"], sec["K"], sec["Kp"], sec["Kp"], sec["t3pan"], sec["rtoff"],
-                                   sec["crow_base"], "row"), (poss[0], poss[-1] + 1)) for (poss, sec, _) in classes]
-            self.d4 = DPanelStage("sigma4", parts, ops, dev, flops, crow=crow, longest_first=True)
+            for kind in ("f64", "f32") if self.precision == "f32" else ("f64",):
+                parts = [(dpanel_units(sec["M"], sec["N"], sec["K"], sec["Kp"], sec["Kp"], sec["t3pan"],
+                                       sec["rtoff"], sec["crow_base"], "row", kind=kind), (poss[0], poss[-1] + 1))
+                         for (poss, sec, _) in classes]
+                st = DPanelStage("sigma4", parts, ops, dev, flops, crow=crow, longest_first=True, kind=kind)
+                self.d4, self.f4 = (st, self.f4) if kind == "f64" else (self.d4, st)
         self._build_rpan_k()
 
     def _setup_panels1(self, tc1_classes, order, L, st1_ops, tc, f64):
@@ -691,8 +694,10 @@ class SigmaOperator(object):
         if f64:
             ops = st1_ops.copy()
             ops["a_base"], ops["b_base"] = base, 0
-            parts, tab = self._dpanel1_units(classes, info, cols)
-            self.d1 = DPanelStage("sigma1", parts, ops, dev, self._stages[0].flops, cols=tab)
+            for kind in ("f64", "f32") if self.precision == "f32" else ("f64",):
+                parts, tab = self._dpanel1_units(classes, info, cols, kind)
+                st = DPanelStage("sigma1", parts, ops, dev, self._stages[0].flops, cols=tab, kind=kind)
+                self.d1, self.f1 = (st, self.f1) if kind == "f64" else (self.d1, st)
         self._lp_descs = numpy.concatenate(descs)
         self._lp_descs_d = upload(self._lp_descs, dev)
         self._lp_ops_d = upload(op_table(L.offsets[order], 0, base, 1.0), dev)
@@ -700,8 +705,8 @@ class SigmaOperator(object):
         self._build_lpan_k()
 
     @staticmethod
-    def _dpanel1_units(classes, info, cols):
-        """Units and column table of L.psi in FP64: the psi panel of a contracted sector times
+    def _dpanel1_units(classes, info, cols, kind):
+        """Units and column table of L.psi: the psi panel of a contracted sector times
         the class's L panel of that sector; column c of psi block j of sector l' is column c of
         the T1 panel at t1pan_j (rows N_j apart)."""
         secs = sorted(info)
@@ -724,14 +729,18 @@ class SigmaOperator(object):
             sec = [int(s) for s in tc["sectors"]]
             N = [info[s][1] for s in sec]
             u = dpanel_units(tc["M"], N, tc["K"], tc["Kp"], [info[s][3] for s in sec], tc["lpoff"],
-                             [info[s][0] for s in sec], [base + col0[s] for s in sec], "col")
+                             [info[s][0] for s in sec], [base + col0[s] for s in sec], "col", kind=kind)
             parts.append((u, (poss[0], poss[-1] + 1)))
         return parts, numpy.concatenate(tabs)
 
     def _build_lpan_k(self):
         """K-major L panels [M x Kp] per sector: FP32 hi plane then lo plane for the tcgen05 kernel,
-        FP64 for the FP64 one."""
+        FP64 and FP32 for the others."""
         n = self._lp_total
+        if self.f1 is not None:
+            self.lpan32 = torch.empty(max(n, 1), dtype=torch.float32, device=self.ws.device)
+            block_permute(self._lp_descs_d, len(self._lp_descs), self._lp_span, self._lp_ops_d, self.L.values,
+                          self.lpan32)
         if self.d1 is not None:
             self.lpan64 = torch.empty(max(n, 1), dtype=torch.float64, device=self.ws.device)
             block_permute(self._lp_descs_d, len(self._lp_descs), self._lp_span, self._lp_ops_d, self.L.values,
@@ -745,8 +754,12 @@ class SigmaOperator(object):
 
     def _build_rpan_k(self):
         """K-major R panels [D_r' x Kp] per sector: FP32 hi plane then lo plane for the tcgen05
-        kernel, FP64 for the FP64 one."""
+        kernel, FP64 and FP32 for the others."""
         n = self._rt_total
+        if self.f4 is not None:
+            self.rpan32 = torch.empty(max(n, 1), dtype=torch.float32, device=self.ws.device)
+            block_permute(self._rt_descs_d, len(self._rt_descs), self._rt_span, self._rt_ops_d, self.R.values,
+                          self.rpan32)
         if self.d4 is not None:
             self.rpan64 = torch.empty(max(n, 1), dtype=torch.float64, device=self.ws.device)
             block_permute(self._rt_descs_d, len(self._rt_descs), self._rt_span, self._rt_ops_d, self.R.values,
@@ -863,6 +876,11 @@ class SigmaOperator(object):
                 out.append((0, native.GROUP_PANEL, self.tc1.d_units.data_ptr(), self.tc1.ntasks, 1, 0, 0))
         return out
 
+    def _x32(self, x):
+        x32 = self.ws.get("x32", self.ndim0, torch.float32)
+        convert(x, x32)
+        return x32
+
     def __call__(self, x, y=None, precision=None):
         """x: device tensor (ndim0,) float64 -> y = H x (float64).
 
@@ -898,9 +916,7 @@ class SigmaOperator(object):
         kind = prec if prec in ("tf32", "tf32x3") else "f32"
         T1 = ws.get("t1", self.tot[0], torch.float32)
         T3 = ws.get("t3", self.tot[2], torch.float32)
-        x32 = ws.get("x32", self.ndim0, torch.float32)
         y32 = ws.get("y32", self.ndim0, torch.float32)
-        convert(x, x32)
         P = ws.get("part32", self.nops * self.ndim0, torch.float32)
         s = self._stages
         if self.tc1 is not None and kind == "tf32x3":
@@ -908,9 +924,13 @@ class SigmaOperator(object):
             gather_split(x, self._psi_gidx, pt[:self._psi_total], pt[self._psi_total:2 * self._psi_total])
             self.tc1.run(self.lpan_tc, pt, T1)
             if self._s0_generic is not None:
-                self._s0_generic.run(self.a1("f32"), x32, T1, "f32")
+                self._s0_generic.run(self.a1("f32"), self._x32(x), T1, "f32")
+        elif self.f1 is not None and kind == "f32":
+            pt = ws.get("psiT", self._psi_total, torch.float32)
+            gather_pad(x, self._psi_gidx, pt)
+            self.f1.run(self.lpan32, pt, T1)
         else:
-            s[0].run(self.a1("f32"), x32, T1, kind)
+            s[0].run(self.a1("f32"), self._x32(x), T1, kind)
         if self.wx is not None:
             self.wx.run(T1, None, T3, "f32")
         else:
@@ -922,6 +942,8 @@ class SigmaOperator(object):
         P[:self.nops * self.ndim0].zero_()
         if self.tc4 is not None and kind == "tf32x3":
             self.tc4.run(T3, self.rpan_tc, P)
+        elif self.f4 is not None and kind == "f32":
+            self.f4.run(T3, self.rpan32, P)
         else:
             s[3].run(T3, self.b4("f32"), P, kind)
         reduce_ops(P, self.nops, self.ndim0, y32)

@@ -78,6 +78,8 @@ _SIGS = {
     "qc_fgemm_f64": (c_int, [c_vp, c_ll, c_vp, c_vp, c_vp, c_vp, c_int, c_int, c_int, c_vp, c_vp, c_vp, c_vp]),
     "qc_fgemm_f32": (c_int, [c_vp, c_ll, c_vp, c_vp, c_vp, c_vp, c_int, c_int, c_int, c_vp, c_vp, c_vp, c_vp]),
     "qc_dpanel_f64": (c_int, [c_vp, c_vp, c_ll] + [c_vp] * 7),
+    "qc_dpanel_f32": (c_int, [c_vp, c_vp, c_ll] + [c_vp] * 7),
+    "qc_gather_pad_f32": (c_int, [c_vp, c_vp, c_ll, c_vp, c_vp]),
     "qc_gather_pad_f64": (c_int, [c_vp, c_vp, c_ll, c_vp, c_vp]),
     "qc_wx_build": (c_int, [c_int] + [c_vp] * 12 + [c_int] + [c_vp] * 7),
     "qc_wx_fetch": (c_int, [c_vp, c_ll, c_int, c_vp, c_vp, c_vp, c_vp, c_vp]),

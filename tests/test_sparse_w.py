@@ -66,7 +66,7 @@ def interpret_panel(st, A, B, C):
     hits = numpy.zeros(len(c), dtype=numpy.int64)
     for w in st.h_work:
         u, o = st.h_units[w[0]], st.host_ops[w[1]]
-        assert 0 < u["mrem"] <= 128 and 0 < u["nrem"] <= 64
+        assert 0 < u["mrem"] <= engine.DP_TILE[st.kind][0] and 0 < u["nrem"] <= engine.DP_TILE[st.kind][1]
         assert (u["a_off"] + o["a_base"]) % 4 == 0 and (u["b_off"] + o["b_base"]) % 4 == 0 and u["lda"] % 4 == 0
         m, n, k = (numpy.arange(u[x]) for x in ("mrem", "nrem", "K"))
         blk = st.h_cols is None and st.h_crow is None
@@ -144,6 +144,11 @@ def test_sparse_records_reproduce_the_separate_stages(tag, monkeypatch):
         assert interpret_panel(sig.d4, tb, sig.rpan64, part).max() == 1
         sig._stages[3].run(tb, sig.b4("f64"), ref4, "f64")
         assert numpy.abs((part - ref4).numpy()).max() <= 1e-13 * max(1.0, ref4.abs().max().item())
+        # the FP32 panels: the same elements, each once; operands rounded to 2^-24, sums below 2^5 terms
+        for st, a, b, out in ((sig.f1, sig.lpan32, psi, T0), (sig.f4, tb, sig.rpan32, ref4)):
+            c = torch.zeros_like(out)
+            assert interpret_panel(st, a, b, c).max() == 1
+            assert numpy.abs((c - out).numpy()).max() <= 1e-5 * max(1.0, out.abs().max().item())
 
 
 @pytest.mark.parametrize("tag", ["SP_K4", "SP_K5"])
