@@ -260,6 +260,31 @@ int qc_wsparse_f32(const void *items, long long nitems, int tile, const void *de
                    const void *rows, const void *dops, const void *octs, const void *ent_w, const void *ent_r,
                    const void *ops, int maxR, int maxO, const float *A, float *C, void *stream);
 
+/* The five steps of a matrix-vector product in panel form as one call: psi panels, L.psi, the
+ * sparse MPO stage, .R, the sum over operators.  All pointers are device memory.  f32: panels,
+ * intermediates and coefficients are FP32 (x and y stay FP64); clear: .R leaves parts of the
+ * partial vectors untouched, which are zeroed first; table: column (first) or row (last) table. */
+typedef struct {
+  const void *units, *work;
+  long long nwork;
+  const void *ops, *table;
+} qc_sigma_panel;
+typedef struct {
+  const void *items;
+  long long n;
+  int tile, maxr, maxo, pad;
+} qc_sigma_tiles;
+typedef struct {
+  int f32, nops, clear, pad;
+  long long ndim, npsi;
+  const long long *psi_idx;
+  qc_sigma_panel first, last;
+  const void *deltas, *groups, *rows, *dops, *octs, *ent_w, *ent_r, *wops;
+  qc_sigma_tiles tiles[3];
+} qc_sigma_plan;
+int qc_sigma_panels(const qc_sigma_plan *p, const void *lpan, const void *rpan, const double *x, void *psi, void *t1,
+                    void *t3, void *part, double *y, void *stream);
+
 /* W panels of the dense fiber-group GEMM assembled from their W blocks (the form the plan
  * compiler emits; the W blocks are those of the pair lists of tensordotSYM for
  * top2 = tensordot(top1, W_i) / top3 = tensordot(top2, W_j), kernelQt.py:301-306):

@@ -200,12 +200,12 @@ __global__ void k_f32_to_f64(const float *__restrict__ s, double *__restrict__ d
     d[i] = (double)s[i];
 }
 
-template <typename T>
-__global__ void k_reduce_ops(const T *__restrict__ part, int nops, long long n, T *__restrict__ out) {
+template <typename T, typename O>
+__global__ void k_reduce_ops(const T *__restrict__ part, int nops, long long n, O *__restrict__ out) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     T acc = T(0);
     for (int o = 0; o < nops; ++o) acc += part[(long long)o * n + i];   // fixed order: reproducible
-    out[i] = acc;
+    out[i] = O(acc);
   }
 }
 
@@ -225,11 +225,14 @@ __attribute__((visibility("hidden"))) int qc_internal_bgemm_f64(const void *task
   return launch_bgemm<double>(tasks, ntasks, opspan, contribs, ops, summed, A, B, C, cfg, s);
 }
 
-__attribute__((visibility("hidden"))) int qc_internal_reduce_f64(const double *part, int nops, long long n,
-                                                                 double *out, cudaStream_t s) {
+__attribute__((visibility("hidden"))) int qc_internal_reduce(const void *part, int f32, int nops, long long n,
+                                                             double *out, cudaStream_t s) {
   if (n <= 0) return QC_OK;
-  k_reduce_ops<double><<<grid_for(n), 256, 0, s>>>(part, nops, n, out);
-  return cuda_fail("qc_internal_reduce_f64");
+  if (f32)
+    k_reduce_ops<float, double><<<grid_for(n), 256, 0, s>>>((const float *)part, nops, n, out);
+  else
+    k_reduce_ops<double, double><<<grid_for(n), 256, 0, s>>>((const double *)part, nops, n, out);
+  return cuda_fail("qc_internal_reduce");
 }
 
 extern "C" int qc_bgemm_f64(const void *tasks, long long ntasks, int opspan, const void *contribs, const void *ops,
@@ -278,13 +281,13 @@ extern "C" int qc_scatter_f64(const double *src, const long long *idx, double *d
 
 extern "C" int qc_reduce_ops_f64(const double *part, int nops, long long n, double *out, void *stream) {
   if (n <= 0) return QC_OK;
-  k_reduce_ops<double><<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(part, nops, n, out);
+  k_reduce_ops<double, double><<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(part, nops, n, out);
   return cuda_fail("qc_reduce_ops_f64");
 }
 
 extern "C" int qc_reduce_ops_f32(const float *part, int nops, long long n, float *out, void *stream) {
   if (n <= 0) return QC_OK;
-  k_reduce_ops<float><<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(part, nops, n, out);
+  k_reduce_ops<float, float><<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(part, nops, n, out);
   return cuda_fail("qc_reduce_ops_f32");
 }
 

@@ -43,7 +43,7 @@ static __device__ __align__(256) double g_noalloc_scratch[QC_NOALLOC_SCRATCH_DOU
 
 int qc_internal_bgemm_f64(const void *tasks, long long ntasks, int opspan, const void *contribs, const void *ops,
                           int summed, const double *A, const double *B, double *C, int cfg, cudaStream_t s);
-int qc_internal_reduce_f64(const double *part, int nops, long long n, double *out, cudaStream_t s);
+int qc_internal_reduce(const void *part, int f32, int nops, long long n, double *out, cudaStream_t s);
 
 static thread_local std::string g_noalloc_err;
 static std::mutex g_noalloc_mu;
@@ -114,7 +114,7 @@ extern "C" int qc_sigma_f64_noalloc(int ngroups, const int *group_stage, const v
                                0, A, B, C, group_cfg[g], s);
     if (rc != QC_OK) return noalloc_fail(rc, "qc_sigma_f64_noalloc: kernel launch failed");
   }
-  rc = qc_internal_reduce_f64(P, nops, ndim0, y, s);
+  rc = qc_internal_reduce(P, 0, nops, ndim0, y, s);
   if (rc != QC_OK) return noalloc_fail(rc, "qc_sigma_f64_noalloc: reduction launch failed");
   return QC_OK;
 }

@@ -25,6 +25,7 @@
 // pipe (75 %); copying alone takes 2.2 and 1.3 ms of it.  Twelve warps of deeper prefetch: 5.99, 4.11.
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
@@ -39,6 +40,7 @@ constexpr int WX_WARPS = 16;
 constexpr int WX_THREADS = 32 * WX_WARPS;
 constexpr int WX_MAXOCT = 512;            // octets of one (delta, operator)
 constexpr int WX_GRPS = 32;               // sector pairs of one tile
+constexpr int WX_MAXSMEM = 224 * 1024;
 
 __device__ __forceinline__ void cp_async_el(float *dst, const float *src, bool valid) {
   const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
@@ -402,12 +404,19 @@ struct WxArgs {
   int maxR, maxO;
 };
 
-template <typename T, typename W, typename K>
-int launch_kernel(K kernel, size_t smem, const WxArgs &x, const T *A, T *C, cudaStream_t s) {
-  if (smem > 224 * 1024) return QC_ERR_ARG;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+template <typename T, typename W, auto Kernel>
+int launch_kernel(size_t smem, const WxArgs &x, const T *A, T *C, cudaStream_t s) {
+  if (smem > WX_MAXSMEM) return QC_ERR_ARG;
+  // the limit belongs to a kernel on a device: raised once for each
+  static std::atomic<bool> raised[64];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess && (dev >= 64 || !raised[dev].load(std::memory_order_relaxed))) {
+    e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WX_MAXSMEM);
+    if (e == cudaSuccess && dev < 64) raised[dev].store(true, std::memory_order_relaxed);
+  }
   if (e == cudaSuccess) {
-    kernel<<<(unsigned)x.nitems, WX_THREADS, smem, s>>>(
+    Kernel<<<(unsigned)x.nitems, WX_THREADS, smem, s>>>(
         (const qc_wxitem *)x.items, (const qc_wxdelta *)x.deltas, (const qc_wxgrp *)x.grps, (const int *)x.rows,
         (const qc_wxdop *)x.dops, (const qc_wxoct *)x.octs, (const W *)x.ent_w, (const int *)x.ent_r,
         (const qc_op *)x.ops, x.maxR, x.maxO, A, C);
@@ -753,9 +762,9 @@ extern "C" int qc_wsparse_f64(const void *items, long long nitems, int tile, con
   if (wx_bad(x)) return QC_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   switch (tile) {
-    case 32: return launch_kernel<double, double>(k_wsparse_f64<32>, wx_smem_bytes<double, 32>(maxR, maxO), x, A, C, s);
-    case 64: return launch_kernel<double, double>(k_wsparse_f64<64>, wx_smem_bytes<double, 64>(maxR, maxO), x, A, C, s);
-    case 128: return launch_kernel<double, double>(k_wsparse_f64<128>, wx_smem_bytes<double, 128>(maxR, maxO), x, A, C, s);
+    case 32: return launch_kernel<double, double, k_wsparse_f64<32>>(wx_smem_bytes<double, 32>(maxR, maxO), x, A, C, s);
+    case 64: return launch_kernel<double, double, k_wsparse_f64<64>>(wx_smem_bytes<double, 64>(maxR, maxO), x, A, C, s);
+    case 128: return launch_kernel<double, double, k_wsparse_f64<128>>(wx_smem_bytes<double, 128>(maxR, maxO), x, A, C, s);
     default: return QC_ERR_ARG;
   }
 }
@@ -769,9 +778,9 @@ extern "C" int qc_wsparse_f32(const void *items, long long nitems, int tile, con
   if (wx_bad(x)) return QC_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   switch (tile) {
-    case 32: return launch_kernel<float, float4>(k_wsparse_f32<32, 32>, wx_smem_bytes<float, 32>(maxR, maxO), x, A, C, s);
-    case 64: return launch_kernel<float, float4>(k_wsparse_f32<64, 64>, wx_smem_bytes<float, 64>(maxR, maxO), x, A, C, s);
-    case 128: return launch_kernel<float, float4>(k_wsparse_f32<128, 64>, wx_smem_bytes<float, 128>(maxR, maxO), x, A, C, s);
+    case 32: return launch_kernel<float, float4, k_wsparse_f32<32, 32>>(wx_smem_bytes<float, 32>(maxR, maxO), x, A, C, s);
+    case 64: return launch_kernel<float, float4, k_wsparse_f32<64, 64>>(wx_smem_bytes<float, 64>(maxR, maxO), x, A, C, s);
+    case 128: return launch_kernel<float, float4, k_wsparse_f32<128, 64>>(wx_smem_bytes<float, 128>(maxR, maxO), x, A, C, s);
     default: return QC_ERR_ARG;
   }
 }

@@ -1778,6 +1778,13 @@ class DPanelStage(object):
             if crow is not None else None
         self.d_cols = upload(cols, device) if cols is not None else None
 
+    def record(self):
+        """The launch as a native.SigmaPanel (pointers to this stage's device tables)."""
+        if self.ntasks == 0:
+            return native.SigmaPanel()
+        return native.SigmaPanel(self.d_units.data_ptr(), self.d_work.data_ptr(), self.ntasks, self.d_ops.data_ptr(),
+                                 (self.d_crow if self.d_cols is None else self.d_cols).data_ptr())
+
     def run(self, A, B, C, stream=None):
         if self.ntasks == 0:
             return

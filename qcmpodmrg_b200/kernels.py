@@ -13,6 +13,8 @@ scratch and the sum over operators done inside the last launch (no atomics).
 Block-pair lists are built per symmetry class of the operator, as the
 reference caches its templates per class.
 """
+import ctypes
+
 import numpy
 import torch
 
@@ -430,6 +432,7 @@ class SigmaOperator(object):
                 self._stages.append(CompositeStage(f + [g], "sigma%d" % (si + 1)))
         # the two MPO-site contractions as one sparse product, T1 -> T3
         self.wx = None
+        self._plans, self._part_full = {}, False
         if sparse_w:
             w1, w2 = Wi.host(), Wj.host()
             parts = [(x, rng, (WSource.of(x["W"][0], w1, Wi.offsets[ops]), WSource.of(x["W"][1], w2, Wj.offsets[ops])))
@@ -642,6 +645,9 @@ class SigmaOperator(object):
         if tc:
             units, maps = tc_sigma4_units(classes, None, t3b, rtb, rts, rt_tot)
             self.tc4 = TCPanelStage("sigma4", units, maps, st4_ops, crow, flops, dev)
+        # .R writes every element of every partial vector (none twice)
+        self._part_full = sum(len(poss) for poss, _, _ in classes) == len(order) and \
+            all(int((sec["M"] * sec["N"]).sum()) == self.psi.size for _, sec, _ in classes)
         self._rt_total = rt_tot
         self._rt_descs = numpy.concatenate(descs)
         self._rt_descs_d = upload(self._rt_descs, dev)
@@ -821,8 +827,8 @@ class SigmaOperator(object):
         self.L = self.R = None
         self.Lpan = self._Lpan32 = None
         self.Rpan = self._Rpan32 = None
-        self.rpan_tc = self.rpan64 = None
-        self.lpan_tc = self.lpan64 = None
+        self.rpan_tc = self.rpan64 = self.rpan32 = None
+        self.lpan_tc = self.lpan64 = self.lpan32 = None
 
     def wij32(self):
         if self._Wij32 is None:
@@ -876,6 +882,39 @@ class SigmaOperator(object):
                 out.append((0, native.GROUP_PANEL, self.tc1.d_units.data_ptr(), self.tc1.ntasks, 1, 0, 0))
         return out
 
+    def _native_plan(self, kind):
+        """The launches of one product in `kind` as a native.SigmaPlan: pointers to device tables
+        that this operator owns."""
+        p = self._plans.get(kind)
+        if p is None:
+            d, w = self.wx.d, self.wx
+            first, last = (self.d1, self.d4) if kind == "f64" else (self.f1, self.f4)
+            p = native.SigmaPlan(int(kind == "f32"), self.nops, int(not self._part_full), 0, self.ndim0,
+                                 self._psi_gidx.numel(), self._psi_gidx.data_ptr(), first.record(), last.record())
+            n = 0
+            if w.ntasks:
+                p.deltas, p.groups, p.rows, p.dops, p.octs, p.ent_r, p.wops = (
+                    d[k].data_ptr() for k in ("deltas", "groups", "rows", "dops", "octs", "ent_r", "ops"))
+                p.ent_w = w._w[kind].data_ptr()
+                for tile, host, dev, maxr, maxo in w.items(kind):
+                    p.tiles[n] = native.SigmaTiles(dev.data_ptr(), len(host), tile, maxr, maxo, 0)
+                    n += 1
+            self._plans[kind] = p = (ctypes.byref(p), p, n + 4)
+        return p
+
+    def _run_panels(self, kind, x, y):
+        dt = torch.float64 if kind == "f64" else torch.float32
+        ws = self.ws
+        ref, _, launches = self._native_plan(kind)
+        lpan, rpan = (self.lpan64, self.rpan64) if kind == "f64" else (self.lpan32, self.rpan32)
+        check(native.lib().qc_sigma_panels(
+            ref, lpan.data_ptr(), rpan.data_ptr(), x.data_ptr(), ws.get("psi_pan", self._psi_total, dt).data_ptr(),
+            ws.get("t1", self.tot[0], dt).data_ptr(), ws.get("t3", self.tot[2], dt).data_ptr(),
+            ws.get("part", self.nops * self.ndim0, dt).data_ptr(), y.data_ptr(), _stream(y.device)),
+            "qc_sigma_panels")
+        LOG.launches += launches
+        return y
+
     def _x32(self, x):
         x32 = self.ws.get("x32", self.ndim0, torch.float32)
         convert(x, x32)
@@ -890,17 +929,22 @@ class SigmaOperator(object):
         prec = precision or self.precision
         if y is None:
             y = torch.empty(self.ndim0, dtype=torch.float64, device=ws.device)
+        # in panel form all through: one native call (the launch log times the stages one by one)
+        if self.wx is not None and (prec == "f64" or (prec == "f32" and self.f1 is not None)) and x.is_cuda \
+                and not LOG.enabled:
+            return self._run_panels(prec, x, y)
         if prec == "f64":
             T1 = ws.get("t1", self.tot[0], torch.float64)
             T3 = ws.get("t3", self.tot[2], torch.float64)
             P = ws.get("part", self.nops * self.ndim0, torch.float64)
             s = self._stages
             if self.wx is not None:
-                pt = ws.get("psiT64", self._psi_total, torch.float64)
+                pt = ws.get("psi_pan", self._psi_total, torch.float64)
                 gather_pad(x, self._psi_gidx, pt)
                 self.d1.run(self.lpan64, pt, T1)
                 self.wx.run(T1, None, T3, "f64")
-                P[:self.nops * self.ndim0].zero_()
+                if not self._part_full:
+                    P[:self.nops * self.ndim0].zero_()
                 self.d4.run(T3, self.rpan64, P)
                 return reduce_ops(P, self.nops, self.ndim0, y)
             else:
@@ -917,7 +961,7 @@ class SigmaOperator(object):
         T1 = ws.get("t1", self.tot[0], torch.float32)
         T3 = ws.get("t3", self.tot[2], torch.float32)
         y32 = ws.get("y32", self.ndim0, torch.float32)
-        P = ws.get("part32", self.nops * self.ndim0, torch.float32)
+        P = ws.get("part", self.nops * self.ndim0, torch.float32)
         s = self._stages
         if self.tc1 is not None and kind == "tf32x3":
             pt = ws.get("psiT", 2 * self._psi_total, torch.float32)
@@ -926,7 +970,7 @@ class SigmaOperator(object):
             if self._s0_generic is not None:
                 self._s0_generic.run(self.a1("f32"), self._x32(x), T1, "f32")
         elif self.f1 is not None and kind == "f32":
-            pt = ws.get("psiT", self._psi_total, torch.float32)
+            pt = ws.get("psi_pan", self._psi_total, torch.float32)
             gather_pad(x, self._psi_gidx, pt)
             self.f1.run(self.lpan32, pt, T1)
         else:

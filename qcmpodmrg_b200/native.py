@@ -31,6 +31,21 @@ def _load(name):
     return ctypes.CDLL(path)
 
 
+class SigmaPanel(ctypes.Structure):
+    _fields_ = [("units", c_vp), ("work", c_vp), ("nwork", c_ll), ("ops", c_vp), ("table", c_vp)]
+
+
+class SigmaTiles(ctypes.Structure):
+    _fields_ = [("items", c_vp), ("n", c_ll), ("tile", c_int), ("maxr", c_int), ("maxo", c_int), ("pad", c_int)]
+
+
+class SigmaPlan(ctypes.Structure):
+    _fields_ = [("f32", c_int), ("nops", c_int), ("clear", c_int), ("pad", c_int), ("ndim", c_ll), ("npsi", c_ll),
+                ("psi_idx", c_vp), ("first", SigmaPanel), ("last", SigmaPanel)] + \
+               [(n, c_vp) for n in ("deltas", "groups", "rows", "dops", "octs", "ent_w", "ent_r", "wops")] + \
+               [("tiles", SigmaTiles * 3)]
+
+
 _lib = None
 _qsym = None
 
@@ -79,6 +94,7 @@ _SIGS = {
     "qc_fgemm_f32": (c_int, [c_vp, c_ll, c_vp, c_vp, c_vp, c_vp, c_int, c_int, c_int, c_vp, c_vp, c_vp, c_vp]),
     "qc_dpanel_f64": (c_int, [c_vp, c_vp, c_ll] + [c_vp] * 7),
     "qc_dpanel_f32": (c_int, [c_vp, c_vp, c_ll] + [c_vp] * 7),
+    "qc_sigma_panels": (c_int, [c_vp] * 10),
     "qc_gather_pad_f32": (c_int, [c_vp, c_vp, c_ll, c_vp, c_vp]),
     "qc_gather_pad_f64": (c_int, [c_vp, c_vp, c_ll, c_vp, c_vp]),
     "qc_wx_build": (c_int, [c_int] + [c_vp] * 12 + [c_int] + [c_vp] * 7),
