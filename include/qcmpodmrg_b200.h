@@ -260,6 +260,12 @@ int qc_wsparse_f32(const void *items, long long nitems, int tile, const void *de
                    const void *rows, const void *dops, const void *octs, const void *ent_w, const void *ent_r,
                    const void *ops, int maxR, int maxO, const float *A, float *C, void *stream);
 
+/* out = r orthonormalised against the m <= 32 rows of V [m x n] in `times` Gram-Schmidt passes
+ * (dvdson_ortho, source/tools/pdvdson.py:350-390, for one vector); work: qc_ortho_work() doubles,
+ * the first of which receives the norm before the normalisation.  out is not r. */
+long long qc_ortho_work(void);
+int qc_ortho(const double *V, int m, long long n, const double *r, double *out, double *work, int times, void *stream);
+
 /* The five steps of a matrix-vector product in panel form as one call: psi panels, L.psi, the
  * sparse MPO stage, .R, the sum over operators.  All pointers are device memory.  f32: panels,
  * intermediates and coefficients are FP32 (x and y stay FP64); clear: .R leaves parts of the

@@ -12,12 +12,23 @@ the reference's HVecs does (:67-78).
 """
 import torch
 
+from . import native
+
 # a start vector of smaller norm carries no usable direction (a projected guess whose
 # weight lies outside the dot's blocks is rounding noise)
 V0_MIN_NORM = 1.e-8
 
 
 def _ortho(vbas, rbas, crit_indp, times=5):
+    if rbas.is_cuda and rbas.dtype == torch.float64 and rbas.shape[0] == 1 and vbas.shape[0] <= 32:
+        # one new vector (a single root): the passes in fused kernels
+        v, r = vbas.contiguous(), rbas.contiguous()
+        out = torch.empty_like(r)
+        work = torch.empty(native.lib().qc_ortho_work(), dtype=r.dtype, device=r.device)
+        native.check(native.lib().qc_ortho(v.data_ptr(), v.shape[0], v.shape[1], r.data_ptr(), out.data_ptr(),
+                                           work.data_ptr(), times, torch.cuda.current_stream(r.device).cuda_stream),
+                     "qc_ortho")
+        return (0, None) if float(work[0]) <= crit_indp else (1, out)
     rbas = rbas.clone()
     for _ in range(times):
         rbas = rbas - (rbas @ vbas.T) @ vbas
@@ -31,7 +42,7 @@ def _ortho(vbas, rbas, crit_indp, times=5):
         r = r / torch.linalg.norm(r)
         out.append(r)
         v2 = torch.stack(out)
-        for _ in range(times):
+        for _ in range(times if i + 1 < rbas.shape[0] else 0):
             rbas[i:] -= (rbas[i:] @ vbas.T) @ vbas
             rbas[i:] -= (rbas[i:] @ v2.T) @ v2
     if not out:

@@ -94,6 +94,8 @@ _SIGS = {
     "qc_fgemm_f32": (c_int, [c_vp, c_ll, c_vp, c_vp, c_vp, c_vp, c_int, c_int, c_int, c_vp, c_vp, c_vp, c_vp]),
     "qc_dpanel_f64": (c_int, [c_vp, c_vp, c_ll] + [c_vp] * 7),
     "qc_dpanel_f32": (c_int, [c_vp, c_vp, c_ll] + [c_vp] * 7),
+    "qc_ortho_work": (c_ll, []),
+    "qc_ortho": (c_int, [c_vp, c_int, c_ll, c_vp, c_vp, c_vp, c_int, c_vp]),
     "qc_sigma_panels": (c_int, [c_vp] * 10),
     "qc_gather_pad_f32": (c_int, [c_vp, c_vp, c_ll, c_vp, c_vp]),
     "qc_gather_pad_f64": (c_int, [c_vp, c_vp, c_ll, c_vp, c_vp]),
