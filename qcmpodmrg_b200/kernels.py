@@ -744,9 +744,9 @@ class SigmaOperator(object):
         FP64 and FP32 for the others."""
         n = self._lp_total
         if self.f1 is not None:
-            self.lpan32 = torch.empty(max(n, 1), dtype=torch.float32, device=self.ws.device)
+            self.lpan_f32 = torch.empty(max(n, 1), dtype=torch.float32, device=self.ws.device)
             block_permute(self._lp_descs_d, len(self._lp_descs), self._lp_span, self._lp_ops_d, self.L.values,
-                          self.lpan32)
+                          self.lpan_f32)
         if self.d1 is not None:
             self.lpan64 = torch.empty(max(n, 1), dtype=torch.float64, device=self.ws.device)
             block_permute(self._lp_descs_d, len(self._lp_descs), self._lp_span, self._lp_ops_d, self.L.values,
@@ -763,9 +763,9 @@ class SigmaOperator(object):
         kernel, FP64 and FP32 for the others."""
         n = self._rt_total
         if self.f4 is not None:
-            self.rpan32 = torch.empty(max(n, 1), dtype=torch.float32, device=self.ws.device)
+            self.rpan_f32 = torch.empty(max(n, 1), dtype=torch.float32, device=self.ws.device)
             block_permute(self._rt_descs_d, len(self._rt_descs), self._rt_span, self._rt_ops_d, self.R.values,
-                          self.rpan32)
+                          self.rpan_f32)
         if self.d4 is not None:
             self.rpan64 = torch.empty(max(n, 1), dtype=torch.float64, device=self.ws.device)
             block_permute(self._rt_descs_d, len(self._rt_descs), self._rt_span, self._rt_ops_d, self.R.values,
@@ -827,8 +827,8 @@ class SigmaOperator(object):
         self.L = self.R = None
         self.Lpan = self._Lpan32 = None
         self.Rpan = self._Rpan32 = None
-        self.rpan_tc = self.rpan64 = self.rpan32 = None
-        self.lpan_tc = self.lpan64 = self.lpan32 = None
+        self.rpan_tc = self.rpan64 = self.rpan_f32 = None
+        self.lpan_tc = self.lpan64 = self.lpan_f32 = None
 
     def wij32(self):
         if self._Wij32 is None:
@@ -906,7 +906,7 @@ class SigmaOperator(object):
         dt = torch.float64 if kind == "f64" else torch.float32
         ws = self.ws
         ref, _, launches = self._native_plan(kind)
-        lpan, rpan = (self.lpan64, self.rpan64) if kind == "f64" else (self.lpan32, self.rpan32)
+        lpan, rpan = (self.lpan64, self.rpan64) if kind == "f64" else (self.lpan_f32, self.rpan_f32)
         check(native.lib().qc_sigma_panels(
             ref, lpan.data_ptr(), rpan.data_ptr(), x.data_ptr(), ws.get("psi_pan", self._psi_total, dt).data_ptr(),
             ws.get("t1", self.tot[0], dt).data_ptr(), ws.get("t3", self.tot[2], dt).data_ptr(),
@@ -972,7 +972,7 @@ class SigmaOperator(object):
         elif self.f1 is not None and kind == "f32":
             pt = ws.get("psi_pan", self._psi_total, torch.float32)
             gather_pad(x, self._psi_gidx, pt)
-            self.f1.run(self.lpan32, pt, T1)
+            self.f1.run(self.lpan_f32, pt, T1)
         else:
             s[0].run(self.a1("f32"), self._x32(x), T1, kind)
         if self.wx is not None:
@@ -987,7 +987,7 @@ class SigmaOperator(object):
         if self.tc4 is not None and kind == "tf32x3":
             self.tc4.run(T3, self.rpan_tc, P)
         elif self.f4 is not None and kind == "f32":
-            self.f4.run(T3, self.rpan32, P)
+            self.f4.run(T3, self.rpan_f32, P)
         else:
             s[3].run(T3, self.b4("f32"), P, kind)
         reduce_ops(P, self.nops, self.ndim0, y32)

@@ -145,7 +145,7 @@ def test_sparse_records_reproduce_the_separate_stages(tag, monkeypatch):
         sig._stages[3].run(tb, sig.b4("f64"), ref4, "f64")
         assert numpy.abs((part - ref4).numpy()).max() <= 1e-13 * max(1.0, ref4.abs().max().item())
         # the FP32 panels: the same elements, each once; operands rounded to 2^-24, sums below 2^5 terms
-        for st, a, b, out in ((sig.f1, sig.lpan32, psi, T0), (sig.f4, tb, sig.rpan32, ref4)):
+        for st, a, b, out in ((sig.f1, sig.lpan_f32, psi, T0), (sig.f4, tb, sig.rpan_f32, ref4)):
             c = torch.zeros_like(out)
             assert interpret_panel(st, a, b, c).max() == 1
             assert numpy.abs((c - out).numpy()).max() <= 1e-5 * max(1.0, out.abs().max().item())
