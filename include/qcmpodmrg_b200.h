@@ -243,16 +243,13 @@ int qc_gather_pad_f64(const double *x, const long long *idx, long long n, double
 
 /* Sparse MPO stage: T3 = T1 . (W_i W_{i+1}) for every operator (records qc_wxitem /
  * qc_wxdelta / qc_wxgrp / qc_wxdop / qc_wxoct of qc_types.h).  qc_wx_build makes the sparse
- * rows of one operator class on the host (w1 / w2: FP64 values, operator o at off1[o] /
- * off2[o]; ns / nd / ioff / allowed: the two layouts), qc_wx_fetch copies them out and frees
+ * rows of operator classes on the host (parts: qc_wxpart records of qc_types.h; nocts, nents: one
+ * count per class), qc_wx_fetch copies them out, class after class, and frees
  * the handle.  qc_wsparse_*: items of one tile width (32, 64 or 128 fibers); ent_w: the
  * coefficients in the precision's order (qc_wx_fetch: w64 / w32); maxR / maxO: most T1 rows /
  * octets of any item's charge difference. */
-int qc_wx_build(int nops, const double *w1, const long long *off1, const int *ns1, const long long *nd1,
-                const long long *ioff1, const int *allowed1, const double *w2, const long long *off2, const int *ns2,
-                const long long *nd2, const long long *ioff2, const int *allowed2, int ndelta, const int *iblk,
-                const int *kblk, const int *row0, const int *R, void **handle, long long *nocts, long long *nents);
-int qc_wx_fetch(void *handle, long long ent0, int oct0, void *dops, void *octs, double *w64, float *w32, int *r);
+int qc_wx_build(int nparts, const void *parts, void **handle, long long *nocts, long long *nents);
+int qc_wx_fetch(void *handle, void *dops, void *octs, double *w64, float *w32, int *r);
 int qc_wsparse_f64(const void *items, long long nitems, int tile, const void *deltas, const void *grps,
                    const void *rows, const void *dops, const void *octs, const void *ent_w, const void *ent_r,
                    const void *ops, int maxR, int maxO, const double *A, double *C, void *stream);

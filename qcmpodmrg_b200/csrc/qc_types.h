@@ -276,6 +276,27 @@ struct alignas(16) qc_dunit {
 };
 static_assert(sizeof(qc_dunit) == 64, "qc_dunit is 64 bytes");
 
+// One operator class of a sparse MPO stage, as its host builder reads it: packed FP64 values of both
+// factors (operator o at off1[o] / off2[o]), their layouts (sector counts, extents of the four
+// axes back to back, block offsets, allowed blocks); iblk / kblk / row0 [ndelta][16]: left
+// (right) MPO sector of every (n1, n2) ((n1', n2')) block of a delta (-1: none) and its first
+// T1 row; R: T1 rows of every delta.
+struct qc_wxpart {
+  const double *w1;
+  const long long *off1;
+  const int *ns1;
+  const long long *nd1, *ioff1;
+  const int *allowed1;
+  const double *w2;
+  const long long *off2;
+  const int *ns2;
+  const long long *nd2, *ioff2;
+  const int *allowed2;
+  const int *iblk, *kblk, *row0, *R;
+  int nops, ndelta;
+};
+static_assert(sizeof(qc_wxpart) == 136, "qc_wxpart is 136 bytes");
+
 struct qc_dcol {
   int off, ld;
 };

@@ -452,7 +452,7 @@ struct SparseW {
 struct OpLists {
   std::vector<qc_wxdop> dops;
   std::vector<qc_wxoct> octs;
-  std::vector<double> w;       // [entry][8]
+  std::vector<double> w;       // four entries a step: [step][row][entry of the step]
   std::vector<int> r;
 };
 
@@ -577,6 +577,8 @@ void build_op(const SparseW &W1, const double *v1, const SparseW &W2, const doub
       // (one step of zero rows for an octet without entries)
       for (bool first = true; first || rest > 0; first = false) {
         bool used[4] = {false, false, false, false};
+        out.w.resize(out.w.size() + 32, 0.0);
+        double *const w = out.w.data() + out.w.size() - 32;
         for (int e = 0; e < 4; ++e) {
           int best = -1;
           for (int b = 0; b < 4; ++b)
@@ -590,7 +592,6 @@ void build_op(const SparseW &W1, const double *v1, const SparseW &W2, const doub
             while (z < 3 && used[(R + z) & 3]) ++z;
             used[(R + z) & 3] = true;
             out.r.push_back(R + z);
-            out.w.insert(out.w.end(), 8, 0.0);
             continue;
           }
           used[best] = true;
@@ -598,7 +599,7 @@ void build_op(const SparseW &W1, const double *v1, const SparseW &W2, const doub
           bucket[best].pop_back();
           --rest;
           out.r.push_back(i);
-          for (int k = 0; k < 8; ++k) out.w.push_back(k < nk ? S[(size_t)perm[k0 + k] * R + i] : 0.0);
+          for (int k = 0; k < nk; ++k) w[4 * k + e] = S[(size_t)perm[k0 + k] * R + i];
         }
       }
       x.cnt = (int)((long long)out.r.size() - rec.ent_b) - x.ent;
@@ -611,143 +612,154 @@ void build_op(const SparseW &W1, const double *v1, const SparseW &W2, const doub
 }
 
 struct WxBuild {
-  std::vector<OpLists> ops;
-  int ndelta;
+  struct Part {
+    SparseW W1, W2;
+    const qc_wxpart *in;
+    long long op0;
+  };
+  std::vector<Part> parts;
+  std::vector<OpLists> ops;      // of all parts
 };
+
+// f(0) .. f(n - 1) on the host's threads; false if one of them threw
+template <typename F>
+bool wx_each(long long n, F f) {
+  std::atomic<long long> next{0};
+  std::atomic<bool> bad{false};
+  auto loop = [&]() {
+    try {
+      for (long long i; (i = next.fetch_add(1)) < n;) f(i);
+    } catch (...) {
+      bad = true;
+    }
+  };
+  const long long hw = std::max(1u, std::thread::hardware_concurrency());
+  std::vector<std::thread> th;
+  try {
+    for (long long k = 1; k < std::min({8ll, hw, n / 4}); ++k) th.emplace_back(loop);
+  } catch (...) {              // no more threads: the others do their share
+  }
+  loop();
+  for (auto &t : th) t.join();
+  return !bad;
+}
 
 }  // namespace
 
-// Sparse rows of W_i W_{i+1} for the operators of one class.  w1 / w2: packed FP64 values
-// (host) of operator o at off1[o] / off2[o]; ns / nd / ioff / allowed: the two layouts'
-// sector counts, sector extents (four arrays back to back), block offsets and allowed
-// blocks; iblk / kblk / row0 [ndelta][16]: left (right) MPO sector of every (n1, n2)
-// ((n1', n2')) block of a delta (-1: none) and its first T1 row; R: T1 rows.  Returns the
-// quads and entries to fetch with qc_wx_fetch, which frees the handle.
-extern "C" int qc_wx_build(int nops, const double *w1, const long long *off1, const int *ns1, const long long *nd1,
-                           const long long *ioff1, const int *allowed1, const double *w2, const long long *off2,
-                           const int *ns2, const long long *nd2, const long long *ioff2, const int *allowed2,
-                           int ndelta, const int *iblk, const int *kblk, const int *row0, const int *R, void **handle,
-                           long long *nocts, long long *nents) {
-  if (nops < 1 || ndelta < 0 || !w1 || !off1 || !ns1 || !nd1 || !ioff1 || !allowed1 || !w2 || !off2 || !ns2 || !nd2 ||
-      !ioff2 || !allowed2 || (ndelta && (!iblk || !kblk || !row0 || !R)) || !handle || !nocts || !nents)
-    return QC_ERR_ARG;
-  if (ns1[2] != 4 || ns1[3] != 4 || ns2[2] != 4 || ns2[3] != 4 || ns1[1] != ns2[0]) return QC_ERR_LAYOUT;
+// Sparse rows of W_i W_{i+1} for the operators of the given classes (qc_wxpart).  Returns per class
+// the octets and entries to fetch with qc_wx_fetch, which frees the handle; the parts' arrays
+// have to stay until then.
+extern "C" int qc_wx_build(int nparts, const void *parts, void **handle, long long *nocts, long long *nents) {
+  if (nparts < 1 || !parts || !handle || !nocts || !nents) return QC_ERR_ARG;
+  const qc_wxpart *in = (const qc_wxpart *)parts;
+  WxBuild *h = nullptr;
   try {
-    SparseW W1, W2;
-    const long long *p1 = nd1, *p2 = nd2;
-    for (int k = 0; k < 4; ++k) {
-      W1.ns[k] = ns1[k];
-      W2.ns[k] = ns2[k];
-      W1.nd[k] = p1;
-      W2.nd[k] = p2;
-      p1 += ns1[k];
-      p2 += ns2[k];
-    }
-    W1.ioff = ioff1;
-    W1.allowed = allowed1;
-    W2.ioff = ioff2;
-    W2.allowed = allowed2;
-    for (int d = 0; d < ndelta; ++d)
-      for (int b = 0; b < 16; ++b) {
-        const int sa = iblk[16 * d + b], sc = kblk[16 * d + b];
-        if (sa >= ns1[0] || sc >= ns2[1]) return QC_ERR_ARG;
-        if (sa >= 0 && (row0[16 * d + b] < 0 || row0[16 * d + b] + W1.nd[0][sa] > R[d])) return QC_ERR_ARG;
+    h = new WxBuild;
+    h->parts.resize(nparts);
+    long long nops = 0;
+    int rc = QC_OK;
+    for (int q = 0; q < nparts && rc == QC_OK; ++q) {
+      const qc_wxpart &x = in[q];
+      if (x.nops < 1 || x.ndelta < 0 || !x.w1 || !x.off1 || !x.ns1 || !x.nd1 || !x.ioff1 || !x.allowed1 || !x.w2 ||
+          !x.off2 || !x.ns2 || !x.nd2 || !x.ioff2 || !x.allowed2 ||
+          (x.ndelta && (!x.iblk || !x.kblk || !x.row0 || !x.R))) {
+        rc = QC_ERR_ARG;
+        break;
       }
-    WxBuild *h = new WxBuild;
-    h->ndelta = ndelta;
-    h->ops.resize(nops);
-    bool bad = false;
-    auto work = [&](int o) {
-      build_op(W1, w1 + off1[o], W2, w2 + off2[o], ndelta, iblk, kblk, row0, R, h->ops[o]);
-    };
-    const int nt = nops >= 4 ? std::min(8, std::min(nops, (int)std::max(1u, std::thread::hardware_concurrency()))) : 1;
-    if (nt > 1) {
-      std::vector<std::thread> th;
-      std::vector<char> fail(nt, 0);
-      int started = 0;
-      try {
-        for (; started < nt; ++started)
-          th.emplace_back([&, started]() {
-            try {
-              for (int o = started; o < nops; o += nt) work(o);
-            } catch (...) {
-              fail[started] = 1;
-            }
-          });
-      } catch (...) {          // no more threads: their operators are done below
+      if (x.ns1[2] != 4 || x.ns1[3] != 4 || x.ns2[2] != 4 || x.ns2[3] != 4 || x.ns1[1] != x.ns2[0]) {
+        rc = QC_ERR_LAYOUT;
+        break;
       }
-      for (auto &t : th) t.join();
-      try {
-        for (int k = started; k < nt; ++k)
-          for (int o = k; o < nops; o += nt) work(o);
-      } catch (...) {
-        bad = true;
+      WxBuild::Part &p = h->parts[q];
+      p.in = &x;
+      p.op0 = nops;
+      nops += x.nops;
+      const long long *p1 = x.nd1, *p2 = x.nd2;
+      for (int k = 0; k < 4; ++k) {
+        p.W1.ns[k] = x.ns1[k];
+        p.W2.ns[k] = x.ns2[k];
+        p.W1.nd[k] = p1;
+        p.W2.nd[k] = p2;
+        p1 += x.ns1[k];
+        p2 += x.ns2[k];
       }
-      for (char f : fail) bad = bad || f;
-    } else {
-      try {
-        for (int o = 0; o < nops; ++o) work(o);
-      } catch (...) {
-        bad = true;
+      p.W1.ioff = x.ioff1;
+      p.W1.allowed = x.allowed1;
+      p.W2.ioff = x.ioff2;
+      p.W2.allowed = x.allowed2;
+      for (int i = 0; i < 16 * x.ndelta; ++i) {
+        const int sa = x.iblk[i], sc = x.kblk[i];
+        if (sa >= x.ns1[0] || sc >= x.ns2[1] ||
+            (sa >= 0 && (x.row0[i] < 0 || x.row0[i] + p.W1.nd[0][sa] > x.R[i / 16])))
+          rc = QC_ERR_ARG;
       }
     }
-    if (bad) {
+    if (rc == QC_OK) {
+      h->ops.resize(nops);
+      const bool ok = wx_each(nops, [&](long long o) {
+        const WxBuild::Part *p = h->parts.data() + nparts - 1;
+        while (p->op0 > o) --p;
+        const qc_wxpart &x = *p->in;
+        build_op(p->W1, x.w1 + x.off1[o - p->op0], p->W2, x.w2 + x.off2[o - p->op0], x.ndelta, x.iblk, x.kblk, x.row0,
+                 x.R, h->ops[o]);
+      });
+      rc = ok ? QC_OK : QC_ERR_CAPACITY;
+    }
+    long long nq = 0;
+    for (int q = 0; q < nparts && rc == QC_OK; ++q) {
+      nocts[q] = nents[q] = 0;
+      for (int o = 0; o < in[q].nops; ++o) {
+        const OpLists &l = h->ops[h->parts[q].op0 + o];
+        nocts[q] += (long long)l.octs.size();
+        nents[q] += (long long)l.r.size();
+      }
+      nq += nocts[q];
+    }
+    if (nq > 0x7fffffffLL) rc = QC_ERR_CAPACITY;
+    if (rc != QC_OK) {
       delete h;
-      return QC_ERR_CAPACITY;
-    }
-    long long nq = 0, ne = 0;
-    for (const OpLists &l : h->ops) {
-      nq += (long long)l.octs.size();
-      ne += (long long)l.r.size();
-    }
-    if (nq > 0x7fffffffLL) {
-      delete h;
-      return QC_ERR_CAPACITY;
+      return rc;
     }
     *handle = h;
-    *nocts = nq;
-    *nents = ne;
     return QC_OK;
   } catch (...) {
+    delete h;
     return QC_ERR_CAPACITY;
   }
 }
 
-// Copies what qc_wx_build made and frees it: dops [ndelta][nops] (entry and octet offsets from
-// ent0 / oct0), octets, T1 rows [nents] and the coefficients in the kernels' orders: FP64
-// fragments (w64: step by step, lane l the coefficient of entry l % 4 and row l / 4) and FP32
-// [nents][8] (w32); either may be null.
-extern "C" int qc_wx_fetch(void *handle, long long ent0, int oct0, void *dops, void *octs, double *w64, float *w32,
-                           int *r) {
+// Copies what qc_wx_build made, class after class, and frees it: dops [ndelta][nops] of every class,
+// octets, T1 rows and the coefficients in the kernels' orders: FP64 fragments (w64: step by
+// step, lane l the coefficient of entry l % 4 and row l / 4) and FP32 [nents][8] (w32); either
+// may be null.
+extern "C" int qc_wx_fetch(void *handle, void *dops, void *octs, double *w64, float *w32, int *r) {
   WxBuild *h = (WxBuild *)handle;
   if (!h) return QC_ERR_ARG;
-  const int nops = (int)h->ops.size();
   qc_wxdop *pd = (qc_wxdop *)dops;
   qc_wxoct *po = (qc_wxoct *)octs;
-  for (int o = 0; o < nops; ++o) {
-    const OpLists &l = h->ops[o];
-    for (int d = 0; d < h->ndelta; ++d) {
-      qc_wxdop x = l.dops[d];
-      x.ent_b += ent0;
-      x.oct_b += oct0;
-      pd[(long long)d * nops + o] = x;
+  long long ent0 = 0;
+  int oct0 = 0;
+  for (const auto &p : h->parts) {
+    const int nops = p.in->nops;
+    for (int o = 0; o < nops; ++o) {
+      const OpLists &l = h->ops[p.op0 + o];
+      for (int d = 0; d < p.in->ndelta; ++d) {
+        qc_wxdop x = l.dops[d];
+        x.ent_b += ent0;
+        x.oct_b += oct0;
+        pd[(long long)d * nops + o] = x;
+      }
+      const size_t n = l.r.size();
+      if (!l.octs.empty()) memcpy(po + oct0, l.octs.data(), l.octs.size() * sizeof(qc_wxoct));
+      if (n) memcpy(r + ent0, l.r.data(), n * sizeof(int));
+      if (w64 && n) memcpy(w64 + 8 * ent0, l.w.data(), 64 * n);
+      if (w32)
+        for (size_t e = 0; e < n; ++e)
+          for (int k = 0; k < 8; ++k) w32[8 * (ent0 + e) + k] = (float)l.w[(e & ~(size_t)3) * 8 + 4 * k + (e & 3)];
+      ent0 += (long long)n;
+      oct0 += (int)l.octs.size();
     }
-    const size_t n = l.r.size();
-    if (!l.octs.empty()) memcpy(po, l.octs.data(), l.octs.size() * sizeof(qc_wxoct));
-    if (n) memcpy(r, l.r.data(), n * sizeof(int));
-    if (w64) {
-      for (size_t e = 0; e < n; ++e)
-        for (int k = 0; k < 8; ++k) w64[(e & ~(size_t)3) * 8 + 4 * k + (e & 3)] = l.w[8 * e + k];
-      w64 += 8 * n;
-    }
-    if (w32) {
-      for (size_t e = 0; e < 8 * n; ++e) w32[e] = (float)l.w[e];
-      w32 += 8 * n;
-    }
-    po += l.octs.size();
-    r += n;
-    ent0 += (long long)n;
-    oct0 += (int)l.octs.size();
+    pd += (long long)p.in->ndelta * nops;
   }
   delete h;
   return QC_OK;

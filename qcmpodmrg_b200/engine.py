@@ -1061,6 +1061,29 @@ def upload(a, device):
     return t.clone() if torch.device(device).type == "cpu" else t.to(device)
 
 
+def upload_all(arrays, device):
+    """Host arrays as device tensors of their bytes, in one copy (each 256-byte aligned)."""
+    sizes = [max(a.nbytes, 16) for a in arrays]
+    at = numpy.cumsum([0] + [(n + 255) // 256 * 256 for n in sizes])
+    blob = torch.empty(int(at[-1]), dtype=torch.uint8)
+    host = blob.numpy()
+    for a, o in zip(arrays, at):
+        host[o:o + a.nbytes] = numpy.ascontiguousarray(a).reshape(-1).view(numpy.uint8)
+    dev = blob if torch.device(device).type == "cpu" else blob.to(device)
+    return [dev[int(o):int(o) + n] for o, n in zip(at, sizes)]
+
+
+def joined(arrays):
+    """numpy.concatenate of record arrays, copied as bytes (record by record it copies field by field)."""
+    dt = arrays[0].dtype
+    return numpy.concatenate([numpy.ascontiguousarray(a).view(numpy.uint8) for a in arrays]).view(dt)
+
+
+def taken(a, index):
+    """a[index] of a contiguous record array of 8-byte multiples, copied as rows of words."""
+    return a.view(numpy.int64).reshape(len(a), -1).take(index, axis=0).reshape(-1).view(a.dtype)
+
+
 def op_table(a_base, b_base, c_base, alpha):
     n = max(numpy.size(x) for x in (a_base, b_base, c_base, alpha))
     t = numpy.zeros(n, dtype=OP_DT)
@@ -1107,6 +1130,9 @@ WXDOP_DT = numpy.dtype([("ent_b", "<i8"), ("oct_b", "<i4"), ("noct", "<i4")])
 WXOCT_DT = numpy.dtype([("ent", "<i4"), ("cnt", "<i4"), ("pad", "<i4", (2,)), ("row", "<i4", (8,))])
 assert WXGRP_DT.itemsize == 208 and WXDELTA_DT.itemsize == 32 and WXITEM_DT.itemsize == 32
 assert WXDOP_DT.itemsize == 16 and WXOCT_DT.itemsize == 48
+WXPART_DT = numpy.dtype([(k + s, "<i8") for s in "12" for k in ("w", "off", "ns", "nd", "ioff", "allowed")] +
+                        [(k, "<i8") for k in ("iblk", "kblk", "row0", "R")] + [("nops", "<i4"), ("ndelta", "<i4")])
+assert WXPART_DT.itemsize == 136
 WX_MAXR = 640             # T1 rows of one charge difference (FP64 rows of a 32-fiber tile: 160 KB)
 WX_MAXOCT = 512           # octets of one (charge difference, operator)
 WX_GRPS = 32              # sector pairs of one tile
@@ -1268,9 +1294,7 @@ class WSource(object):
             # element e of the transposed block is (e / D_a, e % D_a) = (b, a)
             perm = _W_PERM[id(lay)] = (lay, src + (e % d[b, 0]) * d[b, 1] + e // d[b, 0])
         n = len(offsets)
-        vals = numpy.empty((n, lay.size))
-        for k, o in enumerate(offsets):
-            vals[k] = values[o:o + lay.size][perm[1]]
+        vals = numpy.asarray(values)[numpy.asarray(offsets)[:, None] + perm[1][None, :]]
         nd = numpy.concatenate([lay.ndims[1], lay.ndims[0], lay.ndims[2], lay.ndims[3]])
         tr = lambda v: numpy.asarray(v).reshape(ns).transpose(1, 0, 2, 3).ravel()          # noqa: E731
         return WSource(vals.ravel(), numpy.arange(n) * lay.size, [ns[1], ns[0], ns[2], ns[3]], nd, tr(lay.ioff),
@@ -1286,7 +1310,9 @@ class WSource(object):
         k = numpy.arange(ns)
         allowed[k, k, 0, 0] = 1
         ioff[k, k, 0, 0] = numpy.cumsum(n * n) - n * n
-        vals = numpy.concatenate([numpy.eye(int(x)).ravel() for x in n]) if ns else numpy.zeros(0)
+        vals = numpy.zeros(int((n * n).sum()))
+        own, loc = _ranges(n)
+        vals[ioff[own, own, 0, 0] + loc * (n[own] + 1)] = 1.0
         one = numpy.ones(4, dtype=numpy.int64)
         return WSource(vals, numpy.zeros(nops), [ns, ns, 4, 4], numpy.concatenate([n, n, one, one]), ioff.ravel(),
                        allowed.ravel())
@@ -1307,53 +1333,42 @@ class SparseWStage(object):
         self.name, self.device = name, device
         self.host_ops = ops
         self.flops = self.bytes = 0.0
-        grps, dels, rows, dops, octs, w64, w32, rs, self.op_ranges = [], [], [], [], [], [], [], [], []
-        ngrp = nrow = ndop = no = ne = 0
         lib = native.lib()
         i64 = numpy.int64
-        for part, (b, e), factors in parts:
+        rec = numpy.zeros(len(parts), WXPART_DT)
+        dels, self.op_ranges = [], []
+        ngrp = nrow = ndop = 0
+        for k, (part, (b, e), factors) in enumerate(parts):
             d = part["deltas"].copy()
             nops, nd = e - b, len(d)
-            h, co, ce = numpy.zeros(1, dtype=i64), numpy.zeros(1, dtype=i64), numpy.zeros(1, dtype=i64)
-            args = []
-            for w in factors:
-                assert len(w.offsets) == nops
-                args += [ptr(w.values), ptr(w.offsets), ptr(w.nsyms), ptr(w.nd), ptr(w.ioff), ptr(w.allowed)]
-            check(lib.qc_wx_build(nops, *args, nd, ptr(part["iblk"]), ptr(part["kblk"]), ptr(part["row0"]),
-                                  ptr(part["R"]), ptr(h), ptr(co), ptr(ce)), "qc_wx_build")
-            n = int(ce[0])
-            dp, oc = numpy.empty(nd * nops, WXDOP_DT), numpy.empty(int(co[0]), WXOCT_DT)
-            wd = numpy.empty(8 * n) if "f64" in kinds else None
-            ws = numpy.empty(8 * n, dtype=numpy.float32) if "f32" in kinds else None
-            rr = numpy.empty(n, dtype=numpy.int32)
-            check(lib.qc_wx_fetch(int(h[0]), ne, no, ptr(dp), ptr(oc), ptr(wd), ptr(ws), ptr(rr)), "qc_wx_fetch")
+            assert all(len(w.offsets) == nops for w in factors)
+            rec[k] = tuple(ptr(getattr(w, f)) for w in factors
+                           for f in ("values", "offsets", "nsyms", "nd", "ioff", "allowed")) + \
+                tuple(ptr(part[f]) for f in ("iblk", "kblk", "row0", "R")) + (nops, nd)
             d["grp_b"] += ngrp
             d["grp_e"] += ngrp
             d["row_b"] += nrow
             d["dop_b"] = ndop + numpy.arange(nd) * nops
-            grps.append(part["groups"])
             dels.append(d)
-            rows.append(part["rows"])
-            dops.append(dp)
-            octs.append(oc)
-            w64.append(wd)
-            w32.append(ws)
-            rs.append(rr)
             self.op_ranges.append((b, e, nd))
-            ngrp, nrow, ndop, no, ne = ngrp + len(part["groups"]), nrow + len(part["rows"]), ndop + len(dp), \
-                no + len(oc), ne + n
-        self.h_groups, self.h_deltas = numpy.concatenate(grps), numpy.concatenate(dels)
-        self.h_rows, self.h_dops, self.h_octs = (numpy.concatenate(x) for x in (rows, dops, octs))
-        self.h_ent_r = numpy.concatenate(rs)
-        self.h_w = {k: numpy.concatenate(w) for k, w in (("f64", w64), ("f32", w32)) if k in kinds}
+            ngrp, nrow, ndop = ngrp + len(part["groups"]), nrow + len(part["rows"]), ndop + nd * nops
+        h, co, ce = numpy.zeros(1, dtype=i64), numpy.zeros(len(parts), dtype=i64), numpy.zeros(len(parts), dtype=i64)
+        check(lib.qc_wx_build(len(parts), ptr(rec), ptr(h), ptr(co), ptr(ce)), "qc_wx_build")
+        n = int(ce.sum())
+        self.h_dops, self.h_octs = numpy.empty(ndop, WXDOP_DT), numpy.empty(int(co.sum()), WXOCT_DT)
+        self.h_ent_r = numpy.empty(n, dtype=numpy.int32)
+        self.h_w = {k: numpy.empty(8 * n, dtype=dt) for k, dt in (("f64", numpy.float64), ("f32", numpy.float32))
+                    if k in kinds}
+        check(lib.qc_wx_fetch(int(h[0]), ptr(self.h_dops), ptr(self.h_octs), ptr(self.h_w.get("f64")),
+                              ptr(self.h_w.get("f32")), ptr(self.h_ent_r)), "qc_wx_fetch")
+        self.h_groups = joined([p["groups"] for p, _, _ in parts])
+        self.h_deltas, self.h_rows = joined(dels), numpy.concatenate([p["rows"] for p, _, _ in parts])
         self.fibers = numpy.concatenate([p["fibers"] for p, _, _ in parts])
         self.ntasks = len(self.h_groups)
-        up = lambda a, dt: upload(a if len(a) else numpy.zeros(1, dt), device)         # noqa: E731
-        self.d = {"groups": up(self.h_groups, WXGRP_DT), "deltas": up(self.h_deltas, WXDELTA_DT),
-                  "rows": up(self.h_rows, numpy.int32), "dops": up(self.h_dops, WXDOP_DT),
-                  "octs": up(self.h_octs, WXOCT_DT), "ent_r": up(self.h_ent_r, numpy.int32),
-                  "ops": upload(ops, device)}
-        self._w = {k: up(w, w.dtype) for k, w in self.h_w.items()}
+        names = ["groups", "deltas", "rows", "dops", "octs", "ent_r"]
+        dev = upload_all([getattr(self, "h_" + k) for k in names] + [ops] + list(self.h_w.values()), device)
+        self.d = dict(zip(names + ["ops"], dev))
+        self._w = dict(zip(self.h_w, dev[len(names) + 1:]))
         self._launch = {}
         for kind in kinds:
             self.items(kind)
@@ -1410,13 +1425,14 @@ class SparseWStage(object):
         it["op0"] = op0[own]
         cost = (it["op_e"] - it["op_b"]) * (R[own] + 12 * noct[own]) * ft[own]
         out = []
+        fo = ft[own]
         for k in (128, 64, 32):
-            sel = numpy.flatnonzero(ft[own] == k)
+            sel = numpy.flatnonzero(fo == k)
             if len(sel) == 0:
                 continue
             sel = sel[numpy.argsort(-cost[sel], kind="stable")]
-            dd = numpy.unique(own[sel])
-            out.append((k, it[sel], upload(it[sel], self.device), int(d["R"][dd].max()), int(max(1, noct[dd].max()))))
+            its, os = taken(it, sel), own[sel]
+            out.append((k, its, upload(its, self.device), int(d["R"][os].max()), int(max(1, noct[os].max()))))
         self._launch[kind] = out
         return out
 
@@ -1763,20 +1779,21 @@ class DPanelStage(object):
             units.append(u)
             work.append(w.reshape(-1, 2))
             n += len(u)
-        self.h_units = numpy.concatenate(units) if units else numpy.zeros(0, DUNIT_DT)
+        self.h_units = joined(units) if units else numpy.zeros(0, DUNIT_DT)
         self.h_work = numpy.concatenate(work) if work else numpy.zeros((0, 2), dtype=numpy.int32)
         if longest_first and len(self.h_work):
-            x = self.h_units[self.h_work[:, 0]]
-            cost = x["K"].astype(numpy.int64) * ((x["nrem"] + 7) // 8 + 2)
+            cost = (self.h_units["K"].astype(numpy.int64) * ((self.h_units["nrem"] + 7) // 8 + 2))[self.h_work[:, 0]]
             self.h_work = numpy.ascontiguousarray(self.h_work[numpy.argsort(-cost, kind="stable")])
         self.h_crow, self.h_cols = crow, cols
         self.ntasks = len(self.h_work)
         if not self.ntasks:
             return
-        self.d_units, self.d_work, self.d_ops = (upload(x, device) for x in (self.h_units, self.h_work, ops))
-        self.d_crow = torch.from_numpy(numpy.ascontiguousarray(crow, dtype=numpy.int64)).to(device) \
-            if crow is not None else None
-        self.d_cols = upload(cols, device) if cols is not None else None
+        crow = None if crow is None else numpy.ascontiguousarray(crow, dtype=numpy.int64)
+        tab = crow if cols is None else cols
+        self.d_units, self.d_work, self.d_ops, *tab = upload_all(
+            [self.h_units, self.h_work, ops] + ([] if tab is None else [tab]), device)
+        self.d_crow = tab[0] if cols is None and tab else None
+        self.d_cols = tab[0] if cols is not None else None
 
     def record(self):
         """The launch as a native.SigmaPanel (pointers to this stage's device tables)."""

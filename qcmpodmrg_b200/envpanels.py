@@ -148,11 +148,19 @@ class EnvPanels(object):
         self.qx, self.qz = _q2(qx), _q2(qz)
         want = (self.qx[:, None, None, :] - self.qz[None, :, None, :] + qn[None, None, :, :])    # [x, z, n', q]
         self.b = numpy.full((ncls, nx, nz, 4), -1, dtype=i64)
-        for k, wl in enumerate(self.Wl):
-            q = sign * _q2(wl.qsyms[wax])
+        # quantum numbers as one integer each; the largest absolute value bounds every digit
+        qw = [sign * _q2(wl.qsyms[wax]) for wl in self.Wl]
+        top = max([int(abs(want).max())] + [int(abs(q).max()) for q in qw if len(q)])
+        code = lambda q: (q + top) @ ((2 * top + 1) ** numpy.arange(q.shape[-1], dtype=i64))          # noqa: E731
+        cw = code(want)
+        for k, (wl, q) in enumerate(zip(self.Wl, qw)):
+            if len(q) == 0:
+                continue
             self.db[k, :len(q)] = wl.ndims[wax]
-            hit = (want[:, :, :, None, :] == q[None, None, None, :, :]).all(axis=-1)
-            self.b[k] = numpy.where(hit.any(axis=-1), hit.argmax(axis=-1), -1)
+            cq = code(q)
+            o = numpy.argsort(cq, kind="stable")
+            at = o[numpy.minimum(numpy.searchsorted(cq[o], cw), len(q) - 1)]
+            self.b[k] = numpy.where(cq[at] == cw, at, -1)
         self._w = (W, left, wax, qx, qz, da)
 
     @staticmethod

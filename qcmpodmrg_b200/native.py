@@ -99,8 +99,8 @@ _SIGS = {
     "qc_sigma_panels": (c_int, [c_vp] * 10),
     "qc_gather_pad_f32": (c_int, [c_vp, c_vp, c_ll, c_vp, c_vp]),
     "qc_gather_pad_f64": (c_int, [c_vp, c_vp, c_ll, c_vp, c_vp]),
-    "qc_wx_build": (c_int, [c_int] + [c_vp] * 12 + [c_int] + [c_vp] * 7),
-    "qc_wx_fetch": (c_int, [c_vp, c_ll, c_int, c_vp, c_vp, c_vp, c_vp, c_vp]),
+    "qc_wx_build": (c_int, [c_int] + [c_vp] * 4),
+    "qc_wx_fetch": (c_int, [c_vp] * 6),
     "qc_wsparse_f64": (c_int, [c_vp, c_ll, c_int] + [c_vp] * 8 + [c_int, c_int, c_vp, c_vp, c_vp]),
     "qc_wsparse_f32": (c_int, [c_vp, c_ll, c_int] + [c_vp] * 8 + [c_int, c_int, c_vp, c_vp, c_vp]),
     "qc_wpanel_f64": (c_int, [c_vp, c_vp, c_vp, c_ll, c_vp]),
@@ -139,7 +139,7 @@ def ptr(a):
     if a is None:
         return None
     if isinstance(a, numpy.ndarray):
-        return a.ctypes.data
+        return a.__array_interface__["data"][0]
     return a.data_ptr()
 
 
