@@ -16,7 +16,7 @@
 // short panels of L.psi (a few K slices each) do not wait for their first operands.
 //
 // Measured at the mid-chain dot of K=24, D=500 (160 GFLOP each; DFMA kernel before): L.psi
-// 16.8 -> 7.7 ms (20.8 TFLOP/s, 56 % of the pipe), .R 14.5 -> 6.2 ms (25.9, 70 %).  L.psi is
+// 16.8 -> 7.5 ms (21.3 TFLOP/s, 58 % of the pipe), .R 14.5 -> 5.8 ms (27.6, 75 %).  L.psi is
 // held back by its T1 stores and by K extents that end inside a 16-deep slice, .R by the
 // last wave of tiles and the ring's barriers.
 //
@@ -57,12 +57,15 @@ __device__ __forceinline__ void dp_mma(double (&c)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-// One K slice (k4 groups of four k) of a warp's 16 x 8 NT tile.
-template <int NT, bool AT>
+// One K slice (k4 groups of four k) of a warp's 16 x 8 NT tile.  LONG: whole slices have code of
+// their own without the tests of k4, so that the next group's operands are read ahead of the
+// products.  .R (long K): 6.18 -> 5.77 ms at D = 500; L.psi, whose tiles are 1 to 7 slices, lost 3 %.
+template <int NT, bool AT, bool LONG, bool FULL = false>
 __device__ __forceinline__ void dp_slice(const double *as, const double *bs, int k4, double (&acc)[2][DP_NT][2]) {
+  if (LONG && !FULL && k4 == DP_BK / 4) return dp_slice<NT, AT, LONG, true>(as, bs, k4, acc);
 #pragma unroll
   for (int kk = 0; kk < DP_BK / 4; ++kk) {
-    if (kk < k4) {
+    if (FULL || kk < k4) {
       const double a0 = as[4 * kk * (AT ? DP_PT : 1)], a1 = as[4 * kk * (AT ? DP_PT : 1) + 8 * (AT ? 1 : DP_P)];
       double b[NT];
 #pragma unroll
@@ -116,7 +119,7 @@ __global__ void __launch_bounds__(DP_THREADS, 2)
 k_dpanel(const qc_dunit *__restrict__ units, const int2 *__restrict__ work, int nwork,
          const qc_op *__restrict__ ops, const long long *__restrict__ crow, const qc_dcol *__restrict__ cols,
          const T *__restrict__ A, const T *__restrict__ B, T *__restrict__ C) {
-  constexpr bool COLS = MODE == DP_COLS, AT = MODE == DP_BLK, F64 = sizeof(T) == 8;
+  constexpr bool COLS = MODE == DP_COLS, AT = MODE == DP_BLK, LONG = MODE == DP_ROWS, F64 = sizeof(T) == 8;
   constexpr int BM = Dp<T>::BM, BN = Dp<T>::BN, V = Dp<T>::V, STAGE = Dp<T>::STAGE, RP = Dp<T>::RP, EL = sizeof(T);
   extern __shared__ __align__(16) unsigned char dp_raw[];
   T *const dp_smem = reinterpret_cast<T *>(dp_raw);
@@ -163,6 +166,7 @@ k_dpanel(const qc_dunit *__restrict__ units, const int2 *__restrict__ work, int 
     Bb = B + r.o.b_base + r.u.b_off + (long long)r0 * ldb + ck;
     lk = 0;
     // the tile's column (row) records, read by its epilogue
+    if (COLS && tid >= ln && tid < BN) scols[lt & (DP_RECS - 1)][tid].off = -1;
     if (MODE != DP_BLK && (COLS ? tid < ln : tid < lm)) {
       const void *src = COLS ? (const void *)(cols + r.u.c_off + tid) : (const void *)(crow + r.u.c_off + tid);
       const void *dst = COLS ? (const void *)&scols[lt & (DP_RECS - 1)][tid] : (const void *)&srow[lt & (DP_RECS - 1)][tid];
@@ -252,14 +256,14 @@ k_dpanel(const qc_dunit *__restrict__ units, const int2 *__restrict__ work, int 
           const double *as = buf + (AT ? gk * DP_PT + warp * WR + gr : (warp * WR + gr) * DP_P + gk);
           const double *bs = buf + (BM + gr) * DP_P + gk;
           switch (nt) {
-            case 1: dp_slice<1, AT>(as, bs, k4, acc); break;
-            case 2: dp_slice<2, AT>(as, bs, k4, acc); break;
-            case 3: dp_slice<3, AT>(as, bs, k4, acc); break;
-            case 4: dp_slice<4, AT>(as, bs, k4, acc); break;
-            case 5: dp_slice<5, AT>(as, bs, k4, acc); break;
-            case 6: dp_slice<6, AT>(as, bs, k4, acc); break;
-            case 7: dp_slice<7, AT>(as, bs, k4, acc); break;
-            default: dp_slice<8, AT>(as, bs, k4, acc); break;
+            case 1: dp_slice<1, AT, LONG>(as, bs, k4, acc); break;
+            case 2: dp_slice<2, AT, LONG>(as, bs, k4, acc); break;
+            case 3: dp_slice<3, AT, LONG>(as, bs, k4, acc); break;
+            case 4: dp_slice<4, AT, LONG>(as, bs, k4, acc); break;
+            case 5: dp_slice<5, AT, LONG>(as, bs, k4, acc); break;
+            case 6: dp_slice<6, AT, LONG>(as, bs, k4, acc); break;
+            case 7: dp_slice<7, AT, LONG>(as, bs, k4, acc); break;
+            default: dp_slice<8, AT, LONG>(as, bs, k4, acc); break;
           }
         } else {
           const float *as = buf + (warp * WR + gr) * DP_P, *bs = buf + (BM + gk) * DP_P;
@@ -294,22 +298,24 @@ k_dpanel(const qc_dunit *__restrict__ units, const int2 *__restrict__ work, int 
         }
       }
     } else if constexpr (COLS) {
-      const long long m0 = rec.u.m0 + warp * WR + gr;
-      const qc_dcol *cl = scols[ct & (DP_RECS - 1)];
+      // eight columns' records first, then their stores under predicates: with a branch for each
+      // column its record's latency is paid sixteen times (D = 200: 786 -> 729 us, D = 500: 7.67 -> 7.48 ms)
+      const int m = warp * WR + gr, m0 = rec.u.m0 + m;
+      const bool r0 = m < mrem, r1 = m + 8 < mrem;
+      const qc_dcol *cl = scols[ct & (DP_RECS - 1)] + gk;
 #pragma unroll
-      for (int j = 0; j < DP_NT; ++j)
+      for (int j = 0; j < DP_NT; j += 4) {
+        qc_dcol c[8];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int n = 8 * j + 4 * h + gk;
-          if (n < nrem) {
-            const qc_dcol c = cl[n];
-            if (c.off >= 0) {
-              double *dst = Cb + c.off + m0 * c.ld;
-              if (warp * WR + gr < mrem) dst[0] = alpha * acc[0][j][h];
-              if (warp * WR + gr + 8 < mrem) dst[8LL * c.ld] = alpha * acc[1][j][h];
-            }
-          }
+        for (int q = 0; q < 8; ++q) c[q] = cl[8 * j + 4 * q];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          double *dst = Cb + c[q].off + (long long)m0 * c[q].ld;
+          const double v0 = alpha * acc[0][j + q / 2][q & 1], v1 = alpha * acc[1][j + q / 2][q & 1];
+          if (r0 && c[q].off >= 0) dst[0] = v0;
+          if (r1 && c[q].off >= 0) dst[8LL * c[q].ld] = v1;
         }
+      }
     } else if constexpr (AT) {
       const int dr = rec.u.pad0, dc = rec.u.pad1, m0 = rec.u.m0, n0 = rec.u.n0;
 #pragma unroll
