@@ -8,23 +8,24 @@
 // the sigma rows of that sector; the K extent (sum over MPO sectors c of D_c * D_r)
 // is long, the N extent (D_r') short.
 //
-// Persistent, warp-specialised CTA (10 warps):
+// Persistent, warp-specialised CTA (10 warps, or 18 with column segments):
 //   warp 0     one thread issues the TMA loads (cp.async.bulk.tensor, 128-byte swizzle)
 //              of every 32-wide K stage into a ring of S shared-memory stages;
 //   warp 1     owns the tensor memory (2 x BN columns: two accumulators) and one thread
 //              issues tcgen05.mma kind::tf32, 12 per stage: a_lo.b_hi + a_hi.b_lo +
 //              a_hi.b_hi for each 8-wide K step, committed to the stage's "empty"
 //              barrier and, after a unit's last stage, to the accumulator's "full" one;
-//   warps 2-9  split each raw FP32 A stage in place into hi = tf32(x) and a lo plane
+//   warps 2-  split each raw FP32 A stage in place into hi = tf32(x) and a lo plane
 //              tf32(x - hi) (A_SPLIT); every 2 K stages add the TMEM accumulator into FP32
-//              registers (tcgen05.ld: warp w owns TMEM lanes 32*(w%4) .. and one half of the
+//              registers (tcgen05.ld: warp w owns TMEM lanes 32*(w%4) .. and a part of the
 //              columns), and store the finished tile (rows through the row table, or
 //              column segments staged in shared memory); the other TMEM accumulator
 //              meanwhile takes the next chunk.
 // The segment epilogue bounds L.psi, whose K is one or two chunks: with the whole tile staged
 // for all warps (two block barriers, segments copied one by one) a unit took 10 us; with each
 // warp storing its own part, a lane fixed to its columns, 4.7 us (K=24: D=500 5.19 -> 2.38 ms,
-// D=200 1.32 -> 0.39 ms).
+// D=200 1.32 -> 0.39 ms); with the records of a unit fetched ahead of it and sixteen helper warps
+// 2.34 and 0.35 ms.  Without its stores L.psi takes 1.37 and 0.16 ms (15 GB of operand tiles from L2).
 // No cluster, no multicast: every CTA loads its own tiles of this GPU's own memory.
 // Every wait is bounded: on expiry the CTA raises *err, stops issuing work, waits
 // (bounded) for its loads and products in flight and still frees its tensor memory.
@@ -41,8 +42,10 @@ namespace {
 
 constexpr int TP_BM = 128;
 constexpr int TP_BK = 32;                  // 32 FP32 = 128 bytes: one swizzle row
-constexpr int TP_THREADS = 320;             // producer warp, MMA warp, 8 helper warps
-constexpr int TP_HELPERS = 8;
+// helper warps: the segment epilogue gains from sixteen (D = 200: 372 -> 349 us), the row form, whose
+// helpers split and promote in turn, loses 4 %
+__host__ __device__ constexpr int tp_helpers(int epi) { return epi ? 16 : 8; }
+__host__ __device__ constexpr int tp_threads(int epi) { return 64 + 32 * tp_helpers(epi); }     // + producer and MMA warp
 constexpr long long TP_SPIN = 1LL << 26;   // polls before a wait gives up (~seconds)
 constexpr int TP_CHUNK = 2;                 // K stages accumulated in TMEM before promotion to FP32 registers
 
@@ -149,11 +152,12 @@ constexpr int EPI_ROWS = 0;       // rows through a row table, stored from regis
 constexpr int EPI_SEGMENTS = 1;   // column segments, staged in shared memory per warp, coalesced stores
 
 template <bool A_SPLIT, int BN, int S, int EPI>
-__global__ void __launch_bounds__(TP_THREADS, 1)
+__global__ void __launch_bounds__(tp_threads(EPI), 1)
 k_tcpanel(const qc_tcunit *__restrict__ units, int nunits, const CUtensorMap *__restrict__ maps,
           const qc_op *__restrict__ ops, const long long *__restrict__ crow, const qc_tcseg *__restrict__ segs,
           float *__restrict__ C, int *__restrict__ err) {
   static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "UMMA N");
+  constexpr int TP_HELPERS = tp_helpers(EPI);
   extern __shared__ unsigned char tp_smem_raw[];
   // stage s: [A0 (raw / hi) | A1 (lo) | B0 (hi) | B1 (lo)], each 1024-byte aligned
   unsigned char *smem = reinterpret_cast<unsigned char *>(
@@ -201,12 +205,17 @@ k_tcpanel(const qc_tcunit *__restrict__ units, int nunits, const CUtensorMap *__
       int it = 0;
       int issued[S];
       for (int s = 0; s < S; ++s) issued[s] = -1;
+      int am_seen = -1, bm_seen = -1;
+      qc_tcunit tn = units[blockIdx.x];
       for (int u = blockIdx.x; u < nunits && !abort_flag; u += gridDim.x) {
-        const qc_tcunit t = units[u];
+        const qc_tcunit t = tn;
+        if (u + (int)gridDim.x < nunits) tn = units[u + gridDim.x];
         const CUtensorMap *am = maps + t.a_map;
         const CUtensorMap *bm = maps + t.b_map;
-        tmap_acquire(am);
-        tmap_acquire(bm);
+        if (t.a_map != am_seen) tmap_acquire(am);
+        if (t.b_map != bm_seen) tmap_acquire(bm);
+        am_seen = t.a_map;
+        bm_seen = t.b_map;
         for (int k = 0; k < t.nk; ++k, ++it) {
           const int s = it % S;
           const uint32_t ph = (uint32_t)((it / S) & 1);
@@ -236,8 +245,10 @@ k_tcpanel(const qc_tcunit *__restrict__ units, int nunits, const CUtensorMap *__
     if (lane == 0) {
       int it = 0, g = 0;
       bool any = false;
+      int2 tn = make_int2(units[blockIdx.x].nk, units[blockIdx.x].n_valid);
       for (int u = blockIdx.x; u < nunits && !abort_flag; u += gridDim.x) {
-        const qc_tcunit t = units[u];
+        const struct { int nk, n_valid; } t = {tn.x, tn.y};
+        if (u + (int)gridDim.x < nunits) tn = make_int2(units[u + gridDim.x].nk, units[u + gridDim.x].n_valid);
         const int nmma = ((t.n_valid + 15) / 16) * 16;
         const uint32_t idesc = idesc_tf32(nmma > BN ? BN : nmma);
         bool ok = true;
@@ -286,15 +297,15 @@ k_tcpanel(const qc_tcunit *__restrict__ units, int nunits, const CUtensorMap *__
       }
     }
   } else {
-    // ------------------------------------------------------------ split + promotion + epilogue (warps 2-9)
-    // two warpgroups: warp w reads TMEM lanes 32*(w%4) .. (its quarter of the rows) and the
-    // accumulator columns of its group, [BN/2 * gw, BN/2 * (gw + 1))
-    constexpr int HALF = BN / 2;
-    const int hid = threadIdx.x - 64;          // 0 .. 255
+    // ------------------------------------------------------------ split + promotion + epilogue (warps 2 and up)
+    // warpgroups of four: warp w reads TMEM lanes 32*(w%4) .. (its quarter of the rows) and the
+    // accumulator columns of its group, [COLS * gw, COLS * (gw + 1))
+    constexpr int COLS = BN / (TP_HELPERS / 4);
+    const int hid = threadIdx.x - 64;
     const int q = warp & 3;                    // TMEM lane quarter of this warp
-    const int gw = (warp - 2) >> 2;            // column half of this warp's group
+    const int gw = (warp - 2) >> 2;            // column part of this warp's group
     const int row = q * 32 + lane;
-    float acc[HALF];
+    float acc[COLS];
     int it = 0;                                // stages split so far
     // the chunk stream (unit, first stage) in the order the MMA issuer takes it; the next
     // chunk's stages are split before the current chunk is drained, so the tensor core
@@ -337,8 +348,19 @@ k_tcpanel(const qc_tcunit *__restrict__ units, int nunits, const CUtensorMap *__
     };
     bool ok = split_chunk();
     int g = 0;
+    qc_tcunit tn = units[blockIdx.x];
     for (int u = blockIdx.x; u < nunits && ok && !abort_flag; u += gridDim.x) {
-      const qc_tcunit t = units[u];
+      // records that the epilogue and the next unit need, fetched while the products run
+      const qc_tcunit t = tn;
+      if (u + (int)gridDim.x < nunits) tn = units[u + gridDim.x];
+      const qc_op o = ops[t.op];
+      qc_tcseg sg;
+      long long row_off = 0;
+      if (EPI == EPI_ROWS) {
+        if (row < t.m_valid) row_off = crow[t.c_off + row];
+      } else if (lane < t.nseg) {
+        sg = segs[t.c_off + lane];
+      }
       const int ncol = t.n_valid < BN ? t.n_valid : BN;
       for (int k0 = 0; k0 < t.nk; k0 += TP_CHUNK, ++g) {
         ok = split_chunk();
@@ -349,10 +371,10 @@ k_tcpanel(const qc_tcunit *__restrict__ units, int nunits, const CUtensorMap *__
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + gw * HALF);
+        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + gw * COLS);
 #pragma unroll
-        for (int c0 = 0; c0 < HALF; c0 += 16) {
-          if (gw * HALF + c0 < ncol) {
+        for (int c0 = 0; c0 < COLS; c0 += 16) {
+          if (gw * COLS + c0 < ncol) {
             uint32_t r[16];
             tmem_ld16(taddr + (uint32_t)c0, r);
 #pragma unroll
@@ -365,39 +387,37 @@ k_tcpanel(const qc_tcunit *__restrict__ units, int nunits, const CUtensorMap *__
       }
       if (!ok) break;
       // ---- epilogue of unit u from the FP32 registers
-      const qc_op o = ops[t.op];
       const float alpha = (float)o.alpha;
       if (EPI == EPI_ROWS) {
         if (row < t.m_valid) {
-          float *dst = C + o.c_base + crow[t.c_off + row] + t.b_c1 + gw * HALF;
+          float *dst = C + o.c_base + row_off + t.b_c1 + gw * COLS;
 #pragma unroll
-          for (int c = 0; c < HALF; ++c)
-            if (gw * HALF + c < ncol) dst[c] = alpha * acc[c];
+          for (int c = 0; c < COLS; ++c)
+            if (gw * COLS + c < ncol) dst[c] = alpha * acc[c];
         }
       } else {
-        // The warp's 32 rows x BN/2 columns go through its own part of shared memory (row
-        // stride HALF + 1: no bank conflicts) and leave row by row, a lane on the same
+        // The warp's 32 rows x COLS columns go through its own part of shared memory (row
+        // stride COLS + 1: no bank conflicts) and leave row by row, a lane on the same
         // columns throughout: the segment of each is looked up once per unit.
-        float *stg = reinterpret_cast<float *>(smem + S * ST_BYTES) + (warp - 2) * 32 * (HALF + 1);
-        float *dst[HALF / 32];
-        int ldc[HALF / 32];
+        float *stg = reinterpret_cast<float *>(smem + S * ST_BYTES) + (warp - 2) * 32 * (COLS + 1);
+        float *dst[COLS / 32];
+        int ldc[COLS / 32];
         {
-          int cnt[HALF / 32];
+          int cnt[COLS / 32];
 #pragma unroll
-          for (int p = 0; p < HALF / 32; ++p) cnt[p] = -1;
-          qc_tcseg sg;
+          for (int p = 0; p < COLS / 32; ++p) cnt[p] = -1;
           for (int s0 = 0; s0 < t.nseg; s0 += 32) {
             const int ns = min(32, t.nseg - s0);
-            if (lane < ns) sg = segs[t.c_off + s0 + lane];
+            if (s0 > 0 && lane < ns) sg = segs[t.c_off + s0 + lane];
             for (int si = 0; si < ns; ++si) {
               const int c0 = __shfl_sync(0xffffffffu, sg.col0, si);
 #pragma unroll
-              for (int p = 0; p < HALF / 32; ++p) cnt[p] += c0 <= gw * HALF + lane + 32 * p;
+              for (int p = 0; p < COLS / 32; ++p) cnt[p] += c0 <= gw * COLS + lane + 32 * p;
             }
             // columns whose last segment so far is among these 32
 #pragma unroll
-            for (int p = 0; p < HALF / 32; ++p) {
-              const int c = gw * HALF + lane + 32 * p, si = cnt[p] - s0;
+            for (int p = 0; p < COLS / 32; ++p) {
+              const int c = gw * COLS + lane + 32 * p, si = cnt[p] - s0;
               const int from = si & 31;
               const long long off = __shfl_sync(0xffffffffu, sg.off, from);
               const int col0 = __shfl_sync(0xffffffffu, sg.col0, from);
@@ -414,20 +434,20 @@ k_tcpanel(const qc_tcunit *__restrict__ units, int nunits, const CUtensorMap *__
           }
           if (t.nseg == 0) {
 #pragma unroll
-            for (int p = 0; p < HALF / 32; ++p) dst[p] = nullptr, ldc[p] = 0;
+            for (int p = 0; p < COLS / 32; ++p) dst[p] = nullptr, ldc[p] = 0;
           }
         }
-        if (gw * HALF < ncol) {
+        if (gw * COLS < ncol) {
 #pragma unroll
-          for (int c = 0; c < HALF; ++c) stg[lane * (HALF + 1) + c] = alpha * acc[c];
+          for (int c = 0; c < COLS; ++c) stg[lane * (COLS + 1) + c] = alpha * acc[c];
           __syncwarp();
           const int nr = min(32, t.m_valid - q * 32);
 #pragma unroll 4
           for (int m = 0; m < nr; ++m) {
 #pragma unroll
-            for (int p = 0; p < HALF / 32; ++p) {
+            for (int p = 0; p < COLS / 32; ++p) {
               if (dst[p]) {
-                *dst[p] = stg[m * (HALF + 1) + lane + 32 * p];
+                *dst[p] = stg[m * (COLS + 1) + lane + 32 * p];
                 dst[p] += ldc[p];
               }
             }
@@ -477,7 +497,7 @@ constexpr int TP_BN = 128;
 constexpr int TP_S = 3;
 constexpr int tp_stages(int epi) { return epi == EPI_SEGMENTS ? 2 : TP_S; }
 constexpr size_t tp_dsmem(int epi) {
-  return (size_t)tp_stages(epi) * stage_bytes<TP_BN>() + 1024 + (epi == EPI_SEGMENTS ? TP_HELPERS * 32 * (TP_BN / 2 + 1) * 4 : 0);
+  return (size_t)tp_stages(epi) * stage_bytes<TP_BN>() + 1024 + (epi == EPI_SEGMENTS ? tp_helpers(epi) * 32 * (TP_BN / (tp_helpers(epi) / 4) + 1) * 4 : 0);
 }
 bool g_attr[2] = {false, false};
 
@@ -504,7 +524,7 @@ int launch_tcpanel(const void *units, long long nunits, const void *maps, const 
     }
   }
   const int grid = (int)(nunits < (long long)g_nsm ? nunits : (long long)g_nsm);
-  k_tcpanel<A_SPLIT, TP_BN, tp_stages(EPI), EPI><<<grid, TP_THREADS, tp_dsmem(EPI), s>>>(
+  k_tcpanel<A_SPLIT, TP_BN, tp_stages(EPI), EPI><<<grid, tp_threads(EPI), tp_dsmem(EPI), s>>>(
       (const qc_tcunit *)units, (int)nunits, (const CUtensorMap *)maps, (const qc_op *)ops, crow,
       (const qc_tcseg *)segs, C, g_tp_err);
   cudaError_t e = cudaGetLastError();
