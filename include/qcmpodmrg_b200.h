@@ -264,8 +264,9 @@ long long qc_ortho_work(void);
 int qc_ortho(const double *V, int m, long long n, const double *r, double *out, double *work, int times, void *stream);
 
 /* The five steps of a matrix-vector product in panel form as one call: psi panels, L.psi, the
- * sparse MPO stage, .R, the sum over operators.  All pointers are device memory.  f32: panels,
- * intermediates and coefficients are FP32 (x and y stay FP64); clear: .R leaves parts of the
+ * sparse MPO stage, .R, the sum over operators.  All pointers are device memory.  f32 = 1: panels,
+ * intermediates and coefficients are FP32 (x and y stay FP64); f32 = 2: so, with L.psi and .R on
+ * the tensor-core panel GEMM (work unused, lpan and rpan its tensor maps, psi hi and lo planes); clear: .R leaves parts of the
  * partial vectors untouched, which are zeroed first; table: column (first) or row (last) table. */
 typedef struct {
   const void *units, *work;

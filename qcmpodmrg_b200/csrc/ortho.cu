@@ -1,7 +1,7 @@
 // Orthonormalisation of one vector against the rows of a Davidson basis (dvdson_ortho,
 // source/tools/pdvdson.py:350-390): `times` passes of r -= V^T (V r), then r / |r| twice.
 //
-// Bound: launches at small sizes, 2 + times readings of V at large ones (it stays in L2).  A pass
+// Bound: launches at small sizes, times + 1 readings of V at large ones (it stays in L2).  A pass
 // needs all of V r before it can change r, so passes are separate launches; each one finishes
 // the pass before it (sums the blocks' partial products, in a fixed order, and updates its part of
 // r) and forms the next products from the values of V that it holds in registers: 8 launches

@@ -1378,8 +1378,7 @@ class SparseWStage(object):
 
         A tile is 32, 64 or 128 fibers wide: as many as its T1 rows, its offset tables and (in
         FP32) its entry rings leave room for in WX_TILE_BYTES of shared memory, so that two
-        CTAs share an SM.  Dots whose tiles fit
-        the GPU at once use one width, in one launch."""
+        CTAs share an SM.  Dots whose tiles fit the GPU at once use one width, in one launch."""
         hit = self._launch.get(kind)
         if hit is not None:
             return hit
@@ -1519,6 +1518,11 @@ class TCPanelStage(object):
             self._maps = torch.from_numpy(out).to(self.device)
             self._key = key
         return self._maps
+
+    def record(self):
+        """The launch as a native.SigmaPanel (pointers to this stage's device tables; no maps)."""
+        tab = self.d_crow if self.d_segs is None else self.d_segs
+        return native.SigmaPanel(self.d_units.data_ptr(), None, self.ntasks, self.d_ops.data_ptr(), tab.data_ptr())
 
     def run(self, A, B, C, kind="tf32x3", stream=None):
         if self.ntasks == 0:

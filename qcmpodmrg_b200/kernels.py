@@ -888,15 +888,16 @@ class SigmaOperator(object):
         p = self._plans.get(kind)
         if p is None:
             d, w = self.wx.d, self.wx
-            first, last = (self.d1, self.d4) if kind == "f64" else (self.f1, self.f4)
-            p = native.SigmaPlan(int(kind == "f32"), self.nops, int(not self._part_full), 0, self.ndim0,
+            first, last = {"f64": (self.d1, self.d4), "f32": (self.f1, self.f4), "tf32x3": (self.tc1, self.tc4)}[kind]
+            p = native.SigmaPlan(("f64", "f32", "tf32x3").index(kind), self.nops, int(not self._part_full), 0, self.ndim0,
                                  self._psi_gidx.numel(), self._psi_gidx.data_ptr(), first.record(), last.record())
             n = 0
             if w.ntasks:
                 p.deltas, p.groups, p.rows, p.dops, p.octs, p.ent_r, p.wops = (
                     d[k].data_ptr() for k in ("deltas", "groups", "rows", "dops", "octs", "ent_r", "ops"))
-                p.ent_w = w._w[kind].data_ptr()
-                for tile, host, dev, maxr, maxo in w.items(kind):
+                wk = "f64" if kind == "f64" else "f32"
+                p.ent_w = w._w[wk].data_ptr()
+                for tile, host, dev, maxr, maxo in w.items(wk):
                     p.tiles[n] = native.SigmaTiles(dev.data_ptr(), len(host), tile, maxr, maxo, 0)
                     n += 1
             self._plans[kind] = p = (ctypes.byref(p), p, n + 4)
@@ -906,10 +907,15 @@ class SigmaOperator(object):
         dt = torch.float64 if kind == "f64" else torch.float32
         ws = self.ws
         ref, _, launches = self._native_plan(kind)
-        lpan, rpan = (self.lpan64, self.rpan64) if kind == "f64" else (self.lpan_f32, self.rpan_f32)
+        psi = ws.get("psi_pan", self._psi_total * (2 if kind == "tf32x3" else 1), dt)
+        t3 = ws.get("t3", self.tot[2], dt)
+        if kind == "tf32x3":
+            lpan, rpan = self.tc1.maps(self.lpan_tc, psi), self.tc4.maps(t3, self.rpan_tc)
+        else:
+            lpan, rpan = (self.lpan64, self.rpan64) if kind == "f64" else (self.lpan_f32, self.rpan_f32)
         check(native.lib().qc_sigma_panels(
-            ref, lpan.data_ptr(), rpan.data_ptr(), x.data_ptr(), ws.get("psi_pan", self._psi_total, dt).data_ptr(),
-            ws.get("t1", self.tot[0], dt).data_ptr(), ws.get("t3", self.tot[2], dt).data_ptr(),
+            ref, lpan.data_ptr(), rpan.data_ptr(), x.data_ptr(), psi.data_ptr(),
+            ws.get("t1", self.tot[0], dt).data_ptr(), t3.data_ptr(),
             ws.get("part", self.nops * self.ndim0, dt).data_ptr(), y.data_ptr(), _stream(y.device)),
             "qc_sigma_panels")
         LOG.launches += launches
@@ -930,8 +936,9 @@ class SigmaOperator(object):
         if y is None:
             y = torch.empty(self.ndim0, dtype=torch.float64, device=ws.device)
         # in panel form all through: one native call (the launch log times the stages one by one)
-        if self.wx is not None and (prec == "f64" or (prec == "f32" and self.f1 is not None)) and x.is_cuda \
-                and not LOG.enabled:
+        if self.wx is not None and x.is_cuda and not LOG.enabled and (
+                prec == "f64" or (prec == "f32" and self.f1 is not None) or
+                (prec == "tf32x3" and self.tc1 is not None and self.tc4 is not None and self._s0_generic is None)):
             return self._run_panels(prec, x, y)
         if prec == "f64":
             T1 = ws.get("t1", self.tot[0], torch.float64)
