@@ -314,7 +314,7 @@ def stage_kernel(stage, w_path, prec):
     panel = w_path in ("fiber", "fused")
     from qcmpodmrg_b200.engine import FIBER_FGEMM
     fk = "k_fgemm" if FIBER_FGEMM else "k_fiber"
-    tc = "k_tcpanel" if prec == "tf32x3" else "k_pgemm"
+    tc = "k_tcpanel" if prec == "tf32x3" else "k_dpanel"
     return {"sigma1": tc if panel else "k_bgemm", "sigma2": fk if panel else "k_bgemm",
             "sigma3": fk if panel else "k_bgemm", "sigma23": fk if w_path == "fused" else "k_wsparse",
             "sigma4": tc if panel else "k_bgemm"}.get(stage, "k_bgemm")
@@ -327,10 +327,10 @@ def stage_kernel(stage, w_path, prec):
 # traffic grows in proportion to the blocks processed)
 TRAFFIC_RATIO = {("sigma1", "f32"): 0.987, ("sigma2", "f32"): 1.024, ("sigma3", "f32"): 1.007,
                  ("sigma4", "f32"): 1.010,
-                 ("sigma1", "tf32x3"): 1.035, ("sigma2", "tf32x3"): 1.024, ("sigma3", "tf32x3"): 1.007,
-                 ("sigma4", "tf32x3"): 1.146,
-                 ("sigma1", "f64"): 1.083, ("sigma2", "f64"): 1.041, ("sigma3", "f64"): 1.029,
-                 ("sigma4", "f64"): 1.008}
+                 ("sigma1", "tf32x3"): 1.053, ("sigma2", "tf32x3"): 1.024, ("sigma3", "tf32x3"): 1.007,
+                 ("sigma23", "tf32x3"): 0.934, ("sigma4", "tf32x3"): 1.136,
+                 ("sigma1", "f64"): 1.034, ("sigma2", "f64"): 1.041, ("sigma3", "f64"): 1.029,
+                 ("sigma23", "f64"): 0.945, ("sigma4", "f64"): 1.204}
 
 
 def traffic_per_launch(stage, prec, algo_bytes):
