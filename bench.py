@@ -325,8 +325,8 @@ def stage_kernel(stage, w_path, prec):
 # profiles/ holds the captures and the commands); the traffic of a D=500 launch is its
 # algorithmic bytes times this ratio (the kernels stream their operands once, so the
 # traffic grows in proportion to the blocks processed)
-TRAFFIC_RATIO = {("sigma1", "f32"): 0.987, ("sigma2", "f32"): 1.024, ("sigma3", "f32"): 1.007,
-                 ("sigma4", "f32"): 1.010,
+TRAFFIC_RATIO = {("sigma1", "f32"): 1.043, ("sigma2", "f32"): 1.024, ("sigma3", "f32"): 1.007,
+                 ("sigma23", "f32"): 0.934, ("sigma4", "f32"): 1.021,
                  ("sigma1", "tf32x3"): 1.053, ("sigma2", "tf32x3"): 1.024, ("sigma3", "tf32x3"): 1.007,
                  ("sigma23", "tf32x3"): 0.934, ("sigma4", "tf32x3"): 1.136,
                  ("sigma1", "f64"): 1.034, ("sigma2", "f64"): 1.041, ("sigma3", "f64"): 1.029,

@@ -1820,4 +1820,4 @@ class DPanelStage(object):
         LOG.launches += 1
         if LOG.enabled:
             e1.record()
-            LOG.records.append((self.name, e0, e1, self.flops, self.bytes))
+            LOG.records.append((self.name, e0, e1, self.flops, self.bytes * (A.element_size() / 8.0)))
