@@ -58,10 +58,11 @@ class TensorSet(object):
         if isinstance(values, (list, tuple)):
             host = numpy.concatenate([numpy.asarray(v, dtype=numpy.float64) for v in values]) \
                 if values else numpy.zeros(0)
-            values = torch.from_numpy(host).to(device)
-            self._host = (host, values, values._version)
+            ref = torch.from_numpy(host).to(device)
+            values = ref.clone()
+            self._given = (host, ref)               # what host() compares the values with
         else:
-            self._host = None
+            self._given = None
         self.values = values
         self._f32 = None
 
@@ -70,13 +71,19 @@ class TensorSet(object):
             self._f32 = self.values.to(torch.float32)
         return self._f32
 
-    def host(self):
-        """The values as a host array: those the set was made from while the device tensor is
-        that one and unchanged since, else a copy from the device (which waits for it)."""
-        h = self._host
-        if h is not None and h[1] is self.values and h[2] == self.values._version:
-            return h[0]
-        return numpy.ascontiguousarray(self.values.detach().cpu().numpy(), dtype=numpy.float64)
+    def host(self, check=True):
+        """The values as a host array.  Those the set was made from serve while the device values
+        equal them: compared on the device at every call, as a collective, a native kernel or a
+        write through ``.data`` changes values without a trace on the tensor (K=24: 5 MB a site,
+        a comparison instead of a copy); otherwise a copy from the device.  Both wait for the
+        stream.  check=False: as last found, for a caller that compares later (EnvPanels.current)."""
+        if self._given is not None:
+            host, ref = self._given
+            v = self.values
+            if not check or (v.device == ref.device and v.dtype == ref.dtype and torch.equal(v, ref)):
+                return host
+            self._given = None
+        return self.values.detach().to("cpu", torch.float64, copy=True).numpy()
 
     def op_values(self, i):
         o = int(self.offsets[i])
@@ -1198,6 +1205,7 @@ class Renormalizer(object):
     def __init__(self, ws, isite, status, site_layout, E, W, opers, panels=None):
         """panels: the panel form (None: on a GPU, where the blocks allow it)."""
         self.ws, self.status = ws, status
+        self._args = (ws, isite, status, site_layout, E, W, opers, panels)
         dev = ws.device
         groups = _groups(opers, isite, 1)
         nops = len(opers)
@@ -1316,6 +1324,8 @@ class Renormalizer(object):
     def __call__(self, site_values):
         """site_values: packed site tensor (float64, device) -> new TensorSet."""
         ws = self.ws
+        if self.ep is not None and not self.ep.current():
+            self.__init__(*self._args)
         if self.ep is not None:
             out = torch.empty(max(self._nout, 1), dtype=torch.float64, device=ws.device)
             T2, S = self.ep.run(site_values)
@@ -1350,9 +1360,11 @@ class NoiseRDM(object):
         envpanels with the rows (l, n1') of one merged class in one panel, whose Gram matrix
         is one panel GEMM of the panel with itself."""
         self.ws, self.status = ws, status
+        self._args = (ws, isite, status, psi_layout, E, W, opers, qkey, dense_idl, panels)
         dev = ws.device
         groups = _groups(opers, isite, 1)
         nops = len(opers)
+        self.E, self.W = E, W
         self.ep = None
         if panels is None:
             panels = torch.device(dev).type == "cuda"
@@ -1421,7 +1433,6 @@ class NoiseRDM(object):
                 add_parts(st[si], compile_classes(c, t, ax[si]), op_range=rng)
         self.stages = [Stage(st[si], dev, "prdm%d" % (si + 1), tabs[si]) for si in range(3)]
         self.flops = sum(s.flops for s in self.stages)
-        self.E, self.W = E, W
         n = int(numpy.prod(out.shape)) if out is not None else 0
         self.dense_shape = tuple(int(x) for x in out.shape) if out is not None else (0,)
         self.prj = torch.from_numpy(out.prjmap(dense_idl)).to(dev) if out is not None else None
@@ -1496,6 +1507,8 @@ class NoiseRDM(object):
     def __call__(self, psi_values):
         """psi_values: packed rank-3 wavefunction (device FP64) -> dense noise RDM (d x d)."""
         ws = self.ws
+        if self.ep is not None and not self.ep.current():
+            self.__init__(*self._args)
         if self.ep is not None:
             P = ws.get("npart", self.nops * self.size, torch.float64)
             T2, _ = self.ep.run(psi_values)
