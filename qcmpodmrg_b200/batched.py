@@ -221,7 +221,7 @@ class BatchedSigma(object):
         rec = {"deltas": up(numpy.concatenate(dels)), "groups": up(numpy.concatenate(grps)),
                "rows": cat(lambda st: st.h_rows), "dops": up(numpy.concatenate(dops)),
                "octs": cat(lambda st: st.h_octs), "ent_r": cat(lambda st: st.h_ent_r),
-               "w": cat(lambda st: st.h_w[kind])}
+               "w": cat(lambda st: st.host_weights(kind))}
         launches = []
         for tile, xs in sorted(by.items(), reverse=True):
             it = numpy.concatenate([x[0] for x in xs])

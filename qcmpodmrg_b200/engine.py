@@ -1321,6 +1321,12 @@ class WSource(object):
 _W_PERM = {}
 
 
+def f32_weights(w):
+    """FP64 coefficients of a sparse MPO stage (steps of four entries, [step][row][entry]) as the
+    FP32 kernel's, [entry][row], each rounded once."""
+    return w.reshape(-1, 8, 4).transpose(1, 2).reshape(-1).to(torch.float32)
+
+
 class SparseWStage(object):
     """T3 = T1 . (W_i W_{i+1}) for every operator in one sparse product (qc_wsparse_*).
 
@@ -1329,7 +1335,8 @@ class SparseWStage(object):
     stage: it is a plan for these values."""
 
     def __init__(self, parts, device, name, ops, kinds=("f64",)):
-        """kinds: precisions whose work items and coefficients are made now ("f64", "f32")."""
+        """kinds: precisions whose work items and coefficients are made now ("f64", and "f32" or
+        not: an FP32 product of an FP64 plan derives its coefficients and uses the FP64 tiles)."""
         self.name, self.device = name, device
         self.host_ops = ops
         self.flops = self.bytes = 0.0
@@ -1373,13 +1380,27 @@ class SparseWStage(object):
         for kind in kinds:
             self.items(kind)
 
+    def host_weights(self, kind):
+        """The coefficients in the order of ``kind``'s kernel (qc_wx_fetch)."""
+        w = self.h_w.get(kind)
+        return f32_weights(torch.from_numpy(self.h_w["f64"])).numpy() if w is None else w
+
+    def weights(self, kind):
+        """The same on the device; without a copy from the host, which a graph's capture would refuse."""
+        w = self._w.get(kind)
+        if w is None:
+            w = f32_weights(self._w["f64"].view(torch.float64)[:len(self.h_w["f64"])])
+            if not (w.is_cuda and torch.cuda.is_current_stream_capturing()):     # (captured: made by every replay)
+                self._w[kind] = w
+        return w
+
     def items(self, kind):
         """Work items by tile width, [(fibers, items, device items, T1 rows, octets)], longest first.
 
         A tile is 32, 64 or 128 fibers wide: as many as its T1 rows, its offset tables and (in
         FP32) its entry rings leave room for in WX_TILE_BYTES of shared memory, so that two
         CTAs share an SM.  Dots whose tiles fit the GPU at once use one width, in one launch."""
-        hit = self._launch.get(kind)
+        hit = self._launch.get(kind if kind in self.h_w else "f64")
         if hit is not None:
             return hit
         el = 8 if kind == "f64" else 4
@@ -1442,7 +1463,7 @@ class SparseWStage(object):
         lib = native.lib()
         s = stream if stream is not None else torch.cuda.current_stream(C.device).cuda_stream
         k = "f64" if kind == "f64" else "f32"
-        w = self._w[k]
+        w = self.weights(k)
         fn = lib.qc_wsparse_f64 if k == "f64" else lib.qc_wsparse_f32
         if LOG.enabled:
             e0 = torch.cuda.Event(enable_timing=True)

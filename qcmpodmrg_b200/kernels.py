@@ -903,7 +903,7 @@ class SigmaOperator(object):
                 p.deltas, p.groups, p.rows, p.dops, p.octs, p.ent_r, p.wops = (
                     d[k].data_ptr() for k in ("deltas", "groups", "rows", "dops", "octs", "ent_r", "ops"))
                 wk = "f64" if kind == "f64" else "f32"
-                p.ent_w = w._w[wk].data_ptr()
+                p.ent_w = w.weights(wk).data_ptr()
                 for tile, host, dev, maxr, maxo in w.items(wk):
                     p.tiles[n] = native.SigmaTiles(dev.data_ptr(), len(host), tile, maxr, maxo, 0)
                     n += 1
