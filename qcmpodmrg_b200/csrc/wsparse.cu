@@ -486,7 +486,7 @@ void build_op(const SparseW &W1, const double *v1, const SparseW &W2, const doub
   const int nsb = W1.ns[1];
   std::vector<double> S;                 // rows of the current delta, dense in i
   std::vector<uint64_t> mask;
-  std::vector<int> rowid, nnz, perm;
+  std::vector<int> rowid, nnz, perm, reach;
   std::vector<qc_wxoct> os;
   for (int d = 0; d < ndelta; ++d) {
     const int R = Rs[d];
@@ -497,6 +497,7 @@ void build_op(const SparseW &W1, const double *v1, const SparseW &W2, const doub
     S.assign((size_t)nrow * R, 0.0);
     mask.assign((size_t)nrow * words, 0);
     rowid.resize(nrow);
+    reach.assign(nrow, 0);
     int base = 0;
     for (int kb = 0; kb < 16; ++kb) {
       const int sc = kblk[16 * d + kb];
@@ -512,7 +513,9 @@ void build_op(const SparseW &W1, const double *v1, const SparseW &W2, const doub
         for (int sb = 0; sb < nsb; ++sb) {
           const int b1 = ((sa * W1.ns[1] + sb) * W1.ns[2] + n1p) * W1.ns[3] + n1;
           const int b2 = ((sb * W2.ns[1] + sc) * W2.ns[2] + n2p) * W2.ns[3] + n2;
-          if (!W1.allowed[b1] || !W2.allowed[b2] || nz1[b1].empty() || nz2[b2].empty()) continue;
+          if (!W1.allowed[b1] || !W2.allowed[b2]) continue;
+          for (int c = 0; c < nc; ++c) reach[base + c] |= 1 << ib;
+          if (nz1[b1].empty() || nz2[b2].empty()) continue;
           for (int a = 0; a < na; ++a) {
             const int i = r0 + a;
             for (int x = st1[b1][a]; x < st1[b1][a + 1]; ++x) {
@@ -541,10 +544,13 @@ void build_op(const SparseW &W1, const double *v1, const SparseW &W2, const doub
         mask[(size_t)k * words + wd] = live;
         nnz[k] += __builtin_popcountll(live);
       }
-    // rows of like pattern share an octet: longest first, equal patterns side by side
+    // rows of like pattern share an octet: longest first, equal patterns side by side.  A row's zero
+    // coefficients meet the T1 rows of the other seven, so only rows that the same T1 blocks can
+    // reach share one: an Inf or NaN of a T1 row then gets no further than in the two block products
     perm.resize(nrow);
     for (int k = 0; k < nrow; ++k) perm[k] = k;
     std::stable_sort(perm.begin(), perm.end(), [&](int x, int y) {
+      if (reach[x] != reach[y]) return reach[x] > reach[y];
       if (nnz[x] != nnz[y]) return nnz[x] > nnz[y];
       for (int wd = 0; wd < words; ++wd) {
         const uint64_t mx = mask[(size_t)x * words + wd], my = mask[(size_t)y * words + wd];
@@ -556,8 +562,8 @@ void build_op(const SparseW &W1, const double *v1, const SparseW &W2, const doub
     rec.ent_b = (long long)out.r.size();
     rec.oct_b = (int)out.octs.size();
     os.clear();
-    for (int k0 = 0; k0 < nrow; k0 += 8) {
-      const int nk = std::min(8, nrow - k0);
+    for (int k0 = 0, nk; k0 < nrow; k0 += nk) {
+      for (nk = 1; nk < std::min(8, nrow - k0) && reach[perm[k0 + nk]] == reach[perm[k0]];) ++nk;
       qc_wxoct x;
       memset(&x, 0, sizeof(x));
       x.ent = (int)((long long)out.r.size() - rec.ent_b);
@@ -605,6 +611,7 @@ void build_op(const SparseW &W1, const double *v1, const SparseW &W2, const doub
       x.cnt = (int)((long long)out.r.size() - rec.ent_b) - x.ent;
       os.push_back(x);
     }
+    std::stable_sort(os.begin(), os.end(), [](const qc_wxoct &x, const qc_wxoct &y) { return x.cnt > y.cnt; });
     out.octs.insert(out.octs.end(), os.begin(), os.end());
     rec.noct = (int)os.size();
     out.dops.push_back(rec);
