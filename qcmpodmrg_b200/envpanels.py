@@ -202,6 +202,8 @@ class EnvPanels(object):
         # 11.2 instead of 9.0 ms)
         w = W.host(check=False)
         self._mpo = (W, w)
+        if not W.finite(w):
+            raise NoPanelForm
         wp = []
         for k, (g, rng) in enumerate(zip(parts, self.ranges)):
             if g is None:

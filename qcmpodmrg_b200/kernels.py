@@ -65,6 +65,7 @@ class TensorSet(object):
             self._given = None
         self.values = values
         self._f32 = None
+        self._finite = None
 
     def f32(self):
         if self._f32 is None or self._f32.data_ptr() == 0:
@@ -84,6 +85,14 @@ class TensorSet(object):
                 return host
             self._given = None
         return self.values.detach().to("cpu", torch.float64, copy=True).numpy()
+
+    def finite(self, host):
+        """Whether every element of ``host``, an array that host() returned, is finite.  The sparse
+        MPO stage needs that: it multiplies T1 blocks that symmetry leaves out as zeros, and drops
+        zero products."""
+        if self._finite is None or self._finite[0] is not host:
+            self._finite = (host, bool(numpy.isfinite(host).all()))
+        return self._finite[1]
 
     def op_values(self, i):
         o = int(self.offsets[i])
@@ -442,6 +451,10 @@ class SigmaOperator(object):
         self._plans, self._part_full = {}, False
         if sparse_w:
             w1, w2 = Wi.host(), Wj.host()
+            if not (Wi.finite(w1) and Wj.finite(w2)):
+                self.__init__(ws, isite, psi_layout, L, R, Wi, Wj, qkey, opers, hpwts, precision, tensor_cores,
+                              use_fiber, fuse_w, panel1, panel4, live, fg_budget, sparse_w=False)
+                return
             parts = [(x, rng, (WSource.of(x["W"][0], w1, Wi.offsets[ops]), WSource.of(x["W"][1], w2, Wj.offsets[ops])))
                      for x, ops, rng in wx_parts]
             self.wx = SparseWStage(parts, dev, "sigma23", op_table(bases[0][order], 0, bases[2][order], 1.0),
@@ -1205,7 +1218,7 @@ class Renormalizer(object):
     def __init__(self, ws, isite, status, site_layout, E, W, opers, panels=None):
         """panels: the panel form (None: on a GPU, where the blocks allow it)."""
         self.ws, self.status = ws, status
-        self._args = (ws, isite, status, site_layout, E, W, opers, panels)
+        self._args = (ws, isite, status, site_layout, E, W, opers), {"panels": panels}
         dev = ws.device
         groups = _groups(opers, isite, 1)
         nops = len(opers)
@@ -1325,7 +1338,7 @@ class Renormalizer(object):
         """site_values: packed site tensor (float64, device) -> new TensorSet."""
         ws = self.ws
         if self.ep is not None and not self.ep.current():
-            self.__init__(*self._args)
+            self.__init__(*self._args[0], **self._args[1])
         if self.ep is not None:
             out = torch.empty(max(self._nout, 1), dtype=torch.float64, device=ws.device)
             T2, S = self.ep.run(site_values)
@@ -1360,7 +1373,7 @@ class NoiseRDM(object):
         envpanels with the rows (l, n1') of one merged class in one panel, whose Gram matrix
         is one panel GEMM of the panel with itself."""
         self.ws, self.status = ws, status
-        self._args = (ws, isite, status, psi_layout, E, W, opers, qkey, dense_idl, panels)
+        self._args = (ws, isite, status, psi_layout, E, W, opers, qkey, dense_idl), {"panels": panels}
         dev = ws.device
         groups = _groups(opers, isite, 1)
         nops = len(opers)
@@ -1508,7 +1521,7 @@ class NoiseRDM(object):
         """psi_values: packed rank-3 wavefunction (device FP64) -> dense noise RDM (d x d)."""
         ws = self.ws
         if self.ep is not None and not self.ep.current():
-            self.__init__(*self._args)
+            self.__init__(*self._args[0], **self._args[1])
         if self.ep is not None:
             P = ws.get("npart", self.nops * self.size, torch.float64)
             T2, _ = self.ep.run(psi_values)

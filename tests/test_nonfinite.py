@@ -1,4 +1,4 @@
-"""An Inf or NaN gets no further through the sparse MPO stage than through the two block contractions."""
+"""An Inf or NaN gets no further through the sparse MPO stage than through the block contractions."""
 import numpy
 import pytest
 import torch
@@ -33,3 +33,50 @@ def test_a_bad_element_of_t1(tag, monkeypatch):
             bad, may = ~torch.isfinite(new), ~torch.isfinite(old)
             assert not bool((bad & ~may).any())
     assert used
+
+
+@pytest.mark.parametrize("at, bad", [(40, float("nan")), (120, float("inf"))])
+def test_a_bad_element_of_the_mpo(at, bad, monkeypatch):
+    """Operators of such an MPO keep the block contractions: the same non-finite elements, products,
+    environments and noise terms alike."""
+    from helpers import record_noise, record_renormalizer, tensorset
+    from qcmpodmrg_b200 import kernels
+    patch(monkeypatch)
+
+    def spoilt(dicts, device):
+        w = tensorset(dicts, device)
+        if len(w.layouts[0].nsyms) == 4:
+            nz = torch.nonzero(w.values).ravel()
+            w.values[nz[at % len(nz)]] = bad
+        return w
+
+    monkeypatch.setattr("helpers.tensorset", spoilt)
+    monkeypatch.setattr("test_sparse_w.tensorset", spoilt)
+
+    def both(cls, name, run):
+        make, out = cls.__init__, []
+        for on in (True, False):
+            with monkeypatch.context() as m, numpy.errstate(invalid="ignore"):
+                m.setattr(cls, "__init__", lambda self, *a, **k: make(self, *a, **dict({name: on}, **k)))
+                out.append(run())
+        return out
+
+    r = next(r for r in load("kernels_K5.npz")["records"] if numpy.ravel(r["key"])[2] == 1 and "renorm_site" in r)
+    x = torch.from_numpy(numpy.asarray(r["hvec_x"], dtype=numpy.float64))
+    a, b = (sparse_sigma(r, "cpu", on)(x) for on in (True, False))
+    assert not bool(torch.isfinite(b).all()) and torch.equal(torch.isfinite(a), torch.isfinite(b))
+
+    def renorm():
+        op, site = record_renormalizer(r, "cpu")
+        return op(torch.from_numpy(site)).values
+
+    a, b = both(kernels.Renormalizer, "panels", renorm)
+    assert not bool(torch.isfinite(b).all()) and torch.equal(torch.isfinite(a), torch.isfinite(b))
+    rn = next(r for r in load("kernels_NZ_K5.npz")["records"] if "prdm_cimat" in r and numpy.ravel(r["key"])[2] == 1)
+
+    def noise():
+        op, vals = record_noise(rn, "cpu")[:2]
+        return op(torch.as_tensor(vals))
+
+    a, b = both(kernels.NoiseRDM, "panels", noise)
+    assert not bool(torch.isfinite(b).all()) and torch.equal(torch.isfinite(a), torch.isfinite(b))
