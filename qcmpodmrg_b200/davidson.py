@@ -20,7 +20,7 @@ V0_MIN_NORM = 1.e-8
 
 
 def _ortho(vbas, rbas, crit_indp, times=5):
-    if rbas.is_cuda and rbas.dtype == torch.float64 and rbas.shape[0] == 1 and vbas.shape[0] <= 32:
+    if rbas.is_cuda and rbas.dtype == torch.float64 and rbas.shape[0] == 1 and 1 <= vbas.shape[0] <= 32:
         # one new vector (a single root): the passes in fused kernels
         v, r = vbas.contiguous(), rbas.contiguous()
         out = torch.empty_like(r)

@@ -26,3 +26,11 @@ def test_one_vector_against_the_matrix_form(m, n):
     # a vector inside the span has no new direction
     inside = torch.randn(1, m, dtype=torch.float64, generator=gen) @ v
     assert _ortho(v.cuda(), inside.cuda(), 1e-12) == (0, None)
+
+
+@pytest.mark.gpu
+def test_an_empty_basis():
+    """Nothing to remove: the vector, normalised."""
+    r = torch.tensor([[3.0, 4.0]], dtype=torch.float64)
+    k, out = _ortho(torch.zeros(0, 2, dtype=torch.float64, device="cuda"), r.cuda(), 1e-12)
+    assert k == 1 and float((out.cpu() - r / 5.0).abs().max()) <= 2.0 ** -52
