@@ -25,9 +25,10 @@ def _ortho(vbas, rbas, crit_indp, times=5):
         v, r = vbas.contiguous(), rbas.contiguous()
         out = torch.empty_like(r)
         work = torch.empty(native.lib().qc_ortho_work(), dtype=r.dtype, device=r.device)
-        native.check(native.lib().qc_ortho(v.data_ptr(), v.shape[0], v.shape[1], r.data_ptr(), out.data_ptr(),
-                                           work.data_ptr(), times, torch.cuda.current_stream(r.device).cuda_stream),
-                     "qc_ortho")
+        with torch.cuda.device(r.device):       # vectors need not be on the current device
+            native.check(native.lib().qc_ortho(v.data_ptr(), v.shape[0], v.shape[1], r.data_ptr(), out.data_ptr(),
+                                               work.data_ptr(), times,
+                                               torch.cuda.current_stream(r.device).cuda_stream), "qc_ortho")
         return (0, None) if float(work[0]) <= crit_indp else (1, out)
     rbas = rbas.clone()
     for _ in range(times):

@@ -34,3 +34,40 @@ def test_an_empty_basis():
     r = torch.tensor([[3.0, 4.0]], dtype=torch.float64)
     k, out = _ortho(torch.zeros(0, 2, dtype=torch.float64, device="cuda"), r.cuda(), 1e-12)
     assert k == 1 and float((out.cpu() - r / 5.0).abs().max()) <= 2.0 ** -52
+
+
+def test_launches_on_the_device_of_the_vectors(monkeypatch):
+    """Stand-ins for vectors of a device that is not the current one: the kernels are launched with
+    that device current."""
+    from unittest import mock
+    from qcmpodmrg_b200 import davidson
+    current = ["cuda:0"]
+
+    class Device(object):
+        def __init__(self, device):
+            self.device = device
+
+        def __enter__(self):
+            current.append(self.device)
+
+        def __exit__(self, *a):
+            current.pop()
+
+    def vector(rows):
+        t = mock.MagicMock(is_cuda=True, dtype=torch.float64, shape=(rows, 9), device="cuda:1")
+        t.contiguous.return_value = t
+        return t
+
+    seen = []
+    lib = mock.MagicMock()
+    lib.qc_ortho_work.return_value = 1
+    lib.qc_ortho.side_effect = lambda *a: seen.append(current[-1]) or 0
+    monkeypatch.setattr(davidson.native, "lib", lambda: lib)
+    monkeypatch.setattr(torch, "empty_like", lambda r: r)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda d: mock.MagicMock(device=d))
+    monkeypatch.setattr(torch.cuda, "device", Device)
+    work = mock.MagicMock()
+    work.__getitem__.return_value = 1.0
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: work)
+    assert _ortho(vector(3), vector(1), 1e-12)[0] == 1
+    assert seen == ["cuda:1"] and current == ["cuda:0"]
