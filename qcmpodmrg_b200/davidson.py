@@ -13,6 +13,7 @@ the reference's HVecs does (:67-78).
 import torch
 
 from . import native
+from .engine import LOG
 
 # a start vector of smaller norm carries no usable direction (a projected guess whose
 # weight lies outside the dot's blocks is rounding noise)
@@ -29,6 +30,7 @@ def _ortho(vbas, rbas, crit_indp, times=5):
             native.check(native.lib().qc_ortho(v.data_ptr(), v.shape[0], v.shape[1], r.data_ptr(), out.data_ptr(),
                                                work.data_ptr(), times,
                                                torch.cuda.current_stream(r.device).cuda_stream), "qc_ortho")
+        LOG.launches += times + 3
         return (0, None) if float(work[0]) <= crit_indp else (1, out)
     rbas = rbas.clone()
     for _ in range(times):

@@ -3,6 +3,7 @@ import pytest
 import torch
 
 from qcmpodmrg_b200.davidson import _ortho
+from qcmpodmrg_b200.engine import LOG
 
 
 @pytest.mark.gpu
@@ -69,5 +70,7 @@ def test_launches_on_the_device_of_the_vectors(monkeypatch):
     work = mock.MagicMock()
     work.__getitem__.return_value = 1.0
     monkeypatch.setattr(torch, "empty", lambda *a, **k: work)
+    before = LOG.launches
     assert _ortho(vector(3), vector(1), 1e-12)[0] == 1
+    assert LOG.launches - before == 8           # five passes, the last products, two scalings
     assert seen == ["cuda:1"] and current == ["cuda:0"]
