@@ -1023,6 +1023,7 @@ class SigmaOperator(object):
 
 
 _DENSE_STAGES = {}
+PANEL_OPS = 65535         # operators of one panel task: the launch's second grid extent
 
 
 def _diag_stages(dev, nops, A, Ab, Ac, ldim, rdim, hp):
@@ -1039,7 +1040,11 @@ def _diag_stages(dev, nops, A, Ab, Ac, ldim, rdim, hp):
     def stage(name, M, N, K, ops, count, crow=None, lda=None):
         z = numpy.zeros(1, dtype=numpy.int64)
         g = (z, z, z, z + M, z + N, z + K, z if crow is not None else z - 1, z + (K if lda is None else lda))
-        return PanelStage({c: [t] for c, t in compile_panels(g, (0, count)).items()}, dev, name, ops, crow=crow)
+        parts = {}
+        for b in range(0, count, PANEL_OPS):        # (spin projection: 16 x operators x quadrature points)
+            for c, t in compile_panels(g, (b, min(b + PANEL_OPS, count))).items():
+                parts.setdefault(c, []).append(t)
+        return PanelStage(parts, dev, name, ops, crow=crow)
 
     # X[p, n, m][a, c] = sum_b W1[p, n][a, b] W2[p, m][b, c]
     sX = stage("diagX", A, Ac, Ab, op_table((p * 4 + n) * A * Ab, (p * 4 + m) * Ab * Ac, (p * 16 + nm) * A * Ac, 1.0),
