@@ -18,7 +18,9 @@ candidate gives the same sigma (each output element is still one sum over the sa
 contracted rows in the same order; the check allows rounding, 1e-12 relative in FP64 and
 1e-5 otherwise), times the matrix-vector products with CUDA events and keeps the
 fastest.  The choice is cached per (precision, bond dimension) and applied to every later
-plan of the run (DMRG.sigma_opts).
+plan of the run (DMRG.sigma_opts).  A dot whose plan runs both contractions as the sparse
+product (the default where the blocks allow it) has no such stage: the default budgets stay
+and nothing is timed.
 """
 import time
 
@@ -71,6 +73,8 @@ def tune_fiber_budget(d, isite=None, candidates=CANDIDATES, repeats=4, precision
     for cand in candidates:
         d.sigma_opts["fg_budget"] = tuple(int(v) for v in cand)
         lay, idl, sig, dg = d.dot_operators(isite)
+        if sig.wx is not None:          # the sparse product took the place of both fiber stages: nothing to measure
+            break
         if x is None:
             ndim0 = int(sig.ndim0)
             x = torch.from_numpy(numpy.random.default_rng(7).standard_normal(ndim0)).to(d.device)
@@ -83,11 +87,13 @@ def tune_fiber_budget(d, isite=None, candidates=CANDIDATES, repeats=4, precision
                                % (cand, float((y - ref).abs().max())))
         table.append((tuple(int(v) for v in cand), round(ms, 4)))
         del sig, dg
-    best = min(table, key=lambda t: t[1])[0]
+    best = min(table, key=lambda t: t[1])[0] if table else (FG_A_BUDGET, FG_W_BUDGET)
     d.sigma_opts["fg_budget"] = best if best != (FG_A_BUDGET, FG_W_BUDGET) else saved
     d.plan_cache_size = cache_size
     d.plan_cache.clear()
     rep = {"choice": best, "table": table, "dot": isite, "ndim0": ndim0, "precision": prec, "bond": dmax,
            "s": round(time.time() - t0, 2)}
+    if not table:
+        rep["reason"] = "the dot's MPO-site contractions run as one sparse product, which the budgets do not concern"
     _CACHE[key] = rep
     return rep

@@ -43,6 +43,29 @@ def test_fiber_budget_candidates_agree_and_choice_applies(monkeypatch):
         assert (st.a_budget, st.w_budget) == tuple(rep["choice"])
 
 
+def test_nothing_is_timed_with_the_sparse_product(monkeypatch):
+    """Plans without fiber stages: the default budgets, after one plan and no products."""
+    from test_sparse_w import patch
+    patch(monkeypatch)
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda *a, **k: None)
+    monkeypatch.setattr(torch.cuda, "get_device_name", lambda *a, **k: "cpu-interpreter")
+    from qcmpodmrg_b200 import autotune
+    from qcmpodmrg_b200.dmrg import DMRG
+    fx = load("sweep_K6.npz")
+    ham = make_hamiltonian(int(fx["K"]), int(fx["N"]), int(fx["seed"]), None if fx["decay"] < 0 else fx["decay"])
+    d = DMRG(ham, device="cpu", precision="f64")
+    d.sigma_opts["sparse_w"] = True
+    d.load_mps(fx["init_mps"])
+    d.sweep("R", int(fx["D"]), 1e-8)
+    monkeypatch.setattr(autotune, "_time_sigma", lambda *a: 1 / 0)
+    autotune._CACHE.clear()
+    rep = autotune.tune_fiber_budget(d, 2)
+    assert rep["choice"] == (autotune.FG_A_BUDGET, autotune.FG_W_BUDGET) and rep["table"] == [] and rep["reason"]
+    assert d.sigma_opts.get("fg_budget") is None
+    assert autotune.tune_fiber_budget(d, 2)["cached"]
+    autotune._CACHE.clear()
+
+
 def _fiber_stages(sig):
     from qcmpodmrg_b200.engine import FiberStage, CompositeStage
     out = []
