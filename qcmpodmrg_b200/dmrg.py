@@ -155,7 +155,8 @@ class DMRG(object):
         self.psi0 = None
 
     # ------------------------------------------------------------- one dot
-    def dot_operators(self, isite):
+    def dot_operators(self, isite, direct=True):
+        """direct: see SigmaOperator (False for products in lockstep batches)."""
         ql, qr = self.qnuml[isite], self.qnumr[isite + 2]
         cls = [classification(q) for q in (ql, QPHYS, QPHYS, self.qkey - qr)]
         lay = Layout(PSI_STATUS, [c[0] for c in cls], [c[1] for c in cls])
@@ -175,12 +176,13 @@ class DMRG(object):
         if (hit is not None and hit[0] is lay and all(a is b for a, b in zip(hit[1], L.layouts))
                 and all(a is b for a, b in zip(hit[2], R.layouts))):
             sig, dg = hit[3], hit[4]
+            sig.direct = direct
             sig.rebind(L, R)
             dg.rebind(L, R)
             self.stats["plan_hits"] = self.stats.get("plan_hits", 0) + 1
             return lay, idl, sig, dg
         sig = SigmaOperator(self.ws, isite, lay, L, R, Wi, Wj, self.qkey, self.opers, self.hpwts, self.precision,
-                            **self.sigma_opts)
+                            direct=direct, **self.sigma_opts)
         wp = self.stats.setdefault("w_paths", {})
         for k, v in sig.w_paths.items():
             wp[k] = wp.get(k, 0) + v
@@ -259,7 +261,7 @@ class DMRG(object):
     def dot_begin(self, isite, crit_e):
         """Plans, diagonal and a Davidson generator for the dot; returns a context."""
         from .davidson import davidson_steps
-        lay, idl, sig, dg = self.dot_operators(isite)
+        lay, idl, sig, dg = self.dot_operators(isite, direct=False)
         prj = torch.from_numpy(lay.prjmap(idl)).to(self.device)
         diag = dg()
         v0 = None

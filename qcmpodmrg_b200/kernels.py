@@ -219,8 +219,10 @@ class SigmaOperator(object):
 
     def __init__(self, ws, isite, psi_layout, L, R, Wi, Wj, qkey, opers, hpwts, precision="f64",
                  tensor_cores=None, use_fiber=False, fuse_w=True, panel1=True, panel4=True, live=None,
-                 fg_budget=None, sparse_w=None):
-        """sparse_w: the two MPO-site contractions as one sparse product (qc_wsparse, the fiber
+                 fg_budget=None, sparse_w=None, direct=True):
+        """direct: the K-major panels of a product on its own are made now; False: by the first such
+        product (lockstep batches run on the row-major panels and would hold both).
+        sparse_w: the two MPO-site contractions as one sparse product (qc_wsparse, the fiber
         path without fuse_w); None: on a GPU, where the plan's blocks allow it.
         fg_budget: (A, W) shared-memory budgets of the dense fiber-group GEMM (qc_fgemm), as
         chosen by qcmpodmrg_b200.autotune; None keeps the engine's defaults.
@@ -453,7 +455,7 @@ class SigmaOperator(object):
             w1, w2 = Wi.host(), Wj.host()
             if not (Wi.finite(w1) and Wj.finite(w2)):
                 self.__init__(ws, isite, psi_layout, L, R, Wi, Wj, qkey, opers, hpwts, precision, tensor_cores,
-                              use_fiber, fuse_w, panel1, panel4, live, fg_budget, sparse_w=False)
+                              use_fiber, fuse_w, panel1, panel4, live, fg_budget, sparse_w=False, direct=direct)
                 return
             parts = [(x, rng, (WSource.of(x["W"][0], w1, Wi.offsets[ops]), WSource.of(x["W"][1], w2, Wj.offsets[ops])))
                      for x, ops, rng in wx_parts]
@@ -481,11 +483,15 @@ class SigmaOperator(object):
         # the transposed R panels, the wavefunction's panels): split TF32 on the tcgen05 kernel,
         # and FP64 (on the tensor pipe) or FP32 where the sparse product runs between them
         self.tc1 = self.tc4 = self.d1 = self.d4 = self.f1 = self.f4 = None
+        self.direct, self._kmajor = direct, False
+        self.lpan64 = self.lpan_f32 = self.lpan_tc = self.rpan64 = self.rpan_f32 = self.rpan_tc = None
         crow = numpy.concatenate(crow_all) if crow_all else numpy.zeros(1, numpy.int64)
         if tc1_classes:
             self._setup_panels1(tc1_classes, order, L, tabs[0], want_tc1, sparse_w)
         if tc4_classes:
             self._setup_panels4(tc4_classes, order, bases[2], R, tabs[3], crow, want_tc4, sparse_w)
+        if direct:
+            self._build_kmajor()
         # fused W stage (T1 -> T3) and the per-dot two-site MPO blocks it reads
         self.fused = None
         self.wtot = wtot
@@ -630,10 +636,9 @@ class SigmaOperator(object):
             self._build_lpan(self.d1 is not None)
         if self.rperm is not None:
             self._build_rpan(self.d4 is not None)
-        if self.tc4 is not None or self.d4 is not None:
-            self._build_rpan_k()
-        if self.tc1 is not None or self.d1 is not None:
-            self._build_lpan_k()
+        self._kmajor = False
+        if self.direct:
+            self._build_kmajor()
 
     def _setup_panels4(self, tc4_classes, order, t3bases, R, st4_ops, crow, tc, f64):
         from .engine import TCPanelStage, tc_sigma4_units
@@ -685,7 +690,6 @@ class SigmaOperator(object):
                          for (poss, sec, _) in classes]
                 st = DPanelStage("sigma4", parts, ops, dev, flops, crow=crow, longest_first=True, kind=kind)
                 self.d4, self.f4 = (st, self.f4) if kind == "f64" else (self.d4, st)
-        self._build_rpan_k()
 
     def _setup_panels1(self, tc1_classes, order, L, st1_ops, tc, f64):
         from .engine import TCPanelStage, tc_sigma1_units
@@ -728,7 +732,6 @@ class SigmaOperator(object):
         self._lp_descs_d = upload(self._lp_descs, dev)
         self._lp_ops_d = upload(op_table(L.offsets[order], 0, base, 1.0), dev)
         self._lp_span = int(max(len(c[0]) for c in classes))
-        self._build_lpan_k()
 
     @staticmethod
     def _dpanel1_units(classes, info, cols, kind):
@@ -758,6 +761,14 @@ class SigmaOperator(object):
                              [info[s][0] for s in sec], [base + col0[s] for s in sec], "col", kind=kind)
             parts.append((u, (poss[0], poss[-1] + 1)))
         return parts, numpy.concatenate(tabs)
+
+    def _build_kmajor(self):
+        if self.tc4 is not None or self.d4 is not None:
+            self._build_rpan_k()
+        if self.tc1 is not None or self.d1 is not None:
+            self._build_lpan_k()
+        # (made by every replay where a graph is captured)
+        self._kmajor = torch.device(self.ws.device).type != "cuda" or not torch.cuda.is_current_stream_capturing()
 
     def _build_lpan_k(self):
         """K-major L panels [M x Kp] per sector: FP32 hi plane then lo plane for the tcgen05 kernel,
@@ -955,6 +966,8 @@ class SigmaOperator(object):
         prec = precision or self.precision
         if y is None:
             y = torch.empty(self.ndim0, dtype=torch.float64, device=ws.device)
+        if not self._kmajor:
+            self._build_kmajor()
         # in panel form all through: one native call (the launch log times the stages one by one)
         if self.wx is not None and x.is_cuda and not LOG.enabled and (
                 prec == "f64" or (prec == "f32" and self.f1 is not None) or

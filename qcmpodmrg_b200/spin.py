@@ -334,7 +334,7 @@ class SPDMRG(DMRG):
         reference also contracts the zero blocks; skipping them changes no result)."""
         return lay.allowed.astype(bool) if self.prune_zero_blocks else None
 
-    def dot_operators(self, isite):
+    def dot_operators(self, isite, direct=True):
         """H_eff (projected) and its diagonal for the dot; the plan is compiled per dot."""
         lay, idl = self._psi_layout(isite)
         lay_n = reduce_layout(lay)
@@ -342,7 +342,7 @@ class SPDMRG(DMRG):
         L, R = self.lenv[isite - 1], self.renv[isite + 2]
         Wi, Wj = self.mpo[isite], self.mpo[isite + 1]
         inner = SigmaOperator(self.ws, isite, lay_n, L, R, Wi, Wj, self.qkey[:1], self.opers, self.hpwts,
-                              self.precision, live=self._live(lay), **self.sigma_opts)
+                              self.precision, live=self._live(lay), direct=direct, **self.sigma_opts)
         sig = ProjectedOperator(self.ws, inner, red)
         dg = DiagOperator(self.ws, isite, lay, L, R, Wi, Wj, self.qkey, self.opers, self.hpwts)
         return lay, idl, sig, dg
