@@ -26,9 +26,12 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <atomic>
+#include <condition_variable>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <memory>
+#include <mutex>
 #include <new>
 #include <thread>
 #include <vector>
@@ -440,13 +443,33 @@ struct Nz {
   double v;
 };
 
-// A packed W tensor [a, b, n', n] of one class: block (sa, sb, n', n) has its non-zeros
-// listed row by row (row a or, for the second site, row b).
+// A packed W tensor [a, b, n', n] of one class; row0: where an allowed block's rows a stand in a
+// NzRows (-1: not allowed), rows: all of them.
 struct SparseW {
   int ns[4];
   const long long *nd[4];
   const long long *ioff;
   const int *allowed;
+  std::vector<int> row0;
+  int rows = 0;
+  long long size = 0;          // elements of an operator
+
+  void number_rows() {
+    const int per = ns[1] * ns[2] * ns[3], nb = ns[0] * per;
+    row0.assign(nb, -1);
+    for (int b = 0; b < nb; ++b)
+      if (allowed[b]) {
+        row0[b] = rows;
+        rows += (int)nd[0][b / per];
+        size += nd[0][b / per] * nd[1][b / (ns[2] * ns[3]) % ns[1]];
+      }
+  }
+};
+
+// the non-zeros of one operator's tensor, row by row of its allowed blocks
+struct NzRows {
+  std::vector<int> start;
+  std::unique_ptr<Nz[]> nz;
 };
 
 struct OpLists {
@@ -456,81 +479,98 @@ struct OpLists {
   std::vector<int> r;
 };
 
-// rows of the non-zeros of every allowed block: start[block][row], flat lists
-void list_rows(const SparseW &W, const double *val, std::vector<std::vector<int>> &start,
-               std::vector<std::vector<Nz>> &nz) {
-  const int nb = W.ns[0] * W.ns[1] * W.ns[2] * W.ns[3];
-  start.assign(nb, std::vector<int>());
-  nz.assign(nb, std::vector<Nz>());
+void list_rows(const SparseW &W, const double *val, NzRows &out) {
+  const int per = W.ns[1] * W.ns[2] * W.ns[3], nb = W.ns[0] * per;
+  out.start.reserve(W.rows + 1);
+  out.nz.reset(new Nz[W.size + 1]);
+  Nz *q = out.nz.get();
   for (int b = 0; b < nb; ++b) {
-    if (!W.allowed[b]) continue;
-    const int sa = b / (W.ns[1] * W.ns[2] * W.ns[3]), sb = b / (W.ns[2] * W.ns[3]) % W.ns[1];
-    const int na = (int)W.nd[0][sa], nbb = (int)W.nd[1][sb];
+    if (W.row0[b] < 0) continue;
+    const int na = (int)W.nd[0][b / per], nbb = (int)W.nd[1][b / (W.ns[2] * W.ns[3]) % W.ns[1]];
     const double *p = val + W.ioff[b];
-    start[b].resize(na + 1);
-    for (int a = 0; a < na; ++a) {
-      start[b][a] = (int)nz[b].size();
-      for (int j = 0; j < nbb; ++j)
-        if (p[(long long)a * nbb + j] != 0.0) nz[b].push_back(Nz{j, p[(long long)a * nbb + j]});
+    for (int a = 0; a < na; ++a, p += nbb) {
+      out.start.push_back((int)(q - out.nz.get()));
+      for (int j = 0; j < nbb; ++j) {        // (written always: a branch is mispredicted at every other non-zero)
+        *q = Nz{j, p[j]};
+        q += p[j] != 0.0;
+      }
     }
-    start[b][na] = (int)nz[b].size();
   }
+  out.start.push_back((int)(q - out.nz.get()));
 }
 
-void build_op(const SparseW &W1, const double *v1, const SparseW &W2, const double *v2, int ndelta, const int *iblk,
-              const int *kblk, const int *row0, const int *Rs, OpLists &out) {
-  std::vector<std::vector<int>> st1, st2;
-  std::vector<std::vector<Nz>> nz1, nz2;
-  list_rows(W1, v1, st1, nz1);
-  list_rows(W2, v2, st2, nz2);
-  const int nsb = W1.ns[1];
-  std::vector<double> S;                 // rows of the current delta, dense in i
-  std::vector<uint64_t> mask;
-  std::vector<int> rowid, nnz, perm, reach;
-  std::vector<qc_wxoct> os;
+// What the rows of one delta are made of, for every operator of the class: products of the blocks
+// (T1 block ib, MPO sector sb) -> T3 block kb that symmetry allows, and the rows' blocks.
+struct DeltaPlan {
+  struct Product {
+    int k0, i0, na, r1, r2;    // first row k, first row i, rows i, rows of both blocks in their NzRows
+  };
+  int R, nrow = 0;
+  std::vector<Product> products;
+  std::vector<int> rowid, reach;     // block << 16 | c; T1 blocks that reach the row (one bit each)
+};
+
+void plan_deltas(const SparseW &W1, const SparseW &W2, int ndelta, const int *iblk, const int *kblk, const int *row0,
+                 const int *Rs, std::vector<DeltaPlan> &out) {
+  // sectors sb that (sa, n1', n1) connects to
+  std::vector<std::vector<int>> via((size_t)W1.ns[0] * 16);
+  for (int sa = 0; sa < W1.ns[0]; ++sa)
+    for (int sb = 0; sb < W1.ns[1]; ++sb)
+      for (int n = 0; n < 16; ++n)
+        if (W1.row0[(sa * W1.ns[1] + sb) * 16 + n] >= 0) via[16 * sa + n].push_back(sb);
+  out.resize(ndelta);
   for (int d = 0; d < ndelta; ++d) {
-    const int R = Rs[d];
-    const int words = (R + 63) / 64;
-    int nrow = 0;
-    for (int kb = 0; kb < 16; ++kb)
-      if (kblk[16 * d + kb] >= 0) nrow += (int)W2.nd[1][kblk[16 * d + kb]];
-    S.assign((size_t)nrow * R, 0.0);
-    mask.assign((size_t)nrow * words, 0);
-    rowid.resize(nrow);
-    reach.assign(nrow, 0);
-    int base = 0;
+    DeltaPlan &x = out[d];
+    x.R = Rs[d];
     for (int kb = 0; kb < 16; ++kb) {
       const int sc = kblk[16 * d + kb];
       if (sc < 0) continue;
-      const int nc = (int)W2.nd[1][sc];
-      const int n1p = kb >> 2, n2p = kb & 3;
-      for (int c = 0; c < nc; ++c) rowid[base + c] = kb << 16 | c;
+      int reach = 0;
       for (int ib = 0; ib < 16; ++ib) {
         const int sa = iblk[16 * d + ib];
         if (sa < 0) continue;
-        const int n1 = ib >> 2, n2 = ib & 3;
-        const int na = (int)W1.nd[0][sa], r0 = row0[16 * d + ib];
-        for (int sb = 0; sb < nsb; ++sb) {
-          const int b1 = ((sa * W1.ns[1] + sb) * W1.ns[2] + n1p) * W1.ns[3] + n1;
-          const int b2 = ((sb * W2.ns[1] + sc) * W2.ns[2] + n2p) * W2.ns[3] + n2;
-          if (!W1.allowed[b1] || !W2.allowed[b2]) continue;
-          for (int c = 0; c < nc; ++c) reach[base + c] |= 1 << ib;
-          if (nz1[b1].empty() || nz2[b2].empty()) continue;
-          for (int a = 0; a < na; ++a) {
-            const int i = r0 + a;
-            for (int x = st1[b1][a]; x < st1[b1][a + 1]; ++x) {
-              const Nz u = nz1[b1][x];
-              for (int y = st2[b2][u.j]; y < st2[b2][u.j + 1]; ++y) {
-                const Nz w = nz2[b2][y];
-                S[(size_t)(base + w.j) * R + i] += u.v * w.v;
-                mask[(size_t)(base + w.j) * words + (i >> 6)] |= 1ull << (i & 63);
-              }
-            }
+        const int n = 4 * (kb >> 2) + (ib >> 2), m = 4 * (kb & 3) + (ib & 3);       // (n1', n1), (n2', n2)
+        for (int sb : via[16 * sa + n]) {
+          const int r1 = W1.row0[(sa * W1.ns[1] + sb) * 16 + n], r2 = W2.row0[(sb * W2.ns[1] + sc) * 16 + m];
+          if (r2 < 0) continue;
+          reach |= 1 << ib;
+          x.products.push_back({x.nrow, row0[16 * d + ib], (int)W1.nd[0][sa], r1, r2});
+        }
+      }
+      for (int c = 0; c < (int)W2.nd[1][sc]; ++c) x.rowid.push_back(kb << 16 | c);
+      x.nrow = (int)x.rowid.size();
+      x.reach.resize(x.nrow, reach);
+    }
+  }
+}
+
+void build_op(const SparseW &W1, const double *v1, const SparseW &W2, const double *v2,
+              const std::vector<DeltaPlan> &deltas, OpLists &out) {
+  NzRows l1, l2;
+  list_rows(W1, v1, l1);
+  list_rows(W2, v2, l2);
+  std::vector<double> S;                 // rows of the current delta, dense in i
+  std::vector<uint64_t> mask;
+  std::vector<int> nnz, perm, bucket[4];
+  std::vector<qc_wxoct> os;
+  for (const DeltaPlan &dp : deltas) {
+    const int R = dp.R, nrow = dp.nrow;
+    const int words = (R + 63) / 64;
+    const std::vector<int> &rowid = dp.rowid, &reach = dp.reach;
+    S.assign((size_t)nrow * R, 0.0);
+    mask.assign((size_t)nrow * words, 0);
+    for (const auto &p : dp.products)
+      for (int a = 0; a < p.na; ++a) {
+        const int i = p.i0 + a;
+        for (int x = l1.start[p.r1 + a]; x < l1.start[p.r1 + a + 1]; ++x) {
+          const Nz u = l1.nz[x];
+          for (int y = l2.start[p.r2 + u.j]; y < l2.start[p.r2 + u.j + 1]; ++y) {
+            const Nz w = l2.nz[y];
+            S[(size_t)(p.k0 + w.j) * R + i] += u.v * w.v;
+            mask[(size_t)(p.k0 + w.j) * words + (i >> 6)] |= 1ull << (i & 63);
           }
         }
       }
-      base += nc;
-    }
     // products that cancelled exactly are no entries
     nnz.assign(nrow, 0);
     for (int k = 0; k < nrow; ++k)
@@ -569,7 +609,7 @@ void build_op(const SparseW &W1, const double *v1, const SparseW &W2, const doub
       x.ent = (int)((long long)out.r.size() - rec.ent_b);
       for (int k = 0; k < 8; ++k) x.row[k] = k < nk ? rowid[perm[k0 + k]] : -1;
       // the T1 rows any of the eight reads, in fours of different residues mod 4 where possible
-      std::vector<int> bucket[4];
+      for (auto &b : bucket) b.clear();
       for (int wd = 0; wd < words; ++wd) {
         uint64_t m = 0;
         for (int k = 0; k < nk; ++k) m |= mask[(size_t)perm[k0 + k] * words + wd];
@@ -621,6 +661,7 @@ void build_op(const SparseW &W1, const double *v1, const SparseW &W2, const doub
 struct WxBuild {
   struct Part {
     SparseW W1, W2;
+    std::vector<DeltaPlan> deltas;
     const qc_wxpart *in;
     long long op0;
   };
@@ -628,27 +669,44 @@ struct WxBuild {
   std::vector<OpLists> ops;      // of all parts
 };
 
-// f(0) .. f(n - 1) on the host's threads; false if one of them threw
+// f(0) .. f(n - 1) on the host's threads; false if one of them threw.  The caller waits for the
+// items, not for the threads: a CPU of a shared host that has to wake can take a scheduler tick
+// or two to start one, which then finds nothing left.  Renormalisations from the right at K=24, D=16
+// and 60 took 7.9 ms in the median with a join of the threads, in steps of 4 ms; 5.2 and 5.7 ms now
+// (with the deltas planned once a class and the exchanged bonds kept, 7.3 and 7.4 without either).
+// A thread touches f only for an item, and so only while the caller waits for it.
 template <typename F>
-bool wx_each(long long n, F f) {
-  std::atomic<long long> next{0};
-  std::atomic<bool> bad{false};
-  auto loop = [&]() {
-    try {
-      for (long long i; (i = next.fetch_add(1)) < n;) f(i);
-    } catch (...) {
-      bad = true;
+bool wx_each(long long n, const F &f) {
+  struct State {
+    std::atomic<long long> next{0}, done{0};
+    std::atomic<bool> bad{false};
+    std::mutex m;
+    std::condition_variable all;
+  };
+  const auto st = std::make_shared<State>();
+  const F *const fp = &f;
+  auto loop = [st, n, fp]() {
+    for (long long i; (i = st->next.fetch_add(1)) < n;) {
+      try {
+        (*fp)(i);
+      } catch (...) {
+        st->bad = true;
+      }
+      if (st->done.fetch_add(1) + 1 == n) {
+        std::lock_guard<std::mutex> l(st->m);
+        st->all.notify_one();
+      }
     }
   };
   const long long hw = std::max(1u, std::thread::hardware_concurrency());
-  std::vector<std::thread> th;
   try {
-    for (long long k = 1; k < std::min({8ll, hw, n / 4}); ++k) th.emplace_back(loop);
+    for (long long k = 1; k < std::min({8ll, hw, n / 4}); ++k) std::thread(loop).detach();
   } catch (...) {              // no more threads: the others do their share
   }
   loop();
-  for (auto &t : th) t.join();
-  return !bad;
+  std::unique_lock<std::mutex> l(st->m);
+  st->all.wait(l, [&]() { return st->done.load() >= n; });
+  return !st->bad;
 }
 
 }  // namespace
@@ -700,6 +758,10 @@ extern "C" int qc_wx_build(int nparts, const void *parts, void **handle, long lo
             (sa >= 0 && (x.row0[i] < 0 || x.row0[i] + p.W1.nd[0][sa] > x.R[i / 16])))
           rc = QC_ERR_ARG;
       }
+      if (rc != QC_OK) break;
+      p.W1.number_rows();
+      p.W2.number_rows();
+      plan_deltas(p.W1, p.W2, x.ndelta, x.iblk, x.kblk, x.row0, x.R, p.deltas);
     }
     if (rc == QC_OK) {
       h->ops.resize(nops);
@@ -707,8 +769,7 @@ extern "C" int qc_wx_build(int nparts, const void *parts, void **handle, long lo
         const WxBuild::Part *p = h->parts.data() + nparts - 1;
         while (p->op0 > o) --p;
         const qc_wxpart &x = *p->in;
-        build_op(p->W1, x.w1 + x.off1[o - p->op0], p->W2, x.w2 + x.off2[o - p->op0], x.ndelta, x.iblk, x.kblk, x.row0,
-                 x.R, h->ops[o]);
+        build_op(p->W1, x.w1 + x.off1[o - p->op0], p->W2, x.w2 + x.off2[o - p->op0], p->deltas, h->ops[o]);
       });
       rc = ok ? QC_OK : QC_ERR_CAPACITY;
     }

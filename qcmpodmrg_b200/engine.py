@@ -1281,24 +1281,11 @@ class WSource(object):
 
     @staticmethod
     def transposed(lay, values, offsets):
-        """The bonds exchanged: every block transposed in place (values: the operators' packed
-        values back to back, one row of ``lay.size`` per operator)."""
+        """The bonds exchanged; values: those of ``transposed_values``."""
         ns = [int(x) for x in lay.nsyms]
-        perm = _W_PERM.get(id(lay))
-        if perm is None or perm[0] is not lay:
-            d = lay.block_dims(lay.idx_allowed)
-            b, e = _ranges(d[:, 0] * d[:, 1])
-            src = lay.ioff[lay.idx_allowed][b]
-            if len(_W_PERM) > 512:
-                _W_PERM.clear()
-            # element e of the transposed block is (e / D_a, e % D_a) = (b, a)
-            perm = _W_PERM[id(lay)] = (lay, src + (e % d[b, 0]) * d[b, 1] + e // d[b, 0])
-        n = len(offsets)
-        vals = numpy.asarray(values)[numpy.asarray(offsets)[:, None] + perm[1][None, :]]
         nd = numpy.concatenate([lay.ndims[1], lay.ndims[0], lay.ndims[2], lay.ndims[3]])
         tr = lambda v: numpy.asarray(v).reshape(ns).transpose(1, 0, 2, 3).ravel()          # noqa: E731
-        return WSource(vals.ravel(), numpy.arange(n) * lay.size, [ns[1], ns[0], ns[2], ns[3]], nd, tr(lay.ioff),
-                       tr(lay.allowed))
+        return WSource(values, offsets, [ns[1], ns[0], ns[2], ns[3]], nd, tr(lay.ioff), tr(lay.allowed))
 
     @staticmethod
     def identity(ndims, nops):
@@ -1319,6 +1306,27 @@ class WSource(object):
 
 
 _W_PERM = {}
+
+
+def transposed_values(layouts, values, offsets):
+    """A copy of the packed values of MPO tensors with every block [a, b] transposed in its place."""
+    out = numpy.array(values)
+    by = {}
+    for lay, o in zip(layouts, offsets):
+        by.setdefault(id(lay), (lay, []))[1].append(int(o))
+    for lay, off in by.values():
+        perm = _W_PERM.get(id(lay))
+        if perm is None or perm[0] is not lay:
+            d = lay.block_dims(lay.idx_allowed)
+            b, e = _ranges(d[:, 0] * d[:, 1])
+            src = lay.ioff[lay.idx_allowed][b]
+            if len(_W_PERM) > 512:
+                _W_PERM.clear()
+            # element e of the transposed block is (e / D_a, e % D_a) = (b, a)
+            perm = _W_PERM[id(lay)] = (lay, src + (e % d[b, 0]) * d[b, 1] + e // d[b, 0])
+        for o in off:           # (blocks are packed in this order)
+            out[o:o + lay.size] = values[o:o + lay.size][perm[1]]
+    return out
 
 
 def f32_weights(w):

@@ -204,11 +204,13 @@ class EnvPanels(object):
         self._mpo = (W, w)
         if not W.finite(w):
             raise NoPanelForm
+        source = WSource.of if left else WSource.transposed
+        values = w if left else W.transposed(w)
         wp = []
         for k, (g, rng) in enumerate(zip(parts, self.ranges)):
             if g is None:
                 continue
-            f = (WSource.of if left else WSource.transposed)(self.Wl[k], w, W.offsets[self.ops[k]])
+            f = source(self.Wl[k], values, W.offsets[self.ops[k]])
             wp.append((g, rng, (f, WSource.identity(self.Wl[k].ndims[wax], rng[1] - rng[0]))))
         z = numpy.zeros(self.nops, dtype=i64)
         self.wx = SparseWStage(wp, dev, self.name + "2", op_table(self.base_1, 0, self.base_2, 1.0)) if wp else None
