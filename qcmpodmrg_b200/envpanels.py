@@ -65,7 +65,19 @@ class EnvPanels(object):
                     raise NoPanelForm
         dx, dz = (numpy.asarray(site.ndims[k], dtype=i64) for k in (old, new))
         self.dx, self.dz = dx, dz
-        if any(not numpy.array_equal(el.ndims[k], dx) for el in self.El for k in (1, 2)):
+        # contracted indices have the same sectors in the same order (the block contractions, which take
+        # what does not, refuse other ones): E's bond states those of S, its MPO bond W's
+        wk, sign = (0, 1) if left else (1, -1)
+
+        def same(mine, theirs):
+            return [len(v) for v in mine] == [len(v) for v in theirs] and \
+                numpy.array_equal(numpy.concatenate(mine), numpy.concatenate(theirs))
+
+        bonds = [(el, k) for el in self.El for k in (1, 2)]
+        if not (same([el.ndims[k] for el, k in bonds], [dx] * len(bonds))
+                and same([_q2(el.qsyms[k]) for el, k in bonds], [_q2(qx)] * len(bonds))
+                and same([el.ndims[0] for el in self.El], [wl.ndims[wk] for wl in self.Wl])
+                and same([_q2(el.qsyms[0]) for el in self.El], [sign * _q2(wl.qsyms[wk]) for wl in self.Wl])):
             raise NoPanelForm
         ncls, nx, nz = len(self.ops), len(dx), len(dz)
         # ---- S: blocks sorted by contracted sector, side by side as the columns of its panel
@@ -159,6 +171,8 @@ class EnvPanels(object):
             self.db[k, :len(q)] = wl.ndims[wax]
             cq = code(q)
             o = numpy.argsort(cq, kind="stable")
+            if (numpy.diff(cq[o]) == 0).any():          # two sectors of one quantum number
+                raise NoPanelForm
             at = o[numpy.minimum(numpy.searchsorted(cq[o], cw), len(q) - 1)]
             self.b[k] = numpy.where(cq[at] == cw, at, -1)
         self._w = (W, left, wax, qx, qz, da)
