@@ -1106,11 +1106,12 @@ def _ragged(n):
 
 
 def _neutral(lay, axis):
-    """Sector of an MPO bond with quantum number zero (-1: none) and its extent.  Diagonal
-    blocks E[a, l, l] and W[a, b, n, n] between neutral bond states are all that the
-    diagonal of H_eff reads."""
-    z = numpy.flatnonzero((numpy.rint(2 * numpy.asarray(lay.qsyms[axis])) == 0).all(axis=1))
-    return (int(z[0]), int(lay.ndims[axis][z[0]])) if len(z) else (-1, 0)
+    """First neutral state of every sector of an MPO bond among those of quantum number zero (-1:
+    another quantum number), and the number of neutral states.  Diagonal blocks E[a, l, l] and
+    W[a, b, n, n] between them are all that the diagonal of H_eff reads."""
+    z = (numpy.rint(2 * numpy.asarray(lay.qsyms[axis])) == 0).all(axis=1)
+    n = numpy.where(z, numpy.asarray(lay.ndims[axis], dtype=numpy.int64), 0)
+    return numpy.where(z, numpy.cumsum(n) - n, -1), int(n.sum())
 
 
 def _env_diag_map(lay, A, ncol, kfast):
@@ -1119,13 +1120,15 @@ def _env_diag_map(lay, A, ncol, kfast):
     def build():
         idx = lay.idx_allowed
         sa, s1, s2 = numpy.unravel_index(idx, tuple(lay.nsyms))
-        keep = (s1 == s2) & (sa == _neutral(lay, 0)[0])
-        idx, s1 = idx[keep], s1[keep]
+        a0 = _neutral(lay, 0)[0][sa]
+        keep = (s1 == s2) & (a0 >= 0)
+        idx, s1, a0 = idx[keep], s1[keep], a0[keep]
         d = lay.block_dims(idx) if len(idx) else numpy.zeros((0, 3), dtype=numpy.int64)
         da, dl = d[:, 0], d[:, 1]
         b, e = _ragged(da * dl)
         w, u = e // dl[b], e % dl[b]
         src = lay.ioff[idx][b] + w * dl[b] * dl[b] + u * dl[b] + u
+        w = w + a0[b]
         col = lay.secoff[1][s1][b] + u
         out = numpy.full(A * ncol, -1, dtype=numpy.int64)
         out[col * A + w if kfast else w * ncol + col] = src
@@ -1138,14 +1141,15 @@ def _w_diag_map(lay, A, B):
     def build():
         idx = lay.idx_allowed
         sa, sb, n, n_ = numpy.unravel_index(idx, tuple(lay.nsyms))
-        keep = (n == n_) & (sa == _neutral(lay, 0)[0]) & (sb == _neutral(lay, 1)[0])
-        idx, n = idx[keep], n[keep]
+        a0, b0 = _neutral(lay, 0)[0][sa], _neutral(lay, 1)[0][sb]
+        keep = (n == n_) & (a0 >= 0) & (b0 >= 0)
+        idx, n, a0, b0 = idx[keep], n[keep], a0[keep], b0[keep]
         d = lay.block_dims(idx) if len(idx) else numpy.zeros((0, 4), dtype=numpy.int64)
         da, db = d[:, 0], d[:, 1]
         b, e = _ragged(da * db)
         w, v = e // db[b], e % db[b]
         out = numpy.full(4 * A * B, -1, dtype=numpy.int64)
-        out[(n[b] * A + w) * B + v] = lay.ioff[idx][b] + w * db[b] + v
+        out[(n[b] * A + a0[b] + w) * B + b0[b] + v] = lay.ioff[idx][b] + w * db[b] + v
         return out
     return _cached(("w", id(lay), A, B), lay, build)
 
