@@ -69,15 +69,15 @@ class EnvPanels(object):
         # what does not, refuse other ones): E's bond states those of S, its MPO bond W's
         wk, sign = (0, 1) if left else (1, -1)
 
-        def same(mine, theirs):
+        def same(mine, theirs, number=numpy.asarray):
             return [len(v) for v in mine] == [len(v) for v in theirs] and \
-                numpy.array_equal(numpy.concatenate(mine), numpy.concatenate(theirs))
+                numpy.array_equal(number(numpy.concatenate(mine)), number(numpy.concatenate(theirs)))
 
         bonds = [(el, k) for el in self.El for k in (1, 2)]
         if not (same([el.ndims[k] for el, k in bonds], [dx] * len(bonds))
-                and same([_q2(el.qsyms[k]) for el, k in bonds], [_q2(qx)] * len(bonds))
+                and same([el.qsyms[k] for el, k in bonds], [qx] * len(bonds), _q2)
                 and same([el.ndims[0] for el in self.El], [wl.ndims[wk] for wl in self.Wl])
-                and same([_q2(el.qsyms[0]) for el in self.El], [sign * _q2(wl.qsyms[wk]) for wl in self.Wl])):
+                and same([sign * el.qsyms[0] for el in self.El], [wl.qsyms[wk] for wl in self.Wl], _q2)):
             raise NoPanelForm
         ncls, nx, nz = len(self.ops), len(dx), len(dz)
         # ---- S: blocks sorted by contracted sector, side by side as the columns of its panel
