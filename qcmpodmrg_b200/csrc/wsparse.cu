@@ -21,7 +21,8 @@
 // in FP64, 3.0 ms, and half of that in FP32): two dense stages took 30.2 ms in FP64 and 15.5 ms in
 // FP32, lists of four consecutive rows on scalar multiply-adds 8.1 and 4.6 ms (shared-memory pipe
 // 72 % busy: a row read and a coefficient broadcast for every four rows), octets of like rows
-// 6.0 and 4.05 ms (D = 200: 1.37 -> 1.00, 0.78 -> 0.71 ms).  FP32 is still bound by the shared-memory
+// 6.0 and 4.05 ms (D = 200: 1.37 -> 1.00, 0.78 -> 0.71 ms), 6.07 and 4.09 (1.00, 0.72) since an octet
+// ends where the T1 blocks that reach its rows change.  FP32 is still bound by the shared-memory
 // pipe (75 %); copying alone takes 2.2 and 1.3 ms of it.  Twelve warps of deeper prefetch: 5.99, 4.11.
 #include <cuda_runtime.h>
 #include <algorithm>

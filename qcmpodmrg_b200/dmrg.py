@@ -124,8 +124,8 @@ class DMRG(object):
         # vector and both energies are appended here (off when None)
         self.shadow = None
         # mixed precision: one FP64 Davidson step after every accepted low-precision solve.
-        # Off: at K=24, D=500 it cost one more FP64 product per dot (1.36x instead of 1.43x
-        # over FP64) and did not bring converged D=200 energies closer to the FP64 run's
+        # Off: at K=24, D=500 it cost one more FP64 product per dot (before the sparse MPO product
+        # 1.36x instead of 1.43x over FP64) and did not bring converged D=200 energies closer to the FP64 run's
         self.fp64_step = False
 
     # ------------------------------------------------------------- set-up
