@@ -251,11 +251,10 @@ class EnvPanels(object):
     def run(self, values):
         """T2 and the panels of S for the packed values of S."""
         from . import kernels as K
-        get = self.ws.get
-        S = get("ep_site", self.site_size, torch.float64)
-        EP = get("ep_env", self.tot_e, torch.float64)
-        T1 = get("ep_t1", self.tot_1, torch.float64)
-        T2 = get("ep_t2", self.tot_2, torch.float64)
+        # scratch of its own for each kind of contraction: a noise term may run beside a renormalisation
+        get = lambda name, n: self.ws.get(self.name + name, n, torch.float64)          # noqa: E731
+        S, EP = get("_site", self.site_size), get("_env", self.tot_e)
+        T1, T2 = get("_t1", self.tot_1), get("_t2", self.tot_2)
         K.block_permute(self._site_d, len(self.site_descs), 1, self._one, values, S)
         K.block_permute(self._env_d, len(self.env_descs), self._span, self._env_ops, self.E.values, EP)
         self.d1.run(EP, S, T1)

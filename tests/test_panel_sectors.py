@@ -84,3 +84,17 @@ def test_a_repeated_sector_keeps_the_block_contractions(what, status, monkeypatc
     x = torch.from_numpy(rng.standard_normal(a[3].size))
     y, ref = (op(x) if what == "noise" else op(x).values for op in (cls(*a, panels=p) for p in (True, False)))
     assert torch.equal(y, ref)
+
+
+def test_scratch_is_not_shared(monkeypatch):
+    """A renormalisation and a noise term on one workspace use different buffers, as their block
+    contractions do, so that one may run beside the other on a stream of its own."""
+    patch(monkeypatch)
+    names = []
+    for what in ("renorm", "noise"):
+        cls, a = _args(what, "L", monkeypatch)
+        op = cls(*a, panels=True)
+        op(torch.zeros(a[3].size, dtype=torch.float64))
+        assert op.ep is not None
+        names.append(set(a[0].bufs))
+    assert names[0] and names[1] and not names[0] & names[1]
