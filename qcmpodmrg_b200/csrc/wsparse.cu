@@ -749,6 +749,8 @@ extern "C" int qc_wx_build(int nparts, const void *parts, void **handle, long lo
         p1 += x.ns1[k];
         p2 += x.ns2[k];
       }
+      for (int k = 0; k < x.ns1[1]; ++k)
+        if (p.W1.nd[1][k] != p.W2.nd[0][k]) rc = QC_ERR_LAYOUT;        // the bond between the sites
       p.W1.ioff = x.ioff1;
       p.W1.allowed = x.allowed1;
       p.W2.ioff = x.ioff2;

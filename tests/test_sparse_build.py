@@ -2,6 +2,7 @@
 from concurrent.futures import ThreadPoolExecutor
 
 import numpy
+import pytest
 import torch
 
 from helpers import load, record_renormalizer, tensorset
@@ -56,3 +57,25 @@ def _tables(r):
         return []
     return [getattr(wx, n).tobytes() for n in ("h_dops", "h_octs", "h_ent_r", "h_groups", "h_deltas", "h_rows")] + \
         [wx.h_w[k].tobytes() for k in ("f64", "f32")]
+
+
+def test_sites_of_different_bonds_are_refused():
+    """The second site's left bond one state shorter than the first one's right bond."""
+    from qcmpodmrg_b200 import engine, native
+    ones, four = numpy.ones(1, dtype=numpy.int64), numpy.ones(4, dtype=numpy.int64)
+
+    def source(a, b):
+        return engine.WSource(numpy.ones(16 * a * b), [0], [1, 1, 4, 4], numpy.concatenate([a * ones, b * ones, four, four]),
+                              numpy.arange(16) * a * b, numpy.ones(16))
+
+    i32 = numpy.int32
+    part = {"groups": numpy.zeros(1, engine.WXGRP_DT), "deltas": numpy.zeros(1, engine.WXDELTA_DT),
+            "rows": numpy.zeros(2, i32), "fibers": numpy.ones(1, dtype=numpy.int64),
+            "iblk": numpy.array([[0] + [-1] * 15], i32), "kblk": numpy.array([[0] + [-1] * 15], i32),
+            "row0": numpy.zeros((1, 16), i32), "R": numpy.array([2], i32)}
+    part["deltas"]["R"], part["deltas"]["grp_e"] = 2, 1
+    make = lambda b: engine.SparseWStage([(part, (0, 1), (source(2, 3), source(b, 2)))], "cpu", "s",            # noqa: E731
+                                         engine.op_table(0, 0, 0, 1.0))
+    assert len(make(3).h_octs) == 1
+    with pytest.raises(native.NativeError):
+        make(2)
