@@ -73,8 +73,8 @@ def tune_fiber_budget(d, isite=None, candidates=CANDIDATES, repeats=4, precision
     for cand in candidates:
         d.sigma_opts["fg_budget"] = tuple(int(v) for v in cand)
         lay, idl, sig, dg = d.dot_operators(isite)
-        if sig.wx is not None:          # the sparse product took the place of both fiber stages: nothing to measure
-            break
+        if getattr(sig, "inner", sig).wx is not None:       # (inner: spin projection's)
+            break                       # the sparse product took the place of both fiber stages: nothing to measure
         if x is None:
             ndim0 = int(sig.ndim0)
             x = torch.from_numpy(numpy.random.default_rng(7).standard_normal(ndim0)).to(d.device)

@@ -66,6 +66,27 @@ def test_nothing_is_timed_with_the_sparse_product(monkeypatch):
     autotune._CACHE.clear()
 
 
+def test_spin_projection(monkeypatch):
+    """A spin-projected run, whose product wraps the one with the plan: timed with fiber stages, not
+    with the sparse product."""
+    from test_sparse_w import patch
+    patch(monkeypatch)
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda *a, **k: None)
+    monkeypatch.setattr(torch.cuda, "get_device_name", lambda *a, **k: "cpu-interpreter")
+    from qcmpodmrg_b200 import autotune
+    from qcmpodmrg_b200.spin import SPDMRG
+    from qcmpodmrg_b200.synthetic import product_mps
+    d = SPDMRG(make_hamiltonian(4, 4, 1, 3.0), 2, device="cpu")
+    d.load_mps(product_mps(d.ham))
+    d.sweep("R", 8, 1e-7)
+    monkeypatch.setattr(autotune, "_time_sigma", lambda sig, x, p, n: (1.0, sig(x, precision=p)))
+    for sparse, timed in ((False, 2), (True, 0)):
+        d.sigma_opts["sparse_w"] = sparse
+        autotune._CACHE.clear()
+        assert len(autotune.tune_fiber_budget(d, 1, candidates=((4096, 4096), (64, 64)))["table"]) == timed
+    autotune._CACHE.clear()
+
+
 def _fiber_stages(sig):
     from qcmpodmrg_b200.engine import FiberStage, CompositeStage
     out = []
